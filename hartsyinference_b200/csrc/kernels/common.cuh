@@ -480,10 +480,11 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 __device__ __forceinline__ float gelu_tanh(float x) {
+  // 0.5 (1 + tanh u) = 1 / (1 + exp(-2 u)): no cancellation for negative x, and a third of the instructions
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
+  return __fdividef(x, 1.f + __expf(-2.f * k0 * (x + k1 * x * x * x)));
 }
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 __device__ __forceinline__ float relu2(float x) {
   const float r = fmaxf(x, 0.f);
   return r * r;

@@ -32,6 +32,36 @@ __device__ __forceinline__ uint8_t to_e4m3(float v) {
   return static_cast<uint8_t>(__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3));
 }
 
+// Eight values times `inv` as e4m3 bytes: one conversion instruction per pair.
+__device__ __forceinline__ uint2 to_e4m3x8(const float (&y)[8], float inv) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    w[i] = __nv_cvt_float2_to_fp8x2(make_float2(y[2 * i] * inv, y[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+  return make_uint2(w[0] | w[1] << 16, w[2] | w[3] << 16);
+}
+__device__ __forceinline__ void unpack_bf16x8(const uint4& raw, float (&v)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+__device__ __forceinline__ uint4 pack_bf16x8(const float (&v)[8]) {
+  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+// Eight parameters from column c (a multiple of 8): one 16-byte load where the host found the array aligned.
+__device__ __forceinline__ void load_param8(const __nv_bfloat16* w, long long c, bool vec, float (&v)[8]) {
+  if (vec) {
+    unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(w + c)), v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __bfloat162float(w[c + i]);
+  }
+}
+
 // UE8M0 (power-of-two) scale for hardware block scaling: the smallest 2^e >= amax / 448.
 // Returns 2^-e and the biased exponent byte e + 127.
 __device__ __forceinline__ float mx_scale_inv(float amax, uint32_t& e_biased) {
@@ -51,6 +81,22 @@ __device__ __forceinline__ void store_sf(uint8_t* sf, int row, int kb, int tile_
   sf[(blk * 128 + (r & 31) * 4 + (r >> 5)) * 4 + (kb & 3)] = static_cast<uint8_t>(e_biased);
 }
 
+// Eight e4m3 values of vector `vi` of a row of `dim` values, whose 1x128 group has the largest magnitude
+// `amax`; the group's first thread stores its scale.
+__device__ __forceinline__ void store_fp8(const float (&y)[8], float amax, uint8_t* dst, float* scales, int row, int vi,
+                                          int dim, int sf_tile_rows) {
+  if (sf_tile_rows > 0) {
+    uint32_t eb;
+    const float inv = mx_scale_inv(amax, eb);
+    *reinterpret_cast<uint2*>(dst) = to_e4m3x8(y, inv);
+    if ((vi & 15) == 0) store_sf(reinterpret_cast<uint8_t*>(scales), row, vi >> 4, sf_tile_rows, (dim + 511) >> 9, eb);
+  } else {
+    const float sc = fmaxf(amax, 1e-12f) / kFp8Max;
+    *reinterpret_cast<uint2*>(dst) = to_e4m3x8(y, 1.f / sc);
+    if ((vi & 15) == 0) scales[static_cast<long long>(row) * (dim >> 7) + (vi >> 4)] = sc;
+  }
+}
+
 struct NormParams {
   const __nv_bfloat16* x;         // [rows][dim]
   const __nv_bfloat16* residual;  // optional [rows][dim]: h = x + residual
@@ -67,10 +113,15 @@ struct NormParams {
   int layernorm;                  // 0 = RMSNorm, 1 = LayerNorm (mean-centred)
   int weight_plus_one;            // Gemma-style (1 + w)
   int sf_tile_rows;               // > 0: out_scale is a blocked UE8M0 scale-factor array
+  int vec_params;                 // weight, bias, shift and scale can be read in 16-byte pieces
 };
 
-// dim % 8 == 0; blockDim.x * 8 >= dim handled by a strided loop keeping the row in registers for
-// dim <= 8 * 1024 (blockDim 1024) .. generic fallback re-reads the row.
+// One block per row, dim % 8 == 0, the row kept in registers: kMaxVec 16-byte vectors a thread, all loads (the
+// residual's too) in flight before the first use. Bound by HBM. Many rows take several vectors a thread, so that more
+// rows share a processor and one row's loads run under another's reduction; few rows (decoding) take one
+// vector a thread, where the latency of a single row is what counts. Residual + norm + fp8, one vector a
+// thread before: 8192 x 8192 163.6 -> 112.5 us (5.4 TB/s), 14040 x 5120 160 -> 118 us; two vectors instead of
+// four 123 and 118, so four start at rows of 8192.
 template <int kMaxVec>
 __global__ void __launch_bounds__(1024) norm_kernel(const NormParams p) {
   pdl_wait();
@@ -78,51 +129,39 @@ __global__ void __launch_bounds__(1024) norm_kernel(const NormParams p) {
   __shared__ float red[32];
   const int row = blockIdx.x;
   const int nvec = p.dim >> 3;
-  const __nv_bfloat16* xr = p.x + static_cast<long long>(row) * p.dim;
+  const long long base = static_cast<long long>(row) * p.dim;
+  uint4 raw[kMaxVec], res[kMaxVec];
+#pragma unroll
+  for (int it = 0; it < kMaxVec; ++it) {
+    const int vi = threadIdx.x + it * blockDim.x;
+    raw[it] = res[it] = make_uint4(0u, 0u, 0u, 0u);
+    if (vi < nvec) {
+      raw[it] = *reinterpret_cast<const uint4*>(p.x + base + vi * 8);
+      if (p.residual) res[it] = *reinterpret_cast<const uint4*>(p.residual + base + vi * 8);
+    }
+  }
   float v[kMaxVec][8];
   float sum = 0.f, sumsq = 0.f;
 #pragma unroll
   for (int it = 0; it < kMaxVec; ++it) {
     const int vi = threadIdx.x + it * blockDim.x;
-    if (vi < nvec) {
-      uint4 raw = *reinterpret_cast<const uint4*>(xr + vi * 8);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    unpack_bf16x8(raw[it], v[it]);
+    if (p.residual) {
+      float r[8];
+      unpack_bf16x8(res[it], r);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 f = __bfloat1622float2(h[i]);
-        v[it][2 * i] = f.x;
-        v[it][2 * i + 1] = f.y;
-      }
-      if (p.residual) {
-        uint4 rr = *reinterpret_cast<const uint4*>(p.residual + static_cast<long long>(row) * p.dim + vi * 8);
-        const __nv_bfloat162* rh = reinterpret_cast<const __nv_bfloat162*>(&rr);
+      for (int i = 0; i < 8; ++i) v[it][i] += r[i];
+    }
+    if (p.residual_out) {
+      const uint4 o = pack_bf16x8(v[it]);
+      if (vi < nvec) *reinterpret_cast<uint4*>(p.residual_out + base + vi * 8) = o;
+      // the norm must see the value that was stored (bf16-rounded), as the unfused path does
+      unpack_bf16x8(o, v[it]);
+    }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float2 f = __bfloat1622float2(rh[i]);
-          v[it][2 * i] += f.x;
-          v[it][2 * i + 1] += f.y;
-        }
-      }
-      if (p.residual_out) {
-        uint4 o;
-        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ow[i] = pack_bf16x2(v[it][2 * i], v[it][2 * i + 1]);
-        *reinterpret_cast<uint4*>(p.residual_out + static_cast<long long>(row) * p.dim + vi * 8) = o;
-        // the norm must see the value that was stored (bf16-rounded), as the unfused path does
-        const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float2 f = __bfloat1622float2(oh[i]);
-          v[it][2 * i] = f.x;
-          v[it][2 * i + 1] = f.y;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        sum += v[it][i];
-        sumsq += v[it][i] * v[it][i];
-      }
+    for (int i = 0; i < 8; ++i) {
+      sum += v[it][i];
+      sumsq += v[it][i] * v[it][i];
     }
   }
   float mean = 0.f;
@@ -145,123 +184,84 @@ __global__ void __launch_bounds__(1024) norm_kernel(const NormParams p) {
   }
   const float total = block_sum(sumsq, red);
   const float rstd = rsqrtf(total / p.dim + p.eps);
-  const int batch = p.rows_per_batch > 0 ? row / p.rows_per_batch : 0;
+  const long long mod = p.rows_per_batch > 0 ? static_cast<long long>(row / p.rows_per_batch) * p.mod_stride : 0;
 #pragma unroll
   for (int it = 0; it < kMaxVec; ++it) {
     const int vi = threadIdx.x + it * blockDim.x;
     const bool active = vi < nvec;
+    const int c = vi * 8;
     float y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = active ? (v[it][i] - mean) * rstd : 0.f;
     if (active) {
+      float t[8];
+      if (p.weight) {
+        load_param8(p.weight, c, p.vec_params, t);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = vi * 8 + i;
-        float t = (v[it][i] - mean) * rstd;
-        if (p.weight) {
-          const float w = __bfloat162float(p.weight[c]);
-          t *= p.weight_plus_one ? (1.f + w) : w;
-        }
-        if (p.bias) t += __bfloat162float(p.bias[c]);
-        if (p.scale) t *= 1.f + __bfloat162float(p.scale[static_cast<long long>(batch) * p.mod_stride + c]);
-        if (p.shift) t += __bfloat162float(p.shift[static_cast<long long>(batch) * p.mod_stride + c]);
-        y[i] = t;
+        for (int i = 0; i < 8; ++i) y[i] *= p.weight_plus_one ? (1.f + t[i]) : t[i];
       }
-      if (p.out) {
-        uint4 o;
-        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+      if (p.bias) {
+        load_param8(p.bias, c, p.vec_params, t);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ow[i] = pack_bf16x2(y[2 * i], y[2 * i + 1]);
-        *reinterpret_cast<uint4*>(p.out + static_cast<long long>(row) * p.dim + vi * 8) = o;
+        for (int i = 0; i < 8; ++i) y[i] += t[i];
       }
-    } else {
+      if (p.scale) {
+        load_param8(p.scale, mod + c, p.vec_params, t);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = 0.f;
+        for (int i = 0; i < 8; ++i) y[i] *= 1.f + t[i];
+      }
+      if (p.shift) {
+        load_param8(p.shift, mod + c, p.vec_params, t);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] += t[i];
+      }
     }
+    const uint4 o = pack_bf16x8(y);
+    if (p.out && active) *reinterpret_cast<uint4*>(p.out + base + c) = o;
     if (p.out_fp8) {
-      // all 32 lanes take part in the half-warp shuffles; inactive lanes carry zeros and do not
-      // store. dim % 128 == 0 is required for the fp8 output, so a 16-lane group is all-active
-      // or all-inactive.
-      if (active) {
-        // fp8 consumers see the bf16-rounded activations, exactly like the unfused path
-#pragma unroll
-        for (int i = 0; i < 8; ++i) y[i] = __bfloat162float(__float2bfloat16(y[i]));
-      }
+      // fp8 consumers see the bf16-rounded activations, exactly like the unfused path. All 32 lanes
+      // take part in the half-warp shuffles; inactive lanes carry zeros and do not store. dim % 128 == 0
+      // is required for the fp8 output, so a 16-lane group is all-active or all-inactive.
+      unpack_bf16x8(o, y);
       float amax = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(y[i]));
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      if (active) {
-        float sc = fmaxf(amax, 1e-12f) / kFp8Max;
-        float inv = 1.f / sc;
-        uint32_t eb = 0;
-        if (p.sf_tile_rows > 0) inv = mx_scale_inv(amax, eb);
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) lo |= static_cast<uint32_t>(to_e4m3(y[i] * inv)) << (8 * i);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) hi |= static_cast<uint32_t>(to_e4m3(y[4 + i] * inv)) << (8 * i);
-        *reinterpret_cast<uint2*>(p.out_fp8 + static_cast<long long>(row) * p.dim + vi * 8) =
-            make_uint2(lo, hi);
-        if ((vi & 15) == 0) {
-          if (p.sf_tile_rows > 0)
-            store_sf(reinterpret_cast<uint8_t*>(p.out_scale), row, vi >> 4, p.sf_tile_rows, (p.dim + 511) >> 9, eb);
-          else
-            p.out_scale[static_cast<long long>(row) * (p.dim >> 7) + (vi >> 4)] = sc;
-        }
-      }
+      for (int o2 = 8; o2 > 0; o2 >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o2));
+      if (active) store_fp8(y, amax, p.out_fp8 + base + c, p.out_scale, row, vi, p.dim, p.sf_tile_rows);
     }
   }
 }
 
-// fp8 1x128 quantisation of a bf16 matrix [rows][dim] (dim % 128 == 0) with row pitch ld.
-__global__ void quant_fp8_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ out,
+// fp8 1x128 quantisation of a bf16 matrix [rows][dim] (dim % 128 == 0) with row pitch ld. A thread keeps its
+// vector of eight columns and takes kRows rows, whose loads go out together; grid (column blocks, row groups).
+// Bound by HBM: 14040 x 13824 202 -> 130 us (4.5 TB/s), 4608 x 15360 77 -> 51 us (one row a thread 145 and 56).
+template <int kRows>
+__global__ void __launch_bounds__(256) quant_fp8_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ out,
                                  float* __restrict__ scales, int rows, int dim, long long ld,
                                  int sf_tile_rows) {
   pdl_wait();
   pdl_trigger();
-  const int groups = dim >> 7;
-  const long long total = static_cast<long long>(rows) * groups * 16;   // one thread per 8 values
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  // total is a multiple of 16, blockDim is a multiple of 32: a 16-lane group is uniform
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-       i < ((total + 31) / 32) * 32; i += stride) {
-    const bool active = i < total;
-    const long long ii = active ? i : total - 1;
-    const int sub = static_cast<int>(ii & 15);
-    const long long g = ii >> 4;
-    const int row = static_cast<int>(g / groups), grp = static_cast<int>(g % groups);
-    uint4 raw = *reinterpret_cast<const uint4*>(x + row * ld + grp * 128 + sub * 8);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    float v[8];
+  const int vi = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool col = vi < (dim >> 3);            // dim % 128 == 0: a 16-lane group is uniform
+  for (int row0 = blockIdx.y * kRows; row0 < rows; row0 += gridDim.y * kRows) {
+    uint4 raw[kRows];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float2 f = __bfloat1622float2(h[k]);
-      v[2 * k] = f.x;
-      v[2 * k + 1] = f.y;
+    for (int r = 0; r < kRows; ++r) {
+      raw[r] = make_uint4(0u, 0u, 0u, 0u);
+      if (col && row0 + r < rows) raw[r] = *reinterpret_cast<const uint4*>(x + (row0 + r) * ld + vi * 8);
     }
-    float amax = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
+    for (int r = 0; r < kRows; ++r) {
+      float v[8];
+      unpack_bf16x8(raw[r], v);
+      float amax = 0.f;
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (active) {
-      float sc = fmaxf(amax, 1e-12f) / kFp8Max;
-      float inv = 1.f / sc;
-      uint32_t eb = 0;
-      if (sf_tile_rows > 0) inv = mx_scale_inv(amax, eb);
-      uint32_t lo = 0, hi = 0;
+      for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) lo |= static_cast<uint32_t>(to_e4m3(v[k] * inv)) << (8 * k);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) hi |= static_cast<uint32_t>(to_e4m3(v[4 + k] * inv)) << (8 * k);
-      *reinterpret_cast<uint2*>(out + static_cast<long long>(row) * dim + grp * 128 + sub * 8) =
-          make_uint2(lo, hi);
-      if (sub == 0) {
-        if (sf_tile_rows > 0)
-          store_sf(reinterpret_cast<uint8_t*>(scales), row, grp, sf_tile_rows, (dim + 511) >> 9, eb);
-        else
-          scales[static_cast<long long>(row) * groups + grp] = sc;
-      }
+      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      if (col && row0 + r < rows)
+        store_fp8(v, amax, out + static_cast<long long>(row0 + r) * dim + vi * 8, scales, row0 + r, vi, dim, sf_tile_rows);
     }
   }
 }
@@ -317,75 +317,63 @@ __global__ void quant_fp8_weight_kernel(const __nv_bfloat16* __restrict__ w,
   }
 }
 
-// Gated activation: out[r][c] = act(in[r][c]) * in[r][F + c] for in [rows][2F] (gate first, then
-// up), act: 0 = SiLU, 1 = GELU-tanh. Optional fp8 1x128 output (F % 128 == 0).
-__global__ void glu_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+// Gated activation: out[r][c] = act(in[r][c]) * in[r][F + c] for in [rows][2F] (gate first, then up), act:
+// 0 = SiLU, 1 = GELU-tanh. Optional fp8 1x128 output (F % 128 == 0). A thread keeps its vector of eight columns
+// and takes kRows rows, whose loads go out together; grid (column blocks, row groups), so no index is divided.
+// Arithmetic and HBM bind about equally: 8192 x 28672 with fp8 output 485 -> 365 us, bf16 338 -> 270 us
+// (one row a thread 377 and 300, four 490 and 361: too many registers).
+template <int kRows>
+__global__ void __launch_bounds__(256) glu_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
                            uint8_t* __restrict__ out_fp8, float* __restrict__ out_scale, int rows,
                            int f, int act, int sf_tile_rows, const SplitPartials part) {
   pdl_wait();
   pdl_trigger();
-  const int nvec = f >> 3;
-  const long long total = static_cast<long long>(rows) * nvec;
-  const long long padded = ((total + 31) / 32) * 32;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < padded;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const bool active = i < total;
-    const long long ii = active ? i : total - 1;
-    const int row = static_cast<int>(ii / nvec), vi = static_cast<int>(ii % nvec);
-    float gv[8], uv[8];
-    if (part.ws) {
-      // the producing GEMM left its K ranges unsummed: add them here (no reduce kernel in between)
-      split_sum8(part, row, vi * 8, gv);
-      split_sum8(part, row, f + vi * 8, uv);
-    } else {
-      const __nv_bfloat16* g = in + static_cast<long long>(row) * 2 * f + vi * 8;
-      uint4 graw = *reinterpret_cast<const uint4*>(g);
-      uint4 uraw = *reinterpret_cast<const uint4*>(g + f);
-      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&graw);
-      const __nv_bfloat162* uh = reinterpret_cast<const __nv_bfloat162*>(&uraw);
+  const int vi = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool col = vi < (f >> 3);              // f % 128 == 0 with the fp8 output: a 16-lane group is uniform
+  for (int row0 = blockIdx.y * kRows; row0 < rows; row0 += gridDim.y * kRows) {
+    uint4 graw[kRows], uraw[kRows];
+    if (!part.ws) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float2 a = __bfloat1622float2(gh[k]), b = __bfloat1622float2(uh[k]);
-        gv[2 * k] = a.x; gv[2 * k + 1] = a.y;
-        uv[2 * k] = b.x; uv[2 * k + 1] = b.y;
+      for (int r = 0; r < kRows; ++r) {
+        graw[r] = uraw[r] = make_uint4(0u, 0u, 0u, 0u);
+        if (col && row0 + r < rows) {
+          const __nv_bfloat16* g = in + static_cast<long long>(row0 + r) * 2 * f + vi * 8;
+          graw[r] = *reinterpret_cast<const uint4*>(g);
+          uraw[r] = *reinterpret_cast<const uint4*>(g + f);
+        }
       }
     }
-    float y[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) y[k] = (act == 0 ? silu(gv[k]) : gelu_tanh(gv[k])) * uv[k];
-    if (out && active) {
-      uint4 o;
-      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+    for (int r = 0; r < kRows; ++r) {
+      const int row = row0 + r;
+      const bool active = col && row < rows;
+      float gv[8], uv[8];
+      if (part.ws) {
+        // the producing GEMM left its K ranges unsummed: add them here (no reduce kernel in between)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) ow[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
-      *reinterpret_cast<uint4*>(out + static_cast<long long>(row) * f + vi * 8) = o;
-    }
-    if (out_fp8) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) y[k] = __bfloat162float(__float2bfloat16(y[k]));
-      float amax = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(y[k]));
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      if (active) {
-        float sc = fmaxf(amax, 1e-12f) / kFp8Max;
-        float inv = 1.f / sc;
-        uint32_t eb = 0;
-        if (sf_tile_rows > 0) inv = mx_scale_inv(amax, eb);
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) lo |= static_cast<uint32_t>(to_e4m3(y[k] * inv)) << (8 * k);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) hi |= static_cast<uint32_t>(to_e4m3(y[4 + k] * inv)) << (8 * k);
-        *reinterpret_cast<uint2*>(out_fp8 + static_cast<long long>(row) * f + vi * 8) =
-            make_uint2(lo, hi);
-        if ((vi & 15) == 0) {
-          if (sf_tile_rows > 0)
-            store_sf(reinterpret_cast<uint8_t*>(out_scale), row, vi >> 4, sf_tile_rows, (f + 511) >> 9, eb);
-          else
-            out_scale[static_cast<long long>(row) * (f >> 7) + (vi >> 4)] = sc;
+        for (int k = 0; k < 8; ++k) gv[k] = uv[k] = 0.f;
+        if (active) {
+          split_sum8(part, row, vi * 8, gv);
+          split_sum8(part, row, f + vi * 8, uv);
         }
+      } else {
+        unpack_bf16x8(graw[r], gv);
+        unpack_bf16x8(uraw[r], uv);
+      }
+      float y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) y[k] = (act == 0 ? silu(gv[k]) : gelu_tanh(gv[k])) * uv[k];
+      const uint4 o = pack_bf16x8(y);
+      if (out && active) *reinterpret_cast<uint4*>(out + static_cast<long long>(row) * f + vi * 8) = o;
+      if (out_fp8) {
+        unpack_bf16x8(o, y);
+        float amax = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(y[k]));
+#pragma unroll
+        for (int o2 = 8; o2 > 0; o2 >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o2));
+        if (active)
+          store_fp8(y, amax, out_fp8 + static_cast<long long>(row) * f + vi * 8, out_scale, row, vi, f, sf_tile_rows);
       }
     }
   }
@@ -517,6 +505,123 @@ __global__ void rope_kv_kernel(const RopeParams p) {
       const __nv_bfloat16 b = __float2bfloat16(v[i]);
       if (dst) dst[c] = b;
       if (dst2) dst2[c] = b;
+    }
+  }
+}
+
+// Eight values as bf16 to one or two places.
+__device__ __forceinline__ void store_twice(__nv_bfloat16* a, __nv_bfloat16* b, const float (&v)[8]) {
+  const uint4 o = pack_bf16x8(v);
+  if (a) *reinterpret_cast<uint4*>(a) = o;
+  if (b) *reinterpret_cast<uint4*>(b) = o;
+}
+
+// The same for heads of 16, 32, 64, 128 or 256 values with a rotated part that is a multiple of 16, everything on
+// 16-byte boundaries. Angles are the tokens', not the heads': a block works out the sines and cosines of
+// `block_tokens` tokens once (they were 80 sincosf a pair of a 64 + 16 head token, and bound the kernel) and
+// keeps a token's in registers while it walks the heads. A unit of work is two 16-byte vectors of one head:
+// with split halves the vectors whose elements turn together, otherwise two neighbours; d / 16 lanes share a
+// head. Bound by HBM: 8192 tokens x 80 heads x 128 628 -> 86 us (3.9 TB/s), 1935 x 48 83 -> 20 us.
+__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const RopeParams p, int block_tokens, int unit_bits) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ float rope_table[];            // [block_tokens][cos of rot / 2 | sin of rot / 2]
+  __shared__ long long cache_row[8];               // row of the token in a cache of one head's pages, -1: not stored
+  const int heads = p.hq + 2 * p.hkv, half = p.rot >> 1;
+  const int t0 = blockIdx.x * block_tokens, nt = min(block_tokens, p.tokens - t0);
+  for (int i = threadIdx.x; i < nt * half; i += blockDim.x) {
+    const int tt = i / half, j = i - tt * half;
+    const float pos = static_cast<float>(p.positions[t0 + tt]);
+    const float inv = p.inv_freq ? p.inv_freq[j] : __powf(p.theta, -2.f * j / static_cast<float>(p.rot));
+    float sn, cs;
+    sincosf(pos * inv, &sn, &cs);
+    rope_table[tt * p.rot + j] = cs;
+    rope_table[tt * p.rot + half + j] = sn;
+  }
+  if (threadIdx.x < nt) {
+    const long long slot = p.slot_mapping ? p.slot_mapping[t0 + threadIdx.x] : -1;
+    cache_row[threadIdx.x] = slot < 0 ? -1 : slot / p.page * p.hkv * p.page + slot % p.page;
+  }
+  __syncthreads();
+  const int u = threadIdx.x & ((1 << unit_bits) - 1);
+  const int step = blockDim.x >> unit_bits;
+  const int first = blockIdx.y * step + (threadIdx.x >> unit_bits), stride = gridDim.y * step;
+  const bool turns = u < p.rot >> 4;               // this unit's vectors are rotated (of q and k)
+  const int va = turns && p.style == 0 ? u : 2 * u, vb = turns && p.style == 0 ? u + (p.rot >> 4) : 2 * u + 1;
+  for (int tt = 0; tt < nt; ++tt) {
+    const int t = t0 + tt;
+    float cs[8], sn[8];
+    if (turns) {
+      // split halves: the eight pairs of vector u; neighbours: the four pairs of each of the two vectors
+      const float* tab = rope_table + tt * p.rot + u * 8;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { cs[k] = tab[k]; sn[k] = tab[half + k]; }
+    }
+    // every lane of a warp makes the same rounds, since the norm's sum is exchanged between lanes
+    for (int h0 = first; h0 - (first % (32 >> unit_bits)) < heads; h0 += stride) {
+      const bool active = h0 < heads;
+      const int h = active ? h0 : heads - 1;
+      const int kind = h < p.hq ? 0 : (h < p.hq + p.hkv ? 1 : 2);
+      const int ca = (kind == 2 ? 2 * u : va) * 8, cb = (kind == 2 ? 2 * u + 1 : vb) * 8;
+      float a[8], b[8];
+      if (p.part.ws) {
+        split_sum8(p.part, t, h * p.d + ca, a);
+        split_sum8(p.part, t, h * p.d + cb, b);
+      } else {
+        const __nv_bfloat16* src = p.qkv + (static_cast<long long>(t) * heads + h) * p.d;
+        const uint4 ra = *reinterpret_cast<const uint4*>(src + ca), rb = *reinterpret_cast<const uint4*>(src + cb);
+        unpack_bf16x8(ra, a);
+        unpack_bf16x8(rb, b);
+      }
+      if (p.q_norm_w || p.k_norm_w) {
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ss += a[k] * a[k] + b[k] * b[k];
+        for (int o = 1 << unit_bits >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const __nv_bfloat16* nw = kind == 0 ? p.q_norm_w : (kind == 1 ? p.k_norm_w : nullptr);
+        if (nw) {
+          const float rstd = rsqrtf(ss / p.d + p.eps);
+          float w[8];
+          load_param8(nw, ca, true, w);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) a[k] = a[k] * rstd * w[k];
+          load_param8(nw, cb, true, w);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) b[k] = b[k] * rstd * w[k];
+        }
+      }
+      if (turns && kind != 2) {
+        if (p.style == 0) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float x = a[k], y = b[k];
+            a[k] = x * cs[k] - y * sn[k];
+            b[k] = y * cs[k] + x * sn[k];
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float x = a[2 * k], y = a[2 * k + 1], z = b[2 * k], w = b[2 * k + 1];
+            a[2 * k] = x * cs[k] - y * sn[k];
+            a[2 * k + 1] = y * cs[k] + x * sn[k];
+            b[2 * k] = z * cs[4 + k] - w * sn[4 + k];
+            b[2 * k + 1] = w * cs[4 + k] + z * sn[4 + k];
+          }
+        }
+      }
+      if (!active) continue;
+      __nv_bfloat16 *dst = nullptr, *dst2 = nullptr;
+      if (kind == 0) {
+        dst = p.q_out + (static_cast<long long>(t) * p.hq + h) * p.d;
+      } else {
+        const int hk = kind == 1 ? h - p.hq : h - p.hq - p.hkv;
+        __nv_bfloat16* cache = kind == 1 ? p.k_cache : p.v_cache;
+        __nv_bfloat16* lin = kind == 1 ? p.k_out : p.v_out;
+        if (cache && cache_row[tt] >= 0) dst = cache + (cache_row[tt] + static_cast<long long>(hk) * p.page) * p.d;
+        if (lin) dst2 = lin + (static_cast<long long>(t) * p.hkv + hk) * p.d;
+      }
+      store_twice(dst ? dst + ca : nullptr, dst2 ? dst2 + ca : nullptr, a);
+      store_twice(dst ? dst + cb : nullptr, dst2 ? dst2 + cb : nullptr, b);
     }
   }
 }
@@ -676,6 +781,26 @@ inline int grid_for(long long n, int block, int cap_mult = 8) {
   return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// Launch shape of the kernels that give a thread one vector of columns: `most` rows a thread once that still
+// leaves every processor several blocks, one row below.
+struct RowGrid {
+  int rows_each;
+  dim3 block, grid;
+  RowGrid(int rows, int nvec, int most) {
+    const int threads = nvec >= 256 ? 256 : (nvec + 31) / 32 * 32;
+    const int cols = (nvec + threads - 1) / threads;
+    rows_each = static_cast<long long>(rows) * cols >= 148 * 8 * 4 ? most : 1;
+    const int groups = (rows + rows_each - 1) / rows_each;
+    block = dim3(threads);
+    grid = dim3(cols, groups < 65535 ? groups : 65535);
+  }
+};
+
+template <typename... P>
+inline bool aligned16(P... ptrs) {
+  return ((reinterpret_cast<uintptr_t>(ptrs) | ... | uintptr_t{0}) & 15) == 0;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -709,15 +834,14 @@ B200_API int b200_norm(const void* x, const void* residual, void* residual_out, 
   p.rows = rows; p.dim = dim; p.rows_per_batch = rows_per_batch; p.mod_stride = mod_stride;
   p.eps = eps; p.layernorm = layernorm; p.weight_plus_one = weight_plus_one;
   p.sf_tile_rows = sf_tile_rows;
+  p.vec_params = aligned16(weight, bias, shift, scale) && mod_stride % 8 == 0;
   const int nvec = dim / 8;
-  // threads: multiple of 32 covering the row with at most 2 vectors per thread
-  int threads = ((nvec + 31) / 32) * 32;
-  if (threads <= 1024) {
-    launch_pdl(norm_kernel<1>, dim3(rows), dim3(threads < 32 ? 32 : threads), 0, stream, p);
-  } else {
-    threads = (((nvec + 1) / 2 + 31) / 32) * 32;
-    launch_pdl(norm_kernel<2>, dim3(rows), dim3(threads), 0, stream, p);
-  }
+  auto go = [&](auto* kernel, int per) {
+    launch_pdl(kernel, dim3(rows), dim3(((nvec + per - 1) / per + 31) / 32 * 32), 0, stream, p);
+  };
+  if (rows > 296 && nvec >= 1024) go(norm_kernel<4>, 4);
+  else if (nvec > 1024 || (rows > 296 && nvec >= 256)) go(norm_kernel<2>, 2);
+  else go(norm_kernel<1>, 1);
   CHECK_LAUNCH();
   return 0;
 }
@@ -728,9 +852,9 @@ B200_API int b200_quant_fp8(const void* x, void* out, float* scales, int rows, i
                             long long ld, int sf_tile_rows, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (dim % 128 != 0 || ld % 8 != 0) return -2;
-  const long long n = static_cast<long long>(rows) * (dim / 8);
-  launch_pdl(quant_fp8_kernel, dim3(grid_for(n, 256)), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(x),
-             static_cast<uint8_t*>(out), scales, rows, dim, ld, sf_tile_rows);
+  const RowGrid g(rows, dim / 8, 4);
+  launch_pdl(g.rows_each == 4 ? quant_fp8_kernel<4> : quant_fp8_kernel<1>, g.grid, g.block, 0, stream,
+             static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(out), scales, rows, dim, ld, sf_tile_rows);
   CHECK_LAUNCH();
   return 0;
 }
@@ -752,9 +876,9 @@ B200_API int b200_glu(const void* in, void* out, void* out_fp8, float* out_scale
                       cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (f % 8 != 0 || (out_fp8 && f % 128 != 0)) return -2;
-  const long long n = static_cast<long long>(rows) * (f / 8);
+  const RowGrid g(rows, f / 8, 2);
   const SplitPartials part{part_ws, part_splits, part_bn};
-  launch_pdl(glu_kernel, dim3(grid_for(n, 256)), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(in),
+  launch_pdl(g.rows_each == 2 ? glu_kernel<2> : glu_kernel<1>, g.grid, g.block, 0, stream, static_cast<const __nv_bfloat16*>(in),
              static_cast<__nv_bfloat16*>(out), static_cast<uint8_t*>(out_fp8), out_scale, rows, f, act, sf_tile_rows,
              part);
   CHECK_LAUNCH();
@@ -784,7 +908,20 @@ B200_API int b200_rope_kv(const void* qkv, void* q_out, void* k_cache, void* v_c
   p.inv_freq = inv_freq;
   p.tokens = tokens; p.hq = hq; p.hkv = hkv; p.d = d; p.rot = rot; p.style = style; p.page = page;
   p.theta = theta; p.eps = eps;
-  const long long warps = static_cast<long long>(tokens) * (hq + 2 * hkv);
+  const int heads = hq + 2 * hkv;
+  int unit_bits = 0;
+  while (16 << unit_bits < d) ++unit_bits;
+  if (16 << unit_bits == d && rot % 16 == 0 && (style == 0 || style == 1) &&
+      aligned16(qkv, q_out, k_cache, v_cache, k_out, v_out, q_norm_w, k_norm_w, part_ws)) {
+    const int block_heads = 256 >> unit_bits;
+    const int chunks = (heads + block_heads - 1) / block_heads;
+    const int each = tokens >= 148 * 8 ? 4 : 1;      // more tokens a block once every processor has several
+    launch_pdl(rope_kv_vec_kernel, dim3((tokens + each - 1) / each, each == 1 ? chunks : 1), dim3(256),
+               static_cast<size_t>(each) * rot * sizeof(float), stream, p, each, unit_bits);
+    CHECK_LAUNCH();
+    return 0;
+  }
+  const long long warps = static_cast<long long>(tokens) * heads;
   const int block = 256;
   const long long blocks = (warps * 32 + block - 1) / block;
   launch_pdl(rope_kv_kernel, dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, p);
