@@ -202,6 +202,8 @@ struct GemmParams {
   AllReduceParams ar;   // ar.world == 0: plain GEMM
   GatherParams ag;      // ag.world == 0: the A operand is complete when the kernel starts
   int ta_rotate;        // plain GEMM: A tiles are walked starting with this one
+  int row_stores;       // large-token orientation: C (and bias, gate, residual) can be reached in 16-byte pieces
+  int band;             // > 0, plain GEMM: tiles are walked in bands of this many A tiles (see decode_item)
 };
 
 constexpr int kTileA = 128;
@@ -281,8 +283,19 @@ __device__ __forceinline__ WorkItem decode_item(const GemmParams& p, long long w
       it.skip = p.group_counts != nullptr && p.group_counts[it.tb] == 0;
     }
   } else {
-    it.tb = static_cast<int>(tile / tiles_a);
     it.skip = false;
+    if (p.band > 0) {
+      // a band of A tiles meets all B tiles before the next band starts, so the tiles in flight cover a
+      // block of the output that is about square and read fewer different rows of the operands
+      const int tiles_b = p.num_tiles / tiles_a;
+      const int per = p.band * tiles_b;
+      const int t = static_cast<int>(tile), b = t / per, r = t - b * per;
+      const int width = min(p.band, tiles_a - b * p.band);
+      it.tb = r / width;
+      it.ta = b * p.band + (r - it.tb * width);
+      return it;
+    }
+    it.tb = static_cast<int>(tile / tiles_a);
     if (p.ta_rotate > 0) {
       it.ta += p.ta_rotate;
       if (it.ta >= tiles_a) it.ta -= tiles_a;
@@ -302,10 +315,11 @@ __device__ __forceinline__ float apply_epilogue(const GemmParams& p, float v, lo
                                                 long long col) {
   // row = token index, col = output feature, both already bounds-checked
   if (p.bias) v += __bfloat162float(p.bias[col]);
-  if (p.act == 1) v = gelu_tanh(v);
+  if (col < p.act_col) { /* features ahead of the activation's first */ }
+  else if (p.act == 1) v = gelu_tanh(v);
   else if (p.act == 2) v = silu(v);
   else if (p.act == 3) v = relu2(v);
-  else if (p.act == 4 && col >= p.act_col) v = tanhf(v);
+  else if (p.act == 4) v = tanhf(v);
   if (p.gate) v *= __bfloat162float(p.gate[col]);
   if (p.residual) v += __bfloat162float(p.residual[row * p.ldc + col]);
   return v;
@@ -370,6 +384,90 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float (&v
   }
 }
 
+__device__ __forceinline__ void load_cols8(const __nv_bfloat16* src, float (&v)[8]) {
+  const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src));
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+
+// Epilogue of 32 rows x 32 columns of a whole tile in the large-token orientation: lane l holds row
+// row0 + l. The values go through a strip of shared memory that belongs to the warp, so that global
+// memory sees 64-byte runs of a row instead of 16-byte pieces of 32 rows, whose half-written sectors held the
+// tensor core up (fp8 4608 x 21504 x 3072 with the 128 x 256 tile: 1127 -> 326 us, bf16 579 -> 440 us).
+constexpr int kStripPitch = 80;                        // 64 bytes + 16: rows of a strip start in different banks
+constexpr int kStripBytes = 32 * kStripPitch;
+__device__ __forceinline__ void store_chunk_rows(const GemmParams& p, float (&v)[32], int row0, int b0, uint8_t* strip) {
+  const int lane = threadIdx.x & 31;
+  const int pr = lane >> 2, pc = lane & 3;             // this lane's row of eight and 16-byte piece in global accesses
+  const long long at = static_cast<long long>(row0 + pr) * p.ldc + b0 + pc * 8;
+  if (p.residual) {
+    uint4 raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      raw[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (row0 + i * 8 + pr < p.rows_a) raw[i] = *reinterpret_cast<const uint4*>(p.residual + at + i * 8 * p.ldc);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(strip + (i * 8 + pr) * kStripPitch + pc * 16) = raw[i];
+    __syncwarp();
+  }
+  uint8_t* own = strip + lane * kStripPitch;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float t[8];
+    if (p.bias) {
+      load_cols8(p.bias + b0 + q * 8, t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] += t[j];
+    }
+    if (b0 + q * 8 < p.act_col) {
+      // features ahead of the activation's first (a multiple of 8)
+    } else if (p.act == 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] = gelu_tanh(v[q * 8 + j]);
+    } else if (p.act == 2) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] = silu(v[q * 8 + j]);
+    } else if (p.act == 3) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] = relu2(v[q * 8 + j]);
+    } else if (p.act == 4) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] = tanhf(v[q * 8 + j]);
+    }
+    if (p.gate) {
+      load_cols8(p.gate + b0 + q * 8, t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q * 8 + j] *= t[j];
+    }
+    if (p.residual) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(own + q * 16);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        v[q * 8 + 2 * j] += f.x;
+        v[q * 8 + 2 * j + 1] += f.y;
+      }
+    }
+    *reinterpret_cast<uint4*>(own + q * 16) =
+        make_uint4(pack_bf16x2(v[q * 8], v[q * 8 + 1]), pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]),
+                   pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint4 o = *reinterpret_cast<const uint4*>(strip + (i * 8 + pr) * kStripPitch + pc * 16);
+    if (row0 + i * 8 + pr < p.rows_a) *reinterpret_cast<uint4*>(p.out + at + i * 8 * p.ldc) = o;
+  }
+  __syncwarp();                                        // the strip is free for the next chunk
+}
+
 // fp32 partial of a split tile: slot layout [BN columns][128 rows], so that the 32 lanes of a warp
 // (consecutive rows) write and later read consecutive addresses.
 template <int BN>
@@ -381,11 +479,14 @@ __device__ __forceinline__ void store_partial(const GemmParams& p, const float (
     if (col0_local + j < BN) ws[(col0_local + j) * 128 + row_local] = v[j];
 }
 
-// Routes one 32-column chunk of accumulator values of work item `it`.
-template <int BN>
-__device__ __forceinline__ void emit_chunk(const GemmParams& p, const float (&v)[32], const WorkItem& it,
-                                           int row_local, int chunk) {
+// Routes one 32-column chunk of accumulator values of work item `it`. kLarge: the large-token orientation (a
+// compile-time matter, because the code of its epilogue slowed the start of the short decode kernels by 2 us).
+template <int BN, bool kLarge>
+__device__ __forceinline__ void emit_chunk(const GemmParams& p, float (&v)[32], const WorkItem& it,
+                                           int row_local, int chunk, uint8_t* strip) {
   if (it.slot >= 0 && p.ar.world == 0) store_partial<BN>(p, v, row_local, chunk * 32, it);
+  else if (kLarge && p.row_stores && it.tb * BN + chunk * 32 + 32 <= p.rows_b)
+    store_chunk_rows(p, v, it.ta * kTileA + (row_local & ~31), it.tb * BN + chunk * 32, strip);
   else store_chunk(p, v, it.ta * kTileA + row_local, it.tb * BN + chunk * 32, min(p.rows_b, (it.tb + 1) * BN),
                    it.split);
 }
@@ -970,9 +1071,10 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
         if (parts & 2) {
           if (with_sf) {
             const long long tile_b = (static_cast<long long>(it.tb) * BN) / p.sf_tile_b;
+            const long long last_b = (p.rows_b - 1) / p.sf_tile_b;      // rows past the end are not stored: any block will do
 #pragma unroll
             for (int j = 0; j < kSfBlocksB; ++j) {
-              const long long gb = ((tile_b + j) * p.sf_kgroups + (kb >> 2)) * 128;
+              const long long gb = (min(tile_b + j, last_b) * p.sf_kgroups + (kb >> 2)) * 128;
               bulk_load(sa + kSfOffset + 512 * (1 + j), p.sf_b + gb, 512, &bars->full[st]);
             }
           }
@@ -1134,6 +1236,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     constexpr int kChunks = (BN + 31) / 32;
     constexpr int kMine = (kChunks + 1) / 2;
     const int row_local = q * 32 + lane;
+    uint8_t* strip = reinterpret_cast<uint8_t*>(bars + 1) + (warp - 2) * kStripBytes;     // there in the large-token orientation
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     int abuf = 0;
     uint32_t aph = 0;
@@ -1148,6 +1251,27 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
             ok = false;
           } else {
             tc_fence_after_sync();
+            bool drained = false;
+            if constexpr (kAccBufs == 1 && !kI8) drained = !p.cluster_reduce;
+            if (drained) {
+              // a single accumulator: take all of it into registers and give it back before the
+              // epilogue arithmetic, so that the tensor core waits for the loads only
+              uint32_t r[kMine][32];
+#pragma unroll
+              for (int u = 0; u < kMine; ++u) tmem_ld_32x32(lane_base + (hsel + 2 * u) * 32, r[u]);
+              tmem_ld_wait();
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars->tmem_empty[abuf]);
+#pragma unroll
+              for (int u = 0; u < kMine; ++u) {
+                float v[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[u][j]);
+                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, hsel + 2 * u, strip);
+              }
+              aph ^= 1;
+            } else {
 #pragma unroll 1
             for (int c = hsel; c < kChunks; c += 2) {
               uint32_t r[32];
@@ -1174,13 +1298,14 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
                 for (int j = 0; j < 32; ++j)
                   if (c * 32 + j < BN) part[(c * 32 + j) * 128 + row_local] = v[j];
               } else {
-                emit_chunk<BN>(p, v, it, row_local, c);
+                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, c, strip);
               }
             }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->tmem_empty[abuf]);
             if (++abuf == kAccBufs) { abuf = 0; aph ^= 1; }
+            }
           }
         } else {
           float acc[kMine * 32];
@@ -1281,7 +1406,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = acc[i * 32 + j];
-                emit_chunk<BN>(p, v, it, row_local, c);
+                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, c, strip);
               }
             }
           }
@@ -1420,7 +1545,7 @@ template <int kMode, int BN, int kAtoms>
 int launch_gemm(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& tb, int grid,
                 cudaStream_t stream) {
   const int stage_bytes = kAtoms * (kStageBytesA + BN * 128) + (kMode == 2 ? 2048 : 0);
-  const int smem = p.stages * stage_bytes + static_cast<int>(sizeof(GemmBarriers)) + 1024;
+  const int smem = p.stages * stage_bytes + static_cast<int>(sizeof(GemmBarriers)) + 1024 + (p.row_stores ? 8 * kStripBytes : 0);
   static PerDeviceOnce configured;
   if (configured.first_time()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<kMode, BN, kAtoms>,
@@ -1520,7 +1645,6 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.act = act & 255;
   p.act_col = act >> 8;
-  if (p.act_col > 0 && p.act != 4) return -6;
   p.status = static_cast<DeviceStatus*>(status);
   p.swap_out = swap ? 1 : 0;
   if (ar != nullptr) {
@@ -1574,6 +1698,12 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
     p.rows_a = m; p.rows_b = n;
     a_ptr = x; lda = ldx; b_ptr = w; ldb = ldw;
     bn = fp8 && !i8 ? 128 : 256;
+    // A 128 x 256 tile reads three quarters of the operand bytes per product of two 128 x 128 ones, which is
+    // what bounds one-byte operands (8192 x 57344 x 8192: 1.59 -> 2.32 PFLOP/s), but it fills the 512 columns of
+    // TMEM with one accumulator and the scale factors; below one tile per SM the smaller ones balance
+    // better (512 x 9216 x 3072: 30 us against 42 us with the larger tiles cut along K).
+    if (mx && ar == nullptr && ag == nullptr &&
+        static_cast<long long>((m + 127) / 128) * ((n + 255) / 256) >= num_sms()) bn = 256;
     if ((!fp8 || i8) && n <= 128) bn = 128;
     p.scale_a = x_scale; p.sa_gran = 1;   p.sa_ld = k / 128;
     p.scale_b = w_scale; p.sb_gran = 128; p.sb_ld = k / 128;
@@ -1594,6 +1724,11 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
                                : ((p.rows_a + 127) / 128) * ((p.rows_b + bn - 1) / bn);
   const int sms = num_sms();
   p.num_tiles = tiles;
+  // Bands of 16 A tiles (2048 tokens): 148 tiles of 128 x 256 in flight then cover 16 x 9 of them, the squarest
+  // block. Walking all A tiles first re-read them from HBM once per wave when they do not fit L2: bf16
+  // 14040 x 15360 x 5120 1789 -> 1562 us, 1935 x 28672 x 4096 552 -> 391 us; 12 and 24 measure the same.
+  constexpr int kBand = 16;
+  if (!swap && groups == 0 && cs == nullptr && ar == nullptr && ag == nullptr && (p.rows_a + 127) / 128 > kBand) p.band = kBand;
 
   // ---- K-split policy (see the header comment)
   int first_split = tiles, s_eff = 1;
@@ -1656,6 +1791,11 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   if (stages > 12) stages = 12;
   p.stages = stages;
 
+  if (!swap && groups == 0 && ar == nullptr && ldc % 8 == 0 && p.act_col % 8 == 0 &&
+      ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(gate) |
+        reinterpret_cast<uintptr_t>(residual)) & 15) == 0)
+    p.row_stores = 1;
+
   CUtensorMap ta, tb;
   if (cs != nullptr) {
     if (fp8 || groups > 0 || ar != nullptr || cs->taps < 1 || cs->taps > 28 || cs->cin % 64 != 0) return -10;
@@ -1697,8 +1837,10 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
         case 64: rc = launch_gemm<2, 64, 2>(p, ta, tb, grid, stream); break;
         default: rc = launch_gemm<2, 128, 2>(p, ta, tb, grid, stream); break;
       }
-    } else {
+    } else if (bn == 128) {
       rc = launch_gemm<2, 128, 1>(p, ta, tb, grid, stream);
+    } else {
+      rc = launch_gemm<2, 256, 1>(p, ta, tb, grid, stream);
     }
   } else if (fp8) {
     if (swap) {
@@ -1762,8 +1904,7 @@ B200_API long long b200_gemm_workspace_bytes() {
 //   x_scale: [m][k/128] fp32 (per token, per 128-wide K group); w_scale: [ceil(n/128)][k/128] fp32
 //   splits: 0 = automatic (split only the tiles of a partial last wave), 1 = never, > 1 = split
 //           every tile that many ways
-//   act: 0 none, 1 gelu-tanh, 2 silu, 3 relu squared, 4 tanh; tanh can be limited to the output features from
-//           act >> 8 on
+//   act: 0 none, 1 gelu-tanh, 2 silu, 3 relu squared, 4 tanh, for the output features from act >> 8 on
 //   workspace: zero-initialised scratch (see b200_gemm_workspace_bytes), may be null (no splitting)
 // Returns 0 on success, negative on a launch-time error.
 B200_API int b200_gemm(const void* x, const void* w, void* out, int m, int n, int k, long long ldx,

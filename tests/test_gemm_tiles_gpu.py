@@ -1,0 +1,39 @@
+"""Large-token products at the edges of their tiles, bands and strips, against the fp32 statement."""
+import pytest
+import torch
+
+from hartsyinference_b200 import ops
+from hartsyinference_b200.ops import reference as R
+
+pytestmark = pytest.mark.gpu
+
+
+# (tokens, features): the 128 x 256 tile starts at one tile per SM; 2048 tokens are one band; features that are no
+# multiple of 32 or 8 leave chunks to the elementwise store
+@pytest.mark.parametrize("m,n", [(2049, 2432), (2050, 2328), (4097, 1184), (129, 136), (2177, 2180), (300, 20000)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("act,act_from", [(None, 0), ("gelu_tanh", 0), ("gelu_tanh", 128), ("silu", 12), ("tanh", 64)])
+def test_epilogue_and_tiles(m, n, fp8, act, act_from):
+    torch.manual_seed(m)
+    k = 256
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16),
+                                    torch.randn(n, device="cuda").to(torch.bfloat16), fp8=fp8)
+    gate = torch.randn(n, device="cuda").to(torch.bfloat16)
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16)
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    y = ops.linear(xq, w, act=act, act_from=act_from, gate=gate, residual=res).float()
+    ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, w.bias, act, gate, res, torch.float32,
+                   act_from=act_from)
+    assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums of 256
+
+
+def test_output_rows_apart():
+    torch.manual_seed(1)
+    x = torch.randn(260, 192, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight.from_dense((torch.randn(320, 192, device="cuda") * 0.07).to(torch.bfloat16))
+    for pitch in (328, 321):                              # rows on 16-byte boundaries, and not
+        buf = torch.zeros(260, pitch, dtype=torch.bfloat16, device="cuda")
+        ops.linear(x, w, out=buf[:, :320])
+        assert torch.allclose(buf[:, :320].float(), x.float() @ w.weight.float().t(), rtol=2 ** -7, atol=2 ** -7)
+        assert not buf[:, 320:].any()
