@@ -562,6 +562,14 @@ def attn_prefill_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
                                    window=window).to(q.dtype)
         return out
     out = torch.empty_like(q)
+    if (d == 128 and causal and softcap == 0.0 and window <= 0 and scale > 0 and page in (8, 16, 32, 64)
+            and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16 == 0):
+        rc = N.lib().b200_attn_prefill_tc(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
+                                          block_table.data_ptr(), kv_lens.data_ptr(), cu_q.data_ptr(), nseq, tq, max_q_len, hq, hkv,
+                                          page, block_table.shape[1], k_cache.shape[0], scale,
+                                          N.state(q.device).status.data_ptr(), N.stream())
+        N.check(rc, "b200_attn_prefill_tc")
+        return out
     rc = N.lib().b200_attn_prefill(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                    block_table.data_ptr(), kv_lens.data_ptr(), cu_q.data_ptr(), None,
                                    nseq, max_q_len, 0, 0, hq, hkv, d, page, block_table.shape[1], 1,
