@@ -29,8 +29,9 @@
 //                more than 2^8, otherwise the stale maximum keeps being used, which is exact
 //                because the final division by the row sum uses the same maximum.
 //
-// V is consumed transposed ([head dim][keys], keys contiguous) so that both MMAs use K-major
-// operands; the transpose (and the int8 quantisation) is a small kernel of its own in front.
+// One sample's V is read as it lies ([key][head dim], an MN-major operand). In a batch, and in the segmented forms
+// below, V is consumed transposed ([head dim][keys]) and padded; that transpose and the int8 quantisation are small
+// kernels of their own in front.
 #include "comm.cuh"
 
 namespace b200 {
@@ -105,7 +106,9 @@ __device__ __forceinline__ void fa_key_tile(const FaParams& p, int j, int& buf_t
   valid = min(kFaTile, p.seg_len - lt * kFaTile);
 }
 
-template <bool kI8>
+// kDirect: V is read as it lies ([key][dim], an MN-major operand) through tm_vt, nothing is transposed (a compile-time
+// matter: both forms in one kernel made the compiler spill inside the key loop, 15 % at 14040 keys).
+template <bool kI8, bool kDirect>
 __global__ void __launch_bounds__(kFaThreads, 1)
 attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
                const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_vt,
@@ -210,8 +213,9 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
                       col0 + a * 64, k_row0 + tile_at * kFaTile);
         if (!mbar_wait(&bars->v_empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
         mbar_arrive_expect_tx(&bars->v_full[s], kVTileBytes);
-        tma_load_2d(sv + s * kVTileBytes, mv, &bars->v_full[s], tile_at * kFaTile, vt_row0);
-        tma_load_2d(sv + s * kVTileBytes + kVTileBytes / 2, mv, &bars->v_full[s], tile_at * kFaTile + 64, vt_row0);
+        for (int a = 0; a < 2; ++a)
+          tma_load_2d(sv + s * kVTileBytes + a * (kVTileBytes / 2), mv, &bars->v_full[s],
+                      kDirect ? col0 + a * 64 : tile_at * kFaTile + a * 64, kDirect ? tile_at * kFaTile : vt_row0);
       }
       if (!ok) report_status(p.status, kWaitTimeout, kKernelAttnPrefill, 21, blockIdx.x);
     }
@@ -252,12 +256,20 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
           // O_t += P_t V_j: A = P_t in TMEM (64 columns of bf16 pairs), B = V^T tile (two atoms of 64 keys)
           const uint32_t d_tmem = tmem_base + 256 + t * 128;
           const uint32_t a_tmem = tmem_base + t * 128;
+          const uint32_t v_at = smem_u32(sv + s * kVTileBytes);
+          if (kDirect) {
+            const uint64_t bd = make_desc_sw128_mn(v_at, kVTileBytes / 2);      // 16 rows (keys) of the tile per product
 #pragma unroll
-          for (int a = 0; a < 2; ++a) {
-            const uint64_t bd = make_desc_sw128(smem_u32(sv + s * kVTileBytes + a * (kVTileBytes / 2)));
+            for (int k = 0; k < 8; ++k)
+              mma_bf16_ts(d_tmem, a_tmem + k * 8, bd + k * (2048 >> 4), kIdescPV | kIdescBMn, (j | k) != 0);
+          } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              mma_bf16_ts(d_tmem, a_tmem + (a * 4 + k) * 8, bd + 2 * k, kIdescPV, (j | a | k) != 0);
+            for (int a = 0; a < 2; ++a) {
+              const uint64_t bd = make_desc_sw128(v_at + a * (kVTileBytes / 2));
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                mma_bf16_ts(d_tmem, a_tmem + (a * 4 + k) * 8, bd + 2 * k, kIdescPV, (j | a | k) != 0);
+            }
           }
           tc_commit(&bars->o_done[t]);
           if (t == nq - 1) tc_commit(&bars->v_empty[s]);
@@ -285,10 +297,8 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
     const int q_idx = qt2 * 2 * kFaTile + t * kFaTile + row;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t s_col = lane_base + t * 128, o_col = lane_base + 256 + t * 128;
-    // position of the row inside its query segment (a plain call has one segment of sq rows)
-    const int q_seg = p.seg_mode ? q_idx / p.seg_pad : 0;
-    const int q_local = q_idx - q_seg * p.seg_pad;
-    const bool q_valid = p.seg_mode ? q_local < p.seg_len : q_idx < p.sq;
+    // whether the row exists: its position inside its query segment (a plain call has one segment of sq rows)
+    const bool q_valid = p.seg_mode ? q_idx % p.seg_pad < p.seg_len : q_idx < p.sq;
     if (t == 0 || tile1) {
       float m_run = -INFINITY, l_run = 0.f;
       float qs = p.scale_log2;
@@ -401,25 +411,37 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
       } else {
         tc_fence_after_sync();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        __nv_bfloat16* dst = p.seg_mode
-            ? p.out_seg[q_valid ? q_seg + p.q_seg_base : 0] + static_cast<long long>(q_local) * p.ld_out + p.out_col0 + col0
-            : p.out + static_cast<long long>(q_row0 + t * kFaTile + row) * p.ld_out + col0;
+        // The Q tile is no longer read: 32 rows of 64 bytes per warp turn the rows that the lanes hold into
+        // 64-byte runs of the output (16-byte pieces of 32 rows at a time leave half-written sectors). Pieces are
+        // placed by (piece xor row / 2), which keeps the banks apart.
+        uint8_t* strip = sq + t * kQkTileBytes + quarter * 32 * 64;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(o_col + c * 32, r);
+        for (int hc = 0; hc < 4; ++hc) {
+          uint32_t o[32];
+          tmem_ld_32x32(o_col + hc * 32, o);
           tmem_ld_wait();
-          if (q_valid) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 v;
-              uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+          for (int i = 0; i < 4; ++i) {
+            uint32_t w[4];
 #pragma unroll
-              for (int u = 0; u < 4; ++u)
-                w[u] = pack_bf16x2(__uint_as_float(r[i + 2 * u]) * inv, __uint_as_float(r[i + 2 * u + 1]) * inv);
-              *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
+            for (int u = 0; u < 4; ++u)
+              w[u] = pack_bf16x2(__uint_as_float(o[i * 8 + 2 * u]) * inv, __uint_as_float(o[i * 8 + 2 * u + 1]) * inv);
+            *reinterpret_cast<uint4*>(strip + lane * 64 + ((i ^ (lane >> 1 & 3)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rr = i * 8 + (lane >> 2), piece = lane & 3;
+            const int qr = q_idx - lane + rr;                                // the query of that row
+            const int sg = p.seg_mode ? qr / p.seg_pad : 0, local = qr - sg * p.seg_pad;
+            const uint4 v = *reinterpret_cast<const uint4*>(strip + rr * 64 + ((piece ^ (rr >> 1 & 3)) * 16));
+            if (p.seg_mode ? local < p.seg_len : qr < p.sq) {
+              __nv_bfloat16* dst = p.seg_mode ? p.out_seg[sg + p.q_seg_base] + static_cast<long long>(local) * p.ld_out + p.out_col0 + col0
+                                              : p.out + static_cast<long long>(b * p.sq + qr) * p.ld_out + col0;
+              *reinterpret_cast<uint4*>(dst + hc * 32 + piece * 8) = v;
             }
           }
+          __syncwarp();
         }
       }
     }
@@ -824,7 +846,7 @@ using namespace b200;
 
 static inline int fa_pad(int s, int to) { return (s + to - 1) / to * to; }
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,
-                     int int8, cudaStream_t stream, const FaPeerMaps* peers = nullptr);
+                     int int8, cudaStream_t stream, const FaPeerMaps* peers = nullptr, bool direct = false);
 
 // Scratch layout of one call: V^T [batch * heads * 128][sk_pad64] bf16, then (int8 mode) Q8
 // [batch * sq][heads * 128], K8 [batch * sk][heads * 128], q scales [batch * heads][sq_pad128],
@@ -855,21 +877,26 @@ B200_API long long b200_attn_fa_workspace_bytes(int batch, int heads, int sq, in
 // Dense attention, head dim 128: q [batch * sq][heads * 128], k / v [batch * sk][heads * 128] bf16
 // (contiguous), out like q: softmax(q k^T * scale) v per (batch, head). int8 != 0: SageAttention
 // (K mean removal, int8 Q K^T). `scratch`: b200_attn_fa_workspace_bytes bytes.
-B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out, int batch, int sq, int sk,
-                          int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
+static int fa_dense(const void* q, const void* k, const void* v, void* out, long long ld_out, int batch, int sq, int sk,
+                    int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
   if (batch <= 0 || sq <= 0 || sk <= 0) return 0;
   if (scratch == nullptr) return -2;
+  if (ld_out % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15)) return -2;
   const long long ld = static_cast<long long>(heads) * kFaD;
   const FaScratch sc = fa_scratch(batch, heads, sq, sk, int8);
   uint8_t* base = static_cast<uint8_t*>(scratch);
   const int sk_pad64 = fa_pad(sk, 64);
+  // One sample: rows past the end of V arrive as zeros, so V is read in place. In a batch they are the next
+  // sample's rows, whose values times a probability of zero need not be zero: V is transposed with padding there
+  // (36 us of 300 at 4608 keys x 24 heads).
+  const bool direct = batch == 1;
   dim3 tgrid((sk_pad64 + 63) / 64, kFaD / 64, batch * heads);
-  fa_transpose_v_kernel<<<tgrid, dim3(32, 8), 0, stream>>>(static_cast<const __nv_bfloat16*>(v),
+  if (!direct) fa_transpose_v_kernel<<<tgrid, dim3(32, 8), 0, stream>>>(static_cast<const __nv_bfloat16*>(v),
                                                            reinterpret_cast<__nv_bfloat16*>(base + sc.vt), ld, sk,
                                                            sk_pad64, heads);
   FaParams p{};
   p.out = static_cast<__nv_bfloat16*>(out);
-  p.ld_out = ld;
+  p.ld_out = ld_out;
   p.sq = sq; p.sk = sk; p.heads = heads; p.batch = batch;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = static_cast<DeviceStatus*>(status);
@@ -907,30 +934,37 @@ B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out
     rc = make_kmajor_map(&tk, k, 2, static_cast<long long>(batch) * sk, ld, ld, 128);
     if (rc) return rc;
   }
-  rc = make_kmajor_map(&tv, base + sc.vt, 2, static_cast<long long>(batch) * heads * kFaD, sk_pad64, sk_pad64, 128);
+  rc = direct ? make_kmajor_map(&tv, v, 2, sk, ld, ld, 128)
+              : make_kmajor_map(&tv, base + sc.vt, 2, static_cast<long long>(batch) * heads * kFaD, sk_pad64, sk_pad64, 128);
   if (rc) return rc;
-  return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads, batch), int8, stream);
+  return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads, batch), int8, stream, nullptr, direct);
+}
+
+B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out, int batch, int sq, int sk,
+                          int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
+  return fa_dense(q, k, v, out, static_cast<long long>(heads) * kFaD, batch, sq, sk, heads, scale, int8, scratch, status, stream);
+}
+
+// The same with rows of the output ld_out values apart (a multiple of 8, the first on a 16-byte boundary).
+B200_API int b200_attn_fa_ld(const void* q, const void* k, const void* v, void* out, long long ld_out, int batch, int sq, int sk,
+                             int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
+  return fa_dense(q, k, v, out, ld_out, batch, sq, sk, heads, scale, int8, scratch, status, stream);
 }
 
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,
-                     int int8, cudaStream_t stream, const FaPeerMaps* peers) {
+                     int int8, cudaStream_t stream, const FaPeerMaps* peers, bool direct) {
   static const FaPeerMaps no_peers{};
   const FaPeerMaps& pm = peers ? *peers : no_peers;
   const int qk_tile = int8 ? 128 * 128 : 128 * 128 * 2;
   const int stages = int8 ? 3 : 2;
   const int smem = 2 * qk_tile + stages * (qk_tile + 128 * 128 * 2) + static_cast<int>(sizeof(FaBarriers)) + 1024;
-  static PerDeviceOnce configured[2];
-  if (int8) {
-    if (configured[1].first_time() &&
-        cudaFuncSetAttribute(attn_fa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -4;
-    attn_fa_kernel<true><<<grid, kFaThreads, smem, stream>>>(p, tq, tk, tv, pm);
-  } else {
-    if (configured[0].first_time() &&
-        cudaFuncSetAttribute(attn_fa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -4;
-    attn_fa_kernel<false><<<grid, kFaThreads, smem, stream>>>(p, tq, tk, tv, pm);
-  }
+  static PerDeviceOnce configured[4];
+  auto* kernel = int8 ? (direct ? attn_fa_kernel<true, true> : attn_fa_kernel<true, false>)
+                      : (direct ? attn_fa_kernel<false, true> : attn_fa_kernel<false, false>);
+  if (configured[(int8 ? 2 : 0) + (direct ? 1 : 0)].first_time() &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return -4;
+  kernel<<<grid, kFaThreads, smem, stream>>>(p, tq, tk, tv, pm);
   const cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? 0 : -(1000 + static_cast<int>(err));   // the CUDA error number stays readable
 }

@@ -248,12 +248,15 @@ class FluxTransformer:
     def _final_mod(self, temb_act: torch.Tensor) -> torch.Tensor:
         return ops.linear(temb_act, self.norm_out)
 
-    def _attend(self, q, k, v, batch: int) -> torch.Tensor:
-        """q, k, v [B * S, Hl, D] -> [B * S, Hl * D]; one attention call per sample."""
+    def _attend(self, q, k, v, batch: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """q, k, v [B * S, Hl, D] -> [B * S, Hl * D] (``out``: where to, rows may lie apart); one attention call per sample."""
         s = q.shape[0] // batch
-        outs = [ops.attention(q[b * s:(b + 1) * s], k[b * s:(b + 1) * s], v[b * s:(b + 1) * s]) for b in range(batch)]
-        o = outs[0] if batch == 1 else torch.cat(outs, 0)
-        return o.reshape(o.shape[0], -1)
+        if out is None:
+            out = torch.empty(q.shape[0], q.shape[1] * q.shape[2], dtype=q.dtype, device=q.device)
+        for b in range(batch):
+            rows = slice(b * s, (b + 1) * s)
+            ops.attention(q[rows], k[rows], v[rows], out=out[rows])
+        return out
 
     def _gated_add(self, x, y, gate, rows_per_batch):
         return ops.gated_residual(x, y, gate, rows_per_batch)
@@ -374,7 +377,9 @@ class FluxTransformer:
     def _row_parallel(self, a, w, x, gate, rows_per_batch, fused, slot):
         """x + gate * all_reduce(a w^T + bias): one fused kernel where it applies."""
         if fused is not None and gate.shape[0] == 1 and fused.supports_large(a.shape[0], w.weight.shape[0]):
-            return fused.large(a, w, res=x.contiguous(), gate=gate.reshape(-1).contiguous(), slot=slot)
+            return fused.large(a.contiguous(), w, res=x.contiguous(), gate=gate.reshape(-1).contiguous(), slot=slot)
+        if self.tp == 1 and gate.shape[0] == 1 and isinstance(w, LinearWeight):
+            return ops.linear(a, w, gate=gate.reshape(-1).contiguous(), residual=x.contiguous())
         return self._gated_add(x, self._reduce(ops.linear(a, w)), gate, rows_per_batch)
 
     def forward(self, img: torch.Tensor, txt: torch.Tensor, timestep: torch.Tensor, pooled: torch.Tensor,
@@ -417,11 +422,11 @@ class FluxTransformer:
         else:
             x_i, x_t, joint = hidden_in
 
-        def stream_pre(x, w: _StreamWeights, mod, S, c, s):
+        def stream_pre(x, w: _StreamWeights, mod, S, c, s, out=None):
             xn, _, xq = ops.norm(x, None, shift=mod[:, 0:H], scale=mod[:, H:2 * H], rows_per_batch=S, layernorm=True,
                                  emit_fp8=self.fp8 and w.qkv.is_fp8, emit_bf16=not (self.fp8 and w.qkv.is_fp8))
             qkv = ops.linear(xq if xq is not None else xn, w.qkv)
-            return ops.dit_qkv(qkv, self.hl, self.hl, D, q_norm_w=w.q_norm, k_norm_w=w.k_norm, cos=c, sin=s)
+            return ops.dit_qkv(qkv, self.hl, self.hl, D, q_norm_w=w.q_norm, k_norm_w=w.k_norm, cos=c, sin=s, out=out)
 
         # the fused row-parallel kernel hands out views of its own buffers: not while something
         # (ControlNet residual collection, the step cache) keeps the streams beyond the next block
@@ -443,15 +448,17 @@ class FluxTransformer:
             if skip_rest:
                 break
             mod_i, mod_t = self._mod(temb_act, wi.mod, "img", self.block_range[0] + bi), self._mod(temb_act, wt.mod, "txt", self.block_range[0] + bi)
-            qi, ki, vi = stream_pre(x_i, wi, mod_i, S_i, cos_i, sin_i)
-            qt, kt, vt = stream_pre(x_t, wt, mod_t, S_t, cos_t, sin_t)
             # joint sequence per sample: [txt | img]
-            def join(a, b):
-                if B == 1:
-                    return torch.cat([a, b], 0)
-                return torch.cat([torch.cat([a[i * S_t:(i + 1) * S_t], b[i * S_i:(i + 1) * S_i]], 0) for i in range(B)], 0)
-            att = self._attend(join(qt, qi), join(kt, ki), join(vt, vi), B)
             S = S_t + S_i
+            if B == 1:       # both streams write their rows of it
+                qkv = [torch.empty(S, self.hl, D, dtype=dt, device=self.device) for _ in range(3)]
+                stream_pre(x_i, wi, mod_i, S_i, cos_i, sin_i, tuple(y[S_t:] for y in qkv))
+                stream_pre(x_t, wt, mod_t, S_t, cos_t, sin_t, tuple(y[:S_t] for y in qkv))
+            else:
+                img_qkv, txt_qkv = stream_pre(x_i, wi, mod_i, S_i, cos_i, sin_i), stream_pre(x_t, wt, mod_t, S_t, cos_t, sin_t)
+                qkv = [torch.cat([torch.cat([a[i * S_t:(i + 1) * S_t], b[i * S_i:(i + 1) * S_i]], 0) for i in range(B)], 0)
+                       for a, b in zip(txt_qkv, img_qkv)]
+            att = self._attend(*qkv, B)
             if B == 1:
                 a_t, a_i = att[:S_t], att[S_t:]
             else:
@@ -483,12 +490,13 @@ class FluxTransformer:
                 mod = self._mod(temb_act, w.mod, "single", si)
                 xn, _, xq = ops.norm(joint, None, shift=mod[:, 0:H], scale=mod[:, H:2 * H], rows_per_batch=S, layernorm=True,
                                      emit_fp8=self.fp8 and w.qkv_mlp.is_fp8, emit_bf16=not (self.fp8 and w.qkv_mlp.is_fp8))
-                fused = ops.linear(xq if xq is not None else xn, w.qkv_mlp)     # [T, 3 Hl D + mlp_l]
+                # [T, q | k | v | mlp]: the activation of the last part is the product's epilogue; once q, k and v are
+                # split off, the attention output takes the place of v, next to the part it is projected with
+                fused = ops.linear(xq if xq is not None else xn, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols)
                 q, k, v = ops.dit_qkv(fused[:, :qkv_cols], self.hl, self.hl, D, q_norm_w=w.q_norm, k_norm_w=w.k_norm,
                                       cos=cj, sin=sj)
-                att = self._attend(q, k, v, B)
-                mlp = torch.nn.functional.gelu(fused[:, qkv_cols:].float(), approximate="tanh").to(dt)
-                joint = self._row_parallel(torch.cat([att, mlp], 1), w.out, joint, mod[:, 2 * H:3 * H], S, rp_fused, si & 1)
+                self._attend(q, k, v, B, out=fused[:, qkv_cols - self.hl * D:qkv_cols])
+                joint = self._row_parallel(fused[:, qkv_cols - self.hl * D:], w.out, joint, mod[:, 2 * H:3 * H], S, rp_fused, si & 1)
                 if collect is not None or (control is not None and control[1]):
                     img_rows = slice(S_t, S) if B == 1 else None
                     if img_rows is None:

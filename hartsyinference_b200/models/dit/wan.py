@@ -229,10 +229,8 @@ class WanTransformer:
             xn, _, xq = ops.norm(x, None, shift=m[:, 0:H], scale=m[:, H:2 * H], rows_per_batch=S_l, layernorm=True,
                                  eps=cfg.eps, emit_fp8=self.fp8 and blk.qkv.is_fp8, emit_bf16=not (self.fp8 and blk.qkv.is_fp8))
             qkv = ops.linear(xq if xq is not None else xn, blk.qkv)                           # [S_l, 3H]
-            qn, _, _ = ops.norm(qkv[:, 0:H].contiguous(), blk.norm_q, eps=cfg.eps)
-            kn, _, _ = ops.norm(qkv[:, H:2 * H].contiguous(), blk.norm_k, eps=cfg.eps)
-            packed = torch.cat([qn, kn, qkv[:, 2 * H:]], 1)
-            q, k, v = ops.dit_qkv(packed, heads, heads, D, cos=cos, sin=sin)
+            q, k, v = ops.dit_qkv(qkv, heads, heads, D, q_norm_w=blk.norm_q, k_norm_w=blk.norm_k, cos=cos, sin=sin, eps=cfg.eps,
+                                  row_norm=True)
             att = self._self_attention(q, k, v)
             x = ops.linear(att, blk.o, gate=m[0, 2 * H:3 * H].contiguous(), residual=x)
             # cross-attention to the text tokens (no gate, affine LayerNorm)

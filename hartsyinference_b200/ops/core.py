@@ -580,40 +580,48 @@ def attn_prefill_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = False,
               scale: Optional[float] = None, softcap: float = 0.0, window: int = 0,
-              int8: Optional[bool] = None) -> torch.Tensor:
+              int8: Optional[bool] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Dense attention for one sequence: q [Tq, hq, d], k/v [Tk, hkv, d] -> [Tq, hq, d].
-    ``int8`` (default: flag ``sage_attention``) selects the int8 Q K^T mode of the tcgen05 kernel."""
+    ``int8`` (default: flag ``sage_attention``) selects the int8 Q K^T mode of the tcgen05 kernel. ``out``: a
+    [Tq, hq * d] matrix to write, whose rows may lie apart."""
     tq, hq, d = q.shape
     tk, hkv, _ = k.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     if not q.is_cuda:
         return R.attention(q, k, v, causal, scale, softcap, window).to(q.dtype)
     assert q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
-    out = torch.empty_like(q)
+    dst = torch.empty_like(q) if out is None else out
     dense_tc = d == 128 and hq == hkv and not causal and softcap == 0.0 and window <= 0 and tk >= 256 and _tc_attention()
+    if out is not None:
+        from .. import config
+        if not (q.is_cuda and d == 128 and hq == hkv and not causal and softcap == 0.0 and window <= 0 and tk >= 256
+                and _tc_attention() and config.get("fa_attention") and out.stride(1) == 1 and out.stride(0) % 8 == 0
+                and out.data_ptr() % 16 == 0):
+            out.copy_(attention(q, k, v, causal, scale, softcap, window, int8).reshape(tq, hq * d))
+            return out
     from .. import config
     if dense_tc and config.get("fa_attention"):
         # long bidirectional sequences (DiT blocks): two query tiles per CTA, S / P / O in TMEM
         L = N.lib()
         i8 = int(config.get("sage_attention") if int8 is None else int8)
         ws = N.state(q.device).scratch(L.b200_attn_fa_workspace_bytes(1, hq, tq, tk, i8))
-        rc = L.b200_attn_fa(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1, tq, tk, hq, float(scale), i8,
-                            ws.data_ptr(), N.state(q.device).status.data_ptr(), N.stream())
-        N.check(rc, "b200_attn_fa", 5 if i8 else 2)
-        return out
+        rc = L.b200_attn_fa_ld(q.data_ptr(), k.data_ptr(), v.data_ptr(), dst.data_ptr(), hq * d if out is None else out.stride(0),
+                               1, tq, tk, hq, float(scale), i8, ws.data_ptr(), N.state(q.device).status.data_ptr(), N.stream())
+        N.check(rc, "b200_attn_fa", 4 if i8 else 1)
+        return dst
     if dense_tc:
         # long bidirectional sequences (DiT blocks): tcgen05 kernel, V consumed transposed
         L = N.lib()
         vt = torch.empty(L.b200_attn_tc_workspace_bytes(1, hq, tk), dtype=torch.uint8, device=q.device)
-        rc = L.b200_attn_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1, tq, tk, hq, float(scale),
+        rc = L.b200_attn_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), dst.data_ptr(), 1, tq, tk, hq, float(scale),
                             vt.data_ptr(), N.state(q.device).status.data_ptr(), N.stream())
         N.check(rc, "b200_attn_tc")
-        return out
-    rc = N.lib().b200_attn_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None, None,
+        return dst
+    rc = N.lib().b200_attn_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), dst.data_ptr(), None, None,
                                    None, None, 1, tq, tq, tk, hq, hkv, d, 16, 0, 0, int(causal), window,
                                    scale, softcap, N.stream())
     N.check(rc, "b200_attn_prefill")
-    return out
+    return dst
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
@@ -798,18 +806,22 @@ def fill_random_(t: torch.Tensor, seed: int, std: float = 0.02) -> torch.Tensor:
 
 def dit_qkv(qkv: torch.Tensor, hq: int, hkv: int, d: int, *, q_norm_w: Optional[torch.Tensor] = None,
             k_norm_w: Optional[torch.Tensor] = None, cos: Optional[torch.Tensor] = None,
-            sin: Optional[torch.Tensor] = None, eps: float = 1e-6):
+            sin: Optional[torch.Tensor] = None, eps: float = 1e-6, row_norm: bool = False,
+            out: Optional[tuple] = None):
     """Split packed qkv [T, (hq + 2 hkv) d] into q [T, hq, d], k, v [T, hkv, d] with optional per-head
-    RMSNorm on q / k and interleaved-pair rotary embedding from per-token tables cos / sin [T, d/2]."""
+    RMSNorm on q / k and interleaved-pair rotary embedding from per-token tables cos / sin [T, d/2].
+    ``row_norm``: the norms run over all heads of a row at once (weights [hq d] and [hkv d]). ``out``: the three
+    (contiguous) tensors to write."""
     t = qkv.shape[0]
     if not qkv.is_cuda:
         x = qkv.float().reshape(t, hq + 2 * hkv, d)
         q, k, v = x[:, :hq], x[:, hq:hq + hkv], x[:, hq + hkv:]
         if q_norm_w is not None:
-            q = q * torch.rsqrt((q * q).mean(-1, keepdim=True) + eps) * q_norm_w.float()
+            q = q * torch.rsqrt((q * q).mean(dims, keepdim=True) + eps) * q_norm_w.float().reshape(-1, d)
         if k_norm_w is not None:
-            k = k * torch.rsqrt((k * k).mean(-1, keepdim=True) + eps) * k_norm_w.float()
+            k = k * torch.rsqrt((k * k).mean(dims, keepdim=True) + eps) * k_norm_w.float().reshape(-1, d)
         if cos is not None:
+        dims = (-2, -1) if row_norm else -1
             def rot(z):
                 a, b = z[..., 0::2], z[..., 1::2]
                 c, s = cos.float()[:, None, :], sin.float()[:, None, :]
@@ -817,15 +829,28 @@ def dit_qkv(qkv: torch.Tensor, hq: int, hkv: int, d: int, *, q_norm_w: Optional[
             q, k = rot(q), rot(k)
         return q.to(qkv.dtype).contiguous(), k.to(qkv.dtype).contiguous(), v.to(qkv.dtype).contiguous()
     assert qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1
-    q = torch.empty(t, hq, d, dtype=torch.bfloat16, device=qkv.device)
-    k = torch.empty(t, hkv, d, dtype=torch.bfloat16, device=qkv.device)
-    v = torch.empty(t, hkv, d, dtype=torch.bfloat16, device=qkv.device)
+    if out is None:
+        out = tuple(torch.empty(t, h, d, dtype=torch.bfloat16, device=qkv.device) for h in (hq, hkv, hkv))
+    q, k, v = out
+    assert all(o.is_contiguous() and o.dtype == torch.bfloat16 for o in out)
+        if out is not None:
+            for o, y in zip(out, (q, k, v)):
+                o.copy_(y)
+            return out
     if cos is not None:
         assert cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-    N.check(N.lib().b200_dit_qkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), N.ptr(q_norm_w),
-                                 N.ptr(k_norm_w), N.ptr(cos), N.ptr(sin), t, hq, hkv, d, qkv.stride(0), eps,
-                                 N.stream()), "b200_dit_qkv")
-    return q, k, v
+    if row_norm and (d % 8 or max(hq, hkv) * d > 8192 or qkv.stride(0) % 8 or any(
+            p is not None and p.data_ptr() % 16 for p in (qkv, q, k, v, q_norm_w, k_norm_w, cos, sin))):
+        # outside the kernel's sizes: the norms by themselves, then the plain split
+        nq, nk = hq * d, hkv * d
+        qn, kn = qkv[:, :nq].contiguous(), qkv[:, nq:nq + nk].contiguous()
+        qn = qn if q_norm_w is None else norm(qn, q_norm_w, eps=eps)[0]
+        kn = kn if k_norm_w is None else norm(kn, k_norm_w, eps=eps)[0]
+        return dit_qkv(torch.cat([qn, kn, qkv[:, nq + nk:]], 1), hq, hkv, d, cos=cos, sin=sin, out=out)
+    fn = N.lib().b200_dit_qkv_row if row_norm else N.lib().b200_dit_qkv
+    N.check(fn(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), N.ptr(q_norm_w), N.ptr(k_norm_w), N.ptr(cos), N.ptr(sin),
+               t, hq, hkv, d, qkv.stride(0), eps, N.stream()), "b200_dit_qkv")
+    return out
 
 
 # ---------------------------------------------------------------------------------------------

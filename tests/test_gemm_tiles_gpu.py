@@ -37,3 +37,14 @@ def test_output_rows_apart():
         ops.linear(x, w, out=buf[:, :320])
         assert torch.allclose(buf[:, :320].float(), x.float() @ w.weight.float().t(), rtol=2 ** -7, atol=2 ** -7)
         assert not buf[:, 320:].any()
+
+
+def test_attention_into_rows_apart():
+    torch.manual_seed(2)
+    for t, h in ((257, 3), (600, 2)):
+        q, k, v = (torch.randn(t, h, 128, device="cuda").to(torch.bfloat16) for _ in range(3))
+        buf = torch.zeros(t, h * 128 + 24, dtype=torch.bfloat16, device="cuda")
+        ops.attention(q, k, v, out=buf[:, 8:8 + h * 128])
+        ref = R.attention(q, k, v)
+        assert torch.allclose(buf[:, 8:8 + h * 128].float().reshape(t, h, 128), ref.float(), rtol=2e-2, atol=1e-2)
+        assert not buf[:, :8].any() and not buf[:, 8 + h * 128:].any()

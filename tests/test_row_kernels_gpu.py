@@ -76,3 +76,19 @@ def test_rotary_and_cache_write(tokens, d, rot, style, norm):
                              style=style, q_norm_w=cpu[0], k_norm_w=cpu[1], want_kv=True)
     for got, ref in ((q, qr), (k, k2), (v, v2), (kc, kr), (vc, vr)):
         assert torch.allclose(got.float().cpu(), ref.float(), rtol=2 ** -6, atol=2 ** -6)
+
+
+@pytest.mark.parametrize("tokens,hq,hkv,d", [(1, 2, 2, 32), (77, 3, 1, 64), (130, 24, 24, 128), (9, 5, 5, 256), (33, 4, 4, 48), (3, 66, 2, 128)])
+@pytest.mark.parametrize("row_norm", [False, True])
+def test_dit_qkv_forms(tokens, hq, hkv, d, row_norm):
+    torch.manual_seed(tokens)
+    width = (hq + 2 * hkv) * d
+    x = _rand(tokens, width + 64)[:, :width]
+    wq, wk = (_rand(hq * d), _rand(hkv * d)) if row_norm else (_rand(d), _rand(d))
+    ang = torch.randn(tokens, d // 2, device="cuda")
+    out = tuple(torch.empty(tokens + 2, h, d, dtype=torch.bfloat16, device="cuda")[2:] for h in (hq, hkv, hkv))
+    got = ops.dit_qkv(x, hq, hkv, d, q_norm_w=wq, k_norm_w=wk, cos=ang.cos(), sin=ang.sin(), row_norm=row_norm, out=out)
+    ref = ops.dit_qkv(x.cpu(), hq, hkv, d, q_norm_w=wq.cpu(), k_norm_w=wk.cpu(), cos=ang.cos().cpu(), sin=ang.sin().cpu(), row_norm=row_norm)
+    for g, o, r in zip(got, out, ref):
+        assert g.data_ptr() == o.data_ptr()
+        assert torch.allclose(g.float().cpu(), r.float(), rtol=2 ** -6, atol=2 ** -6)
