@@ -9,7 +9,11 @@
 // The two order statistics are found by a radix search on the bit pattern of w (positive floats
 // order like their bits): three passes of 11 + 11 + 10 bits, each one histogram of counts and of
 // (fixed-point) masses in shared memory. The draw walks the vocabulary in index order with a block-wide prefix
-// sum of the kept masses. Eight passes over a row that stays in L2.
+// sum of the kept masses.
+//
+// A row of up to 262144 logits belongs to a cluster of eight blocks that keep it in registers: one read of
+// the row, histograms and prefix sums met through distributed shared memory. Longer rows (and the rare device
+// without clusters) go through one block that makes eight passes over a row in L2.
 //
 // The reference applies the same chain on the host, one request at a time, after copying the logits
 // back (src/HartsyInference.LLM/Sampling/SamplerChain.cs:26-85, TopKSampler.cs, TopPSampler.cs,
@@ -336,6 +340,306 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
   }
 }
 
+// ---- one row per cluster -------------------------------------------------------------------------
+constexpr int kRowBlocks = 8;          // blocks of a row's cluster (the portable size)
+constexpr int kRowThreads = 512;
+
+__device__ __forceinline__ uint32_t dsmem_addr(const void* local, int block) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(local)), "r"(block));
+  return r;
+}
+__device__ __forceinline__ unsigned long long ld_dsmem_u64(uint32_t addr) {
+  unsigned long long v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_dsmem_u32x4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// A block's histogram: counts in `lo`, or masses (up to 2^41 each, 2^15 of them) as three 32-bit sums of 14-bit
+// pieces, because 32-bit adds are what shared memory does by itself; 64-bit ones are compare-and-swap loops that
+// the few bins of a peaked row keep failing.
+struct RowHist {
+  unsigned lo[kSampleBins], mid[kSampleBins], hi[kSampleBins];
+};
+struct RowShared {
+  RowHist hist[2];                                    // levels alternate
+  unsigned long long part[kSampleBins];               // the draw's masses per step and warp
+  unsigned long long scan[kRowThreads / 32];
+  unsigned long long front;                           // what lies in front of the chosen bin
+  unsigned long long meet[3];                         // this block's words of the exchanges: (max, index), kept mass, drawn mass
+  unsigned long long all[kRowBlocks];
+  int bin;
+};
+
+// All blocks' words of exchange `n` in sh.all (thread 0 has written sh.meet[n], which is used once).
+__device__ __forceinline__ void row_exchange(RowShared& sh, int n) {
+  cluster_sync_all();
+  if (threadIdx.x < kRowBlocks) sh.all[threadIdx.x] = ld_dsmem_u64(dsmem_addr(&sh.meet[n], threadIdx.x));
+  __syncthreads();
+}
+
+// Sum of `x` over the threads in front of this one; the block's sum in `total`.
+__device__ __forceinline__ unsigned long long row_scan(RowShared& sh, unsigned long long x, unsigned long long& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long incl = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  __syncthreads();
+  if (lane == 31) sh.scan[wid] = incl;
+  __syncthreads();
+  unsigned long long base = 0;
+  total = 0;
+#pragma unroll
+  for (int w = 0; w < kRowThreads / 32; ++w) {
+    const unsigned long long y = sh.scan[w];
+    if (w < wid) base += y;
+    total += y;
+  }
+  return base + incl - x;
+}
+
+// Order statistic of the row's values >= floor_w (see radix_level): by count the `target`-th largest value, by
+// mass the first value, from the largest down, with more than `target` up to and including it. 0 when there is
+// no such value.
+template <int V>
+__device__ __forceinline__ float row_select(RowShared& sh, int& level, const float (&v)[V], float floor_w, bool by_count,
+                                            unsigned long long target) {
+  unsigned prefix = 0u, hi_mask = 0u;
+  unsigned long long before = 0;
+#pragma unroll 1
+  for (int lv = 0; lv < 3; ++lv) {
+    const int shift = lv == 0 ? 21 : lv == 1 ? 10 : 0, bits = lv == 2 ? 10 : 11, nb = 1 << bits;
+    RowHist& hist = sh.hist[level & 1];
+    ++level;
+    for (int b = threadIdx.x; b < kSampleBins; b += kRowThreads) {
+      hist.lo[b] = 0u;
+      if (!by_count) hist.mid[b] = hist.hi[b] = 0u;
+    }
+    if (threadIdx.x == 0) sh.bin = -1;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const unsigned u = __float_as_uint(v[i]);
+      if (v[i] >= floor_w && (u & hi_mask) == prefix) {
+        const int b = (u >> shift) & (nb - 1);
+        if (by_count) {
+          atomicAdd(hist.lo + b, 1u);
+        } else {
+          const unsigned long long m = static_cast<unsigned long long>(v[i] * kMassScale);
+          if (m & 0x3fffu) atomicAdd(hist.lo + b, static_cast<unsigned>(m) & 0x3fffu);
+          if (m >> 14) atomicAdd(hist.mid + b, static_cast<unsigned>(m >> 14) & 0x3fffu);
+          if (m >> 28) atomicAdd(hist.hi + b, static_cast<unsigned>(m >> 28));
+        }
+      }
+    }
+    cluster_sync_all();
+    // every block adds up all blocks' bins; thread t takes four of them, the top ones first
+    const int b0 = kSampleBins - 4 - 4 * static_cast<int>(threadIdx.x);
+    unsigned long long c[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+    for (int k = 0; k < kRowBlocks; ++k) {
+      const uint4 x = ld_dsmem_u32x4(dsmem_addr(hist.lo + b0, k));
+      uint4 y = make_uint4(0u, 0u, 0u, 0u), z = y;
+      if (!by_count) {
+        y = ld_dsmem_u32x4(dsmem_addr(hist.mid + b0, k));
+        z = ld_dsmem_u32x4(dsmem_addr(hist.hi + b0, k));
+      }
+      const unsigned xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w}, zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        c[j] += xs[j] + (static_cast<unsigned long long>(ys[j]) << 14) + (static_cast<unsigned long long>(zs[j]) << 28);
+    }
+    unsigned long long total;
+    unsigned long long front = before + row_scan(sh, c[0] + c[1] + c[2] + c[3], total);
+#pragma unroll
+    for (int j = 3; j >= 0; --j) {
+      const unsigned long long upto = front + c[j];
+      // one bin at most: what lies in front has not reached the target, with it it has
+      const bool hit = c[j] != 0ull && (by_count ? front < target && upto >= target : front <= target && upto > target);
+      if (hit) { sh.bin = b0 + j; sh.front = front; }
+      front = upto;
+    }
+    __syncthreads();
+    const int chosen = sh.bin;
+    if (chosen < 0) return 0.f;
+    before = sh.front;
+    prefix |= static_cast<unsigned>(chosen) << shift;
+    hi_mask |= static_cast<unsigned>(nb - 1) << shift;
+    __syncthreads();
+  }
+  return __uint_as_float(prefix);
+}
+
+// The filter chain and the draw of sample_kernel with the row in registers: thread t of block b holds the values
+// (b * V + i) * 512 + t. Masses are 2^-40 fixed point throughout, so sums do not depend on their order.
+// Bound by the adds into the first histogram of a search, whose bins are few, and by the chain of exchanges, not by
+// memory. 64 rows of 128256: top-k 388 -> 95 us, top-p 432 -> 205, both 483 -> 257, neither 90 -> 42; one row with both
+// 469 -> 73 us.
+template <int V>
+__global__ void __launch_bounds__(kRowThreads, V <= 40 ? 2 : 1) sample_row_kernel(const SampleParams p) {
+  extern __shared__ __align__(16) uint8_t row_smem[];
+  RowShared& sh = *reinterpret_cast<RowShared*>(row_smem);
+  const int row = blockIdx.x / kRowBlocks, block = blockIdx.x % kRowBlocks;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long row_off = static_cast<long long>(row) * p.ld;
+  const int first = block * V * kRowThreads + threadIdx.x;
+  float v[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int at = first + i * kRowThreads;
+    v[i] = at < p.vocab ? sample_logit(p, row_off, at) : -INFINITY;
+  }
+  // ---- maximum and its first index: ordered so that the largest word is the largest logit, then the lowest index
+  float mx = -INFINITY;
+  int arg = 0x7fffffff;
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (v[i] > mx) { mx = v[i]; arg = first + i * kRowThreads; }
+  auto word = [](float f, int i) {
+    const unsigned u = __float_as_uint(f), key = u & 0x80000000u ? ~u : u | 0x80000000u;
+    return static_cast<unsigned long long>(key) << 32 | static_cast<unsigned>(0x7fffffff - i);
+  };
+  if (mx == 0.f) mx = 0.f;                     // -0 and +0 tie
+  unsigned long long best = word(mx, arg);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, best, o);
+    best = y > best ? y : best;
+  }
+  if (lane == 0) sh.scan[wid] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kRowThreads / 32; ++w) best = sh.scan[w] > best ? sh.scan[w] : best;
+    sh.meet[0] = best;
+  }
+  row_exchange(sh, 0);
+  best = sh.all[0];
+#pragma unroll
+  for (int k = 1; k < kRowBlocks; ++k) best = sh.all[k] > best ? sh.all[k] : best;
+  const unsigned key = static_cast<unsigned>(best >> 32);
+  const float bmx = __uint_as_float(key & 0x80000000u ? key & 0x7fffffffu : ~key);
+  const int top = 0x7fffffff - static_cast<int>(static_cast<unsigned>(best));
+  const float temp = p.temperature[row];
+  if (temp <= 0.f || !(bmx > -INFINITY)) {
+    if (block == 0 && threadIdx.x == 0) p.out[row] = top == 0x7fffffff ? 0 : top;
+    cluster_sync_all();                        // nobody leaves while a peer may still read its words
+    return;
+  }
+  const float inv_t = 1.f / fmaxf(temp, 1e-6f);
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    v[i] = first + i * kRowThreads < p.vocab ? __expf((v[i] - bmx) * inv_t) : -1.f;      // below every threshold
+
+  int level = 0;
+  float tau = 0.f;
+  const int k = p.top_k[row];
+  if (k > 0 && k < p.vocab) tau = row_select<V>(sh, level, v, 0.f, true, static_cast<unsigned long long>(k));
+  const float tp = p.top_p[row];
+  if (tp > 0.f && tp < 1.f) {
+    unsigned long long mine = 0, total;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (v[i] >= tau) mine += static_cast<unsigned long long>(v[i] * kMassScale);
+    row_scan(sh, mine, total);
+    if (threadIdx.x == 0) sh.meet[1] = total;
+    row_exchange(sh, 1);
+    total = 0;
+#pragma unroll
+    for (int b = 0; b < kRowBlocks; ++b) total += sh.all[b];
+    const unsigned long long limit = static_cast<unsigned long long>(static_cast<double>(tp) * static_cast<double>(total));
+    tau = fmaxf(tau, row_select<V>(sh, level, v, tau, false, limit));
+  }
+  const float mp = p.min_p[row];
+  if (mp > 0.f) tau = fmaxf(tau, fminf(mp, 1.f));
+
+  // ---- draw: index-ordered prefix sums of the kept masses, per warp and step first
+  __syncthreads();
+  unsigned long long* part = sh.part;                      // [V steps][16 warps]
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    unsigned long long m = v[i] >= tau ? static_cast<unsigned long long>(v[i] * kMassScale) : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    if (lane == 0) part[i * (kRowThreads / 32) + wid] = m;
+  }
+  __syncthreads();
+  constexpr int kParts = V * (kRowThreads / 32), kEach = (kParts + kRowThreads - 1) / kRowThreads;
+  unsigned long long mine = 0, total;
+#pragma unroll
+  for (int e = 0; e < kEach; ++e) {
+    const int at = threadIdx.x * kEach + e;
+    if (at < kParts) mine += part[at];
+  }
+  const unsigned long long own = row_scan(sh, mine, total);      // parts in front of this thread's
+  if (threadIdx.x == 0) { sh.meet[2] = total; sh.bin = -1; }
+  row_exchange(sh, 2);
+  unsigned long long before = 0, all = 0;
+#pragma unroll
+  for (int b = 0; b < kRowBlocks; ++b) {
+    if (b < block) before += sh.all[b];
+    all += sh.all[b];
+  }
+  // u in [0, all): the 24-bit uniform number times the whole mass
+  const unsigned long long bits = static_cast<unsigned long long>(sample_uniform(p.seed[row], p.counter[row]) * 16777216.f);
+  const unsigned long long u = __umul64hi(all, bits << 40);
+  unsigned long long run = before + own;
+#pragma unroll
+  for (int e = 0; e < kEach; ++e) {
+    const int at = threadIdx.x * kEach + e;
+    const unsigned long long m = at < kParts ? part[at] : 0ull;
+    if (m != 0ull && u >= run && u < run + m) { sh.bin = at; sh.front = run; }
+    run += m;
+  }
+  __syncthreads();
+  const int at = sh.bin;
+  if (at >= 0 && wid == at % (kRowThreads / 32)) {
+    const int step = at / (kRowThreads / 32);
+    float w = -1.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (i == step) w = v[i];
+    const unsigned long long m = w >= tau ? static_cast<unsigned long long>(w * kMassScale) : 0ull;
+    unsigned long long incl = m;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    incl += sh.front;
+    if (m != 0ull && u >= incl - m && u < incl) p.out[row] = first + step * kRowThreads;
+  }
+  if (all == 0ull && block == 0 && threadIdx.x == 0) p.out[row] = top;      // no finite mass: the most probable token
+  cluster_sync_all();
+}
+
+template <int V>
+static int launch_rows(const SampleParams& p, int rows, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * kRowBlocks);
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.dynamicSmemBytes = sizeof(RowShared);
+  cfg.stream = stream;
+  static PerDeviceOnce configured;
+  if (configured.first_time() &&
+      cudaFuncSetAttribute(sample_row_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(RowShared)) != cudaSuccess)
+    return -200;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kRowBlocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, sample_row_kernel<V>, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -300;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -350,6 +654,14 @@ B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows,
   p.logits = logits; p.is_f32 = is_f32; p.ld = ld; p.vocab = vocab;
   p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.min_p = min_p;
   p.seed = seed; p.counter = counter; p.out = out;
+  const int each = (vocab + kRowBlocks * kRowThreads - 1) / (kRowBlocks * kRowThreads);      // values a thread holds
+  if (rows < (1 << 27)) {
+    if (each <= 8) return launch_rows<8>(p, rows, stream);
+    if (each <= 16) return launch_rows<16>(p, rows, stream);
+    if (each <= 32) return launch_rows<32>(p, rows, stream);
+    if (each <= 40) return launch_rows<40>(p, rows, stream);
+    if (each <= 64) return launch_rows<64>(p, rows, stream);
+  }
   sample_kernel<<<rows, kSampleThreads, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -300;
 }
