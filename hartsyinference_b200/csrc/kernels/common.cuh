@@ -451,24 +451,47 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
 struct SplitPartials {
   const float* ws;     // nullptr: the consumer reads its ordinary bf16 input
   int splits, bn;
+  const __nv_bfloat16* bias = nullptr;      // per feature, added ahead of the rounding (16-byte aligned)
 };
 __device__ __forceinline__ float split_sum(const SplitPartials& sp, int token, int feature) {
   const float* base = sp.ws + (static_cast<long long>(feature >> 7) * sp.splits * sp.bn + token) * 128 + (feature & 127);
   float acc = 0.f;
   for (int s = 0; s < sp.splits; ++s) acc += __ldcg(base + static_cast<long long>(s) * sp.bn * 128);
+  if (sp.bias) acc += __bfloat162float(sp.bias[feature]);
   return __bfloat162float(__float2bfloat16(acc));
 }
 // eight consecutive features (feature0 a multiple of 8)
 __device__ __forceinline__ void split_sum8(const SplitPartials& sp, int token, int feature0, float (&out)[8]) {
   const float* base = sp.ws + (static_cast<long long>(feature0 >> 7) * sp.splits * sp.bn + token) * 128 + (feature0 & 127);
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-  for (int s = 0; s < sp.splits; ++s) {
-    const float4 x = __ldcg(reinterpret_cast<const float4*>(base + static_cast<long long>(s) * sp.bn * 128));
-    const float4 y = __ldcg(reinterpret_cast<const float4*>(base + static_cast<long long>(s) * sp.bn * 128 + 4));
-    a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-    b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+  // four ranges' loads at a time: the ranges are few, and their latency is what counts
+  for (int s0 = 0; s0 < sp.splits; s0 += 4) {
+    float4 x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (s0 + u < sp.splits) {
+        x[u] = __ldcg(reinterpret_cast<const float4*>(base + static_cast<long long>(s0 + u) * sp.bn * 128));
+        y[u] = __ldcg(reinterpret_cast<const float4*>(base + static_cast<long long>(s0 + u) * sp.bn * 128 + 4));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      a.x += x[u].x; a.y += x[u].y; a.z += x[u].z; a.w += x[u].w;
+      b.x += y[u].x; b.y += y[u].y; b.z += y[u].z; b.w += y[u].w;
+    }
   }
-  const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (sp.bias) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(sp.bias + feature0));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      v[2 * i] += f.x;
+      v[2 * i + 1] += f.y;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) out[i] = __bfloat162float(__float2bfloat16(v[i]));
 }

@@ -99,6 +99,7 @@ __device__ __forceinline__ void store_fp8(const float (&y)[8], float amax, uint8
 
 struct NormParams {
   const __nv_bfloat16* x;         // [rows][dim]
+  SplitPartials part;             // ws != null: x comes as unsummed K ranges of the producing GEMM
   const __nv_bfloat16* residual;  // optional [rows][dim]: h = x + residual
   __nv_bfloat16* residual_out;    // optional: receives h
   const __nv_bfloat16* weight;    // optional [dim]
@@ -121,8 +122,9 @@ struct NormParams {
 // rows share a processor and one row's loads run under another's reduction; few rows (decoding) take one
 // vector a thread, where the latency of a single row is what counts. Residual + norm + fp8, one vector a
 // thread before: 8192 x 8192 163.6 -> 112.5 us (5.4 TB/s), 14040 x 5120 160 -> 118 us; two vectors instead of
-// four 123 and 118, so four start at rows of 8192.
-template <int kMaxVec>
+// four 123 and 118, so four start at rows of 8192. Unsummed K ranges are read by instances of their own (kParts):
+// the branch alone kept the loads of the others apart (131 us).
+template <int kMaxVec, bool kParts>
 __global__ void __launch_bounds__(1024) norm_kernel(const NormParams p) {
   pdl_wait();
   pdl_trigger();   // a GEMM launched behind this kernel may start fetching its weights now
@@ -136,7 +138,13 @@ __global__ void __launch_bounds__(1024) norm_kernel(const NormParams p) {
     const int vi = threadIdx.x + it * blockDim.x;
     raw[it] = res[it] = make_uint4(0u, 0u, 0u, 0u);
     if (vi < nvec) {
-      raw[it] = *reinterpret_cast<const uint4*>(p.x + base + vi * 8);
+      if (kParts) {
+        float sum8[8];
+        split_sum8(p.part, row, vi * 8, sum8);
+        raw[it] = pack_bf16x8(sum8);
+      } else {
+        raw[it] = *reinterpret_cast<const uint4*>(p.x + base + vi * 8);
+      }
       if (p.residual) res[it] = *reinterpret_cast<const uint4*>(p.residual + base + vi * 8);
     }
   }
@@ -321,18 +329,20 @@ __global__ void quant_fp8_weight_kernel(const __nv_bfloat16* __restrict__ w,
 // 0 = SiLU, 1 = GELU-tanh. Optional fp8 1x128 output (F % 128 == 0). A thread keeps its vector of eight columns
 // and takes kRows rows, whose loads go out together; grid (column blocks, row groups), so no index is divided.
 // Arithmetic and HBM bind about equally: 8192 x 28672 with fp8 output 485 -> 365 us, bf16 338 -> 270 us
-// (one row a thread 377 and 300, four 490 and 361: too many registers).
+// (one row a thread 377 and 300, four 490 and 361: too many registers; blocks that walk rows with three in flight
+// 383 and 256).
 template <int kRows>
 __global__ void __launch_bounds__(256) glu_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
                            uint8_t* __restrict__ out_fp8, float* __restrict__ out_scale, int rows,
                            int f, int act, int sf_tile_rows, const SplitPartials part) {
   pdl_wait();
   pdl_trigger();
+  constexpr bool kParts = kRows == 1;          // unsummed K ranges come from small batches only
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   const bool col = vi < (f >> 3);              // f % 128 == 0 with the fp8 output: a 16-lane group is uniform
   for (int row0 = blockIdx.y * kRows; row0 < rows; row0 += gridDim.y * kRows) {
     uint4 graw[kRows], uraw[kRows];
-    if (!part.ws) {
+    if (!(kParts && part.ws)) {
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
         graw[r] = uraw[r] = make_uint4(0u, 0u, 0u, 0u);
@@ -348,7 +358,7 @@ __global__ void __launch_bounds__(256) glu_kernel(const __nv_bfloat16* __restric
       const int row = row0 + r;
       const bool active = col && row < rows;
       float gv[8], uv[8];
-      if (part.ws) {
+      if (kParts && part.ws) {
         // the producing GEMM left its K ranges unsummed: add them here (no reduce kernel in between)
 #pragma unroll
         for (int k = 0; k < 8; ++k) gv[k] = uv[k] = 0.f;
@@ -648,16 +658,36 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const __nv_bfloat1
   }
 }
 
-// argmax over the last dim of bf16 / fp32 logits [rows][vocab]; ties -> lowest index.
+// argmax over the last dim of bf16 / fp32 logits [rows][vocab]; ties -> lowest index. One block per row; with rows on
+// 16-byte boundaries (vec) a thread reads 16 bytes at a time, four in flight: one row of 151936 bf16 42 -> 8 us.
 template <typename T>
-__global__ void argmax_kernel(const T* __restrict__ logits, int* __restrict__ out, int vocab,
-                              long long ld) {
+__global__ void __launch_bounds__(1024) argmax_kernel(const T* __restrict__ logits, int* __restrict__ out, int vocab,
+                              long long ld, int vec) {
   __shared__ float sval[32];
   __shared__ int sidx[32];
   const T* row = logits + blockIdx.x * ld;
   float best = -INFINITY;
   int bi = 0x7fffffff;
-  for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
+  constexpr int kPer = 16 / sizeof(T);
+  const int nvec = vec ? vocab / kPer : 0;
+  for (int i0 = threadIdx.x; i0 < nvec; i0 += 4 * blockDim.x) {
+    uint4 raw[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * blockDim.x < nvec) raw[u] = __ldg(reinterpret_cast<const uint4*>(row) + i0 + u * blockDim.x);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * blockDim.x;
+      if (i >= nvec) break;
+      const T* e = reinterpret_cast<const T*>(&raw[u]);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const float v = static_cast<float>(e[k]);
+        if (v > best) { best = v; bi = i * kPer + k; }       // a thread's indices ascend
+      }
+    }
+  }
+  for (int i = nvec * kPer + threadIdx.x; i < vocab; i += blockDim.x) {
     const float v = static_cast<float>(row[i]);
     if (v > best || (v == best && i < bi)) { best = v; bi = i; }
   }
@@ -811,17 +841,19 @@ using namespace b200;
     if (e__ != cudaSuccess) return -static_cast<int>(e__) - 300;  \
   } while (0)
 
-// (residual +) RMSNorm / LayerNorm with optional affine, AdaLN modulation, bf16 and/or fp8 output.
+// (residual +) RMSNorm / LayerNorm with optional affine, AdaLN modulation, bf16 and/or fp8 output. part_ws != null: x
+// is ignored and the rows are read as unsummed K ranges (see b200_glu).
 B200_API int b200_norm(const void* x, const void* residual, void* residual_out, const void* weight,
                        const void* bias, const void* shift, const void* scale, void* out,
                        void* out_fp8, float* out_scale, int rows, int dim, int rows_per_batch,
                        int mod_stride, float eps, int layernorm, int weight_plus_one,
-                       int sf_tile_rows, cudaStream_t stream) {
+                       int sf_tile_rows, const float* part_ws, int part_splits, int part_bn, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (dim % 8 != 0 || dim > 16384) return -2;
   if (out_fp8 && dim % 128 != 0) return -3;
   NormParams p{};
   p.x = static_cast<const __nv_bfloat16*>(x);
+  p.part = SplitPartials{part_ws, part_splits, part_bn};
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.residual_out = static_cast<__nv_bfloat16*>(residual_out);
   p.weight = static_cast<const __nv_bfloat16*>(weight);
@@ -839,9 +871,10 @@ B200_API int b200_norm(const void* x, const void* residual, void* residual_out, 
   auto go = [&](auto* kernel, int per) {
     launch_pdl(kernel, dim3(rows), dim3(((nvec + per - 1) / per + 31) / 32 * 32), 0, stream, p);
   };
-  if (rows > 296 && nvec >= 1024) go(norm_kernel<4>, 4);
-  else if (nvec > 1024 || (rows > 296 && nvec >= 256)) go(norm_kernel<2>, 2);
-  else go(norm_kernel<1>, 1);
+  if (part_ws != nullptr) nvec > 1024 ? go(norm_kernel<2, true>, 2) : go(norm_kernel<1, true>, 1);
+  else if (rows > 296 && nvec >= 1024) go(norm_kernel<4, false>, 4);
+  else if (nvec > 1024 || (rows > 296 && nvec >= 256)) go(norm_kernel<2, false>, 2);
+  else go(norm_kernel<1, false>, 1);
   CHECK_LAUNCH();
   return 0;
 }
@@ -876,7 +909,7 @@ B200_API int b200_glu(const void* in, void* out, void* out_fp8, float* out_scale
                       cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (f % 8 != 0 || (out_fp8 && f % 128 != 0)) return -2;
-  const RowGrid g(rows, f / 8, 2);
+  const RowGrid g(rows, f / 8, part_ws != nullptr ? 1 : 2);
   const SplitPartials part{part_ws, part_splits, part_bn};
   launch_pdl(g.rows_each == 2 ? glu_kernel<2> : glu_kernel<1>, g.grid, g.block, 0, stream, static_cast<const __nv_bfloat16*>(in),
              static_cast<__nv_bfloat16*>(out), static_cast<uint8_t*>(out_fp8), out_scale, rows, f, act, sf_tile_rows,
@@ -890,11 +923,11 @@ B200_API int b200_rope_kv(const void* qkv, void* q_out, void* k_cache, void* v_c
                           const void* q_norm_w, const void* k_norm_w, const float* inv_freq,
                           int tokens, int hq, int hkv, int d, int rot, int style, int page,
                           float theta, float eps, const float* part_ws, int part_splits, int part_bn,
-                          cudaStream_t stream) {
+                          const void* part_bias, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (d > 256 || rot > d || (rot & 1)) return -2;
   RopeParams p{};
-  p.part = SplitPartials{part_ws, part_splits, part_bn};
+  p.part = SplitPartials{part_ws, part_splits, part_bn, static_cast<const __nv_bfloat16*>(part_bias)};
   p.qkv = static_cast<const __nv_bfloat16*>(qkv);
   p.q_out = static_cast<__nv_bfloat16*>(q_out);
   p.k_cache = static_cast<__nv_bfloat16*>(k_cache);
@@ -912,7 +945,7 @@ B200_API int b200_rope_kv(const void* qkv, void* q_out, void* k_cache, void* v_c
   int unit_bits = 0;
   while (16 << unit_bits < d) ++unit_bits;
   if (16 << unit_bits == d && rot % 16 == 0 && (style == 0 || style == 1) &&
-      aligned16(qkv, q_out, k_cache, v_cache, k_out, v_out, q_norm_w, k_norm_w, part_ws)) {
+      aligned16(qkv, q_out, k_cache, v_cache, k_out, v_out, q_norm_w, k_norm_w, part_ws, part_bias)) {
     const int block_heads = 256 >> unit_bits;
     const int chunks = (heads + block_heads - 1) / block_heads;
     const int each = tokens >= 148 * 8 ? 4 : 1;      // more tokens a block once every processor has several
@@ -943,10 +976,11 @@ B200_API int b200_embedding(const int* ids, const void* table, void* out, int to
 B200_API int b200_argmax(const void* logits, int* out, int rows, int vocab, long long ld,
                          int is_fp32, cudaStream_t stream) {
   if (rows <= 0) return 0;
+  const int vec = aligned16(logits) && ld * (is_fp32 ? 4 : 2) % 16 == 0 ? 1 : 0;
   if (is_fp32)
-    argmax_kernel<float><<<rows, 1024, 0, stream>>>(static_cast<const float*>(logits), out, vocab, ld);
+    argmax_kernel<float><<<rows, 1024, 0, stream>>>(static_cast<const float*>(logits), out, vocab, ld, vec);
   else
-    argmax_kernel<__nv_bfloat16><<<rows, 1024, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), out, vocab, ld);
+    argmax_kernel<__nv_bfloat16><<<rows, 1024, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), out, vocab, ld, vec);
   CHECK_LAUNCH();
   return 0;
 }
@@ -1016,6 +1050,18 @@ struct DitQkvParams {
   float eps;
 };
 
+// Four neighbouring pairs times their (cos, sin).
+__device__ __forceinline__ void turn_pairs(float (&v)[8], const float* cos, const float* sin) {
+  const float4 c = __ldg(reinterpret_cast<const float4*>(cos)), s = __ldg(reinterpret_cast<const float4*>(sin));
+  const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float x = v[2 * k], y = v[2 * k + 1];
+    v[2 * k] = x * cs[k] - y * sn[k];
+    v[2 * k + 1] = y * cs[k] + x * sn[k];
+  }
+}
+
 __global__ void dit_qkv_kernel(const DitQkvParams p) {
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1050,18 +1096,6 @@ __global__ void dit_qkv_kernel(const DitQkvParams p) {
         b[i] *= rstd * __bfloat162float(nw[2 * pi + 1]);
       }
     }
-// Four neighbouring pairs times their (cos, sin).
-__device__ __forceinline__ void turn_pairs(float (&v)[8], const float* cos, const float* sin) {
-  const float4 c = __ldg(reinterpret_cast<const float4*>(cos)), s = __ldg(reinterpret_cast<const float4*>(sin));
-  const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float x = v[2 * k], y = v[2 * k + 1];
-    v[2 * k] = x * cs[k] - y * sn[k];
-    v[2 * k + 1] = y * cs[k] + x * sn[k];
-  }
-}
-
   }
   __nv_bfloat16* dst;
   if (kind == 0) dst = p.q + (static_cast<long long>(t) * p.hq + h) * p.d;
@@ -1081,28 +1115,6 @@ __device__ __forceinline__ void turn_pairs(float (&v)[8], const float* cos, cons
       *reinterpret_cast<__nv_bfloat162*>(dst + 2 * pi) = __floats2bfloat162_rn(x, y);
     }
   }
-}
-}  // namespace b200
-
-B200_API int b200_dit_qkv(const void* qkv, void* q, void* k, void* v, const void* q_norm_w,
-                          const void* k_norm_w, const float* cos, const float* sin, int tokens, int hq,
-                          int hkv, int d, long long ld, float eps, cudaStream_t stream) {
-  if (tokens <= 0) return 0;
-  if (d > 256 || (d & 1)) return -2;
-  DitQkvParams p{};
-  p.qkv = static_cast<const __nv_bfloat16*>(qkv);
-  p.q = static_cast<__nv_bfloat16*>(q);
-  p.k = static_cast<__nv_bfloat16*>(k);
-  p.v = static_cast<__nv_bfloat16*>(v);
-  p.q_norm_w = static_cast<const __nv_bfloat16*>(q_norm_w);
-  p.k_norm_w = static_cast<const __nv_bfloat16*>(k_norm_w);
-  p.cos = cos; p.sin = sin;
-  p.tokens = tokens; p.hq = hq; p.hkv = hkv; p.d = d; p.ld = ld; p.eps = eps;
-  const long long warps = static_cast<long long>(tokens) * (hq + 2 * hkv);
-  const long long blocks = (warps * 32 + 255) / 256;
-  dit_qkv_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p);
-  CHECK_LAUNCH();
-  return 0;
 }
 
 // The same for heads of 32, 64, 128 or 256 values with everything on 16-byte boundaries: a thread takes 16
@@ -1213,6 +1225,23 @@ __global__ void __launch_bounds__(256) dit_qkv_row_kernel(const DitQkvParams p) 
   for (int at = threadIdx.x; at < nk; at += 256)
     reinterpret_cast<uint4*>(p.v + static_cast<long long>(t) * nk * 8)[at] = src[nq + nk + at];
 }
+}  // namespace b200
+
+B200_API int b200_dit_qkv(const void* qkv, void* q, void* k, void* v, const void* q_norm_w,
+                          const void* k_norm_w, const float* cos, const float* sin, int tokens, int hq,
+                          int hkv, int d, long long ld, float eps, cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if (d > 256 || (d & 1)) return -2;
+  DitQkvParams p{};
+  p.qkv = static_cast<const __nv_bfloat16*>(qkv);
+  p.q = static_cast<__nv_bfloat16*>(q);
+  p.k = static_cast<__nv_bfloat16*>(k);
+  p.v = static_cast<__nv_bfloat16*>(v);
+  p.q_norm_w = static_cast<const __nv_bfloat16*>(q_norm_w);
+  p.k_norm_w = static_cast<const __nv_bfloat16*>(k_norm_w);
+  p.cos = cos; p.sin = sin;
+  p.tokens = tokens; p.hq = hq; p.hkv = hkv; p.d = d; p.ld = ld; p.eps = eps;
+  const long long warps = static_cast<long long>(tokens) * (hq + 2 * hkv);
   int unit_bits = 1;
   while (16 << unit_bits < d) ++unit_bits;
   if (16 << unit_bits == d && ld % 8 == 0 && aligned16(qkv, q, k, v, q_norm_w, k_norm_w, cos, sin) && warps << unit_bits < 1ll << 31) {
@@ -1220,6 +1249,11 @@ __global__ void __launch_bounds__(256) dit_qkv_row_kernel(const DitQkvParams p) 
     CHECK_LAUNCH();
     return 0;
   }
+  const long long blocks = (warps * 32 + 255) / 256;
+  dit_qkv_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p);
+  CHECK_LAUNCH();
+  return 0;
+}
 
 // b200_dit_qkv with the norms taken over the whole rows of q and k (weights [hq * d] and [hkv * d]). Returns -2 for
 // sizes or alignments that it does not take.

@@ -1869,7 +1869,7 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   }
   if (defer_info != nullptr) {
     // the caller's consumer kernel sums the K ranges itself: report their layout, launch no reduce
-    const bool deferred = rc == 0 && p.external_reduce && swap && groups == 0 && bias == nullptr &&
+    const bool deferred = rc == 0 && p.external_reduce && swap && groups == 0 &&
                           gate == nullptr && residual == nullptr && act == 0 && m <= bn;
     defer_info[0] = deferred ? 1 : 0;
     defer_info[1] = p.splits;
@@ -1917,15 +1917,15 @@ B200_API int b200_gemm(const void* x, const void* w, void* out, int m, int n, in
 }
 
 // b200_gemm for a consumer that can add split-K ranges itself (b200_glu, b200_rope_kv): when the
-// policy cuts every tile along K (small-token GEMMs with fewer tiles than SMs) and no epilogue term
-// is asked for, the reduce kernel is NOT launched and `out` is left untouched; info[0] = 1 then and
+// policy cuts every tile along K (small-token GEMMs with fewer tiles than SMs), the reduce kernel is NOT
+// launched (the consumer adds `bias` too) and `out` is left untouched; info[0] = 1 then and
 // the partials sit at workspace + 16384 bytes as [feature tile][info[1] K ranges][info[2] tokens][128]
 // fp32. Otherwise info[0] = 0 and `out` holds the result as usual.
 B200_API int b200_gemm_deferred(const void* x, const void* w, void* out, int m, int n, int k, long long ldx,
                                 long long ldw, long long ldc, int dtype, const float* x_scale,
-                                const float* w_scale, void* workspace, long long workspace_bytes, int* info,
+                                const float* w_scale, const void* bias, void* workspace, long long workspace_bytes, int* info,
                                 void* status, cudaStream_t stream) {
-  return gemm_impl(x, w, out, m, n, k, ldx, ldw, ldc, dtype, x_scale, w_scale, nullptr, nullptr, nullptr, 0, 0,
+  return gemm_impl(x, w, out, m, n, k, ldx, ldw, ldc, dtype, x_scale, w_scale, bias, nullptr, nullptr, 0, 0,
                    workspace, workspace_bytes, status, stream, nullptr, nullptr, nullptr, info);
 }
 

@@ -106,16 +106,21 @@ class MlaAttention:
         lens = batch.kv_lens.to(torch.int64)[seq] - (last - rows)
         return seq.to(torch.int32), lens.clamp_(min=0).to(torch.int32)
 
-    def __call__(self, h: torch.Tensor, batch, li: int, model) -> torch.Tensor:
+    defers = True          # takes ``defer``, see DecoderModel._reduce_linear
+
+    def __call__(self, h: torch.Tensor, batch, li: int, model, defer: bool = False) -> torch.Tensor:
         cfg, m, w = self.cfg, self.m, self.w
         t = h.shape[0]
+        fold = w.q_fold is not None and t <= FOLD_MAX_TOKENS
         qin = h
         if w.q_a is not None:
             qa = ops.linear(h, w.q_a)
-            qin, _, _ = ops.norm(qa, w.q_a_norm, eps=cfg.rms_eps)
+            q8 = qa.is_cuda and (w.q_fold if fold else w.q_b).is_fp8       # the norm emits the next product's input itself
+            qin, _, qin8 = ops.norm(qa, w.q_a_norm, eps=cfg.rms_eps, emit_fp8=q8, emit_bf16=not q8)
+            qin = qin8 if q8 else qin
         kv = ops.linear(h, w.kv_a)
         cache = model.kv_cache[li] if model.kv_cache is not None else None      # [pages, page, 576]
-        if w.q_fold is not None and t <= FOLD_MAX_TOKENS:
+        if fold:
             # absorbed queries straight from the folded projection; the rotary part is rotated in place
             q_abs = ops.linear(qin, w.q_fold).view(t, self.heads, ROW)
             ops.mla_prep(kv, w.kv_a_norm, q_abs.view(t, self.heads * ROW), q_abs, cache, batch.positions,
@@ -131,7 +136,9 @@ class MlaAttention:
                            max_kv_len=batch.max_kv_len or None)
         v = torch.empty(t, self.heads * m.v_head_dim, dtype=h.dtype, device=h.device)
         ops.colbatched_linear(lat.view(t, self.heads * LATENT), w.w_uv.weight, self.heads, LATENT, v, m.v_head_dim)
-        return model._reduce_linear(v, w.o) if self.reduce_output else ops.linear(v, w.o)
+        if not self.reduce_output:
+            return ops.linear(v, w.o)
+        return model._reduce_linear(v, w.o, defer=True) if defer else model._reduce_linear(v, w.o)
 
 
 def mla_reference(h: torch.Tensor, positions: torch.Tensor, cfg: TransformerConfig, full: dict,

@@ -636,8 +636,9 @@ class DecoderModel:
         s = self.cfg.attn_scale if self.cfg.attn_scale > 0 else 1.0 / math.sqrt(self.cfg.head_dim)
         return s * self.rope_attn_factor * self.rope_attn_factor if self.rope_attn_factor != 1.0 else s
 
-    def _reduce_linear(self, x, w: LinearWeight) -> torch.Tensor:
-        """Row-parallel linear: local partial product, then sum over the TP group. In order of
+    def _reduce_linear(self, x, w: LinearWeight, defer: bool = False) -> torch.Tensor:
+        """Row-parallel linear: local partial product, then sum over the TP group. ``defer``: a norm is the only reader
+        (single rank: K ranges may stay unsummed, see ops.SplitSum). In order of
         preference: the fused GEMM + all-reduce kernel (up to 128 tokens), GEMM written straight
         into the peer-memory all-reduce kernel's input buffer, GEMM + NCCL."""
         if self.tp > 1:
@@ -654,15 +655,17 @@ class DecoderModel:
             if self.custom_ar is not None and self.custom_ar.fits(m * n):
                 ops.linear(x, w, out=self.custom_ar.input(m, n))
                 return self.custom_ar.reduce(m, n)
-        y = ops.linear(x, w)
+        y = ops.linear(x, w, defer=defer and self.tp == 1)
         return self.all_reduce(y) if self.tp > 1 else y
 
     # ------------------------------------------------------------------------------ layer pieces
-    def _attention(self, lw: LayerWeights, li: int, h: torch.Tensor, hq8, batch: ForwardBatch, scale: float) -> torch.Tensor:
+    def _attention(self, lw: LayerWeights, li: int, h: torch.Tensor, hq8, batch: ForwardBatch, scale: float,
+                   defer: bool = False) -> torch.Tensor:
         """qkv projection, (q/k norm,) rotary + KV-cache write, paged attention, output projection."""
         if lw.attn_module is not None:
-            return lw.attn_module(h, batch, li, self)
-        return self._reduce_linear(self._attention_core(lw, li, h, hq8, batch, scale), lw.o)
+            return lw.attn_module(h, batch, li, self, defer) if defer and getattr(lw.attn_module, "defers", False) else \
+                lw.attn_module(h, batch, li, self)
+        return self._reduce_linear(self._attention_core(lw, li, h, hq8, batch, scale), lw.o, defer)
 
     def _attention_core(self, lw: LayerWeights, li: int, h: Optional[torch.Tensor], hq8, batch: ForwardBatch,
                         scale: float) -> torch.Tensor:
@@ -673,7 +676,7 @@ class DecoderModel:
         # decode-size batches: a fully K-split qkv GEMM leaves its ranges to the rotary kernel
         simple = (not cfg.qk_norm_full and not cfg.qk_norm_after_rope and not (cfg.mrope_section and batch.positions3 is not None)
                   and self.kv_cache is not None)
-        qkv = ops.linear(hq8 if hq8 is not None else h, lw.qkv, defer=simple and t <= 128 and x_is_cuda(hq8 if hq8 is not None else h))
+        qkv = ops.linear(hq8 if hq8 is not None else h, lw.qkv, defer=simple and t <= 128 and x_is_cuda(hq8 if hq8 is not None else h), defer_bias=True)
         q_norm_w, k_norm_w = lw.q_norm, lw.k_norm
         if cfg.qk_norm_full and q_norm_w is not None:
             # RMSNorm over all heads of q (and of k) at once, before the heads are split
@@ -1068,17 +1071,22 @@ class DecoderModel:
         if hidden_in is None and x.is_cuda and self._fused_tp_ok(x.shape[0]):
             return self._forward_fused_tp(batch, x)
 
+        # small batches: what goes straight into a norm is left as unsummed K ranges that the norm adds
+        rows, on_device = x.shape[0], x.is_cuda
+        plain = on_device and rows <= 128 and cfg.residual_multiplier == 1.0
+        last = len(self.layers) - 1
         for li, lw in enumerate(self.layers):
-            # ---- attention block
+            # ---- attention block (the bf16 normed rows are written only where something reads them)
+            qkv_fp8 = fp8 and lw.qkv is not None and lw.qkv.is_fp8
+            need_h = not qkv_fp8 or lw.attn_module is not None
             if res is None:
                 h, _, hq8 = ops.norm(x, lw.in_norm, eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one,
-                                     emit_fp8=fp8 and lw.qkv is not None and lw.qkv.is_fp8, emit_bf16=True)
+                                     emit_fp8=qkv_fp8, emit_bf16=need_h)
                 res = x
             else:
                 h, res, hq8 = ops.norm(x, lw.in_norm, residual=res, eps=cfg.rms_eps,
-                                       weight_plus_one=cfg.norm_plus_one,
-                                       emit_fp8=fp8 and lw.qkv is not None and lw.qkv.is_fp8, emit_bf16=True)
-            a = self._attention(lw, li, h, hq8, batch, scale)
+                                       weight_plus_one=cfg.norm_plus_one, emit_fp8=qkv_fp8, emit_bf16=need_h)
+            a = self._attention(lw, li, h, hq8, batch, scale, defer=plain)
             if lw.post_attn_norm is not None:
                 a, _, _ = ops.norm(a, lw.post_attn_norm, eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one)
             if cfg.residual_multiplier != 1.0:
@@ -1086,19 +1094,21 @@ class DecoderModel:
             # ---- feed-forward block
             dense_fp8 = fp8 and lw.gate_up is not None and lw.gate_up.is_fp8
             h2, res, h2q8 = ops.norm(a, lw.post_norm, residual=res, eps=cfg.rms_eps,
-                                     weight_plus_one=cfg.norm_plus_one, emit_fp8=dense_fp8, emit_bf16=True)
+                                     weight_plus_one=cfg.norm_plus_one, emit_fp8=dense_fp8,
+                                     emit_bf16=not dense_fp8 or lw.ffn_module is not None)
             if lw.ffn_module is not None:
                 f = lw.ffn_module(h2, self)
             else:
                 gated_fast = cfg.gated_ffn and cfg.activation in ("silu", "gelu_tanh")
                 gu = ops.linear(h2q8 if h2q8 is not None else h2, lw.gate_up,
-                                defer=gated_fast and x.is_cuda and x.shape[0] <= 128)
+                                defer=gated_fast and on_device and rows <= 128)
+                defer = plain and (li < last or self.last_stage)
                 if cfg.gated_ffn:
                     act, act8 = ops.glu(gu, cfg.activation, emit_fp8=fp8 and lw.down.is_fp8,
                                         emit_bf16=not (fp8 and lw.down.is_fp8))
-                    f = self._reduce_linear(act8 if act8 is not None else act, lw.down)
+                    f = self._reduce_linear(act8 if act8 is not None else act, lw.down, defer)
                 else:
-                    f = self._reduce_linear(gu, lw.down)
+                    f = self._reduce_linear(gu, lw.down, defer)
             if lw.post_ffn_norm is not None:
                 f, _, _ = ops.norm(f, lw.post_ffn_norm, eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one)
             if cfg.residual_multiplier != 1.0:

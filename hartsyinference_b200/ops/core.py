@@ -246,12 +246,13 @@ def quant_fp8_weight(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
 @dataclass
 class SplitSum:
     """Result of a small-token GEMM whose K ranges were left unsummed in the GEMM scratch
-    (``linear(..., defer=True)``): the consumer kernel (``glu``, ``rope_kv``) adds them while it
+    (``linear(..., defer=True)``): the consumer kernel (``glu``, ``rope_kv``, ``norm``) adds them while it
     reads, so no reduce kernel runs in between. Valid until the next GEMM on the device."""
     ws: torch.Tensor          # the device's GEMM scratch
     splits: int
     bn: int
     shape: tuple              # (tokens, features) of the product
+    bias: Optional[torch.Tensor] = None       # still to be added (``rope_kv`` only)
 
     def part_args(self):
         return self.ws.data_ptr() + 16384, self.splits, self.bn
@@ -275,14 +276,15 @@ def _scale_ptrs(x, w: LinearWeight):
 
 def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.Tensor] = None,
            residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-           splits: Optional[int] = None, defer: bool = False, act_from: int = 0):
+           splits: Optional[int] = None, defer: bool = False, act_from: int = 0, defer_bias: bool = False):
     """y = residual + gate * act(x @ W^T + bias), bf16 output [M, N]. ``act`` applies to the output features from
     ``act_from`` on.
 
     ``x`` is a bf16 tensor [M, K] or an :class:`Fp8Act`. With an fp8 weight a bf16 ``x`` is
     quantised on the fly (1x128 groups). ``gate`` is a per-output-feature vector [N].
     ``defer=True`` (device, plain product only): when the GEMM cuts all its tiles along K, return a
-    :class:`SplitSum` for a consumer that adds the ranges itself instead of running the reduce kernel.
+    :class:`SplitSum` for a consumer that adds the ranges itself instead of running the reduce kernel;
+    ``defer_bias``: also where the weight has a bias, which the consumer then adds (``rope_kv``).
     """
     if isinstance(w, GgufWeight):
         if act is not None or gate is not None or residual is not None or isinstance(x, Fp8Act):
@@ -323,14 +325,14 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
     st = N.state(xd.device)
     ws = st.gemm_workspace()
     xs_ptr, ws_ptr = _scale_ptrs(x, w)
-    if defer and m <= 128 and w.bias is None and act is None and gate is None and residual is None and splits is None:
+    if defer and m <= 128 and (w.bias is None or defer_bias) and act is None and gate is None and residual is None and splits is None:
         import ctypes as C
         info = (C.c_int * 4)()
         rc = L.b200_gemm_deferred(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k, xd.stride(0),
-                                  w.weight.stride(0), out.stride(0), _gemm_dtype(w), xs_ptr, ws_ptr, ws.data_ptr(),
+                                  w.weight.stride(0), out.stride(0), _gemm_dtype(w), xs_ptr, ws_ptr, N.ptr(w.bias), ws.data_ptr(),
                                   ws.numel(), info, st.status.data_ptr(), N.stream())
         N.check(rc, "b200_gemm_deferred")
-        return SplitSum(ws, int(info[1]), int(info[2]), (m, n)) if info[0] else out
+        return SplitSum(ws, int(info[1]), int(info[2]), (m, n), w.bias) if info[0] else out
     rc = L.b200_gemm(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k,
                      xd.stride(0), w.weight.stride(0), out.stride(0), _gemm_dtype(w),
                      xs_ptr, ws_ptr,
@@ -348,11 +350,12 @@ def norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, *, bias: Option
     """(residual add +) RMSNorm / LayerNorm (+ affine) (+ AdaLN ``y * (1 + scale) + shift``).
 
     x [rows, dim] bf16. ``shift``/``scale`` are [batch, >= dim] with ``rows_per_batch`` rows
-    sharing a batch entry. Returns ``(y, h, y_fp8)``: y bf16 (or None), h = x + residual (or
+    sharing a batch entry. ``x`` may be a :class:`SplitSum` without a bias. Returns ``(y, h, y_fp8)``: y bf16 (or None), h = x + residual (or
     None), y_fp8 an :class:`Fp8Act` (or None).
     """
     rows, dim = x.shape
-    if not x.is_cuda:
+    part = x if isinstance(x, SplitSum) else None
+    if part is None and not x.is_cuda:
         yf, h = R.norm(x, weight, bias, residual, shift, scale, rows_per_batch, eps, layernorm, weight_plus_one)
         y = yf.to(x.dtype)
         fq = None
@@ -360,23 +363,25 @@ def norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, *, bias: Option
             q, s = R.quant_fp8_act(y, pow2=fp8_mx())
             fq = Fp8Act(q, s)
         return (y if emit_bf16 else None), h, fq
-    assert x.dtype == torch.bfloat16 and x.is_contiguous()
-    y = torch.empty_like(x) if emit_bf16 else None
-    h = torch.empty_like(x) if residual is not None else None
+    assert part is not None or (x.dtype == torch.bfloat16 and x.is_contiguous())
+    assert part is None or part.bias is None
+    dev = part.ws.device if part is not None else x.device
+    y = torch.empty(rows, dim, dtype=torch.bfloat16, device=dev) if emit_bf16 else None
+    h = torch.empty(rows, dim, dtype=torch.bfloat16, device=dev) if residual is not None else None
     q = s = None
     mx = emit_fp8 and fp8_mx()
     if emit_fp8:
-        q = torch.empty(rows, dim, dtype=torch.uint8, device=x.device)
-        s = _alloc_sf(rows, dim, fp8_tile_rows, x.device) if mx else \
-            torch.empty(rows, dim // 128, dtype=torch.float32, device=x.device)
+        q = torch.empty(rows, dim, dtype=torch.uint8, device=dev)
+        s = _alloc_sf(rows, dim, fp8_tile_rows, dev) if mx else \
+            torch.empty(rows, dim // 128, dtype=torch.float32, device=dev)
     mod_stride = 0
     if shift is not None or scale is not None:
         ref = shift if shift is not None else scale
         mod_stride = ref.stride(0) if ref.dim() > 1 else 0
-    rc = N.lib().b200_norm(x.data_ptr(), N.ptr(residual), N.ptr(h), N.ptr(weight), N.ptr(bias),
+    rc = N.lib().b200_norm(None if part is not None else x.data_ptr(), N.ptr(residual), N.ptr(h), N.ptr(weight), N.ptr(bias),
                            N.ptr(shift), N.ptr(scale), N.ptr(y), N.ptr(q), N.ptr(s), rows, dim,
                            rows_per_batch, mod_stride, eps, int(layernorm), int(weight_plus_one),
-                           fp8_tile_rows if mx else 0, N.stream())
+                           fp8_tile_rows if mx else 0, *_part_args(x), N.stream())
     N.check(rc, "b200_norm")
     if not emit_fp8:
         return y, h, None
@@ -468,7 +473,7 @@ def rope_kv(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: in
     rc = N.lib().b200_rope_kv(None if part is not None else qkv.data_ptr(), q.data_ptr(), N.ptr(k_cache), N.ptr(v_cache),
                               N.ptr(k), N.ptr(v), positions.data_ptr(), N.ptr(slot_mapping), N.ptr(q_norm_w),
                               N.ptr(k_norm_w), N.ptr(inv_freq), t, hq, hkv, d, rot, style, page, theta, eps,
-                              *_part_args(qkv), N.stream())
+                              *_part_args(qkv), N.ptr(part.bias) if part is not None else None, N.stream())
     N.check(rc, "b200_rope_kv")
     return q, k, v
 
@@ -587,11 +592,6 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
     tq, hq, d = q.shape
     tk, hkv, _ = k.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
-    if not q.is_cuda:
-        return R.attention(q, k, v, causal, scale, softcap, window).to(q.dtype)
-    assert q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
-    dst = torch.empty_like(q) if out is None else out
-    dense_tc = d == 128 and hq == hkv and not causal and softcap == 0.0 and window <= 0 and tk >= 256 and _tc_attention()
     if out is not None:
         from .. import config
         if not (q.is_cuda and d == 128 and hq == hkv and not causal and softcap == 0.0 and window <= 0 and tk >= 256
@@ -599,6 +599,11 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
                 and out.data_ptr() % 16 == 0):
             out.copy_(attention(q, k, v, causal, scale, softcap, window, int8).reshape(tq, hq * d))
             return out
+    if not q.is_cuda:
+        return R.attention(q, k, v, causal, scale, softcap, window).to(q.dtype)
+    assert q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
+    dst = torch.empty_like(q) if out is None else out
+    dense_tc = d == 128 and hq == hkv and not causal and softcap == 0.0 and window <= 0 and tk >= 256 and _tc_attention()
     from .. import config
     if dense_tc and config.get("fa_attention"):
         # long bidirectional sequences (DiT blocks): two query tiles per CTA, S / P / O in TMEM
@@ -816,27 +821,27 @@ def dit_qkv(qkv: torch.Tensor, hq: int, hkv: int, d: int, *, q_norm_w: Optional[
     if not qkv.is_cuda:
         x = qkv.float().reshape(t, hq + 2 * hkv, d)
         q, k, v = x[:, :hq], x[:, hq:hq + hkv], x[:, hq + hkv:]
+        dims = (-2, -1) if row_norm else -1
         if q_norm_w is not None:
             q = q * torch.rsqrt((q * q).mean(dims, keepdim=True) + eps) * q_norm_w.float().reshape(-1, d)
         if k_norm_w is not None:
             k = k * torch.rsqrt((k * k).mean(dims, keepdim=True) + eps) * k_norm_w.float().reshape(-1, d)
         if cos is not None:
-        dims = (-2, -1) if row_norm else -1
             def rot(z):
                 a, b = z[..., 0::2], z[..., 1::2]
                 c, s = cos.float()[:, None, :], sin.float()[:, None, :]
                 return torch.stack([a * c - b * s, b * c + a * s], dim=-1).flatten(-2)
             q, k = rot(q), rot(k)
+        if out is not None:
+            for o, y in zip(out, (q, k, v)):
+                o.copy_(y)
+            return out
         return q.to(qkv.dtype).contiguous(), k.to(qkv.dtype).contiguous(), v.to(qkv.dtype).contiguous()
     assert qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1
     if out is None:
         out = tuple(torch.empty(t, h, d, dtype=torch.bfloat16, device=qkv.device) for h in (hq, hkv, hkv))
     q, k, v = out
     assert all(o.is_contiguous() and o.dtype == torch.bfloat16 for o in out)
-        if out is not None:
-            for o, y in zip(out, (q, k, v)):
-                o.copy_(y)
-            return out
     if cos is not None:
         assert cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
     if row_norm and (d % 8 or max(hq, hkv) * d > 8192 or qkv.stride(0) % 8 or any(
