@@ -34,6 +34,10 @@ class Flag:
 
 
 _REGISTRY: dict[str, Flag] = {}
+# the environment as the interpreter itself holds it: flags are read on every op, and the mapping in front of it
+# encodes the name and decodes the value each time
+_ENV = getattr(os.environ, "_data", None)
+_ENV_KEYS: dict[str, Any] = {}
 _OVERRIDES: dict[str, Any] = {}
 
 
@@ -42,6 +46,8 @@ def declare(name: str, type_: type, default: Any, doc: str) -> Flag:
         raise ValueError(f"flag {name} declared twice")
     f = Flag(name, type_, default, doc)
     _REGISTRY[name] = f
+    if _ENV is not None:
+        _ENV_KEYS[name] = os.environ.encodekey(f.env)
     return f
 
 
@@ -49,6 +55,8 @@ def get(name: str) -> Any:
     f = _REGISTRY[name]
     if name in _OVERRIDES:
         return _OVERRIDES[name]
+    if _ENV is not None and _ENV_KEYS[name] not in _ENV:
+        return f.default
     raw = os.environ.get(f.env)
     if raw is None:
         return f.default

@@ -164,7 +164,8 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, without building the Python object around it (4 us of a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # number of kernels of this library launched so far by this process (ops report their own count)
