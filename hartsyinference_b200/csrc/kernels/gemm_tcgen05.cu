@@ -1607,6 +1607,9 @@ struct ConvSpec {
   int shift[28];
 };
 
+int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long long ldx, long long ldw, long long ldc,
+              const void* bias, const void* gate, const void* residual, int act, cudaStream_t stream);
+
 int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long long ldx,
                      long long ldw, long long ldc, int dtype, const float* x_scale,
                      const float* w_scale, const void* bias, const void* gate, const void* residual,
@@ -1618,9 +1621,6 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   // grouped: x is [groups * m][k], w is [groups * n][k], out is [groups * m][n]; m = tokens per group
   const bool i8 = dtype == 3;           // int8 operands, one fp32 scale per x row and per w row
   const bool fp8 = dtype != 0;          // one-byte operands. 1: fp32 block scales, 2: UE8M0 scale factors (blocked layout)
-int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long long ldx, long long ldw, long long ldc,
-              const void* bias, const void* gate, const void* residual, int act, cudaStream_t stream);
-
   const bool mx = dtype == 2;
   const int esz = fp8 ? 1 : 2;
   const int kelems = fp8 ? 128 : 64;
@@ -1752,7 +1752,21 @@ int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long
     const int q = tiles / sms, r = tiles % sms;
     // worthwhile when the partial wave is a visible share of the run: always for the
     // bandwidth-bound orientation, for the other only when there are few waves
-    if (r != 0 && (swap || q < 4)) {
+    if (swap && q == 0 && 2 * r > sms && groups == 0 && ar == nullptr && ag == nullptr) {
+      // More than half of the SMs have a tile, too many for two ranges each in one wave: up to four ranges in as many waves
+      // as they take, where the slowest SM is then done earlier (a tile's weights count as 1, and the writing and the
+      // second reading of the ranges' sums is added). fp8 64 x 10240 x 8192 36.4 -> 24.9 us, bf16 16 x 9728 x 896 13.8 ->
+      // 10.2 us. The same count for fewer tiles chose more ranges than fit one wave and lost (bf16 6 x 4096 x 4096 9.7 ->
+      // 12.3 us): there the ranges that fill one wave stay. Sixteen loads in flight in the last arriver's sums, tried for
+      // the tail of larger products, lost too (fp8 64 x 57344 x 8192 103 -> 115 us).
+      const double part = static_cast<double>(bn) * 128 * 4 / (128.0 * k * esz);
+      double best = 1.0;
+      for (int s = 2; s <= 4 && s <= total_kblocks / 2; ++s) {
+        const double cost = ((r * s + sms - 1) / sms) * (1.0 / s + part) + static_cast<double>(r) * s / sms * part;
+        if (cost < 0.9 * best) { best = cost; s_eff = s; }
+      }
+      if (s_eff > 1) first_split = 0;
+    } else if (r != 0 && (swap || q < 4)) {
       int s = sms / r;
       if (s > total_kblocks / 2) s = total_kblocks / 2;   // at least two k-blocks per range
       // after full waves a modest split already shrinks the tail to 1/s of a tile; without full

@@ -48,3 +48,18 @@ def test_attention_into_rows_apart():
         ref = R.attention(q, k, v)
         assert torch.allclose(buf[:, 8:8 + h * 128].float().reshape(t, h, 128), ref.float(), rtol=2e-2, atol=1e-2)
         assert not buf[:, :8].any() and not buf[:, 8 + h * 128:].any()
+
+
+# 75 to 147 tiles of 128 features for few tokens: ranges of K in more than one wave, down to depths that leave no ranges
+@pytest.mark.parametrize("m,n,k", [(5, 9600, 128), (64, 9596, 512), (33, 10240, 1152), (16, 9728, 896), (7, 18816, 4096), (128, 12288, 2048)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_few_tokens_more_than_half_a_wave(m, n, k, fp8):
+    torch.manual_seed(m)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16),
+                                    torch.randn(n, device="cuda").to(torch.bfloat16), fp8=fp8)
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16)
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    y = ops.linear(xq, w, act="silu", residual=res).float()
+    ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, w.bias, "silu", None, res, torch.float32)
+    assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums
