@@ -1099,16 +1099,14 @@ class DecoderModel:
             if lw.ffn_module is not None:
                 f = lw.ffn_module(h2, self)
             else:
-                gated_fast = cfg.gated_ffn and cfg.activation in ("silu", "gelu_tanh")
-                gu = ops.linear(h2q8 if h2q8 is not None else h2, lw.gate_up,
-                                defer=gated_fast and on_device and rows <= 128)
                 defer = plain and (li < last or self.last_stage)
+                hx = h2q8 if h2q8 is not None else h2
                 if cfg.gated_ffn:
-                    act, act8 = ops.glu(gu, cfg.activation, emit_fp8=fp8 and lw.down.is_fp8,
-                                        emit_bf16=not (fp8 and lw.down.is_fp8))
+                    down8 = fp8 and lw.down.is_fp8
+                    act, act8 = ops.linear_glu(hx, lw.gate_up, cfg.activation, emit_fp8=down8, emit_bf16=not down8)
                     f = self._reduce_linear(act8 if act8 is not None else act, lw.down, defer)
                 else:
-                    f = self._reduce_linear(gu, lw.down, defer)
+                    f = self._reduce_linear(ops.linear(hx, lw.gate_up), lw.down, defer)
             if lw.post_ffn_norm is not None:
                 f, _, _ = ops.norm(f, lw.post_ffn_norm, eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one)
             if cfg.residual_multiplier != 1.0:

@@ -25,6 +25,7 @@ from .core import (  # noqa: F401
     fp8_mx,
     gated_residual,
     glu,
+    linear_glu,
     gguf_linear,
     int8_linear,
     grouped_linear,

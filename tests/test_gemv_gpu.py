@@ -33,3 +33,15 @@ def test_values_that_are_not_finite_stay_where_they_are():
     y = ops.linear(x, ops.LinearWeight(w))
     assert torch.isnan(y[0, 3]) and torch.isfinite(y[0, [0, 1, 2, 4, 5, 6, 7, 8]]).all()
     assert torch.isinf(y[1, [0, 1, 2, 4, 5, 6, 7, 8]]).all()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("f,k", [(8, 8), (4864, 896), (4104, 264), (1000, 4096)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gated_product(m, f, k, act):
+    torch.manual_seed(f + m)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight((torch.randn(2 * f, k, device="cuda") * k ** -0.5).to(torch.bfloat16))
+    y, q = ops.linear_glu(x, w, act)
+    ref = R.glu(x.float() @ w.weight.float().t(), act)
+    assert q is None and torch.allclose(y.float(), ref, rtol=2 ** -6, atol=2 ** -8)      # five tokens round both halves first
