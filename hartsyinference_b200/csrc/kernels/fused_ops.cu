@@ -15,8 +15,6 @@
 
 namespace b200 {
 
-constexpr float kFp8Max = 448.f;
-
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
@@ -60,25 +58,6 @@ __device__ __forceinline__ void load_param8(const __nv_bfloat16* w, long long c,
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __bfloat162float(w[c + i]);
   }
-}
-
-// UE8M0 (power-of-two) scale for hardware block scaling: the smallest 2^e >= amax / 448.
-// Returns 2^-e and the biased exponent byte e + 127.
-__device__ __forceinline__ float mx_scale_inv(float amax, uint32_t& e_biased) {
-  const uint32_t bits = __float_as_uint(amax / kFp8Max);
-  int e = static_cast<int>(bits >> 23) - 127 + ((bits & 0x7fffffu) != 0 ? 1 : 0);
-  e = max(-126, min(126, e));
-  e_biased = static_cast<uint32_t>(e + 127);
-  return __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-}
-// Blocked scale-factor layout read by the block-scaled GEMM: rows are grouped in tiles of
-// `tile_rows` (<= 128, each padded to a 128-row block), K in groups of four 128-wide blocks; a
-// block is 128 x uint32 with row r at word (r % 32) * 4 + r / 32 and K block kb at byte kb % 4.
-__device__ __forceinline__ void store_sf(uint8_t* sf, int row, int kb, int tile_rows, int kgroups,
-                                         uint32_t e_biased) {
-  const int tile = row / tile_rows, r = row - tile * tile_rows;
-  const long long blk = static_cast<long long>(tile) * kgroups + (kb >> 2);
-  sf[(blk * 128 + (r & 31) * 4 + (r >> 5)) * 4 + (kb & 3)] = static_cast<uint8_t>(e_biased);
 }
 
 // Eight e4m3 values of vector `vi` of a row of `dim` values, whose 1x128 group has the largest magnitude

@@ -202,6 +202,12 @@ struct GemmParams {
   AllReduceParams ar;   // ar.world == 0: plain GEMM
   GatherParams ag;      // ag.world == 0: the A operand is complete when the kernel starts
   int ta_rotate;        // plain GEMM: A tiles are walked starting with this one
+  // Gated product (kGlu instances): w holds f gate rows, then f up rows; a tile's columns are 128 of either, and
+  // act(gate) * up leaves as bf16 (out) or as e4m3 with 1x128 UE8M0 scales in the blocked layout (glu_q, glu_sf)
+  int glu_f, glu_act;   // act: 0 = SiLU, 1 = GELU-tanh
+  uint8_t* glu_q;
+  uint8_t* glu_sf;
+  int glu_sf_rows;      // rows per block of the scale layout
   int row_stores;       // large-token orientation: C (and bias, gate, residual) can be reached in 16-byte pieces
   int band;             // > 0, plain GEMM: tiles are walked in bands of this many A tiles (see decode_item)
 };
@@ -957,7 +963,65 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, 
   reduce_partials<8>(p, it, bn, e4);
 }
 
-template <int kMode, int BN, int kAtoms>
+// Epilogue of a gated tile: this warp's 32 rows and, of the tile's 128 output features, the half `hsel`. r holds
+// the gate values of those 64 features, then the up values. The scale of a row's 128 features needs both halves, which
+// sit in two warps: they exchange maxima through `amax` ([2][128], one of two buffers) behind a barrier of their
+// own, which a warp whose accumulator did not come (got = false) still meets.
+__device__ __forceinline__ void store_glu_tile(const GemmParams& p, uint32_t (&r)[4][32], int row0, int tb, int hsel, int quarter,
+                                               float* amax, uint8_t* strip, bool got) {
+  const int lane = threadIdx.x & 31, pr = lane >> 2, pc = lane & 3;
+  uint32_t y[32];                                      // 64 features as bf16 pairs
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float g0 = __uint_as_float(r[c][2 * j]), g1 = __uint_as_float(r[c][2 * j + 1]);
+      y[c * 16 + j] = pack_bf16x2((p.glu_act == 0 ? silu(g0) : gelu_tanh(g0)) * __uint_as_float(r[2 + c][2 * j]),
+                                  (p.glu_act == 0 ? silu(g1) : gelu_tanh(g1)) * __uint_as_float(r[2 + c][2 * j + 1]));
+    }
+  auto leave = [&](const uint32_t* words, uint8_t* dst, long long pitch) {      // 64 bytes per row through the strip
+    uint8_t* own = strip + lane * kStripPitch;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4*>(own + q * 16) = make_uint4(words[4 * q], words[4 * q + 1], words[4 * q + 2], words[4 * q + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 v = *reinterpret_cast<const uint4*>(strip + (i * 8 + pr) * kStripPitch + pc * 16);
+      if (got && row0 + i * 8 + pr < p.rows_a) *reinterpret_cast<uint4*>(dst + (i * 8 + pr) * pitch + pc * 16) = v;
+    }
+    __syncwarp();
+  };
+  if (p.glu_q == nullptr) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      leave(y + c * 16, reinterpret_cast<uint8_t*>(p.out + static_cast<long long>(row0) * p.ldc + tb * 128 + hsel * 64 + c * 32), p.ldc * 2);
+    return;
+  }
+  float mx = 0.f;
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(y[j] << 16)), fabsf(__uint_as_float(y[j] & 0xffff0000u))));
+  const int row = quarter * 32 + lane;
+  amax[hsel * 128 + row] = mx;
+  asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+  mx = fmaxf(mx, amax[(hsel ^ 1) * 128 + row]);
+  uint32_t eb;
+  const float inv = mx_scale_inv(mx, eb);
+  uint32_t q[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t a = y[2 * j], b = y[2 * j + 1];
+    q[j] = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(a << 16) * inv, __uint_as_float(a & 0xffff0000u) * inv),
+                                                          __NV_SATFINITE, __NV_E4M3)) |
+           static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(b << 16) * inv, __uint_as_float(b & 0xffff0000u) * inv),
+                                                          __NV_SATFINITE, __NV_E4M3)) << 16;
+  }
+  leave(q, p.glu_q + static_cast<long long>(row0) * p.glu_f + tb * 128 + hsel * 64, p.glu_f);
+  if (hsel == 0 && got && row0 + lane < p.rows_a) store_sf(p.glu_sf, row0 + lane, tb, p.glu_sf_rows, (p.glu_f + 511) >> 9, eb);
+}
+
+template <int kMode, int BN, int kAtoms, bool kGlu = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a,
                     const __grid_constant__ CUtensorMap tm_b) {
@@ -1074,13 +1138,21 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
             const long long last_b = (p.rows_b - 1) / p.sf_tile_b;      // rows past the end are not stored: any block will do
 #pragma unroll
             for (int j = 0; j < kSfBlocksB; ++j) {
-              const long long gb = (min(tile_b + j, last_b) * p.sf_kgroups + (kb >> 2)) * 128;
+              const long long blk = kGlu ? it.tb + (j ? p.glu_f >> 7 : 0) : min(tile_b + j, last_b);
+              const long long gb = (blk * p.sf_kgroups + (kb >> 2)) * 128;
               bulk_load(sa + kSfOffset + 512 * (1 + j), p.sf_b + gb, 512, &bars->full[st]);
             }
           }
-          for (int a = 0; a < na; ++a)
+          for (int a = 0; a < na; ++a) {
+            if (kGlu) {
+              for (int j = 0; j < 2; ++j)
+                tma_load_2d(sb + a * kAtomBytesB + j * (kAtomBytesB / 2), &tm_b, &bars->full[st], (kb + a) * kElemsPerAtom,
+                            it.tb * (BN / 2) + j * p.glu_f);
+              continue;
+            }
             tma_load_2d(sb + a * kAtomBytesB, &tm_b, &bars->full[st], (kb + a) * kElemsPerAtom + it.bk,
                         it.tb * BN);
+          }
         }
       };
       // Programmatic dependent launch: this grid may start while the kernel before it is still
@@ -1241,9 +1313,31 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     int abuf = 0;
     uint32_t aph = 0;
     bool ok = true;
+    uint32_t glu_round = 0;
     for (long long w = blockIdx.x; w < work_items; w += gridDim.x) {
       const WorkItem it = decode_item(p, w, tiles_a, total_kblocks);
       if (it.skip) continue;
+      if constexpr (kGlu) {
+        if (ok && !__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[abuf], aph, abort_flag))) {
+          if (lane == 0) report_status(p.status, kWaitTimeout, kKernelGemm, 5, blockIdx.x);
+          ok = false;
+        }
+        uint32_t r[4][32];
+        if (ok) {
+          tc_fence_after_sync();
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            tmem_ld_32x32(lane_base + abuf * kBufStride + (u >> 1) * (BN / 2) + hsel * 64 + (u & 1) * 32, r[u]);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->tmem_empty[abuf]);
+          if (++abuf == kAccBufs) { abuf = 0; aph ^= 1; }
+        }
+        store_glu_tile(p, r, it.ta * kTileA + q * 32, it.tb, hsel, q, &bars->cs_bcast[0][0][0] + (glu_round & 1) * 256, strip, ok);
+        ++glu_round;
+        continue;
+      }
       if (ok) {
         if constexpr (!kFp8) {
           if (!__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[abuf], aph, abort_flag))) {
@@ -1541,14 +1635,14 @@ namespace b200 {
 static bool g_cluster_reduce = false;   // measured slower than the other two ways; opt-in
 static bool g_external_reduce = true;    // fully split GEMMs: second kernel (true) or last-arriving CTA (false)
 
-template <int kMode, int BN, int kAtoms>
+template <int kMode, int BN, int kAtoms, bool kGlu = false>
 int launch_gemm(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& tb, int grid,
                 cudaStream_t stream) {
   const int stage_bytes = kAtoms * (kStageBytesA + BN * 128) + (kMode == 2 ? 2048 : 0);
   const int smem = p.stages * stage_bytes + static_cast<int>(sizeof(GemmBarriers)) + 1024 + (p.row_stores ? 8 * kStripBytes : 0);
   static PerDeviceOnce configured;
   if (configured.first_time()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<kMode, BN, kAtoms>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return -static_cast<int>(e) - 200;
   }
@@ -1569,7 +1663,7 @@ int launch_gemm(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& t
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
   }
-  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kMode, BN, kAtoms>, p, ta, tb) != cudaSuccess) return -300;
+  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu>, p, ta, tb) != cudaSuccess) return -300;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 300;
 }
@@ -1940,6 +2034,54 @@ B200_API int b200_gemm(const void* x, const void* w, void* out, int m, int n, in
                        long long workspace_bytes, void* status, cudaStream_t stream) {
   return gemm_impl(x, w, out, m, n, k, ldx, ldw, ldc, dtype, x_scale, w_scale, bias, gate, residual,
                    act, splits, workspace, workspace_bytes, status, stream, nullptr);
+}
+
+// The first half of a gated feed-forward for more than 128 tokens in one launch: act(x w_gate^T) * (x w_up^T) for w [2f][k],
+// gate rows first. dtype 0: bf16 operands, out [m][ldc] bf16; dtype 2: e4m3 operands with UE8M0 scales, result as
+// e4m3 [m][f] (out_q) with 1x128 scales in the blocked layout of sf_rows rows per block (out_sf). A tile reads 128 gate
+// and 128 up rows, so neither product goes to memory: 8192 x 28672 of k 8192 writes 0.24 GB instead of 0.94, which the
+// activation kernel would read again (both 3740 us, this one 3287, fp8; bf16 8192 x 14336 of k 4096 1609 -> 1402). Bound
+// by the tensor core. Returns -12 for sizes that it does not take (f a multiple of 128, at least one tile per SM).
+B200_API int b200_gemm_glu(const void* x, const void* w, void* out, void* out_q, void* out_sf, int m, int f, int k, long long ldx,
+                           long long ldw, long long ldc, int dtype, const float* x_scale, const float* w_scale, int act, int sf_rows,
+                           void* status, cudaStream_t stream) {
+  const bool mx = dtype == 2;
+  const int esz = mx ? 1 : 2, kelems = mx ? 128 : 64;
+  const long long tiles = static_cast<long long>((m + 127) / 128) * (f / 128);
+  if (m <= 128 || f % 128 != 0 || k < 1 || tiles < num_sms() || tiles >= 1ll << 31 || (dtype != 0 && !mx)) return -12;
+  if ((ldx * esz) % 16 != 0 || (ldw * esz) % 16 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15)) return -12;
+  if (mx ? k % 16 != 0 || !x_scale || !w_scale || !out_q || !out_sf || sf_rows < 1 || sf_rows > 128 || (reinterpret_cast<uintptr_t>(out_q) & 15)
+         : !out || ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15))
+    return -12;
+  GemmParams p{};
+  p.k = k;
+  p.rows_a = m;
+  p.rows_b = 2 * f;
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.ldc = ldc;
+  p.status = static_cast<DeviceStatus*>(status);
+  p.glu_f = f;
+  p.glu_act = act;
+  p.glu_q = mx ? static_cast<uint8_t*>(out_q) : nullptr;
+  p.glu_sf = static_cast<uint8_t*>(out_sf);
+  p.glu_sf_rows = sf_rows;
+  p.row_stores = 1;                                    // the strips are there
+  p.sf_a = reinterpret_cast<const uint32_t*>(x_scale);
+  p.sf_b = reinterpret_cast<const uint32_t*>(w_scale);
+  p.sf_kgroups = (k + 511) / 512;
+  p.sf_tile_b = 128;
+  p.num_tiles = p.first_split_tile = static_cast<int>(tiles);
+  p.splits = 1;
+  p.kblocks_per_split = (k + kelems - 1) / kelems;
+  if ((m + 127) / 128 > 16) p.band = 16;
+  const int stage_bytes = kStageBytesA + 256 * 128 + (mx ? 2048 : 0);
+  p.stages = (200 * 1024) / stage_bytes;
+  CUtensorMap ta, tb;
+  int rc = make_kmajor_map(&ta, x, esz, m, k, ldx, kTileA);
+  if (rc == 0) rc = make_kmajor_map(&tb, w, esz, 2ll * f, k, ldw, 128);
+  if (rc) return rc;
+  const int grid = static_cast<int>(tiles < num_sms() ? tiles : num_sms());
+  return mx ? launch_gemm<2, 256, 1, true>(p, ta, tb, grid, stream) : launch_gemm<0, 256, 1, true>(p, ta, tb, grid, stream);
 }
 
 // b200_gemm for a consumer that can add split-K ranges itself (b200_glu, b200_rope_kv): when the

@@ -63,3 +63,32 @@ def test_few_tokens_more_than_half_a_wave(m, n, k, fp8):
     y = ops.linear(xq, w, act="silu", residual=res).float()
     ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, w.bias, "silu", None, res, torch.float32)
     assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums
+
+
+@pytest.mark.parametrize("m,f,k", [(129, 23808, 64), (300, 15872, 136), (2177, 2688, 1024), (4737, 1280, 328)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gated_tiles(m, f, k, act):
+    torch.manual_seed(m)
+    x = (torch.randn(m, k, device="cuda")).to(torch.bfloat16)
+    w = ops.LinearWeight((torch.randn(2 * f, k, device="cuda") * 2 * k ** -0.5).to(torch.bfloat16))
+    y, q = ops.linear_glu(x, w, act)
+    ref = R.glu(x.float() @ w.weight.float().t(), act)
+    assert q is None and torch.allclose(y.float(), ref, rtol=2 ** -7, atol=2 ** -8)      # fp32 sums, one rounding to bf16
+
+
+@pytest.mark.parametrize("m,f,k", [(129, 23808, 128), (300, 15872, 640), (2177, 2688, 1024), (4737, 1280, 384)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gated_tiles_fp8(m, f, k, act):
+    if not ops.fp8_mx():
+        pytest.skip("block scales in fp32")
+    torch.manual_seed(m)
+    w = ops.LinearWeight.from_dense((torch.randn(2 * f, k, device="cuda") * 2 * k ** -0.5).to(torch.bfloat16), fp8=True)
+    x = ops.quant_fp8_act(torch.randn(m, k, device="cuda").to(torch.bfloat16))
+    y, q = ops.linear_glu(x, w, act, emit_fp8=True, emit_bf16=False)
+    ref = R.glu(R.linear(x.data.cpu(), w.weight.cpu(), w.scale.cpu(), x.scales_fp32().cpu(), out_dtype=torch.float32), act)
+    assert y is None and q.data.shape == (m, f)
+    got, s = R.dequant_fp8_act(q.data.cpu(), q.scales_fp32().cpu()), q.scales_fp32().cpu().repeat_interleave(128, 1)
+    # half a step of e4m3 (2^-4 of a value, 2^-10 scales at least) and the rounding to bf16 ahead of it
+    assert ((got - ref).abs() <= ref.abs() * (2 ** -4 + 2 ** -7) + s * 2 ** -10 + 2 ** -9).all()
+    mx = ref.abs().reshape(m, -1, 128).amax(-1)
+    assert (q.scales_fp32().cpu() * 448 * (1 + 2 ** -6) + 2 ** -9 >= mx).all() and (q.scales_fp32().cpu() * 448 <= 2 * (1 + 2 ** -6) * mx + 2 ** -8).all()
