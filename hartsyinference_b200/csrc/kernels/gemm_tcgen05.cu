@@ -24,7 +24,7 @@
 // Work items. Output tiles are dealt round-robin to the CTAs. When the tile count is not a
 // multiple of the grid, the tiles of the last, partial wave are split along K so that this wave
 // also covers every SM (a bandwidth-bound GEMM otherwise loses up to half its throughput to wave
-// quantisation). The CTAs of a split tile write fp32 partials to a scratch buffer and bump a
+// quantisation); after full waves of 128 x 256 tiles only where rows are long. The CTAs of a split tile write fp32 partials to a scratch buffer and bump a
 // counter; whoever arrives last sums the partials in split order (deterministic) and runs the
 // epilogue. A GEMM with fewer tiles than SMs is split completely; its partials are summed by a
 // second, machine-wide kernel (splitk_reduce_kernel) or, optionally, through the distributed
@@ -1845,7 +1845,11 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   } else if (splits <= 0 && !(groups > 0 && gs->block_group)) {   // automatic (never with a device block list)
     const int q = tiles / sms, r = tiles % sms;
     // worthwhile when the partial wave is a visible share of the run: always for the
-    // bandwidth-bound orientation, for the other only when there are few waves
+    // bandwidth-bound orientation, for the other only when there are few waves. After a full wave of 128 x 256 tiles the one
+    // CTA that adds a tile's ranges takes 50 to 75 us, so a whole wave more is faster up to rows of 24 KB in bf16 and 16 KB in
+    // 8 bits (152 tiles, cut -> whole: bf16 k 1024 97 -> 21 us, k 8192 157 -> 114, k 12288 184 -> 166; fp8 k 1024 65 -> 26,
+    // k 8192 103 -> 82, k 16384 150 -> 148, k 24576 194 -> 213).
+    const bool long_rows = static_cast<long long>(k) * esz > (esz == 1 ? 16384 : 24576);
     if (swap && q == 0 && 2 * r > sms && groups == 0 && ar == nullptr && ag == nullptr) {
       // More than half of the SMs have a tile, too many for two ranges each in one wave: up to four ranges in as many waves
       // as they take, where the slowest SM is then done earlier (a tile's weights count as 1, and the writing and the
@@ -1860,7 +1864,7 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
         if (cost < 0.9 * best) { best = cost; s_eff = s; }
       }
       if (s_eff > 1) first_split = 0;
-    } else if (r != 0 && (swap || q < 4)) {
+    } else if (r != 0 && (swap || (q < 4 && (q == 0 || bn < 256 || long_rows)))) {
       int s = sms / r;
       if (s > total_kblocks / 2) s = total_kblocks / 2;   // at least two k-blocks per range
       // after full waves a modest split already shrinks the tail to 1/s of a tile; without full

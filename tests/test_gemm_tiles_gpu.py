@@ -50,6 +50,19 @@ def test_attention_into_rows_apart():
         assert not buf[:, :8].any() and not buf[:, 8 + h * 128:].any()
 
 
+# a wave of 128 x 256 tiles and a few more: rows up to the line between a wave of whole tiles and ranges of K, and beyond it
+@pytest.mark.parametrize("k,fp8", [(512, False), (12288, False), (12296, False), (512, True), (16384, True), (16512, True)])
+def test_tail_after_a_full_wave(k, fp8):
+    torch.manual_seed(k)
+    m, n = 250, 19456
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16), fp8=fp8)
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    y = ops.linear(xq, w).float()
+    ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, out_dtype=torch.float32)
+    assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums
+
+
 # 75 to 147 tiles of 128 features for few tokens: ranges of K in more than one wave, down to depths that leave no ranges
 @pytest.mark.parametrize("m,n,k", [(5, 9600, 128), (64, 9596, 512), (33, 10240, 1152), (16, 9728, 896), (7, 18816, 4096), (128, 12288, 2048)])
 @pytest.mark.parametrize("fp8", [False, True])
