@@ -637,6 +637,25 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const __nv_bfloat1
   }
 }
 
+// The block's largest value and the lowest index that has it, in every thread; 0x7fffffff: no thread had one.
+__device__ __forceinline__ void block_argmax(float& best, int& bi, float* sval, int* sidx) {
+  auto warp_best = [&] {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+    }
+  };
+  warp_best();
+  if ((threadIdx.x & 31) == 0) { sval[threadIdx.x >> 5] = best; sidx[threadIdx.x >> 5] = bi; }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  best = lane < nw ? sval[lane] : -INFINITY;
+  bi = lane < nw ? sidx[lane] : 0x7fffffff;
+  warp_best();
+}
+
 // argmax over the last dim of bf16 / fp32 logits [rows][vocab]; ties -> lowest index. One block per row; with rows on
 // 16-byte boundaries (vec) a thread reads 16 bytes at a time, four in flight: one row of 151936 bf16 42 -> 8 us.
 template <typename T>
@@ -668,28 +687,19 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const T* __restrict__ logi
   }
   for (int i = nvec * kPer + threadIdx.x; i < vocab; i += blockDim.x) {
     const float v = static_cast<float>(row[i]);
-    if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+    if (v > best) { best = v; bi = i; }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+  block_argmax(best, bi, sval, sidx);
+  if (bi == 0x7fffffff) {
+    // Nothing above -infinity: the first value that equals it (a mask that allows no token), 0 for a row of NaN. Apart
+    // from the loops above, where the second comparison costs 1 to 2 us of 10.
+    for (int i = threadIdx.x; i < vocab && bi == 0x7fffffff; i += blockDim.x)
+      if (static_cast<float>(row[i]) == -INFINITY) bi = i;
+    __syncthreads();
+    block_argmax(best, bi, sval, sidx);
+    if (bi == 0x7fffffff) bi = 0;
   }
-  if ((threadIdx.x & 31) == 0) { sval[threadIdx.x >> 5] = best; sidx[threadIdx.x >> 5] = bi; }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int nw = blockDim.x >> 5;
-    best = threadIdx.x < nw ? sval[threadIdx.x] : -INFINITY;
-    bi = threadIdx.x < nw ? sidx[threadIdx.x] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = bi;
-  }
+  if (threadIdx.x == 0) out[blockIdx.x] = bi;
 }
 
 // logits[b][tok] /= penalty when > 0 else *= penalty, for every token in the row's history.

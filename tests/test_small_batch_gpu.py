@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from hartsyinference_b200 import ops
-from hartsyinference_b200.ops import reference as R
+from hartsyinference_b200.engine.sampling import SamplingParams, sample_row
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,14 @@ def test_argmax_takes_the_first_of_equals(vocab, dtype):
     want = torch.tensor([int((r == r.max()).nonzero()[0]) for r in x.cpu()])
     for y in (x, x.contiguous(), x[:, :]):
         assert torch.equal(ops.argmax(y).cpu().long(), want)
+
+
+@pytest.mark.parametrize("vocab,pitch", [(1, 8), (8, 8), (1025, 1032), (1025, 1033), (32777, 32784), (151936, 151936)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_argmax_of_rows_without_a_finite_value(vocab, pitch, dtype):
+    x = torch.full((3, pitch), float("-inf"), device="cuda", dtype=dtype)[:, :vocab]
+    x[1, vocab - 1] = torch.finfo(dtype).min
+    assert ops.argmax(x).tolist() == [0, vocab - 1, 0]
+    p = SamplingParams(greedy=True, logits_mask=lambda history: torch.zeros(vocab, dtype=torch.bool))
+    lg = torch.randn(vocab)
+    assert sample_row(lg.cuda(), p, [], None) == sample_row(lg, p, [], None) == 0      # a grammar that allows nothing
