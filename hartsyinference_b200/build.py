@@ -44,8 +44,8 @@ NVCC_FLAGS = [
     "--expt-relaxed-constexpr",
     "-diag-suppress", "550,177",
 ]
-# sources that make a smaller library for one kind of model; no source refers to a symbol of another one
-# except the launch switch that gemm_tcgen05.cu defines
+# sources that make a smaller library for one kind of model; what a source uses of another one is in gemm_tcgen05.cu
+# (the launch switch, the number of processors, tensor maps) or used by it (gemv_bf16)
 KERNEL_GROUPS = {
     "decoder": ("gemm_tcgen05", "gemv_bf16", "attention", "attention_pf", "delta", "delta_general", "fused_ops", "latent", "linear_f32", "mla", "moe", "residual_norm", "rotary", "sampling", "ssm"),
 }

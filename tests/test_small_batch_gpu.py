@@ -52,6 +52,8 @@ def test_argmax_takes_the_first_of_equals(vocab, dtype):
     want = torch.tensor([int((r == r.max()).nonzero()[0]) for r in x.cpu()])
     for y in (x, x.contiguous(), x[:, :]):
         assert torch.equal(ops.argmax(y).cpu().long(), want)
+    many = x.repeat(40, 1) if vocab < 40000 else x                     # more rows than processors: smaller blocks
+    assert torch.equal(ops.argmax(many).cpu().long(), want.repeat(many.shape[0] // 9))
 
 
 @pytest.mark.parametrize("vocab,pitch", [(1, 8), (8, 8), (1025, 1032), (1025, 1033), (32777, 32784), (151936, 151936)])
