@@ -29,8 +29,8 @@
 //                more than 2^8, otherwise the stale maximum keeps being used, which is exact
 //                because the final division by the row sum uses the same maximum.
 //
-// One sample's V is read as it lies ([key][head dim], an MN-major operand). In a batch, and in the segmented forms
-// below, V is consumed transposed ([head dim][keys]) and padded; that transpose and the int8 quantisation are small
+// One sample's V is read as it lies ([key][head dim], an MN-major operand) where it starts on a 16-byte boundary.
+// Otherwise, in a batch and in the segmented forms below, V is consumed transposed ([head dim][keys]) and padded; that transpose and the int8 quantisation are small
 // kernels of their own in front.
 #include "comm.cuh"
 
@@ -848,17 +848,18 @@ static inline int fa_pad(int s, int to) { return (s + to - 1) / to * to; }
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,
                      int int8, cudaStream_t stream, const FaPeerMaps* peers = nullptr, bool direct = false);
 
-// Scratch layout of one call: V^T [batch * heads * 128][sk_pad64] bf16, then (int8 mode) Q8
+// Scratch layout of one call: (unless V is read in place) V^T [batch * heads * 128][sk_pad64] bf16, then (int8 mode) Q8
 // [batch * sq][heads * 128], K8 [batch * sk][heads * 128], q scales [batch * heads][sq_pad128],
 // K tile scales [batch * heads][key tiles] fp32, K sums [batch * heads][128] fp32.
 struct FaScratch {
   long long vt, q8, k8, qs, ks, ksum, total;
 };
-static FaScratch fa_scratch(int batch, int heads, int sq, int sk, int int8) {
+static FaScratch fa_scratch(int batch, int heads, int sq, int sk, int int8, bool direct) {
   FaScratch s{};
   auto up = [](long long v) { return (v + 255) / 256 * 256; };
   long long off = 0;
-  s.vt = off; off = up(off + static_cast<long long>(batch) * heads * kFaD * fa_pad(sk, 64) * 2);
+  s.vt = off;
+  if (!direct) off = up(off + static_cast<long long>(batch) * heads * kFaD * fa_pad(sk, 64) * 2);
   if (int8) {
     s.q8 = off; off = up(off + static_cast<long long>(batch) * sq * heads * kFaD);
     s.k8 = off; off = up(off + static_cast<long long>(batch) * sk * heads * kFaD);
@@ -870,8 +871,13 @@ static FaScratch fa_scratch(int batch, int heads, int sq, int sk, int int8) {
   return s;
 }
 
-B200_API long long b200_attn_fa_workspace_bytes(int batch, int heads, int sq, int sk, int int8) {
-  return fa_scratch(batch, heads, sq, sk, int8).total;
+// One sample: rows past the end of V arrive as zeros, so V is read in place. In a batch they are the next
+// sample's rows, whose values times a probability of zero need not be zero: V is transposed with padding there
+// (36 us of 300 at 4608 keys x 24 heads). A tensor map takes no V between 16-byte boundaries either.
+static bool fa_direct(int batch, const void* v) { return batch == 1 && (reinterpret_cast<uintptr_t>(v) & 15) == 0; }
+
+B200_API long long b200_attn_fa_workspace_bytes(int batch, int heads, int sq, int sk, int int8, const void* v) {
+  return fa_scratch(batch, heads, sq, sk, int8, fa_direct(batch, v)).total;
 }
 
 // Dense attention, head dim 128: q [batch * sq][heads * 128], k / v [batch * sk][heads * 128] bf16
@@ -880,16 +886,13 @@ B200_API long long b200_attn_fa_workspace_bytes(int batch, int heads, int sq, in
 static int fa_dense(const void* q, const void* k, const void* v, void* out, long long ld_out, int batch, int sq, int sk,
                     int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
   if (batch <= 0 || sq <= 0 || sk <= 0) return 0;
-  if (scratch == nullptr) return -2;
+  const bool direct = fa_direct(batch, v);
+  const FaScratch sc = fa_scratch(batch, heads, sq, sk, int8, direct);
+  if (scratch == nullptr && sc.total > 0) return -2;
   if (ld_out % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15)) return -2;
   const long long ld = static_cast<long long>(heads) * kFaD;
-  const FaScratch sc = fa_scratch(batch, heads, sq, sk, int8);
   uint8_t* base = static_cast<uint8_t*>(scratch);
   const int sk_pad64 = fa_pad(sk, 64);
-  // One sample: rows past the end of V arrive as zeros, so V is read in place. In a batch they are the next
-  // sample's rows, whose values times a probability of zero need not be zero: V is transposed with padding there
-  // (36 us of 300 at 4608 keys x 24 heads).
-  const bool direct = batch == 1;
   dim3 tgrid((sk_pad64 + 63) / 64, kFaD / 64, batch * heads);
   if (!direct) fa_transpose_v_kernel<<<tgrid, dim3(32, 8), 0, stream>>>(static_cast<const __nv_bfloat16*>(v),
                                                            reinterpret_cast<__nv_bfloat16*>(base + sc.vt), ld, sk,

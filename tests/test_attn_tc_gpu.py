@@ -93,3 +93,20 @@ def test_fa_attention_rescale_path_and_determinism():
                 assert (a.float().cpu() - ref).abs().max().item() < 3e-2
     finally:
         config.set_override("fa_attention", None)
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("tq,tk,heads,shift", [(77, 333, 4, 1), (300, 257, 2, 4), (128, 256, 1, 8)])
+def test_values_between_boundaries(tq, tk, heads, shift, int8):
+    """V as a view that starts off (1, 4) and on (8) a 16-byte boundary: the same result as from its own copy."""
+    torch.manual_seed(tk)
+    q, k = (torch.randn(t, heads, 128, device="cuda").to(torch.bfloat16) for t in (tq, tk))
+    store = torch.full((tk * heads * 128 + 16,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    v = store[shift:shift + tk * heads * 128].view(tk, heads, 128)
+    v.copy_(torch.randn(tk, heads, 128))
+    out = ops.attention(q, k, v, int8=int8)
+    N.check_status()
+    assert (out.float() - ops.attention(q, k, v.clone(), int8=int8).float()).abs().max() < 2 ** -9      # sums of 16 keys at a time in either form
+    rows = torch.empty(tq, heads * 128 + 8, dtype=torch.bfloat16, device="cuda")[:, :heads * 128]
+    ops.attention(q, k, v, int8=int8, out=rows)
+    assert torch.equal(rows.reshape(tq, heads, 128), out)
