@@ -171,7 +171,7 @@ def quant_int8_act(x: torch.Tensor, convrot_group: int = 0, inv_smooth: Optional
 
 
 def int8_linear(x: torch.Tensor, w: Int8Weight, act: Optional[str] = None, gate: Optional[torch.Tensor] = None,
-                residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, act_from: int = 0) -> torch.Tensor:
     """y = residual + gate * act((x H) (W H^T)^T + bias) with int8 operands and s32 accumulation on the
     tensor core (tcgen05 kind::i8); the two scale vectors are applied by the GEMM epilogue. Replaces the
     reference's cublasLt int8 GEMM + dequant pass (src/HartsyInference.Cuda/Kernels/dequant/w8a8.cu,
@@ -183,10 +183,7 @@ def int8_linear(x: torch.Tensor, w: Int8Weight, act: Optional[str] = None, gate:
         y = (q.float() @ w.weight.float().t()) * sc[:, None] * w.row_scale.float()[None, :]
         if w.bias is not None:
             y = y + w.bias.float()
-        if act == "gelu_tanh":
-            y = R.gelu_tanh(y)
-        elif act == "silu":
-            y = torch.nn.functional.silu(y)
+        y = R.activation(y, act, act_from)
         if gate is not None:
             y = y * gate.float()
         if residual is not None:
@@ -202,7 +199,7 @@ def int8_linear(x: torch.Tensor, w: Int8Weight, act: Optional[str] = None, gate:
     ws = st.gemm_workspace()
     rc = N.lib().b200_gemm(q.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k, q.stride(0), w.weight.stride(0),
                            out.stride(0), 3, sc.data_ptr(), w.row_scale.data_ptr(), N.ptr(w.bias), N.ptr(gate), N.ptr(residual),
-                           _ACT[act], 0, ws.data_ptr(), ws.numel(), st.status.data_ptr(), N.stream())
+                           act_code(act, act_from), 0, ws.data_ptr(), ws.numel(), st.status.data_ptr(), N.stream())
     N.check(rc, "b200_gemm")
     return out
 
@@ -293,14 +290,14 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
     if isinstance(w, Int8Weight):
         if isinstance(x, Fp8Act):
             raise ValueError("int8 weights take bf16 activations")
-        return int8_linear(x, w, act, gate, residual, out)
+        return int8_linear(x, w, act, gate, residual, out, act_from)
     xd = x.data if isinstance(x, Fp8Act) else x
     if not xd.is_cuda:
         if isinstance(x, Fp8Act):
-            y = R.linear(x.data, w.weight, w.scale, x.scale, w.bias, act, gate, residual)
+            y = R.linear(x.data, w.weight, w.scale, x.scale, w.bias, act, gate, residual, act_from=act_from)
         elif w.is_fp8:
             q, s = R.quant_fp8_act(x, pow2=fp8_mx())
-            y = R.linear(q, w.weight, w.scale, s, w.bias, act, gate, residual)
+            y = R.linear(q, w.weight, w.scale, s, w.bias, act, gate, residual, act_from=act_from)
         else:
             y = R.linear(x, w.host_f32(), None, None, w.bias, act, gate, residual, act_from=act_from)
         if out is not None:

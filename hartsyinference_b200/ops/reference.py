@@ -97,6 +97,20 @@ def gelu_tanh(x: torch.Tensor) -> torch.Tensor:
     return torch.nn.functional.gelu(x, approximate="tanh")
 
 
+def activation(y: torch.Tensor, act: Optional[str], act_from: int = 0) -> torch.Tensor:
+    """The activation of a product's epilogue, for the features from ``act_from`` on."""
+    plain, y = y[..., :act_from], y[..., act_from:]
+    if act == "gelu_tanh":
+        y = gelu_tanh(y)
+    elif act == "silu":
+        y = torch.nn.functional.silu(y)
+    elif act == "relu2":
+        y = torch.relu(y) ** 2
+    elif act == "tanh":
+        y = torch.tanh(y)
+    return torch.cat([plain, y], -1) if act_from else y
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, w_scale: Optional[torch.Tensor] = None,
            x_scale: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None,
            act: Optional[str] = None, gate: Optional[torch.Tensor] = None,
@@ -107,17 +121,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, w_scale: Optional[torch.Tensor] = N
     y = xf @ wf.t()
     if bias is not None:
         y = y + bias.float()
-    plain, y = y[..., :act_from], y[..., act_from:]
-    if act == "gelu_tanh":
-        y = gelu_tanh(y)
-    elif act == "silu":
-        y = torch.nn.functional.silu(y)
-    elif act == "relu2":
-        y = torch.relu(y) ** 2
-    elif act == "tanh":
-        y = torch.tanh(y)
-    if act_from:
-        y = torch.cat([plain, y], -1)
+    y = activation(y, act, act_from)
     if gate is not None:
         y = y * gate.float()
     if residual is not None:

@@ -38,6 +38,32 @@ def test_weight_round_trip_and_cpu_linear():
         assert _rel(y, x.float() @ w.t() + lw.bias.float()) < 0.03, g
 
 
+def _features_ahead_stay(x, w, act, act_from):
+    y, plain, whole = (ops.linear(x, w, act=a, act_from=f) for a, f in ((act, act_from), (None, 0), (act, 0)))
+    assert torch.equal(y[:, :act_from], plain[:, :act_from]) and torch.equal(y[:, act_from:], whole[:, act_from:])
+    assert not torch.equal(whole[:, :act_from], plain[:, :act_from])
+
+
+@pytest.mark.parametrize("act", ["gelu_tanh", "silu", "relu2", "tanh"])
+def test_activation_from_a_feature_on_the_host(act):
+    """8-bit weights apply the activation from ``act_from`` on, as bf16 ones do."""
+    torch.manual_seed(1)
+    x, w = torch.randn(5, 256).to(torch.bfloat16), torch.randn(96, 256) * 0.1
+    _features_ahead_stay(x, ops.Int8Weight.from_dense(w), act, 40)
+    fp8 = ops.LinearWeight.from_dense(w, fp8=True)
+    _features_ahead_stay(x, fp8, act, 40)
+    _features_ahead_stay(ops.quant_fp8_act(x, mx=fp8.is_mx), fp8, act, 40)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 64, 300])
+@pytest.mark.parametrize("act,act_from", [("gelu_tanh", 128), ("silu", 12), ("tanh", 64)])
+def test_activation_from_a_feature_on_the_device(m, act, act_from):
+    torch.manual_seed(m)
+    w = ops.Int8Weight.from_dense(torch.randn(512, 256, device="cuda") * 0.1)
+    _features_ahead_stay(torch.randn(m, 256, device="cuda").to(torch.bfloat16), w, act, act_from)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(64, 512, 1024), (300, 768, 512), (1, 256, 256), (1000, 1536, 2048)])
 @pytest.mark.parametrize("group", [0, 16, 256])
