@@ -901,7 +901,7 @@ B200_API int b200_quant_fp8_weight(const void* w, void* out, float* scales, int 
 }
 
 // part_ws != null: `in` is ignored and the [rows][2f] input is read as the unsummed K ranges a
-// deferred small-token GEMM left in its scratch (see SplitPartials; b200_gemm_deferred).
+// deferred small-token GEMM left unsummed (see SplitPartials; b200_gemm_deferred).
 B200_API int b200_glu(const void* in, void* out, void* out_fp8, float* out_scale, int rows, int f,
                       int act, int sf_tile_rows, const float* part_ws, int part_splits, int part_bn,
                       cudaStream_t stream) {

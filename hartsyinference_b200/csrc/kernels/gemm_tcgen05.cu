@@ -1704,12 +1704,75 @@ struct ConvSpec {
 int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long long ldx, long long ldw, long long ldc,
               const void* bias, const void* gate, const void* residual, int act, cudaStream_t stream);
 
+// A handful of tokens with bf16 weights: a product on the ordinary cores that needs one launch and no scratch. One
+// token is faster at every size (28672 x 4096 44.2 -> 39.8 us, 896 x 896 6.4 -> 2.2 us), two up to a depth of 8192
+// (4096 x 14336 24.3 -> 27.1 us, taken back); three and four only where the launch, not the weights, is what
+// counts (896 x 4864 7.5 -> 6.1 us, 3072 x 3072 9.4 -> 9.3 us, 28672 x 4096 45 -> 67 us, taken back).
+static bool handful(int m, int n, int k, int dtype) {
+  return dtype == 0 && k % 8 == 0 && (m == 1 || (m == 2 && k <= 8192) || (m <= 4 && static_cast<long long>(n) * k <= 1ll << 23));
+}
+
+// K-split policy (see the header comment): tiles from first_split on are cut into `count` ranges of `kblocks` K blocks.
+// plain: no groups and no peers. splits: 0 = automatic, 1 = never, more = every tile that many ways.
+struct KRanges {
+  int first_split, count, kblocks;
+};
+static KRanges plan_k_ranges(int tiles, int bn, int k, int dtype, bool swap, bool plain, int splits) {
+  const bool mx = dtype == 2;
+  const int esz = dtype != 0 ? 1 : 2, kelems = dtype != 0 ? 128 : 64;
+  const int total_kblocks = (k + kelems - 1) / kelems, sms = num_sms();
+  int first_split = tiles, s_eff = 1;
+  if (splits > 1) {                                  // caller-forced uniform split
+    first_split = 0;
+    s_eff = splits;
+  } else if (splits <= 0) {                          // automatic
+    const int q = tiles / sms, r = tiles % sms;
+    // worthwhile when the partial wave is a visible share of the run: always for the
+    // bandwidth-bound orientation, for the other only when there are few waves. After a full wave of 128 x 256 tiles the one
+    // CTA that adds a tile's ranges takes 50 to 75 us, so a whole wave more is faster up to rows of 24 KB in bf16 and 16 KB in
+    // 8 bits (152 tiles, cut -> whole: bf16 k 1024 97 -> 21 us, k 8192 157 -> 114, k 12288 184 -> 166; fp8 k 1024 65 -> 26,
+    // k 8192 103 -> 82, k 16384 150 -> 148, k 24576 194 -> 213).
+    const bool long_rows = static_cast<long long>(k) * esz > (esz == 1 ? 16384 : 24576);
+    if (swap && q == 0 && 2 * r > sms && plain) {
+      // More than half of the SMs have a tile, too many for two ranges each in one wave: up to four ranges in as many waves
+      // as they take, where the slowest SM is then done earlier (a tile's weights count as 1, and the writing and the
+      // second reading of the ranges' sums is added). fp8 64 x 10240 x 8192 36.4 -> 24.9 us, bf16 16 x 9728 x 896 13.8 ->
+      // 10.2 us. The same count for fewer tiles chose more ranges than fit one wave and lost (bf16 6 x 4096 x 4096 9.7 ->
+      // 12.3 us): there the ranges that fill one wave stay. Sixteen loads in flight in the last arriver's sums, tried for
+      // the tail of larger products, lost too (fp8 64 x 57344 x 8192 103 -> 115 us).
+      const double part = static_cast<double>(bn) * 128 * 4 / (128.0 * k * esz);
+      double best = 1.0;
+      for (int s = 2; s <= 4 && s <= total_kblocks / 2; ++s) {
+        const double cost = ((r * s + sms - 1) / sms) * (1.0 / s + part) + static_cast<double>(r) * s / sms * part;
+        if (cost < 0.9 * best) { best = cost; s_eff = s; }
+      }
+      if (s_eff > 1) first_split = 0;
+    } else if (r != 0 && (swap || (q < 4 && (q == 0 || bn < 256 || long_rows)))) {
+      int s = sms / r;
+      if (s > total_kblocks / 2) s = total_kblocks / 2;   // at least two k-blocks per range
+      // after full waves a modest split already shrinks the tail to 1/s of a tile; without full
+      // waves the split is what fills the machine
+      const int cap = q >= 1 ? 8 : 16;
+      if (s > cap) s = cap;
+      if (s > 1) { first_split = q * sms; s_eff = s; }
+    }
+  }
+  if (s_eff > total_kblocks) s_eff = total_kblocks;
+  int kblocks = (total_kblocks + s_eff - 1) / s_eff;
+  if (mx) kblocks = (kblocks + 3) / 4 * 4;   // ranges start on a scale-factor group
+  s_eff = (total_kblocks + kblocks - 1) / kblocks;
+  if (s_eff <= 1) { first_split = tiles; s_eff = 1; kblocks = total_kblocks; }
+  return {first_split, s_eff, kblocks};
+}
+
+static int small_tile_width(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
+
 int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long long ldx,
                      long long ldw, long long ldc, int dtype, const float* x_scale,
                      const float* w_scale, const void* bias, const void* gate, const void* residual,
                      int act, int splits, void* workspace, long long workspace_bytes, void* status,
                      cudaStream_t stream, const AllReduceParams* ar, const GroupSpec* gs = nullptr,
-                     const ConvSpec* cs = nullptr, int* defer_info = nullptr, const GatherParams* ag = nullptr) {
+                     const ConvSpec* cs = nullptr, void* defer_ws = nullptr, const GatherParams* ag = nullptr) {
   const int groups = gs ? gs->groups : 0;
   if (m <= 0 || n <= 0 || k <= 0) return 0;
   // grouped: x is [groups * m][k], w is [groups * n][k], out is [groups * m][n]; m = tokens per group
@@ -1742,13 +1805,8 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.act = act & 255;
   p.act_col = act >> 8;
-  // A handful of tokens with bf16 weights: a product on the ordinary cores that needs one launch and no scratch. One
-  // token is faster at every size (28672 x 4096 44.2 -> 39.8 us, 896 x 896 6.4 -> 2.2 us), two up to a depth of 8192
-  // (4096 x 14336 24.3 -> 27.1 us, taken back); three and four only where the launch, not the weights, is what
-  // counts (896 x 4864 7.5 -> 6.1 us, 3072 x 3072 9.4 -> 9.3 us, 28672 x 4096 45 -> 67 us, taken back).
-  const bool handful = m == 1 || (m == 2 && k <= 8192) || (m <= 4 && static_cast<long long>(n) * k <= 1ll << 23);
-  if (dtype == 0 && handful && k % 8 == 0 && splits == 0 && groups == 0 && cs == nullptr && ar == nullptr && ag == nullptr) {
-    if (defer_info != nullptr) defer_info[0] = 0;
+  if (handful(m, n, k, dtype) && splits == 0 && groups == 0 && cs == nullptr && ar == nullptr && ag == nullptr) {
+    if (defer_ws != nullptr) return -13;
     return gemv_bf16(x, w, out, m, n, k, ldx, ldw, ldc, bias, gate, residual, act, stream);
   }
   p.status = static_cast<DeviceStatus*>(status);
@@ -1791,13 +1849,13 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
     // with a device block list `chunks` is the total number of blocks the buffers can hold
     p.rows_b = gs->b_koff > 0 ? m : (gs->block_group ? p.group_chunks * m : groups * p.group_chunks * m);
     a_ptr = w; lda = ldw; b_ptr = x; ldb = ldx;
-    bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    bn = small_tile_width(m);
     p.scale_a = w_scale; p.sa_gran = 128; p.sa_ld = k / 128;
     p.scale_b = x_scale; p.sb_gran = 1;   p.sb_ld = k / 128;
   } else if (swap) {
     p.rows_a = n; p.rows_b = m;
     a_ptr = w; lda = ldw; b_ptr = x; ldb = ldx;
-    bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    bn = small_tile_width(m);
     p.scale_a = w_scale; p.sa_gran = 128; p.sa_ld = k / 128;
     p.scale_b = x_scale; p.sb_gran = 1;   p.sb_ld = k / 128;
   } else {
@@ -1836,49 +1894,11 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   constexpr int kBand = 16;
   if (!swap && groups == 0 && cs == nullptr && ar == nullptr && ag == nullptr && (p.rows_a + 127) / 128 > kBand) p.band = kBand;
 
-  // ---- K-split policy (see the header comment)
-  int first_split = tiles, s_eff = 1;
+  const bool plain = groups == 0 && ar == nullptr && ag == nullptr;
+  const KRanges plan = plan_k_ranges(tiles, bn, k, dtype, swap, plain, groups > 0 && gs->block_group && splits <= 0 ? 1 : splits);      // automatic: never with a device block list
+  int first_split = plan.first_split, s_eff = plan.count;
+  p.kblocks_per_split = plan.kblocks;
   const long long slot_bytes = static_cast<long long>(bn) * 128 * 4;
-  if (splits > 1) {                                  // caller-forced uniform split
-    first_split = 0;
-    s_eff = splits;
-  } else if (splits <= 0 && !(groups > 0 && gs->block_group)) {   // automatic (never with a device block list)
-    const int q = tiles / sms, r = tiles % sms;
-    // worthwhile when the partial wave is a visible share of the run: always for the
-    // bandwidth-bound orientation, for the other only when there are few waves. After a full wave of 128 x 256 tiles the one
-    // CTA that adds a tile's ranges takes 50 to 75 us, so a whole wave more is faster up to rows of 24 KB in bf16 and 16 KB in
-    // 8 bits (152 tiles, cut -> whole: bf16 k 1024 97 -> 21 us, k 8192 157 -> 114, k 12288 184 -> 166; fp8 k 1024 65 -> 26,
-    // k 8192 103 -> 82, k 16384 150 -> 148, k 24576 194 -> 213).
-    const bool long_rows = static_cast<long long>(k) * esz > (esz == 1 ? 16384 : 24576);
-    if (swap && q == 0 && 2 * r > sms && groups == 0 && ar == nullptr && ag == nullptr) {
-      // More than half of the SMs have a tile, too many for two ranges each in one wave: up to four ranges in as many waves
-      // as they take, where the slowest SM is then done earlier (a tile's weights count as 1, and the writing and the
-      // second reading of the ranges' sums is added). fp8 64 x 10240 x 8192 36.4 -> 24.9 us, bf16 16 x 9728 x 896 13.8 ->
-      // 10.2 us. The same count for fewer tiles chose more ranges than fit one wave and lost (bf16 6 x 4096 x 4096 9.7 ->
-      // 12.3 us): there the ranges that fill one wave stay. Sixteen loads in flight in the last arriver's sums, tried for
-      // the tail of larger products, lost too (fp8 64 x 57344 x 8192 103 -> 115 us).
-      const double part = static_cast<double>(bn) * 128 * 4 / (128.0 * k * esz);
-      double best = 1.0;
-      for (int s = 2; s <= 4 && s <= total_kblocks / 2; ++s) {
-        const double cost = ((r * s + sms - 1) / sms) * (1.0 / s + part) + static_cast<double>(r) * s / sms * part;
-        if (cost < 0.9 * best) { best = cost; s_eff = s; }
-      }
-      if (s_eff > 1) first_split = 0;
-    } else if (r != 0 && (swap || (q < 4 && (q == 0 || bn < 256 || long_rows)))) {
-      int s = sms / r;
-      if (s > total_kblocks / 2) s = total_kblocks / 2;   // at least two k-blocks per range
-      // after full waves a modest split already shrinks the tail to 1/s of a tile; without full
-      // waves the split is what fills the machine
-      const int cap = q >= 1 ? 8 : 16;
-      if (s > cap) s = cap;
-      if (s > 1) { first_split = q * sms; s_eff = s; }
-    }
-  }
-  if (s_eff > total_kblocks) s_eff = total_kblocks;
-  p.kblocks_per_split = (total_kblocks + s_eff - 1) / s_eff;
-  if (mx) p.kblocks_per_split = (p.kblocks_per_split + 3) / 4 * 4;   // ranges start on a scale-factor group
-  s_eff = (total_kblocks + p.kblocks_per_split - 1) / p.kblocks_per_split;
-  if (s_eff <= 1) { first_split = tiles; s_eff = 1; p.kblocks_per_split = total_kblocks; }
   const int split_tiles = tiles - first_split;
   if (split_tiles > 0 && ar == nullptr) {
     const long long need = kSplitCounterBytes + static_cast<long long>(split_tiles) * s_eff * slot_bytes;
@@ -1907,6 +1927,11 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   }
   p.split_counter = static_cast<uint32_t*>(workspace);
   p.split_ws = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kSplitCounterBytes);
+
+  if (defer_ws != nullptr) {
+    if (!(p.external_reduce && swap && plain && gate == nullptr && residual == nullptr && act == 0)) return -13;
+    p.split_ws = static_cast<float*>(defer_ws);
+  }
 
   // two atoms per stage for the bandwidth-bound small-token orientation
   const int atoms = swap ? 2 : 1;
@@ -1991,15 +2016,7 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
       rc = launch_gemm<0, 256, 1>(p, ta, tb, grid, stream);
     }
   }
-  if (defer_info != nullptr) {
-    // the caller's consumer kernel sums the K ranges itself: report their layout, launch no reduce
-    const bool deferred = rc == 0 && p.external_reduce && swap && groups == 0 &&
-                          gate == nullptr && residual == nullptr && act == 0 && m <= bn;
-    defer_info[0] = deferred ? 1 : 0;
-    defer_info[1] = p.splits;
-    defer_info[2] = bn;
-    if (deferred) return rc;
-  }
+  if (defer_ws != nullptr) return rc;      // the caller's consumer kernel sums the K ranges itself: no reduce
   if (rc == 0 && p.external_reduce) {
     const dim3 rgrid((bn * 32 + 255) / 256, tiles);
     if (launch_pdl(splitk_reduce_kernel, rgrid, dim3(256), 0, stream, p, bn, (p.rows_a + kTileA - 1) / kTileA,
@@ -2020,7 +2037,9 @@ B200_API void b200_gemm_set_cluster_reduce(int enabled) { g_cluster_reduce = ena
 B200_API void b200_gemm_set_external_reduce(int enabled) { g_external_reduce = enabled != 0; }
 
 B200_API long long b200_gemm_workspace_bytes() {
-  return 64ll << 20;   // the automatic policy needs at most 16 KB + 148 slots of 64 KB
+  // On 148 processors the automatic policy needs at most 37 MB: 16 KB of counters and 588 slots of 64 KB (147 tiles of 128
+  // tokens in four ranges each); the ranges of 128 x 256 tiles are one wave of 128 KB, 19 MB.
+  return 64ll << 20;
 }
 
 // out[m][n] (bf16, leading dim ldc) = epilogue(x[m][k] * w[n][k]^T)
@@ -2088,17 +2107,28 @@ B200_API int b200_gemm_glu(const void* x, const void* w, void* out, void* out_q,
   return mx ? launch_gemm<2, 256, 1, true>(p, ta, tb, grid, stream) : launch_gemm<0, 256, 1, true>(p, ta, tb, grid, stream);
 }
 
-// b200_gemm for a consumer that can add split-K ranges itself (b200_glu, b200_rope_kv): when the
-// policy cuts every tile along K (small-token GEMMs with fewer tiles than SMs), the reduce kernel is NOT
-// launched (the consumer adds `bias` too) and `out` is left untouched; info[0] = 1 then and
-// the partials sit at workspace + 16384 bytes as [feature tile][info[1] K ranges][info[2] tokens][128]
-// fp32. Otherwise info[0] = 0 and `out` holds the result as usual.
-B200_API int b200_gemm_deferred(const void* x, const void* w, void* out, int m, int n, int k, long long ldx,
-                                long long ldw, long long ldc, int dtype, const float* x_scale,
-                                const float* w_scale, const void* bias, void* workspace, long long workspace_bytes, int* info,
-                                void* status, cudaStream_t stream) {
-  return gemm_impl(x, w, out, m, n, k, ldx, ldw, ldc, dtype, x_scale, w_scale, bias, nullptr, nullptr, 0, 0,
-                   workspace, workspace_bytes, status, stream, nullptr, nullptr, nullptr, info);
+// For a consumer that can add split-K ranges itself (b200_glu, b200_rope_kv, b200_norm): whether the policy cuts every tile of
+// a product without epilogue along K (small-token GEMMs with fewer tiles than SMs). 0: it does not, use b200_gemm.
+// Otherwise the number of ranges in the low half and the tokens per range in the high half; b200_gemm_deferred then leaves the
+// partials at part_ws as [feature tile][ranges][tokens][128] fp32 and launches no reduce kernel (the consumer adds a
+// bias, too). The memory is the consumer's to keep: in the scratch of all products another one, of another thread or stream or
+// launched in between, would write there before it has read.
+B200_API int b200_gemm_deferred_plan(int m, int n, int k, int dtype, long long workspace_bytes) {
+  if (m < 1 || m > 128 || n < 1 || k < 1 || !g_external_reduce || g_cluster_reduce || handful(m, n, k, dtype)) return 0;
+  const int bn = small_tile_width(m), tiles = (n + 127) / 128;
+  const KRanges r = plan_k_ranges(tiles, bn, k, dtype, true, true, 0);
+  if (r.first_split != 0 || r.count < 2 || tiles > 4096) return 0;
+  if (kSplitCounterBytes + static_cast<long long>(tiles) * r.count * bn * 128 * 4 > workspace_bytes) return 0;
+  return bn << 16 | r.count;
+}
+
+// workspace as for b200_gemm (its size takes part in the policy). -13: the plan for these sizes is 0.
+B200_API int b200_gemm_deferred(const void* x, const void* w, int m, int n, int k, long long ldx, long long ldw, int dtype,
+                                const float* x_scale, const float* w_scale, void* workspace, long long workspace_bytes,
+                                float* part_ws, void* status, cudaStream_t stream) {
+  if (part_ws == nullptr) return -13;
+  return gemm_impl(x, w, nullptr, m, n, k, ldx, ldw, n, dtype, x_scale, w_scale, nullptr, nullptr, nullptr, 0, 0,
+                   workspace, workspace_bytes, status, stream, nullptr, nullptr, nullptr, part_ws);
 }
 
 // Row-parallel linear of a tensor-parallel group fused with the all-reduce of its output, the

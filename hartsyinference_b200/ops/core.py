@@ -242,17 +242,17 @@ def quant_fp8_weight(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
 
 @dataclass
 class SplitSum:
-    """Result of a small-token GEMM whose K ranges were left unsummed in the GEMM scratch
-    (``linear(..., defer=True)``): the consumer kernel (``glu``, ``rope_kv``, ``norm``) adds them while it
-    reads, so no reduce kernel runs in between. Valid until the next GEMM on the device."""
-    ws: torch.Tensor          # the device's GEMM scratch
+    """Result of a small-token GEMM whose K ranges were left unsummed (``linear(..., defer=True)``): the consumer
+    kernel (``glu``, ``rope_kv``, ``norm``) adds them while it reads, so no reduce kernel runs in between. The ranges are
+    in memory of their own, like any result: other products, also of other threads and streams, leave them alone."""
+    ws: torch.Tensor          # fp32 [feature tile][splits][bn][128]
     splits: int
     bn: int
     shape: tuple              # (tokens, features) of the product
     bias: Optional[torch.Tensor] = None       # still to be added (``rope_kv`` only)
 
     def part_args(self):
-        return self.ws.data_ptr() + 16384, self.splits, self.bn
+        return self.ws.data_ptr(), self.splits, self.bn
 
 
 def _part_args(x):
@@ -315,21 +315,21 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
     n = w.weight.shape[0]
     assert w.weight.shape[1] == k, (w.weight.shape, xd.shape)
     assert xd.stride(1) == 1 and w.weight.stride(1) == 1
-    if out is None:
-        out = torch.empty(m, n, dtype=torch.bfloat16, device=xd.device)
-    fp8 = w.is_fp8
     L = N.lib()
     st = N.state(xd.device)
     ws = st.gemm_workspace()
     xs_ptr, ws_ptr = _scale_ptrs(x, w)
     if defer and m <= 128 and (w.bias is None or defer_bias) and act is None and gate is None and residual is None and splits is None:
-        import ctypes as C
-        info = (C.c_int * 4)()
-        rc = L.b200_gemm_deferred(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k, xd.stride(0),
-                                  w.weight.stride(0), out.stride(0), _gemm_dtype(w), xs_ptr, ws_ptr, N.ptr(w.bias), ws.data_ptr(),
-                                  ws.numel(), info, st.status.data_ptr(), N.stream())
-        N.check(rc, "b200_gemm_deferred")
-        return SplitSum(ws, int(info[1]), int(info[2]), (m, n), w.bias) if info[0] else out
+        plan = L.b200_gemm_deferred_plan(m, n, k, _gemm_dtype(w), ws.numel())
+        if plan:
+            ranges, bn = plan & 0xffff, plan >> 16
+            part = torch.empty((n + 127) // 128 * ranges * bn * 128, dtype=torch.float32, device=xd.device)
+            rc = L.b200_gemm_deferred(xd.data_ptr(), w.weight.data_ptr(), m, n, k, xd.stride(0), w.weight.stride(0), _gemm_dtype(w), xs_ptr, ws_ptr,
+                                      ws.data_ptr(), ws.numel(), part.data_ptr(), st.status.data_ptr(), N.stream())
+            N.check(rc, "b200_gemm_deferred")
+            return SplitSum(part, ranges, bn, (m, n), w.bias)
+    if out is None:
+        out = torch.empty(m, n, dtype=torch.bfloat16, device=xd.device)
     rc = L.b200_gemm(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k,
                      xd.stride(0), w.weight.stride(0), out.stride(0), _gemm_dtype(w),
                      xs_ptr, ws_ptr,

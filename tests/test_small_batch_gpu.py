@@ -40,6 +40,20 @@ def test_rotary_adds_ranges_and_bias(m, d, style):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 896, 4864), (64, 1024, 1024), (128, 9600, 4096), (17, 9600, 2048)])
+def test_ranges_outlive_other_products(m, n, k):
+    """A second product that is cut along K, between the first one and its consumer: the ranges are the consumer's."""
+    torch.manual_seed(n)
+    x, x2 = (torch.randn(m, k, device="cuda").to(torch.bfloat16) for _ in range(2))
+    w, w2 = (ops.LinearWeight((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16)) for _ in range(2))
+    want, want2 = ops.norm(ops.linear(x, w))[0], ops.norm(ops.linear(x2, w2))[0]
+    part = ops.linear(x, w, defer=True)
+    assert isinstance(part, ops.core.SplitSum)
+    assert torch.equal(ops.norm(ops.linear(x2, w2))[0], want2)
+    assert torch.equal(ops.norm(ops.linear(x2, w2, defer=True))[0], want2)
+    assert torch.equal(ops.norm(part)[0], want)
+
+
 @pytest.mark.parametrize("vocab", [1, 7, 8, 1025, 32768, 32777, 151936])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_argmax_takes_the_first_of_equals(vocab, dtype):
