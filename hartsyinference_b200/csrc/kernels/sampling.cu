@@ -12,8 +12,9 @@
 // sum of the kept masses.
 //
 // A row of up to 262144 logits belongs to a cluster of eight blocks that keep it in registers: one read of
-// the row, histograms and prefix sums met through distributed shared memory. Longer rows (and the rare device
-// without clusters) go through one block that makes eight passes over a row in L2.
+// the row, histograms and prefix sums met through distributed shared memory. Longer rows go through one block that makes
+// eight passes over a row in L2, and so do short rows and many rows of moderate length, where the exchanges of a
+// cluster cost more than the passes (see b200_sample).
 //
 // The reference applies the same chain on the host, one request at a time, after copying the logits
 // back (src/HartsyInference.LLM/Sampling/SamplerChain.cs:26-85, TopKSampler.cs, TopPSampler.cs,
@@ -22,6 +23,8 @@
 #include "common.cuh"
 
 namespace b200 {
+
+int num_sms();      // of the current device, see gemm_tcgen05.cu
 
 constexpr int kSampleThreads = 1024;
 constexpr int kSampleBins = 2048;
@@ -655,7 +658,18 @@ B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows,
   p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.min_p = min_p;
   p.seed = seed; p.counter = counter; p.out = out;
   const int each = (vocab + kRowBlocks * kRowThreads - 1) / (kRowBlocks * kRowThreads);      // values a thread holds
-  if (rows < (1 << 27)) {
+  // A block of its own per row takes 24 us + a us per 350 logits with every filter, all rows of a wave at once. A cluster takes 58 to
+  // 105 us however short its rows are, and 37 of them (18 of the widest) fill the machine; from 16 to 40 values a thread a
+  // wave gets up to 1.4 times longer. Which filters a row asks for is known on the device only: with every one (us, block /
+  // cluster) 1 x 4096 34 / 54, 1 x 16384 69 / 54, 64 x 32000 121 / 208, 64 x 65536 252 / 214, 512 x 4096 136 / 1549,
+  // 128 x 100352 349 / 489, 128 x 202048 686 / 774; without filters 64 x 32000 32 / 18, 128 x 100352 74 / 73; greedy rows leave a
+  // wave of clusters early, while a wave of blocks waits for its slowest. So clusters may be up to 1.35 times the slower
+  // by the full chain.
+  const int sms = num_sms(), per_wave = (each <= 40 ? 2 * sms : sms) / kRowBlocks;
+  const double block_us = (24. + vocab / 350.) * ((rows + sms - 1) / sms);
+  const double cluster_us = rows <= 8 ? 58. : 2 * rows <= per_wave ? 75. :
+      105. * ((rows + per_wave - 1) / per_wave) * (each > 16 && each <= 40 ? 1. + (each - 16) / 64. : 1.);
+  if (rows < (1 << 27) && per_wave > 0 && cluster_us <= 1.35 * block_us) {
     if (each <= 8) return launch_rows<8>(p, rows, stream);
     if (each <= 16) return launch_rows<16>(p, rows, stream);
     if (each <= 32) return launch_rows<32>(p, rows, stream);

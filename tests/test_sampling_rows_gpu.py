@@ -57,3 +57,23 @@ def test_ties_and_infinities():
     tok = _sample(x, 0.7, 50, 0.9, 0.1).tolist()
     assert tok[0] in (123, 39999) and tok[1:] == [777, 0, 5]
     assert set(_sample(x[:1].repeat(200, 1).contiguous(), 1.0, 1, 0.0, 0.0).tolist()) == {123, 39999}     # ties at the k-th value all stay
+
+
+@pytest.mark.parametrize("rows,vocab", [(300, 32000), (64, 8193), (9, 5000)])
+def test_many_rows_as_few(rows, vocab):
+    """Batches that a block per row is faster for, against the same rows a few at a time and the sampler's statement."""
+    torch.manual_seed(rows)
+    logits = torch.randn(rows, vocab, device="cuda") * 3
+    ids = torch.arange(rows, device="cuda")
+    col = lambda values, dt: torch.tensor(values, dtype=dt, device="cuda").repeat((rows + 5) // 6)[:rows]
+    args = (col([0.0, 0.8, 1.0, 0.7, 1.3, 1.0], torch.float32), col([0, 40, 0, 50, 0, 1], torch.int32), col([0.9, 0.95, 0.9, 0.0, 1.0, 0.0], torch.float32),
+            col([0.0, 0.0, 0.05, 0.0, 0.1, 0.0], torch.float32), ids, ids * 3)
+    tok = ops.sample_tokens(logits, *args)
+    few = torch.cat([ops.sample_tokens(logits[i:i + 4], *(a[i:i + 4] for a in args)) for i in range(0, rows, 4)])
+    greedy = args[0] <= 0
+    assert torch.equal(tok[greedy], logits[greedy].argmax(-1).to(torch.int32))
+    for r in range(rows):
+        if not greedy[r]:
+            assert bool(R.sampling_keep_mask(logits[r], *(float(a[r]) if a.is_floating_point() else int(a[r]) for a in args[:4]))[int(tok[r])])
+    # the two forms sum masses in fp32 and in 2^-40: a draw falls between them with 2^-20 or so a row
+    assert int((tok != few).sum()) <= 1
