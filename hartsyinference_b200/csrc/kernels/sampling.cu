@@ -14,7 +14,8 @@
 // A row of up to 262144 logits belongs to a cluster of eight blocks that keep it in registers: one read of
 // the row, histograms and prefix sums met through distributed shared memory. Longer rows go through one block that makes
 // eight passes over a row in L2, and so do short rows and many rows of moderate length, where the exchanges of a
-// cluster cost more than the passes (see b200_sample).
+// cluster cost more than the passes (see b200_sample). Both forms sum masses in 2^-40, so a row's token is the
+// same whatever batch it comes in (fp32 sums in the one block drew other tokens than the cluster in one of 50 flat rows of 100000).
 //
 // The reference applies the same chain on the host, one request at a time, after copying the logits
 // back (src/HartsyInference.LLM/Sampling/SamplerChain.cs:26-85, TopKSampler.cs, TopPSampler.cs,
@@ -55,6 +56,12 @@ __device__ __forceinline__ float sample_uniform(unsigned long long seed, unsigne
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   z ^= z >> 31;
   return static_cast<float>(z >> 40) * (1.f / 16777216.f);
+}
+
+// The row's uniform number (24 bits) times its whole mass: in [0, total).
+__device__ __forceinline__ unsigned long long draw_point(const SampleParams& p, int row, unsigned long long total) {
+  const unsigned long long bits = static_cast<unsigned long long>(sample_uniform(p.seed[row], p.counter[row]) * 16777216.f);
+  return __umul64hi(total, bits << 40);
 }
 
 __device__ __forceinline__ float block_reduce_max(float v, float* red) {
@@ -172,12 +179,32 @@ __device__ void radix_level(const SampleParams& p, long long row_off, float mx, 
   __syncthreads();
 }
 
+// Sum of `x` over the threads of the block in front of this one; the block's sum in `total`. `sums` may be used again.
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long x, unsigned long long* sums, unsigned long long& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto warp_scan = [&](unsigned long long incl) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    return incl;
+  };
+  const unsigned long long incl = warp_scan(x);
+  __syncthreads();
+  if (lane == 31) sums[wid] = incl;
+  __syncthreads();
+  const unsigned long long own = sums[lane], upto = warp_scan(own);      // 32 warps
+  total = __shfl_sync(0xffffffffu, upto, 31);
+  return __shfl_sync(0xffffffffu, upto - own, wid) + incl - x;
+}
+
 __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleParams p) {
   __shared__ float red[32];
   __shared__ unsigned hist_cnt[kSampleBins];
   __shared__ unsigned long long hist_mass[kSampleBins];
   __shared__ RadixShared rsh;
-  __shared__ float s_scan[kSampleThreads / 32];
+  __shared__ unsigned long long s_scan[kSampleThreads / 32];
   __shared__ int s_pick;
   const int row = blockIdx.x;
   const long long row_off = static_cast<long long>(row) * p.ld;
@@ -211,7 +238,6 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
 
   // ---- top-k: the k-th largest w
   const int k = p.top_k[row];
-  float kept_mass = -1.f;
   if (k > 0 && k < p.vocab) {
     RadixState st{0u};
     if (threadIdx.x == 0) { rsh.count_before = 0u; rsh.mass_before = 0ull; }
@@ -232,33 +258,18 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
     if (!open_end) tau = __uint_as_float(st.prefix);
   }
 
-  // ---- mass of the survivors so far
-  {
-    float local = 0.f;
-    for (int i = threadIdx.x; i < p.vocab; i += blockDim.x) {
-      const float w = __expf((sample_logit(p, row_off, i) - bmx) * inv_t);
-      if (w >= tau) local += w;
-    }
-    local = warp_sum(local);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (int w = 0; w < kSampleThreads / 32; ++w) t += red[w];
-      red[0] = t;
-    }
-    __syncthreads();
-    kept_mass = red[0];
-    __syncthreads();
-  }
-
   // ---- top-p over the survivors: the smallest w whose mass in front is <= p * kept_mass
   const float tp = p.top_p[row];
   if (tp > 0.f && tp < 1.f) {
-    const unsigned long long limit = static_cast<unsigned long long>(static_cast<double>(tp) * static_cast<double>(kept_mass) *
-                                                                   static_cast<double>(kMassScale));
+    unsigned long long kept = 0;
+    for (int i = threadIdx.x; i < p.vocab; i += blockDim.x) {
+      const float w = __expf((sample_logit(p, row_off, i) - bmx) * inv_t);
+      if (w >= tau) kept += static_cast<unsigned long long>(w * kMassScale);
+    }
+    unsigned long long total;
+    block_scan(kept, s_scan, total);
+    const unsigned long long limit = static_cast<unsigned long long>(static_cast<double>(tp) * static_cast<double>(total));
     RadixState st{0u};
-    __syncthreads();
     if (threadIdx.x == 0) { rsh.count_before = 0u; rsh.mass_before = 0ull; }
     __syncthreads();
     unsigned hi_mask = 0u;
@@ -282,56 +293,35 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
   const float mp = p.min_p[row];
   if (mp > 0.f) tau = fmaxf(tau, fminf(mp, 1.f));
 
-  // ---- draw: index-ordered prefix sums of the kept masses
+  // ---- draw: index-ordered prefix sums of the kept masses, in 2^-40 as in sample_row_kernel: the token of a row does not
+  // depend on which of the two its batch takes
   const int per = (p.vocab + kSampleThreads - 1) / kSampleThreads;
   const int i0 = threadIdx.x * per, i1 = min(p.vocab, i0 + per);
-  float local = 0.f;
+  unsigned long long local = 0;
   for (int i = i0; i < i1; ++i) {
     const float w = __expf((sample_logit(p, row_off, i) - bmx) * inv_t);
-    if (w >= tau) local += w;
+    if (w >= tau) local += static_cast<unsigned long long>(w * kMassScale);
   }
-  // block-wide exclusive scan of `local`
-  float incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, incl, o);
-    if ((threadIdx.x & 31) >= o) incl += t;
-  }
-  if ((threadIdx.x & 31) == 31) s_scan[threadIdx.x >> 5] = incl;
+  unsigned long long total;
+  unsigned long long front = block_scan(local, s_scan, total);
   if (threadIdx.x == 0) s_pick = -1;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float run = 0.f;
-    for (int w = 0; w < kSampleThreads / 32; ++w) {
-      const float t = s_scan[w];
-      s_scan[w] = run;
-      run += t;
-    }
-    red[0] = run;
-  }
-  __syncthreads();
-  const float total = red[0];
-  const float excl = s_scan[threadIdx.x >> 5] + incl - local;
-  const float u = sample_uniform(p.seed[row], p.counter[row]) * total;
-  if (local > 0.f && u >= excl && u < excl + local) {
+  const unsigned long long u = draw_point(p, row, total);
+  if (u >= front && u < front + local) {
     // walk this thread's chunk
-    float acc = excl;
-    int pick = -1;
     for (int i = i0; i < i1; ++i) {
       const float w = __expf((sample_logit(p, row_off, i) - bmx) * inv_t);
       if (w >= tau) {
-        pick = i;
-        acc += w;
-        if (u < acc) break;
+        front += static_cast<unsigned long long>(w * kMassScale);
+        if (u < front) { s_pick = i; break; }
       }
     }
-    if (pick >= 0) atomicMax(&s_pick, pick);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int pick = s_pick;
     if (pick < 0) {
-      // rounding at the very end of the range: fall back to the most probable token
+      // no finite mass: the most probable token
       pick = 0;
       float best = -INFINITY;
       for (int i = 0; i < p.vocab; ++i) {
@@ -590,9 +580,7 @@ __global__ void __launch_bounds__(kRowThreads, V <= 40 ? 2 : 1) sample_row_kerne
     if (b < block) before += sh.all[b];
     all += sh.all[b];
   }
-  // u in [0, all): the 24-bit uniform number times the whole mass
-  const unsigned long long bits = static_cast<unsigned long long>(sample_uniform(p.seed[row], p.counter[row]) * 16777216.f);
-  const unsigned long long u = __umul64hi(all, bits << 40);
+  const unsigned long long u = draw_point(p, row, all);
   unsigned long long run = before + own;
 #pragma unroll
   for (int e = 0; e < kEach; ++e) {
