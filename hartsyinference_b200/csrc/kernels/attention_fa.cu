@@ -30,8 +30,8 @@
 //                because the final division by the row sum uses the same maximum.
 //
 // One sample's V is read as it lies ([key][head dim], an MN-major operand) where it starts on a 16-byte boundary.
-// Otherwise, in a batch and in the segmented forms below, V is consumed transposed ([head dim][keys]) and padded; that transpose and the int8 quantisation are small
-// kernels of their own in front.
+// Otherwise, and in the segmented forms below, V is consumed transposed ([head dim][keys]) and padded; that transpose and
+// the int8 quantisation are small kernels of their own in front.
 #include "comm.cuh"
 
 namespace b200 {
@@ -848,59 +848,58 @@ static inline int fa_pad(int s, int to) { return (s + to - 1) / to * to; }
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,
                      int int8, cudaStream_t stream, const FaPeerMaps* peers = nullptr, bool direct = false);
 
-// Scratch layout of one call: (unless V is read in place) V^T [batch * heads * 128][sk_pad64] bf16, then (int8 mode) Q8
-// [batch * sq][heads * 128], K8 [batch * sk][heads * 128], q scales [batch * heads][sq_pad128],
-// K tile scales [batch * heads][key tiles] fp32, K sums [batch * heads][128] fp32.
+// Scratch layout of one call: (unless V is read in place) V^T [heads * 128][sk_pad64] bf16, then (int8 mode) Q8
+// [sq][heads * 128], K8 [sk][heads * 128], q scales [heads][sq_pad128], K tile scales [heads][key tiles] fp32,
+// K sums [heads][128] fp32.
 struct FaScratch {
   long long vt, q8, k8, qs, ks, ksum, total;
 };
-static FaScratch fa_scratch(int batch, int heads, int sq, int sk, int int8, bool direct) {
+static FaScratch fa_scratch(int heads, int sq, int sk, int int8, bool direct) {
   FaScratch s{};
   auto up = [](long long v) { return (v + 255) / 256 * 256; };
   long long off = 0;
   s.vt = off;
-  if (!direct) off = up(off + static_cast<long long>(batch) * heads * kFaD * fa_pad(sk, 64) * 2);
+  if (!direct) off = up(off + static_cast<long long>(heads) * kFaD * fa_pad(sk, 64) * 2);
   if (int8) {
-    s.q8 = off; off = up(off + static_cast<long long>(batch) * sq * heads * kFaD);
-    s.k8 = off; off = up(off + static_cast<long long>(batch) * sk * heads * kFaD);
-    s.qs = off; off = up(off + static_cast<long long>(batch) * heads * fa_pad(sq, 128) * 4);
-    s.ks = off; off = up(off + static_cast<long long>(batch) * heads * (fa_pad(sk, 128) / 128) * 4);
-    s.ksum = off; off = up(off + static_cast<long long>(batch) * heads * kFaD * 4);
+    s.q8 = off; off = up(off + static_cast<long long>(sq) * heads * kFaD);
+    s.k8 = off; off = up(off + static_cast<long long>(sk) * heads * kFaD);
+    s.qs = off; off = up(off + static_cast<long long>(heads) * fa_pad(sq, 128) * 4);
+    s.ks = off; off = up(off + static_cast<long long>(heads) * (fa_pad(sk, 128) / 128) * 4);
+    s.ksum = off; off = up(off + static_cast<long long>(heads) * kFaD * 4);
   }
   s.total = off;
   return s;
 }
 
-// One sample: rows past the end of V arrive as zeros, so V is read in place. In a batch they are the next
-// sample's rows, whose values times a probability of zero need not be zero: V is transposed with padding there
-// (36 us of 300 at 4608 keys x 24 heads). A tensor map takes no V between 16-byte boundaries either.
-static bool fa_direct(int batch, const void* v) { return batch == 1 && (reinterpret_cast<uintptr_t>(v) & 15) == 0; }
+// Rows past the end of V arrive as zeros, so V is read in place (its transposition took 36 us of 300 at 4608 keys x 24
+// heads). A tensor map takes no V between 16-byte boundaries: transposed there.
+static bool fa_direct(const void* v) { return (reinterpret_cast<uintptr_t>(v) & 15) == 0; }
 
-B200_API long long b200_attn_fa_workspace_bytes(int batch, int heads, int sq, int sk, int int8, const void* v) {
-  return fa_scratch(batch, heads, sq, sk, int8, fa_direct(batch, v)).total;
+B200_API long long b200_attn_fa_workspace_bytes(int heads, int sq, int sk, int int8, const void* v) {
+  return fa_scratch(heads, sq, sk, int8, fa_direct(v)).total;
 }
 
-// Dense attention, head dim 128: q [batch * sq][heads * 128], k / v [batch * sk][heads * 128] bf16
-// (contiguous), out like q: softmax(q k^T * scale) v per (batch, head). int8 != 0: SageAttention
-// (K mean removal, int8 Q K^T). `scratch`: b200_attn_fa_workspace_bytes bytes.
-static int fa_dense(const void* q, const void* k, const void* v, void* out, long long ld_out, int batch, int sq, int sk,
-                    int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
-  if (batch <= 0 || sq <= 0 || sk <= 0) return 0;
-  const bool direct = fa_direct(batch, v);
-  const FaScratch sc = fa_scratch(batch, heads, sq, sk, int8, direct);
+// Dense attention of one sample, head dim 128: q [sq][heads * 128], k / v [sk][heads * 128] bf16 (contiguous), out like q
+// with rows ld_out values apart (a multiple of 8, the first on a 16-byte boundary): softmax(q k^T * scale) v per head.
+// int8 != 0: SageAttention (K mean removal, int8 Q K^T). `scratch`: b200_attn_fa_workspace_bytes bytes.
+B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out, long long ld_out, int sq, int sk,
+                          int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
+  if (sq <= 0 || sk <= 0) return 0;
+  const bool direct = fa_direct(v);
+  const FaScratch sc = fa_scratch(heads, sq, sk, int8, direct);
   if (scratch == nullptr && sc.total > 0) return -2;
   if (ld_out % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15)) return -2;
   const long long ld = static_cast<long long>(heads) * kFaD;
   uint8_t* base = static_cast<uint8_t*>(scratch);
   const int sk_pad64 = fa_pad(sk, 64);
-  dim3 tgrid((sk_pad64 + 63) / 64, kFaD / 64, batch * heads);
+  dim3 tgrid((sk_pad64 + 63) / 64, kFaD / 64, heads);
   if (!direct) fa_transpose_v_kernel<<<tgrid, dim3(32, 8), 0, stream>>>(static_cast<const __nv_bfloat16*>(v),
                                                            reinterpret_cast<__nv_bfloat16*>(base + sc.vt), ld, sk,
                                                            sk_pad64, heads);
   FaParams p{};
   p.out = static_cast<__nv_bfloat16*>(out);
   p.ld_out = ld_out;
-  p.sq = sq; p.sk = sk; p.heads = heads; p.batch = batch;
+  p.sq = sq; p.sk = sk; p.heads = heads; p.batch = 1;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = static_cast<DeviceStatus*>(status);
   p.n_tiles = fa_pad(sk, 128) / 128;
@@ -915,43 +914,32 @@ static int fa_dense(const void* q, const void* k, const void* v, void* out, long
     float* ksum = reinterpret_cast<float*>(base + sc.ksum);
     float* qs = reinterpret_cast<float*>(base + sc.qs);
     float* ks = reinterpret_cast<float*>(base + sc.ks);
-    if (cudaMemsetAsync(ksum, 0, static_cast<size_t>(batch) * heads * kFaD * 4, stream) != cudaSuccess) return -3;
-    sage_k_sum_kernel<<<dim3((sk + 255) / 256, batch * heads), 128, 0, stream>>>(
+    if (cudaMemsetAsync(ksum, 0, static_cast<size_t>(heads) * kFaD * 4, stream) != cudaSuccess) return -3;
+    sage_k_sum_kernel<<<dim3((sk + 255) / 256, heads), 128, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(k), ksum, ld, sk, heads);
-    const long long wq = static_cast<long long>(batch) * sq * heads;
+    const long long wq = static_cast<long long>(sq) * heads;
     sage_quant_rows_kernel<<<static_cast<unsigned>((wq + 7) / 8), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(q), reinterpret_cast<int8_t*>(base + sc.q8), qs, nullptr, 1.f, ld, sq, sq_pad,
-        heads, batch);
-    sage_quant_k_tiles_kernel<<<dim3(n_tiles, batch * heads), 256, 0, stream>>>(
+        heads, 1);
+    sage_quant_k_tiles_kernel<<<dim3(n_tiles, heads), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(k), reinterpret_cast<int8_t*>(base + sc.k8), ks, ksum, ld, sk, heads);
     p.q_scale = qs;
     p.k_scale = ks;
     p.sq_pad = sq_pad;
-    rc = make_kmajor_map(&tq, base + sc.q8, 1, static_cast<long long>(batch) * sq, ld, ld, 128);
+    rc = make_kmajor_map(&tq, base + sc.q8, 1, sq, ld, ld, 128);
     if (rc) return rc;
-    rc = make_kmajor_map(&tk, base + sc.k8, 1, static_cast<long long>(batch) * sk, ld, ld, 128);
+    rc = make_kmajor_map(&tk, base + sc.k8, 1, sk, ld, ld, 128);
     if (rc) return rc;
   } else {
-    rc = make_kmajor_map(&tq, q, 2, static_cast<long long>(batch) * sq, ld, ld, 128);
+    rc = make_kmajor_map(&tq, q, 2, sq, ld, ld, 128);
     if (rc) return rc;
-    rc = make_kmajor_map(&tk, k, 2, static_cast<long long>(batch) * sk, ld, ld, 128);
+    rc = make_kmajor_map(&tk, k, 2, sk, ld, ld, 128);
     if (rc) return rc;
   }
   rc = direct ? make_kmajor_map(&tv, v, 2, sk, ld, ld, 128)
-              : make_kmajor_map(&tv, base + sc.vt, 2, static_cast<long long>(batch) * heads * kFaD, sk_pad64, sk_pad64, 128);
+              : make_kmajor_map(&tv, base + sc.vt, 2, static_cast<long long>(heads) * kFaD, sk_pad64, sk_pad64, 128);
   if (rc) return rc;
-  return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads, batch), int8, stream, nullptr, direct);
-}
-
-B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out, int batch, int sq, int sk,
-                          int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
-  return fa_dense(q, k, v, out, static_cast<long long>(heads) * kFaD, batch, sq, sk, heads, scale, int8, scratch, status, stream);
-}
-
-// The same with rows of the output ld_out values apart (a multiple of 8, the first on a 16-byte boundary).
-B200_API int b200_attn_fa_ld(const void* q, const void* k, const void* v, void* out, long long ld_out, int batch, int sq, int sk,
-                             int heads, float scale, int int8, void* scratch, void* status, cudaStream_t stream) {
-  return fa_dense(q, k, v, out, ld_out, batch, sq, sk, heads, scale, int8, scratch, status, stream);
+  return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads), int8, stream, nullptr, direct);
 }
 
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,

@@ -651,9 +651,9 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
         # long bidirectional sequences (DiT blocks): two query tiles per CTA, S / P / O in TMEM
         L = N.lib()
         i8 = int(config.get("sage_attention") if int8 is None else int8)
-        ws = N.state(q.device).scratch(L.b200_attn_fa_workspace_bytes(1, hq, tq, tk, i8, v.data_ptr()))
-        rc = L.b200_attn_fa_ld(q.data_ptr(), k.data_ptr(), v.data_ptr(), dst.data_ptr(), hq * d if out is None else out.stride(0),
-                               1, tq, tk, hq, float(scale), i8, ws.data_ptr(), N.state(q.device).status.data_ptr(), N.stream())
+        ws = N.state(q.device).scratch(L.b200_attn_fa_workspace_bytes(hq, tq, tk, i8, v.data_ptr()))
+        rc = L.b200_attn_fa(q.data_ptr(), k.data_ptr(), v.data_ptr(), dst.data_ptr(), hq * d if out is None else out.stride(0),
+                            tq, tk, hq, float(scale), i8, ws.data_ptr(), N.state(q.device).status.data_ptr(), N.stream())
         N.check(rc, "b200_attn_fa", (4 if i8 else 1) + (v.data_ptr() % 16 != 0))
         return dst
     if dense_tc:
