@@ -2059,6 +2059,21 @@ B200_API int b200_gemm(const void* x, const void* w, void* out, int m, int n, in
                    act, splits, workspace, workspace_bytes, status, stream, nullptr);
 }
 
+// Form of act(x w_gate^T) * (x w_up^T) with f features of either: 1 = b200_gemv_glu, 2 = b200_gemm_glu, 0 = the product and
+// then b200_glu. dtype 0 (bf16) or 2 (UE8M0 fp8 with fp8 result). A handful of tokens: where the product itself leaves the
+// tensor core (1 x 9728 x 896 6.6 -> 5.1 us against the two kernels, 2 x 28672 x 4096 43.0 -> 41.0, 4 x 9728 x 896 10.5
+// both). Many: whole tiles only, from three full waves (bf16 512 x 28672 x 4096 170 -> 118 us, 8192 x 28672 x 4096 1609 ->
+// 1402, fp8 8192 x 57344 x 8192 3740 -> 3287), and from two where the plain product would not cut its last wave along K
+// (1187 x 9728 x 896 46 -> 40; swept from 376 to 690 tiles at depths 1024 to 8192, never slower). One wave and a half lost
+// (bf16 129 x 28672 x 4096 69.3 -> 71.4).
+B200_API int b200_glu_form(int m, int f, int k, int dtype) {
+  if (m < 1 || f < 1 || k < 1) return 0;
+  if (f <= (1 << 30) && f % 8 == 0 && handful(m, 2 * f, k, dtype)) return 1;
+  if (m <= 128 || f % 128 != 0 || (dtype != 0 && dtype != 2)) return 0;
+  const long long tiles = (m + 127ll) / 128 * (f / 128), full = tiles / num_sms(), rest = tiles % num_sms();
+  return full >= 3 || (full == 2 && (rest == 0 || 2 * rest > num_sms())) ? 2 : 0;
+}
+
 // The first half of a gated feed-forward for more than 128 tokens in one launch: act(x w_gate^T) * (x w_up^T) for w [2f][k],
 // gate rows first. dtype 0: bf16 operands, out [m][ldc] bf16; dtype 2: e4m3 operands with UE8M0 scales, result as
 // e4m3 [m][f] (out_q) with 1x128 scales in the blocked layout of sf_rows rows per block (out_sf). A tile reads 128 gate

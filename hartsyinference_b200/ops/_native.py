@@ -82,6 +82,7 @@ _SIGNATURES = {
     "b200_delta": (i32, [vp] * 13 + [i32] * 9 + [i64, i32, i64, i32, f32, i32, vp]),
     "b200_attn_biased": (i32, [vp] * 7 + [i32] * 10 + [vp, f32, f32, i32, i32, vp, i32, vp, vp, i64, i64, i32, i32, vp, i32, i64, vp]),
     "b200_kv_store": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i32, vp]),
+    "b200_glu_form": (i32, [i32, i32, i32, i32]),
     "b200_gemm_glu": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp, vp, i32, i32, vp, vp]),
     "b200_gemv_glu": (i32, [vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp]),
     "b200_norm": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32, i32, vp, i32, i32, vp]),

@@ -429,46 +429,34 @@ def glu(x: torch.Tensor, act: str = "silu", emit_fp8: bool = False, emit_bf16: b
 
 def linear_glu(x, w: LinearWeight, act: str = "silu", emit_fp8: bool = False, emit_bf16: bool = True):
     """``glu(linear(x, w), act)``; ``x`` bf16 or :class:`Fp8Act`. A handful of rows with bf16 weights is one kernel, in
-    which neither product is rounded (the sizes at which ``linear`` leaves the tensor core, see b200_gemm); decode-size
+    which neither product is rounded (the sizes at which ``linear`` leaves the tensor core, see b200_glu_form); decode-size
     batches leave the K ranges of the product to the activation kernel; large batches (bf16, or UE8M0 fp8 with fp8 result) keep
     both products in the tensor core's tile."""
-    bf16 = isinstance(w, LinearWeight) and not w.is_fp8 and isinstance(x, torch.Tensor) and x.is_cuda and w.bias is None
-    if bf16 and not emit_fp8 and act in ("silu", "gelu_tanh"):
-        m, k = x.shape
-        n = w.weight.shape[0]
-        # 1 x 9728 x 896 6.6 -> 5.1 us against the two kernels, 2 x 28672 x 4096 43.0 -> 41.0, 4 x 9728 x 896 10.5 both
-        if ((m == 1 or (m == 2 and k <= 8192) or (m <= 4 and n * k <= 1 << 23)) and k % 8 == 0 and n % 16 == 0
-                and w.weight.shape[1] == k and x.dtype == torch.bfloat16 and x.stride(1) == 1
-                and w.weight.stride(1) == 1 and (x.stride(0) | w.weight.stride(0)) % 8 == 0 and (x.data_ptr() | w.weight.data_ptr()) % 16 == 0):
-            y = torch.empty(m, n // 2, dtype=torch.bfloat16, device=x.device)
-            N.check(N.lib().b200_gemv_glu(x.data_ptr(), w.weight.data_ptr(), y.data_ptr(), m, n // 2, k, x.stride(0), w.weight.stride(0),
-                                          n // 2, 0 if act == "silu" else 1, N.stream()), "b200_gemv_glu")
-            return y, None
     xd = x.data if isinstance(x, Fp8Act) else x
-    mx = (isinstance(w, LinearWeight) and w.is_mx and isinstance(x, Fp8Act) and x.sf is not None and x.tile_rows == 128
-          and emit_fp8 and not emit_bf16)
-    if ((mx or (bf16 and not emit_fp8)) and xd.is_cuda and xd.shape[0] > 128 and w.bias is None
-            and xd.dtype == (torch.uint8 if mx else torch.bfloat16) and act in ("silu", "gelu_tanh")):
-        m, k = xd.shape
-        f = w.weight.shape[0] // 2
-        # Whole tiles only: from three full waves (bf16 512 x 28672 x 4096 170 -> 118 us, 8192 x 28672 x 4096 1609 -> 1402, fp8
-        # 8192 x 57344 x 8192 3740 -> 3287), and from two where the plain product would not cut its last wave along K
-        # (1187 x 9728 x 896 46 -> 40; swept from 376 to 690 tiles at depths 1024 to 8192, never slower). One wave and a half
-        # lost (bf16 129 x 28672 x 4096 69.3 -> 71.4).
-        full, rest = divmod((m + 127) // 128 * (f // 128), 148)
-        if (w.weight.shape[0] % 256 == 0 and w.weight.shape[1] == k and (full >= 3 or (full == 2 and (rest == 0 or rest > 74)))
-                and xd.stride(1) == 1 and w.weight.stride(1) == 1):
-            y = q = sf = None
-            if mx:
-                q, sf = torch.empty(m, f, dtype=torch.uint8, device=xd.device), _alloc_sf(m, f, 128, xd.device)
-            else:
-                y = torch.empty(m, f, dtype=torch.bfloat16, device=xd.device)
-            xs, ws = _scale_ptrs(x, w)
-            rc = N.lib().b200_gemm_glu(xd.data_ptr(), w.weight.data_ptr(), N.ptr(y), N.ptr(q), N.ptr(sf), m, f, k, xd.stride(0), w.weight.stride(0),
-                                       f, 2 if mx else 0, xs, ws, 0 if act == "silu" else 1, 128, N.state(xd.device).status.data_ptr(), N.stream())
-            if rc != -12:                                # -12: sizes or alignments that it does not take
-                N.check(rc, "b200_gemm_glu")
-                return y, (Fp8Act(q, None, sf, 128) if mx else None)
+    form = 0
+    if (isinstance(w, LinearWeight) and w.bias is None and act in ("silu", "gelu_tanh") and xd.is_cuda and w.weight.shape[0] % 2 == 0
+            and w.weight.shape[1] == xd.shape[1] and xd.stride(1) == 1 and w.weight.stride(1) == 1):
+        mx = w.is_mx and isinstance(x, Fp8Act) and x.sf is not None and x.tile_rows == 128 and emit_fp8 and not emit_bf16
+        if mx or (not w.is_fp8 and x is xd and x.dtype == torch.bfloat16 and not emit_fp8):
+            (m, k), f = xd.shape, w.weight.shape[0] // 2
+            form = N.lib().b200_glu_form(m, f, k, 2 if mx else 0)
+    if form == 1 and (x.stride(0) | w.weight.stride(0)) % 8 == 0 and (x.data_ptr() | w.weight.data_ptr()) % 16 == 0:
+        y = torch.empty(m, f, dtype=torch.bfloat16, device=x.device)
+        N.check(N.lib().b200_gemv_glu(x.data_ptr(), w.weight.data_ptr(), y.data_ptr(), m, f, k, x.stride(0), w.weight.stride(0),
+                                      f, 0 if act == "silu" else 1, N.stream()), "b200_gemv_glu")
+        return y, None
+    if form == 2:
+        y = q = sf = None
+        if mx:
+            q, sf = torch.empty(m, f, dtype=torch.uint8, device=xd.device), _alloc_sf(m, f, 128, xd.device)
+        else:
+            y = torch.empty(m, f, dtype=torch.bfloat16, device=xd.device)
+        xs, ws = _scale_ptrs(x, w)
+        rc = N.lib().b200_gemm_glu(xd.data_ptr(), w.weight.data_ptr(), N.ptr(y), N.ptr(q), N.ptr(sf), m, f, k, xd.stride(0), w.weight.stride(0),
+                                   f, 2 if mx else 0, xs, ws, 0 if act == "silu" else 1, 128, N.state(xd.device).status.data_ptr(), N.stream())
+        if rc != -12:                                # -12: alignments that it does not take
+            N.check(rc, "b200_gemm_glu")
+            return y, (Fp8Act(q, None, sf, 128) if mx else None)
     return glu(linear(x, w, defer=xd.is_cuda and xd.shape[0] <= 128), act, emit_fp8=emit_fp8, emit_bf16=emit_bf16)
 
 
