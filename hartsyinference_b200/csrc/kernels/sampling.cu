@@ -15,7 +15,7 @@
 // the row, histograms and prefix sums met through distributed shared memory. Longer rows go through one block that makes
 // eight passes over a row in L2, and so do short rows and many rows of moderate length, where the exchanges of a
 // cluster cost more than the passes (see b200_sample). Both forms sum masses in 2^-40, so a row's token is the
-// same whatever batch it comes in (fp32 sums in the one block drew other tokens than the cluster in one of 50 flat rows of 100000).
+// same whatever batch it comes in (fp32 sums in the one block drew another token than the cluster in two or three of 1000 flat rows of 100000).
 //
 // The reference applies the same chain on the host, one request at a time, after copying the logits
 // back (src/HartsyInference.LLM/Sampling/SamplerChain.cs:26-85, TopKSampler.cs, TopPSampler.cs,

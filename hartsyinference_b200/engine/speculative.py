@@ -5,7 +5,10 @@ recent match first, within ``lookback`` tokens) and the tokens that followed the
 proposed. One forward pass over ``[last token, draft...]`` (causal, on top of the cached prefix)
 verifies the whole draft: position i's greedy token must equal draft token i. The accepted prefix
 plus the first correction are kept; the KV entries of rejected positions are cut off with the
-allocator's ``truncate``. Outputs are identical to plain greedy decoding of the same model.
+allocator's ``truncate``. Every kept token is the greedy token of the same model at its position. A pass over several
+tokens takes other kernels on the device than a decode step (attention of a chunk, products of more rows), which
+round differently, so where two logits are that close together plain greedy decoding may keep the other one; on
+the host the outputs are identical.
 
 Reference behaviour: src/HartsyInference.LLM/Generation/TextGenerationPipeline.cs
 (GenerateSpeculative:403-463; n-gram 3, draft length 8, look-back 4096).

@@ -79,3 +79,9 @@ def test_argmax_of_rows_without_a_finite_value(vocab, pitch, dtype):
     p = SamplingParams(greedy=True, logits_mask=lambda history: torch.zeros(vocab, dtype=torch.bool))
     lg = torch.randn(vocab)
     assert sample_row(lg.cuda(), p, [], None) == sample_row(lg, p, [], None) == 0      # a grammar that allows nothing
+
+
+def test_gated_product_of_no_rows():
+    w = ops.LinearWeight(torch.randn(512, 256, device="cuda").to(torch.bfloat16))
+    y, q = ops.linear_glu(torch.empty(0, 256, device="cuda", dtype=torch.bfloat16), w)
+    assert tuple(y.shape) == (0, 256) and q is None
