@@ -650,14 +650,13 @@ B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows,
   // 105 us however short its rows are, and 37 of them (18 of the widest) fill the machine; from 16 to 40 values a thread a
   // wave gets up to 1.4 times longer. Which filters a row asks for is known on the device only: with every one (us, block /
   // cluster) 1 x 4096 34 / 54, 1 x 16384 69 / 54, 64 x 32000 121 / 208, 64 x 65536 252 / 214, 512 x 4096 136 / 1549,
-  // 128 x 100352 349 / 489, 128 x 202048 686 / 774; without filters 64 x 32000 32 / 18, 128 x 100352 74 / 73; greedy rows leave a
-  // wave of clusters early, while a wave of blocks waits for its slowest. So clusters may be up to 1.35 times the slower
-  // by the full chain.
+  // 128 x 100352 349 / 489, 128 x 202048 686 / 774, 148 x 128256 460 / 587; without filters 64 x 32000 32 / 18, 128 x 100352
+  // 74 / 73. The full chain, the longest a batch can take, decides.
   const int sms = num_sms(), per_wave = (each <= 40 ? 2 * sms : sms) / kRowBlocks;
   const double block_us = (24. + vocab / 350.) * ((rows + sms - 1) / sms);
   const double cluster_us = rows <= 8 ? 58. : 2 * rows <= per_wave ? 75. :
       105. * ((rows + per_wave - 1) / per_wave) * (each > 16 && each <= 40 ? 1. + (each - 16) / 64. : 1.);
-  if (rows < (1 << 27) && per_wave > 0 && cluster_us <= 1.35 * block_us) {
+  if (rows < (1 << 27) && per_wave > 0 && cluster_us <= block_us) {
     if (each <= 8) return launch_rows<8>(p, rows, stream);
     if (each <= 16) return launch_rows<16>(p, rows, stream);
     if (each <= 32) return launch_rows<32>(p, rows, stream);
