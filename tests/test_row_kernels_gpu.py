@@ -92,3 +92,16 @@ def test_dit_qkv_forms(tokens, hq, hkv, d, row_norm):
     for g, o, r in zip(got, out, ref):
         assert g.data_ptr() == o.data_ptr()
         assert torch.allclose(g.float().cpu(), r.float(), rtol=2 ** -6, atol=2 ** -6)
+
+
+@pytest.mark.parametrize("rows,f", [(1, 40), (5, 64), (1183, 64), (1185, 72), (2369, 128), (9473, 384), (37889, 128)])
+def test_narrow_rows_share_a_block(rows, f):
+    torch.manual_seed(rows)
+    x, n8 = _rand(rows, 2 * f, scale=3.0), f % 128 == 0
+    y, q = ops.glu(x, "silu", emit_fp8=n8)
+    assert torch.allclose(y.float().cpu(), R.glu(x.cpu(), "silu"), rtol=2 ** -7, atol=1e-5)
+    if n8:
+        again = ops.quant_fp8_act(y)
+        qr, sr = R.quant_fp8_act(y.cpu(), pow2=q.sf is not None)
+        assert torch.equal(q.data, again.data) and torch.equal(q.scales_fp32(), again.scales_fp32())
+        assert torch.equal(again.data.cpu(), qr) and torch.equal(again.scales_fp32().cpu(), sr)
