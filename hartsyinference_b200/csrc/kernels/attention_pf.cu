@@ -25,6 +25,7 @@
 
 namespace b200 {
 
+int num_sms();      // of the current device, see gemm_tcgen05.cu
 int make_kmajor_map(CUtensorMap* out, const void* base, int elem_bytes, long long rows, long long k, long long ld, int box_rows);
 
 constexpr int kPfD = 128;
@@ -367,11 +368,11 @@ attn_prefill_tc_kernel(const PfParams p, const __grid_constant__ CUtensorMap tm_
 using namespace b200;
 
 // q, out [total_q][hq][128] bf16; k_pool, v_pool [pages][hkv][page][128] bf16; block_table [seqs][max_pages], kv_lens [seqs]
-// and cu_q [seqs + 1] int32 on the device. Causal, scale > 0; page of 8, 16, 32 or 64 rows. Returns -2 .. -6 for
-// what it does not take.
+// and cu_q [seqs + 1] int32 on the device. Causal, scale > 0; page of 8, 16, 32 or 64 rows; max_kv_len: no sequence has
+// more keys. Returns -2 .. -6 for what it does not take, 1 (nothing launched) where b200_attn_prefill is faster.
 B200_API int b200_attn_prefill_tc(const void* q, const void* k_pool, const void* v_pool, void* out, const int* block_table,
                                   const int* kv_lens, const int* cu_q, int seqs, int total_q, int max_q_len, int hq, int hkv,
-                                  int page, int max_pages, long long pages, float scale, void* status, cudaStream_t stream) {
+                                  int page, int max_pages, long long pages, int max_kv_len, float scale, void* status, cudaStream_t stream) {
   if (seqs <= 0 || max_q_len <= 0 || total_q <= 0) return 0;
   if (hkv <= 0 || hq % hkv != 0) return -3;
   PfParams p{};
@@ -387,6 +388,17 @@ B200_API int b200_attn_prefill_tc(const void* q, const void* k_pool, const void*
   p.pool_rows = static_cast<int>(rows);
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = static_cast<DeviceStatus*>(status);
+  const int rows_each = p.pair_heads ? kPfTile : 2 * kPfTile;
+  const int q_tiles = (max_q_len + rows_each - 1) / rows_each;
+  if (q_tiles > 65535) return -5;
+  // A block fills a processor and starts up for 7.5 us before its keys (0.015 us each) count; b200_attn_prefill has several small
+  // blocks of 64 rows and one head on a processor, 1.6 us each and 0.028 us a key, and takes at least 4.7 us and 0.045 us a
+  // key. So it stays faster for short prompts (32 heads on 8, this / that: 17 tokens 11.4 / 6.6 us, 64 10.8 / 7.3, 100 of 5 behind
+  // 10 98 / 53; 8 heads 64 of 64 behind 64 31 / 23) and slower from about 150 keys on (9 behind 400 17 / 24).
+  const double sms = num_sms(), keys = max_kv_len;
+  const double here = 2.5 + ((static_cast<long long>(p.pair_heads ? hq / 2 : hq) * q_tiles * seqs + num_sms() - 1) / num_sms()) * (7.5 + 0.015 * keys);
+  const double rows_us = (static_cast<double>((max_q_len + 63) / 64) * hq * seqs / sms) * (1.6 + 0.028 * keys);
+  if (fmax(4.7 + 0.045 * keys, rows_us) < here) return 1;
   CUtensorMap tq, tk, tv;
   int rc = make_kmajor_map(&tq, q, 2, total_q, static_cast<long long>(hq) * kPfD, static_cast<long long>(hq) * kPfD, kPfTile);
   if (rc == 0) rc = make_kmajor_map(&tk, k_pool, 2, rows, kPfD, kPfD, page);
@@ -397,9 +409,6 @@ B200_API int b200_attn_prefill_tc(const void* q, const void* k_pool, const void*
   if (configured.first_time() &&
       cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return -200;
-  const int rows_each = p.pair_heads ? kPfTile : 2 * kPfTile;
-  const int q_tiles = (max_q_len + rows_each - 1) / rows_each;
-  if (q_tiles > 65535) return -5;
   attn_prefill_tc_kernel<<<dim3(p.pair_heads ? hq / 2 : hq, q_tiles, seqs), kPfThreads, smem, stream>>>(p, tq, tk, tv);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 300;

@@ -726,7 +726,7 @@ class DecoderModel:
         else:
             att = ops.attn_prefill_paged(q, kc, vc, batch.block_table, batch.kv_lens, batch.cu_q,
                                          batch.max_q_len, causal=True, scale=scale,
-                                         softcap=cfg.attn_softcap, window=window)
+                                         softcap=cfg.attn_softcap, window=window, max_kv_len=batch.max_kv_len or None)
         return att.reshape(t, self.hq * d)
 
     def _mrope(self, qkv: torch.Tensor, positions3: torch.Tensor, inv_freq: torch.Tensor) -> torch.Tensor:

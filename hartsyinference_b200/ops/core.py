@@ -579,9 +579,10 @@ def attn_paged_biased(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 def attn_prefill_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                        block_table: torch.Tensor, kv_lens: torch.Tensor, cu_q: torch.Tensor,
                        max_q_len: int, causal: bool = True, scale: Optional[float] = None,
-                       softcap: float = 0.0, window: int = 0) -> torch.Tensor:
+                       softcap: float = 0.0, window: int = 0, max_kv_len: Optional[int] = None) -> torch.Tensor:
     """Variable-length (chunked) prefill: q [total_q, hq, d] packed by cu_q; keys come from the page
-    pool and include any cached prefix (kv_lens[i] >= q_len[i])."""
+    pool and include any cached prefix (kv_lens[i] >= q_len[i]). ``max_kv_len``: the longest of them, where the host
+    knows it (the width of the block table otherwise); it chooses between two kernels, nothing else."""
     tq, hq, d = q.shape
     hkv, page = k_cache.shape[1], k_cache.shape[2]
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
@@ -601,10 +602,12 @@ def attn_prefill_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
             and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16 == 0):
         rc = N.lib().b200_attn_prefill_tc(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                           block_table.data_ptr(), kv_lens.data_ptr(), cu_q.data_ptr(), nseq, tq, max_q_len, hq, hkv,
-                                          page, block_table.shape[1], k_cache.shape[0], scale,
+                                          page, block_table.shape[1], k_cache.shape[0],
+                                          max_kv_len or block_table.shape[1] * page, scale,
                                           N.state(q.device).status.data_ptr(), N.stream())
-        N.check(rc, "b200_attn_prefill_tc")
-        return out
+        if rc != 1:                                      # 1: short prompts, for which the kernel below is faster
+            N.check(rc, "b200_attn_prefill_tc")
+            return out
     rc = N.lib().b200_attn_prefill(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                    block_table.data_ptr(), kv_lens.data_ptr(), cu_q.data_ptr(), None,
                                    nseq, max_q_len, 0, 0, hq, hkv, d, page, block_table.shape[1], 1,

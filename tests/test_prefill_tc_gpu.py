@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
     (16, [(1, 1), (127, 127), (128, 128), (129, 129), (300, 300)]),     # (query tokens, keys): ends of query tiles
     (16, [(1, 128), (1, 129), (2, 257), (64, 500), (257, 1000)]),       # chunks behind a cached prefix, ends of key tiles
     (8, [(17, 41), (130, 136)]), (32, [(256, 256), (33, 97)]), (64, [(5, 5), (200, 391)])])
-def test_against_fp32(hq, hkv, page, lens):
+@pytest.mark.parametrize("most", [1 << 16, None])                     # keys that a sequence may have: tcgen05 at any size, or as sizes have it
+def test_against_fp32(hq, hkv, page, lens, most):
     torch.manual_seed(len(lens) + page + hq)
     d = 128
     need = [(n + page - 1) // page for _, n in lens]
@@ -37,7 +38,7 @@ def test_against_fp32(hq, hkv, page, lens):
     q = torch.randn(sum(q_lens), hq, d).to(torch.bfloat16)
     cu = torch.tensor([0] + q_lens).cumsum(0).to(torch.int32)
     out = ops.attn_prefill_paged(q.cuda(), kc, vc, table.cuda(), torch.tensor([n for _, n in lens], dtype=torch.int32, device="cuda"),
-                                 cu.cuda(), max(q_lens)).float().cpu()
+                                 cu.cuda(), max(q_lens), max_kv_len=most).float().cpu()
     for i in range(len(lens)):
         ref = R.attention(q[cu[i]:cu[i + 1]], keys[i], values[i], causal=True).float()
         got = out[cu[i]:cu[i + 1]]
