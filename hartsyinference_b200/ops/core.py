@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 from dataclasses import dataclass
 from typing import Optional
@@ -271,6 +272,12 @@ def _scale_ptrs(x, w: LinearWeight):
     return x.scale.data_ptr(), w.scale.data_ptr()
 
 
+@functools.lru_cache(maxsize=4096)
+def _deferred_plan(m: int, n: int, k: int, dtype: int, workspace_bytes: int, device: int) -> int:
+    """The policy for a product of these sizes, which asking again would cost 1 us of every small product."""
+    return N.lib().b200_gemm_deferred_plan(m, n, k, dtype, workspace_bytes)
+
+
 def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.Tensor] = None,
            residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
            splits: Optional[int] = None, defer: bool = False, act_from: int = 0, defer_bias: bool = False):
@@ -320,14 +327,15 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
     ws = st.gemm_workspace()
     xs_ptr, ws_ptr = _scale_ptrs(x, w)
     if defer and m <= 128 and (w.bias is None or defer_bias) and act is None and gate is None and residual is None and splits is None:
-        plan = L.b200_gemm_deferred_plan(m, n, k, _gemm_dtype(w), ws.numel())
+        plan = _deferred_plan(m, n, k, _gemm_dtype(w), ws.numel(), xd.device.index)
         if plan:
             ranges, bn = plan & 0xffff, plan >> 16
             part = torch.empty((n + 127) // 128 * ranges * bn * 128, dtype=torch.float32, device=xd.device)
             rc = L.b200_gemm_deferred(xd.data_ptr(), w.weight.data_ptr(), m, n, k, xd.stride(0), w.weight.stride(0), _gemm_dtype(w), xs_ptr, ws_ptr,
                                       ws.data_ptr(), ws.numel(), part.data_ptr(), st.status.data_ptr(), N.stream())
-            N.check(rc, "b200_gemm_deferred")
-            return SplitSum(part, ranges, bn, (m, n), w.bias)
+            if rc != -13:                            # -13: the reduce form was switched since the plan was asked for
+                N.check(rc, "b200_gemm_deferred")
+                return SplitSum(part, ranges, bn, (m, n), w.bias)
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=xd.device)
     rc = L.b200_gemm(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k,
