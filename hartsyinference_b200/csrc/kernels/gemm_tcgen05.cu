@@ -1710,11 +1710,12 @@ int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long
               const void* bias, const void* gate, const void* residual, int act, cudaStream_t stream);
 
 // A handful of tokens with bf16 weights: a product on the ordinary cores that needs one launch and no scratch. One
-// token is faster at every size (28672 x 4096 44.2 -> 39.8 us, 896 x 896 6.4 -> 2.2 us), two up to a depth of 8192
-// (4096 x 14336 24.3 -> 27.1 us, taken back); three and four only where the launch, not the weights, is what
-// counts (896 x 4864 7.5 -> 6.1 us, 3072 x 3072 9.4 -> 9.3 us, 28672 x 4096 45 -> 67 us, taken back).
+// token and two are faster up to a depth of 8192 (28672 x 4096 44.2 -> 39.8 us, 896 x 896 6.4 -> 2.2 us; one of 8192 x 28672
+// 78 -> 101 us, of 3072 x 15360 18.0 -> 20.5, two of 4096 x 14336 24.3 -> 27.1); up to four where the launch, not the
+// weights, is what counts (one of 384 x 18432 11.3 -> 5.6 us, three of 896 x 4864 7.5 -> 6.1, 3072 x 3072 9.4 -> 9.3, but
+// 28672 x 4096 45 -> 67 us).
 static bool handful(int m, int n, int k, int dtype) {
-  return dtype == 0 && k % 8 == 0 && (m == 1 || (m == 2 && k <= 8192) || (m <= 4 && static_cast<long long>(n) * k <= 1ll << 23));
+  return dtype == 0 && k % 8 == 0 && ((m <= 2 && k <= 8192) || (m <= 4 && static_cast<long long>(n) * k <= 1ll << 23));
 }
 
 // K-split policy (see the header comment): tiles from first_split on are cut into `count` ranges of `kblocks` K blocks.
