@@ -874,10 +874,21 @@ B200_API int b200_norm(const void* x, const void* residual, void* residual_out, 
   p.sf_tile_rows = sf_tile_rows;
   p.vec_params = aligned16(weight, bias, shift, scale) && mod_stride % 8 == 0;
   const int nvec = dim / 8;
-  auto go = [&](auto* kernel, int per) {
-    launch_pdl(kernel, dim3(rows), dim3(((nvec + per - 1) / per + 31) / 32 * 32), 0, stream, p);
+  auto go = [&](auto* kernel, int per, int smem = 0) {
+    launch_pdl(kernel, dim3(rows), dim3(((nvec + per - 1) / per + 31) / 32 * 32), smem, stream, p);
   };
-  if (part_ws != nullptr) nvec > 1024 ? go(norm_kernel<2, true>, 2) : go(norm_kernel<1, true>, 1);
+  if (part_ws != nullptr) {
+    // Blocks of this launch start while the product runs, on the processors that it leaves free. Where those are few, they would
+    // take most of the rows and read their ranges alone (144 of 148 processors busy: 33 x 3072 x 3072 13.9 us with the reduce
+    // kernel, 15.9 so, 11.1 with one row a processor at a time). The shared memory is not used.
+    constexpr int kAlone = 116 * 1024;
+    static PerDeviceOnce configured;
+    if (configured.first_time() &&
+        (cudaFuncSetAttribute(norm_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone) != cudaSuccess ||
+         cudaFuncSetAttribute(norm_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone) != cudaSuccess))
+      return -4;
+    nvec > 1024 ? go(norm_kernel<2, true>, 2, kAlone) : go(norm_kernel<1, true>, 1, kAlone);
+  }
   else if (rows > 296 && nvec >= 1024) go(norm_kernel<4, false>, 4);
   else if (nvec > 1024 || (rows > 296 && nvec >= 256)) go(norm_kernel<2, false>, 2);
   else go(norm_kernel<1, false>, 1);
