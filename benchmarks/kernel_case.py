@@ -14,6 +14,8 @@
     python benchmarks/kernel_case.py qk_rope 8192 16 4
     python benchmarks/kernel_case.py general_delta 4 2048 16
     python benchmarks/kernel_case.py input_conv 8192 2048
+    python benchmarks/kernel_case.py attn_prompt 2048 6144 32 8
+    python benchmarks/kernel_case.py gated fp8 2048 14336 4096
 
 Inputs are larger than the L2 cache where the op is bandwidth bound but stay far below a few GB,
 so a full-metric capture (dozens of replays per launch) ends in about a minute. The status word is
@@ -172,6 +174,31 @@ def _attn_dense(argv):
     ms = _time(lambda: ops.attention(q, k, v, int8=mode == "fa8"))
     print(f"attention {mode}: {tokens} tokens x {heads} heads: {ms:.3f} ms, "
           f"{4.0 * tokens * tokens * 128 * heads / ms / 1e9:.0f} TFLOP/s")
+
+
+def _attn_prompt(argv):
+    """attn_prompt QUERIES CONTEXT HEADS KV_HEADS: causal attention of one prompt chunk behind CONTEXT cached tokens, pages of 16,
+    head dim 128; prints the device time and TFLOP/s of what the mask leaves."""
+    ql, ctx, hq, hkv = (int(v) for v in argv[:4])
+    pages = (ql + ctx + 15) // 16
+    q = torch.randn(ql, hq, 128, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn(pages, hkv, 16, 128, device="cuda").to(torch.bfloat16) for _ in range(2))
+    table = torch.randperm(pages, device="cuda").to(torch.int32)[None].contiguous()
+    lens, cu = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([ql + ctx], [0, ql]))
+    ms = _time(lambda: ops.attn_prefill_paged(q, kc, vc, table, lens, cu, ql))
+    print(f"prompt attention {ql} + {ctx}, {hq} heads on {hkv}: {ms * 1e3:.1f} us, {4.0 * ql * (ctx + (ql + 1) / 2) * 128 * hq / ms / 1e9:.0f} TFLOP/s")
+
+
+def _gated(argv):
+    """gated bf16|fp8 M F K: act(x w_gate^T) * (x w_up^T) in one launch, against the product and the activation kernel."""
+    fp8 = argv[0] == "fp8"
+    m, f, k = (int(v) for v in argv[1:4])
+    x = (torch.randn(m, k, device="cuda") * 0.5).to(torch.bfloat16)
+    lw = ops.LinearWeight.from_dense((torch.randn(2 * f, k, device="cuda") * 0.1).to(torch.bfloat16), fp8=fp8)
+    xin = ops.quant_fp8_act(x) if fp8 else x
+    one = _time(lambda: ops.linear_glu(xin, lw, emit_fp8=fp8, emit_bf16=not fp8))
+    two = _time(lambda: ops.glu(ops.linear(xin, lw), emit_fp8=fp8, emit_bf16=not fp8))
+    print(f"gated {argv[0]} {m}x{f}x{k}: {one * 1e3:.1f} us, {4.0 * m * f * k / one / 1e9:.0f} TFLOP/s; two kernels {two * 1e3:.1f} us")
 
 
 def _gemm_ar(argv):
@@ -446,7 +473,7 @@ def _input_conv(argv):
 
 CASES = {"general_delta": _general_delta, "input_conv": _input_conv, "qk_rope": _qk_rope, "latent_rot": _latent_rot, "channel_scan": _channel_scan, "head_scan": _head_scan, "latent": _latent, "delta": _delta, "attn_window": _attn_window, "mla_proj": _mla_proj, "gemm_ar_large": _gemm_ar_large, "ag_gemm": _ag_gemm, "ulysses": _ulysses, "allreduce": _allreduce, "sample": _sample,
          "int8": _int8, "triplane": _triplane,
-         "gemm_ar": _gemm_ar, "attn_dense": _attn_dense, "gemm": _gemm, "grouped": _grouped, "attn_decode": _attn_decode, "mla": _mla}
+         "attn_prompt": _attn_prompt, "gated": _gated, "gemm_ar": _gemm_ar, "attn_dense": _attn_dense, "gemm": _gemm, "grouped": _grouped, "attn_decode": _attn_decode, "mla": _mla}
 
 
 def main(argv=None) -> int:
