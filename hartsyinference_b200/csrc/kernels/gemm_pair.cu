@@ -1,0 +1,495 @@
+// Dense product of many tokens on CTA pairs (tcgen05 cta_group::2): C = A * B^T, tiles of 256 tokens x 256 features.
+//
+// Replaces the same calls of the reference as gemm_tcgen05.cu (src/HartsyInference.Cuda/CudaBackend.cs:1769-2425), for
+// sizes that give most of the processors a tile.
+//
+// Why pairs: a 128 x 256 tile of one SM takes 48 KB of operands from L2 for every 512 cycles of its tensor core
+// (96 bytes a cycle, more than an SM gets), so it ran at 0.6 of the core's rate in 8 and in 16 bits. Two SMs on one tile each
+// keep 128 rows of A and 128 rows of B, and the tensor cores read the other half of B from the neighbour's shared
+// memory: 32 KB for the same cycles, a third less, and a third less energy where the power limit holds the clock.
+//
+// Structure of one CTA (320 threads; persistent, pair i takes tiles i, i + pairs, ...):
+//   warp 0      one thread issues TMA loads of this CTA's 128 rows of either operand into its own shared memory; their
+//               bytes are counted on the barrier of the pair's first CTA
+//   warp 1      allocates TMEM; in the first CTA one thread issues tcgen05.mma (M = 256, N = 256) for both and
+//               commits to the barriers of both
+//   warps 2..9  epilogue of this CTA's 128 rows x 256 columns
+// Bound by the tensor core and the power limit: fp8 4096 x 9216 x 3072 116 -> 92 us (one-SM tiles before), 8192 x 8192 x
+// 28672 1691 -> 1317 us (2.9 PFLOP/s, then held by power), bf16 2048 x 28672 x 4096 gated 364 -> 300 us (1.6 PFLOP/s).
+// Two accumulators: the epilogue of a tile runs beside the products of the next. With scale factors in TMEM (8 bits)
+// 480 columns are left, so the two overlap by 32 columns, which the epilogue takes out first.
+#include "gemm_common.cuh"
+
+namespace b200 {
+
+constexpr int kPairStages = 6;
+constexpr int kPairBand = 8;                           // tiles of 256 tokens in a band: 74 tiles in flight cover 8 x 9 of them
+
+__device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+// Loads into this CTA's shared memory; the bytes are counted on `bar`, a shared::cluster address in either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int32_t c0, int32_t c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+// Arrival at a barrier of either CTA. What it announces are reads of TMEM, which tcgen05.wait::ld has seen done; a release at
+// cluster scope also waits for the thread's stores to global memory (1200 cycles behind the epilogue's).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pair_commit(uint64_t* bar, uint16_t ctas) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)),
+               "h"(ctas)
+               : "memory");
+}
+__device__ __forceinline__ void pair_cp_sf(uint32_t taddr, uint64_t sdesc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+// The issuing thread's own instructions bounded the 8-bit products (690 cycles a K block of four 128-cycle instructions), so
+// the descriptors' upper halves are constants and only the lower ones are counted on (see make_desc_sw128).
+#define B200_PAIR_DESCS                          \
+  "{\n\t"                                        \
+  ".reg .pred p;\n\t"                            \
+  ".reg .b64 da, db;\n\t"                        \
+  "mov.b64 da, {%1, 0x40004040};\n\t"            \
+  "mov.b64 db, {%2, 0x40004040};\n\t"            \
+  "setp.ne.b32 p, %4, 0;\n\t"
+__device__ __forceinline__ void pair_mma_bf16(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(B200_PAIR_DESCS "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(acc)
+               : "memory");
+}
+__device__ __forceinline__ void pair_mma_mx(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
+  asm volatile(B200_PAIR_DESCS "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], da, db, %3, [%5], [%6], p;\n\t}" ::"r"(d), "r"(a),
+               "r"(b), "r"(idesc), "r"(acc), "r"(sfa), "r"(sfb)
+               : "memory");
+}
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// 32 bytes a lane, one sector: what an epilogue of whole rows per lane writes without passing through shared memory, whose
+// 128 bytes a cycle the operands take (64 in by TMA, 64 out to the tensor core).
+__device__ __forceinline__ void store_words8(void* dst, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+__device__ __forceinline__ void load_words8(uint32_t* w, const void* src) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+               : "l"(src)
+               : "memory");
+}
+// Epilogue of 32 columns from b0 on (all of them there) of one row: bias, activation, gate and residual, rounded to bf16 pairs.
+__device__ __forceinline__ void finish_row32(const GemmParams& p, const uint32_t (&r)[32], int row, int b0, uint32_t (&out)[16]) {
+  uint32_t res[16];
+  const bool inside = row < p.rows_a;
+  if (p.residual && inside) {
+    const __nv_bfloat16* src = p.residual + static_cast<long long>(row) * p.ldc + b0;
+    load_words8(res, src);
+    load_words8(res + 8, src + 16);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float v[8], t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[q * 8 + j]);
+    if (p.bias) {
+      load_cols8(p.bias + b0 + q * 8, t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] += t[j];
+    }
+    if (b0 + q * 8 < p.act_col) {
+      // features ahead of the activation's first (a multiple of 8)
+    } else if (p.act == 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = gelu_tanh(v[j]);
+    } else if (p.act == 2) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = silu(v[j]);
+    } else if (p.act == 3) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = relu2(v[j]);
+    } else if (p.act == 4) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = tanhf(v[j]);
+    }
+    if (p.gate) {
+      load_cols8(p.gate + b0 + q * 8, t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] *= t[j];
+    }
+    if (p.residual && inside) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[2 * j] += __uint_as_float(res[q * 4 + j] << 16);
+        v[2 * j + 1] += __uint_as_float(res[q * 4 + j] & 0xffff0000u);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[q * 4 + j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+  }
+}
+
+struct alignas(16) PairBarriers {
+  uint64_t full[kPairStages], empty[kPairStages];        // full: counted in the first CTA of the pair; empty: in each
+  uint64_t tmem_full[2];             // in each
+  uint64_t tmem_empty[2], shared_empty[2];   // in the first: accumulator read; its columns that the other one shares read
+  uint64_t drain;
+  uint32_t tmem_base, abort_flag;
+  float amax[2][256];                // gated tiles: maxima of a row's two halves
+};
+
+template <int kMode>
+constexpr int pair_stage_bytes() { return 2 * kStageBytesA + (kMode == 2 ? 2048 : 0); }
+
+template <int kMode, bool kGlu>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+                 const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb) {
+  constexpr bool kMx = kMode == 2;
+  constexpr int kStages = kPairStages, kStageBytes = pair_stage_bytes<kMode>();
+  constexpr int kElems = kMx ? 128 : 64;               // K elements in one 128-byte swizzle atom
+  constexpr int kAccStride = kMx ? 224 : 256;          // first column of the second accumulator
+  constexpr uint32_t kSfCol = 480;
+  constexpr uint32_t kIdesc = kMx ? make_idesc_mx(256, 256) : make_idesc(256, 256, kFmtBf16, kFmtBf16);
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  PairBarriers* bars = reinterpret_cast<PairBarriers*>(smem + kStages * kStageBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int tiles_a = (p.rows_a + 255) / 256, kblocks = (p.k + kElems - 1) / kElems;
+  const int first = static_cast<int>(blockIdx.x >> 1), step = static_cast<int>(gridDim.x >> 1);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars->tmem_full[b], 1);
+      mbar_init(&bars->tmem_empty[b], 16);             // one arrival per epilogue warp of the pair
+      mbar_init(&bars->shared_empty[b], 8);            // per warp that holds a shared chunk
+    }
+    mbar_init(&bars->drain, 1);
+    bars->abort_flag = 0;
+    fence_mbar_init();
+    prefetch_tensormap(&tm_a);
+    prefetch_tensormap(&tm_b);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                                  // the barriers of both CTAs are set up
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  volatile uint32_t* abort_flag = &bars->abort_flag;
+  pdl_trigger();
+
+  auto tile_of = [&](int w, int& ta, int& tb) {        // as in decode_item of gemm_tcgen05.cu
+    const int per = kPairBand * (p.num_tiles / tiles_a), b = w / per, r = w - b * per;
+    const int width = min(kPairBand, tiles_a - b * kPairBand);
+    tb = r / width;
+    ta = b * kPairBand + (r - tb * width);
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      pdl_wait();
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      long long issued = 0;
+      for (int w = first; w < p.num_tiles && ok; w += step) {
+        int ta, tb;
+        tile_of(w, ta, tb);
+        const int a_row = ta * 256 + static_cast<int>(rank) * 128;
+        const int b_row = kGlu ? tb * 128 + static_cast<int>(rank) * p.glu_f : tb * 256 + static_cast<int>(rank) * 128;
+        const int sfa = (2 * ta + static_cast<int>(rank)) * p.sf_kgroups;
+        const int sfb0 = (kGlu ? tb : 2 * tb) * p.sf_kgroups, sfb1 = (kGlu ? tb + (p.glu_f >> 7) : 2 * tb + 1) * p.sf_kgroups;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&bars->empty[s], ph ^ 1, abort_flag)) {
+            report_status(p.status, kWaitTimeout, kKernelGemm, 21, blockIdx.x);
+            ok = false;
+            break;
+          }
+          uint8_t* sa = smem + s * kStageBytes;
+          const uint32_t bar = map_to_rank(&bars->full[s], 0);
+          const bool with_sf = kMx && (kb & 3) == 0;   // a stage that starts a group of four K blocks carries their scale factors
+          if (rank == 0) mbar_arrive_expect_tx(&bars->full[s], 2 * (2 * kStageBytesA + (with_sf ? 1536 : 0)));
+          if (with_sf) {
+            uint8_t* sf = sa + 2 * kStageBytesA;
+            tma_load_2d_pair(sf, &tm_sfa, bar, 0, sfa + (kb >> 2));
+            tma_load_2d_pair(sf + 512, &tm_sfb, bar, 0, sfb0 + (kb >> 2));
+            tma_load_2d_pair(sf + 1024, &tm_sfb, bar, 0, sfb1 + (kb >> 2));
+          }
+          tma_load_2d_pair(sa, &tm_a, bar, kb * kElems, a_row);
+          tma_load_2d_pair(sa + kStageBytesA, &tm_b, bar, kb * kElems, b_row);
+          ++issued;
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+      }
+      if (!ok && rank == 0) {
+        // let the copies in flight land before the CTAs leave
+        for (int i = 0; i < kStages && i < issued; ++i) {
+          int ss = s - 1 - i;
+          uint32_t pp = ph;
+          if (ss < 0) { ss += kStages; pp ^= 1; }
+          uint32_t dummy = 0;
+          mbar_wait(&bars->full[ss], pp, &dummy, 4000000ll);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0 && rank == 0) {
+      pdl_wait();
+      const uint32_t smem_base = smem_u32(smem);
+      int s = 0, t = 0;
+      uint32_t ph = 0;
+      bool ok = true, issued_any = false;
+      for (int w = first; w < p.num_tiles && ok; w += step, ++t) {
+        const int b = t & 1;
+        if (!mbar_wait(&bars->tmem_empty[b], ((t >> 1) & 1) ^ 1, abort_flag) ||
+            (kMx && t > 0 && !mbar_wait(&bars->shared_empty[b ^ 1], ((t - 1) >> 1) & 1, abort_flag))) {
+          report_status(p.status, kWaitTimeout, kKernelGemm, 22, blockIdx.x);
+          ok = false;
+          break;
+        }
+        const uint32_t d = tmem_base + b * kAccStride;
+        bool ready = mbar_test(&bars->full[s], ph);
+        for (int kg = 0; kg < kblocks && ok; kg += 4) {
+          const uint32_t slot = tmem_base + kSfCol + ((kg >> 2) & 1) * 16;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (kg + j >= kblocks || !ok) break;
+            if (!ready && !mbar_wait(&bars->full[s], ph, abort_flag)) {
+              report_status(p.status, kWaitTimeout, kKernelGemm, 23, blockIdx.x);
+              ok = false;
+              break;
+            }
+            tc_fence_after_sync();
+            const uint32_t sa = smem_base + s * kStageBytes, lo = (sa >> 4) | 1u << 16;
+            if (kMx && j == 0) {
+              pair_cp_sf(slot, make_desc_sf(sa + 2 * kStageBytesA));
+              pair_cp_sf(slot + 4, make_desc_sf(sa + 2 * kStageBytesA + 512));
+              pair_cp_sf(slot + 8, make_desc_sf(sa + 2 * kStageBytesA + 1024));
+            }
+            uint64_t* const done = &bars->empty[s];
+            if (++s == kStages) { s = 0; ph ^= 1; }
+            ready = mbar_test(&bars->full[s], ph);     // asked here, needed behind the four instructions
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t acc = j > 0 || k > 0 || kg > 0;
+              if (kMx)
+                pair_mma_mx(d, lo + 2 * k, lo + (kStageBytesA >> 4) + 2 * k, kIdesc | (j << 29) | (j << 4), acc, slot, slot + 4);
+              else
+                pair_mma_bf16(d, lo + 2 * k, lo + (kStageBytesA >> 4) + 2 * k, kIdesc, acc);
+            }
+            issued_any = true;
+            pair_commit(done, 3);
+          }
+        }
+        if (ok) pair_commit(&bars->tmem_full[b], 3);
+      }
+      if (!ok && issued_any) {
+        pair_commit(&bars->drain, 1);
+        uint32_t dummy = 0;
+        mbar_wait(&bars->drain, 0, &dummy, 4000000ll);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue warps 2..9
+    pdl_wait();
+    const int q = warp & 3, hsel = (warp - 2) >> 2;
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    bool ok = true;
+    int t = 0;
+    for (int w = first; w < p.num_tiles; w += step, ++t) {
+      int ta, tb;
+      tile_of(w, ta, tb);
+      const int b = t & 1, row0 = ta * 256 + static_cast<int>(rank) * 128 + q * 32;
+      // the accumulator's chunk of 32 columns that it shares with the other one: 7 of the first, 0 of the second
+      const bool holds_shared = kMx && hsel == (b ^ 1);
+      const uint32_t acc = lane_base + b * kAccStride;
+      if (ok && !__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[b], (t >> 1) & 1, abort_flag))) {
+        if (lane == 0) report_status(p.status, kWaitTimeout, kKernelGemm, 24, blockIdx.x);
+        ok = false;
+      }
+      const int row = row0 + lane;
+      auto taken = [&](bool shared) {                  // the columns loaded so far are in registers
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_rank(shared ? &bars->shared_empty[b] : &bars->tmem_empty[b], 0));
+      };
+      if constexpr (kGlu) {
+        // 64 features in two runs of 32, gate and up, the run with the shared chunk first
+        uint32_t y[2][16];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int c = hsel * 64 + (u ^ b ^ 1) * 32;
+          if (ok) {
+            uint32_t g[32], up[32];
+            if (u == 0) tc_fence_after_sync();
+            tmem_ld_32x32(acc + c, g);
+            tmem_ld_32x32(acc + 128 + c, up);
+            tmem_ld_wait();
+            if (u == 0 && holds_shared) taken(true);
+            if (u == 1) taken(false);
+            glu_words(p, g, up, y[u]);
+            if (!kMx && row < p.rows_a) {
+              __nv_bfloat16* dst = p.out + static_cast<long long>(row) * p.ldc + tb * 128 + c;
+              store_words8(dst, y[u]);
+              store_words8(dst + 16, y[u] + 8);
+            }
+          }
+        }
+        if constexpr (kMx) {
+          // the scale of a row's 128 features needs both halves, which sit in two warps: they exchange maxima behind a barrier of
+          // their own, which a warp whose accumulator did not come still meets
+          float mx = 0.f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(y[j >> 4][j & 15] << 16)), fabsf(__uint_as_float(y[j >> 4][j & 15] & 0xffff0000u))));
+          bars->amax[b][hsel * 128 + q * 32 + lane] = mx;
+          asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+          mx = fmaxf(mx, bars->amax[b][(hsel ^ 1) * 128 + q * 32 + lane]);
+          uint32_t eb;
+          const float inv = mx_scale_inv(mx, eb);
+          if (ok && row < p.rows_a) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              uint32_t w[8];
+              fp8_words(y[u], inv, w);
+              store_words8(p.glu_q + static_cast<long long>(row) * p.glu_f + tb * 128 + hsel * 64 + (u ^ b ^ 1) * 32, w);
+            }
+            if (hsel == 0) store_sf(p.glu_sf, row, tb, p.glu_sf_rows, (p.glu_f + 511) >> 9, eb);
+          }
+        }
+      } else if (ok) {
+        tc_fence_after_sync();
+        const int turn = holds_shared && b == 0 ? 3 : 0;
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+          const int c = hsel * 4 + ((u + turn) & 3), b0 = tb * 256 + c * 32;
+          uint32_t r[32];
+          tmem_ld_32x32(acc + c * 32, r);
+          tmem_ld_wait();
+          if (u == 0 && holds_shared) taken(true);
+          if (u == 3) taken(false);
+          if (b0 + 32 <= p.rows_b) {
+            uint32_t y[16];
+            finish_row32(p, r, row, b0, y);
+            if (row < p.rows_a) {
+              __nv_bfloat16* dst = p.out + static_cast<long long>(row) * p.ldc + b0;
+              store_words8(dst, y);
+              store_words8(dst + 16, y + 8);
+            }
+          } else {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            store_chunk(p, v, row, b0, p.rows_b);
+          }
+        }
+      }
+    }
+  }
+
+  __syncwarp();                                        // the single-lane roles rejoin their warps
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                                  // no signal from the other CTA is on its way any more
+  if (warp == 1) {
+    tc_fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------------------------------ host side
+template <int kMode, bool kGlu>
+static int launch_pair(const GemmParams& p, const CUtensorMap (&maps)[4], cudaStream_t stream) {
+  const int smem = kPairStages * pair_stage_bytes<kMode>() + static_cast<int>(sizeof(PairBarriers)) + 1024;
+  static PerDeviceOnce configured;
+  if (configured.first_time()) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<kMode, kGlu>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (e != cudaSuccess) return -static_cast<int>(e) - 200;
+  }
+  const int pairs = num_sms() / 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * (p.num_tiles < pairs ? p.num_tiles : pairs));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = g_b200_pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kMode, kGlu>, p, maps[0], maps[1], maps[2], maps[3]) != cudaSuccess) return -300;
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 300;
+}
+
+// Whether a product of `tokens` rows by `rows_b` weight rows runs here and not on the tiles of one SM (gemm_tcgen05.cu). Both sides
+// measured over 24 shapes at depths 1024 to 12288 (bf16 256 x 9216 x 3072 47.4 -> 23.7 us, 2600 x 28672 x 4096 gated 535 -> 417,
+// fp8 600 x 4096 x 3072 56.5 -> 17.0, 8192 x 8192 x 8192 480 -> 377, 4096 x 9216 x 3072 116 -> 92):
+//  - a wave of pair tiles takes 0.8 of the time of a wave of 128 x 256 tiles in bf16 and 0.6 to 0.7 in 8 bits, so tokens that leave
+//    the last 256 rows half empty stay there where that costs more waves (300 x 12288 x 4096, two waves against one: bf16
+//    47.1 us here and 38.7 there; fp8 16.3 and 15.0 at depth 1024, 25.4 and 26.7 at 3072)
+//  - few tiles of a long row are cut along K there (bf16 k 12288: 16 tiles 64.9 here and 45.4 there, 24 tiles 65.0 and 59.0, 32 tiles
+//    64.8 and 71.3; k 4096: 16 tiles 27.9 and 28.5), 8-bit ones of a short row are as fast (k 1024: 36 tiles 12.1 and 11.5, 40 tiles
+//    11.9 and 48.5, k 3072: 24 tiles 15.8 and 16.8).
+// Rows of the output (and residual) start on 32-byte boundaries: the epilogue's accesses.
+bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual) {
+  if (tokens <= 128 || (dtype != 0 && dtype != 2)) return false;
+  if (ldc % 16 != 0 || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 31)) return false;
+  const long long sms = num_sms(), cols = (rows_b + 255) / 256;
+  const long long tiles = (tokens + 255) / 256 * cols, waves = (tiles + sms / 2 - 1) / (sms / 2);
+  const long long waves_one = ((tokens + 127) / 128 * cols + sms - 1) / sms;
+  if (tiles < 16 || tiles >= 1ll << 30) return false;
+  if (dtype == 0) return 4 * waves <= 5 * waves_one && (tiles >= 32 || k <= 4096);
+  return (3 * waves <= 5 * waves_one || k >= 3072) && (k >= 2048 || tiles > 36) && (tiles >= 32 || k <= 12288);
+}
+
+int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream) {
+  const bool mx = dtype == 2, gated = p.glu_f > 0;
+  const int esz = mx ? 1 : 2;
+  p.num_tiles = (p.rows_a + 255) / 256 * (gated ? p.glu_f / 128 : (p.rows_b + 255) / 256);
+  CUtensorMap maps[4];
+  int rc = make_kmajor_map(&maps[0], x, esz, p.rows_a, p.k, ldx, 128);
+  if (rc == 0) rc = make_kmajor_map(&maps[1], w, esz, p.rows_b, p.k, ldw, 128);
+  maps[2] = maps[3] = maps[0];
+  if (rc == 0 && mx) rc = make_sf_map(&maps[2], p.sf_a, (p.rows_a + 127ll) / 128 * p.sf_kgroups);
+  if (rc == 0 && mx) rc = make_sf_map(&maps[3], p.sf_b, (p.rows_b + 127ll) / 128 * p.sf_kgroups);
+  if (rc) return rc;
+  if (mx) return gated ? launch_pair<2, true>(p, maps, stream) : launch_pair<2, false>(p, maps, stream);
+  return gated ? launch_pair<0, true>(p, maps, stream) : launch_pair<0, false>(p, maps, stream);
+}
+
+}  // namespace b200

@@ -28,6 +28,26 @@ def test_epilogue_and_tiles(m, n, fp8, act, act_from):
     assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums of 256
 
 
+# tiles of CTA pairs: the fewest that go there, one K block, a K tail, rows and features that end inside a tile, both
+# accumulators in turn
+@pytest.mark.parametrize("m,n,k", [(256, 4096, 64), (257, 4104, 192), (385, 9232, 136), (2100, 1984, 4096), (5000, 3856, 328), (9473, 2304, 1024)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("full", [False, True])
+def test_pair_tiles(m, n, k, fp8, full):
+    torch.manual_seed(m)
+    k = -(-k // 128) * 128 if fp8 else k
+    n = n if not fp8 else -(-n // 16) * 16
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    vec = lambda: torch.randn(n, device="cuda").to(torch.bfloat16) if full else None
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16), vec(), fp8=fp8)
+    gate, act = vec(), "gelu_tanh" if full else None
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16) if full else None
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    y = ops.linear(xq, w, act=act, gate=gate, residual=res).float()
+    ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, w.bias, act, gate, res, torch.float32)
+    assert torch.allclose(y, ref, rtol=2 ** -7, atol=2 ** -7), (y - ref).abs().max()      # one rounding to bf16; fp32 sums
+
+
 def test_output_rows_apart():
     torch.manual_seed(1)
     x = torch.randn(260, 192, device="cuda").to(torch.bfloat16)
