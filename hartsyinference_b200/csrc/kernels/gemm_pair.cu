@@ -52,8 +52,9 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar, uint16_t ctas) {
 __device__ __forceinline__ void pair_cp_sf(uint32_t taddr, uint64_t sdesc) {
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
-// The issuing thread's own instructions bounded the 8-bit products (690 cycles a K block of four 128-cycle instructions), so
-// the descriptors' upper halves are constants and only the lower ones are counted on (see make_desc_sw128).
+// The issuing thread bounded the 8-bit products in a first form, with waits that acquire at cluster scope and descriptors counted on
+// in 64 bits: 690 cycles a K block of four 128-cycle instructions. With waits at CTA scope, the next stage asked for ahead of
+// this one's instructions and the descriptors' upper halves as constants (only the lower ones change, see make_desc_sw128): 511.
 #define B200_PAIR_DESCS                          \
   "{\n\t"                                        \
   ".reg .pred p;\n\t"                            \
