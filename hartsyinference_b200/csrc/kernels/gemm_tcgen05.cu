@@ -1344,7 +1344,7 @@ int gemv_bf16(const void* x, const void* w, void* out, int m, int n, int k, long
 // 78 -> 101 us, of 3072 x 15360 18.0 -> 20.5, two of 4096 x 14336 24.3 -> 27.1); up to four where the launch, not the
 // weights, is what counts (one of 384 x 18432 11.3 -> 5.6 us, three of 896 x 4864 7.5 -> 6.1, 3072 x 3072 9.4 -> 9.3, but
 // 28672 x 4096 45 -> 67 us).
-static bool handful(int m, int n, int k, int dtype) {
+bool handful(int m, int n, int k, int dtype) {
   return dtype == 0 && k % 8 == 0 && ((m <= 2 && k <= 8192) || (m <= 4 && static_cast<long long>(n) * k <= 1ll << 23));
 }
 

@@ -1043,6 +1043,43 @@ class DecoderModel:
             h = ex.reduce(res, self.final_norm if li == last else self.layers[li + 1].in_norm, cfg.rms_eps)
         return self.comm.all_gather(h.contiguous(), dim=0)
 
+    def _few_ok(self, batch: ForwardBatch, x: torch.Tensor) -> bool:
+        """True when this decode step is one token through a plain stack of bf16 layers, whose products take the norm in front of
+        them along (five launches a layer instead of eight). One token: 24 layers of 896 features 630 -> 488 us, four of 4096
+        features 375 both; two tokens 751 -> 750 and 408 -> 421, so they stay with the kernels apart."""
+        cfg = self.cfg
+        if (not batch.is_decode or not x.is_cuda or x.shape[0] != 1 or self.tp > 1 or self.fp8 or cfg.residual_multiplier != 1.0
+                or cfg.mixed_layers or not (self.first_stage and self.last_stage) or self.alibi_slopes is not None
+                or self.inv_freq_local is not None or batch.slot_mapping is None or self.kv_cache is None or not x.is_contiguous()):
+            return False
+        if (batch.positions.dtype != torch.int32 or batch.slot_mapping.dtype != torch.int64 or self.inv_freq.dtype != torch.float32
+                or self.kv_cache.dim() != 6 or not self.kv_cache.is_contiguous() or cfg.rotary_dim % 2):
+            return False
+        fits, rows = ops.few_fits, (self.hq + 2 * self.hkv) * cfg.head_dim
+        return all(lw.ffn_module is None and lw.attn_module is None and lw.sinks is None and lw.q_norm is None and lw.k_norm is None
+                   and lw.post_attn_norm is None and lw.post_ffn_norm is None and fits(x, lw.in_norm, lw.qkv) and fits(x, lw.post_norm, lw.gate_up)
+                   and lw.qkv.weight.shape[0] == rows and (lw.qkv.bias is None or lw.qkv.bias.dtype == torch.bfloat16) and lw.gate_up.bias is None
+                   and isinstance(lw.o, LinearWeight) and isinstance(lw.down, LinearWeight) for lw in self.layers)
+
+    def _forward_few(self, batch: ForwardBatch, x: torch.Tensor) -> torch.Tensor:
+        """Layer loop of one decoded token (``_few_ok``): norm + qkv + rotation and cache write, attention, o + residual,
+        norm + gated product, down + residual. HBM would idle through the short kernels, so the first and the fourth bring the
+        weights of the ones behind them to L2."""
+        cfg, scale = self.cfg, self._attn_scale()
+        kw = dict(eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one)
+        t = x.shape[0]
+        for li, lw in enumerate(self.layers):
+            kc, vc = self.kv_cache[li, 0], self.kv_cache[li, 1]
+            q = ops.norm_qkv_few(x, lw.in_norm, lw.qkv, batch.positions, self.hq, self.hkv, cfg.head_dim, k_cache=kc, v_cache=vc,
+                                 slot_mapping=batch.slot_mapping, rot=cfg.rotary_dim, inv_freq=self.inv_freq, style=cfg.rope_style,
+                                 ahead=(lw.o, lw.gate_up), **kw)
+            att = ops.attn_decode(q, kc, vc, batch.block_table, batch.kv_lens, scale=scale, softcap=cfg.attn_softcap,
+                                  window=cfg.layer_window(self.layer0 + li), max_kv_len=batch.max_kv_len or None)
+            x = ops.linear(att.reshape(t, -1), lw.o, residual=x)
+            then = self.layers[li + 1].qkv if li + 1 < len(self.layers) else None
+            x = ops.linear(ops.norm_glu_few(x, lw.post_norm, lw.gate_up, cfg.activation, ahead=(lw.down, then), **kw), lw.down, residual=x)
+        return ops.norm(x, self.final_norm, **kw)[0]
+
     def forward_hidden(self, batch: ForwardBatch, hidden_in: Optional[tuple] = None):
         """Runs this instance's layers. The last pipeline stage (the only one by default) returns the
         final-normed hidden states [T, H]; an earlier stage returns ``(x, residual)`` for the next
@@ -1070,6 +1107,9 @@ class DecoderModel:
             return self._forward_general(batch, x if res is None else (x.float() + res.float()).to(x.dtype), scale)
         if hidden_in is None and x.is_cuda and self._fused_tp_ok(x.shape[0]):
             return self._forward_fused_tp(batch, x)
+
+        if hidden_in is None and self._few_ok(batch, x):
+            return self._forward_few(batch, x)
 
         # small batches: what goes straight into a norm is left as unsummed K ranges that the norm adds
         rows, on_device = x.shape[0], x.is_cuda

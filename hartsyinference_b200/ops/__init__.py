@@ -21,6 +21,7 @@ from .core import (  # noqa: F401
     colbatched_linear,
     dit_qkv,
     embedding,
+    few_fits,
     fill_random_,
     fp8_mx,
     gated_residual,
@@ -44,6 +45,8 @@ from .core import (  # noqa: F401
     lincomb,
     msda,
     norm,
+    norm_glu_few,
+    norm_qkv_few,
     quant_fp8_act,
     quant_int8_act,
     quant_fp8_weight,

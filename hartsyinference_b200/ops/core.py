@@ -468,6 +468,57 @@ def linear_glu(x, w: LinearWeight, act: str = "silu", emit_fp8: bool = False, em
     return glu(linear(x, w, defer=xd.is_cuda and xd.shape[0] <= 128), act, emit_fp8=emit_fp8, emit_bf16=emit_bf16)
 
 
+def few_fits(x: torch.Tensor, norm_w, w) -> bool:
+    """Whether the products of a handful of tokens that norm their input themselves take these operands."""
+    if not (isinstance(w, LinearWeight) and isinstance(norm_w, torch.Tensor)) or w.is_fp8 or not x.is_cuda:
+        return False
+    wt = w.weight
+    return (x.dtype == wt.dtype == norm_w.dtype == torch.bfloat16 and x.dim() == 2 and wt.shape[1] == x.shape[1] == norm_w.numel()
+            and x.stride(1) == wt.stride(1) == 1 and norm_w.is_contiguous() and wt.is_cuda and (x.stride(0) | wt.stride(0)) % 8 == 0
+            and (x.data_ptr() | wt.data_ptr() | norm_w.data_ptr()) % 16 == 0 and bool(N.lib().b200_gemv_norm_fits(x.shape[0], wt.shape[0], x.shape[1])))
+
+
+def _ahead(weights) -> tuple:
+    """Pointer and size of up to two weights that a later product reads and a kernel in front of it brings to L2."""
+    out = []
+    for w in weights[:2]:
+        t = w.weight if isinstance(w, LinearWeight) and w.weight.is_cuda and w.weight.is_contiguous() else None
+        out += [None, 0] if t is None else [t.data_ptr(), t.numel() * t.element_size()]
+    return tuple(out + [None, 0] * (2 - len(weights)))
+
+
+def norm_qkv_few(x: torch.Tensor, norm_w: torch.Tensor, w: LinearWeight, positions: torch.Tensor, hq: int, hkv: int, d: int, *,
+                 k_cache: torch.Tensor, v_cache: torch.Tensor, slot_mapping: torch.Tensor, rot: int, inv_freq: torch.Tensor, style: int = 0,
+                 eps: float = 1e-6, weight_plus_one: bool = False, ahead: tuple = ()) -> Optional[torch.Tensor]:
+    """``rope_kv(linear(norm(x), w))`` for a handful of decoded tokens with bf16 weights, in one launch: q [T, hq, d]. None (and
+    nothing is done) for operands that it does not take. ``ahead``: up to two weights of products further on, for L2."""
+    if not (few_fits(x, norm_w, w) and w.weight.shape[0] == (hq + 2 * hkv) * d and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and positions.dtype == torch.int32 and slot_mapping.dtype == torch.int64 and inv_freq is not None and inv_freq.dtype == torch.float32
+            and (w.bias is None or w.bias.dtype == torch.bfloat16)):
+        return None
+    t, k = x.shape
+    q = torch.empty(t, hq, d, dtype=torch.bfloat16, device=x.device)
+    rc = N.lib().b200_gemv_norm_qkv(x.data_ptr(), norm_w.data_ptr(), w.weight.data_ptr(), N.ptr(w.bias), q.data_ptr(), k_cache.data_ptr(),
+                                    v_cache.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(), inv_freq.data_ptr(), t, k, x.stride(0),
+                                    w.weight.stride(0), hq, hkv, d, rot, style, k_cache.shape[2], eps, int(weight_plus_one), *_ahead(ahead), N.stream())
+    N.check(rc, "b200_gemv_norm_qkv")
+    return q
+
+
+def norm_glu_few(x: torch.Tensor, norm_w: torch.Tensor, w: LinearWeight, act: str = "silu", eps: float = 1e-6,
+                 weight_plus_one: bool = False, ahead: tuple = ()) -> Optional[torch.Tensor]:
+    """``linear_glu(norm(x), w, act)`` for a handful of tokens with bf16 weights, in one launch. None for operands that it does not
+    take. ``ahead`` as in :func:`norm_qkv_few`."""
+    if not (few_fits(x, norm_w, w) and w.bias is None and act in ("silu", "gelu_tanh") and w.weight.shape[0] % 2 == 0):
+        return None
+    (t, k), f = x.shape, w.weight.shape[0] // 2
+    y = torch.empty(t, f, dtype=torch.bfloat16, device=x.device)
+    rc = N.lib().b200_gemv_norm_glu(x.data_ptr(), norm_w.data_ptr(), w.weight.data_ptr(), y.data_ptr(), t, f, k, x.stride(0), w.weight.stride(0), f,
+                                    0 if act == "silu" else 1, eps, int(weight_plus_one), *_ahead(ahead), N.stream())
+    N.check(rc, "b200_gemv_norm_glu")
+    return y
+
+
 def rope_kv(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: int, *,
             k_cache: Optional[torch.Tensor] = None, v_cache: Optional[torch.Tensor] = None,
             slot_mapping: Optional[torch.Tensor] = None, rot: Optional[int] = None,

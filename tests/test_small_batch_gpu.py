@@ -1,9 +1,14 @@
 """Small-batch forms: K ranges summed by the norm and the rotary kernel, argmax in 16-byte reads."""
+from dataclasses import replace
+
 import pytest
 import torch
 
 from hartsyinference_b200 import ops
 from hartsyinference_b200.engine.sampling import SamplingParams, sample_row
+from hartsyinference_b200.models.llm import config as C
+from hartsyinference_b200.models.llm.transformer import DecoderModel, ForwardBatch
+from hartsyinference_b200.ops import reference as R
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +90,62 @@ def test_gated_product_of_no_rows():
     w = ops.LinearWeight(torch.randn(512, 256, device="cuda").to(torch.bfloat16))
     y, q = ops.linear_glu(torch.empty(0, 256, device="cuda", dtype=torch.bfloat16), w)
     assert tuple(y.shape) == (0, 256) and q is None
+
+
+# the product that norms its input and rotates its output: depths that leave lanes idle, heads with and without an unrotated rest
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+@pytest.mark.parametrize("k,hq,hkv,d,rot,style,bias", [(896, 14, 2, 64, 64, 0, True), (512, 4, 4, 96, 96, 1, False), (2056, 8, 2, 128, 64, 0, True),
+                                                      (128, 2, 1, 64, 32, 1, False), (64, 2, 2, 32, 0, 0, False)])
+def test_one_launch_of_norm_projection_and_rotation(m, k, hq, hkv, d, rot, style, bias):
+    torch.manual_seed(k + m)
+    bf = torch.bfloat16
+    x = torch.randn(m, k, device="cuda").to(bf)
+    nw = (1 + 0.1 * torch.randn(k, device="cuda")).to(bf)
+    n = (hq + 2 * hkv) * d
+    w = ops.LinearWeight((torch.randn(n, k, device="cuda") * k ** -0.5).to(bf), bias=torch.randn(n, device="cuda").to(bf) if bias else None)
+    pos = torch.randint(0, 30000, (m,), device="cuda", dtype=torch.int32)
+    inv = R.rope_inv_freq(max(rot, 2), 10000.0, torch.device("cuda")).float()
+    slots = torch.tensor([5, -1, 17, 40][:m], device="cuda")
+    caches = [torch.zeros(2, 3, hkv, 16, d, dtype=bf, device="cuda") for _ in range(2)]
+    q = ops.norm_qkv_few(x, nw, w, pos, hq, hkv, d, k_cache=caches[0][0], v_cache=caches[0][1], slot_mapping=slots, rot=rot, inv_freq=inv, style=style, ahead=(w,))
+    h = ops.norm(x, nw)[0]
+    y = (h.float() @ w.weight.float().t() + (w.bias.float() if bias else 0)).to(bf)
+    ref = ops.rope_kv(y, pos, hq, hkv, d, k_cache=caches[1][0], v_cache=caches[1][1], slot_mapping=slots, rot=rot, inv_freq=inv, style=style)[0]
+    # the sums of k products in fp32 differ in order, so a value may round to the neighbouring bf16 in front of the rotation and behind it
+    for a, b in ((q, ref), (caches[0], caches[1])):
+        assert (a.float() - b.float()).abs().max() <= 2 ** -6 * max(1.0, b.float().abs().max().item())
+        assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm() + 1e-6
+
+
+@pytest.mark.parametrize("m,f,k", [(1, 4864, 896), (2, 40, 512), (3, 1000, 2056), (4, 13, 64), (1, 14336, 4096), (1, 8, 8192)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_one_launch_of_norm_and_gated_product(m, f, k, act):
+    torch.manual_seed(f)
+    bf = torch.bfloat16
+    x = torch.randn(m, k, device="cuda").to(bf)
+    nw = (1 + 0.1 * torch.randn(k, device="cuda")).to(bf)
+    w = ops.LinearWeight((torch.randn(2 * f, k, device="cuda") * k ** -0.5).to(bf))
+    y = ops.norm_glu_few(x, nw, w, act, weight_plus_one=f == 40, ahead=(w, w))
+    ref = R.glu(ops.norm(x, nw, weight_plus_one=f == 40)[0].float() @ w.weight.float().t(), act)
+    assert torch.allclose(y.float(), ref, rtol=2 ** -7, atol=2 ** -8)      # fp32 sums, one rounding to bf16
+
+
+def test_one_token_through_the_stack():
+    for preset in ("qwen2.5-0.5b", "llama-3-8b"):
+        cfg = replace(C.PRESETS[preset], num_layers=2, vocab_size=512)
+        model = DecoderModel(cfg, "cuda")
+        model.random_init(seed=1)
+        model.alloc_kv(4, 16)
+        model.kv_cache.normal_()
+        dev = lambda *v, dtype=torch.int32: torch.tensor(v, dtype=dtype, device="cuda")
+        batch = ForwardBatch(tokens=dev(7), positions=dev(40), slot_mapping=dev(2 * 16 + 8, dtype=torch.int64), block_table=dev(0, 1, 2).reshape(1, 3),
+                             kv_lens=dev(41), is_decode=True, max_kv_len=48)
+        assert model._few_ok(batch, torch.zeros(1, cfg.hidden_size, dtype=torch.bfloat16, device="cuda"))
+        before = model.kv_cache.clone()
+        y, cache = model.forward_hidden(batch), model.kv_cache.clone()
+        model.kv_cache.copy_(before)
+        model._few_ok = lambda *a: False
+        ref = model.forward_hidden(batch)
+        # two layers of bf16 roundings that fall differently (one sum is no longer rounded ahead of the residual add)
+        assert (y.float() - ref.float()).norm() <= 2e-2 * ref.float().norm()
+        assert (cache.float() - model.kv_cache.float()).norm() <= 2e-3 * model.kv_cache.float().norm()
