@@ -297,11 +297,12 @@ class LLMEngine:
         # requests that re-computed their context after a pre-emption continue decoding without sampling
         return done + [(req, -1) for req in rebuilt]
 
-    def _read_tokens(self, dev_tokens: torch.Tensor, n: int) -> list[int]:
+    def _read_tokens(self, dev_tokens: Optional[torch.Tensor], n: int) -> list[int]:
         """Sampled ids and the kernels' status word come back in the same synchronising read. A
         recorded wait timeout (a peer that stopped signalling) fails this step's requests instead
         of letting them continue on garbage."""
-        self.h_out[:n].copy_(dev_tokens[:n], non_blocking=True)
+        if n:
+            self.h_out[:n].copy_(dev_tokens[:n], non_blocking=True)
         self.h_status.copy_(N.state(self.device).status, non_blocking=True)
         torch.cuda.current_stream().synchronize()
         self.d2h_bytes_last += n * 4 + 16
@@ -510,7 +511,13 @@ class LLMEngine:
                                  block_table=st["table"], kv_lens=st["kv_lens"], is_decode=True,
                                  max_kv_len=self.max_model_len, state_slots=st["state"] if self.kv.state_slots else None)
             st["hidden"] = self.model.forward_hidden(batch)
-            self.model.greedy_tokens(st["hidden"], st["out"])
+            # logits that the greedy token is taken from, kept where they are what ``full_logits`` gives: the product over the
+            # vocabulary then runs once a step also where they are asked for
+            if isinstance(self.model, DecoderModel) and self.model.tp == 1 and not self.mixed:
+                st["logits"] = self.model.full_logits(st["hidden"])
+                ops.argmax(st["logits"], st["out"])
+            else:
+                self.model.greedy_tokens(st["hidden"], st["out"])
 
         # warm up on a side stream (loads kernels, sizes scratch) before capturing
         s = torch.cuda.Stream(device=dev)
@@ -653,16 +660,21 @@ class LLMEngine:
             if len(runs) <= self.max_batch and all(start > 0 and count == 1 for _, start, count in runs):
                 rids = [rid for rid, _, _ in runs]
                 if self.use_graphs and not self._graphs_disabled:
-                    hidden = self._run_decode_graph(rids)[0]["hidden"]
+                    st = self._run_decode_graph(rids)[0]
+                    hidden = st["hidden"]
+                    if rows and "logits" in st:        # the step's own, copied out of its buffer
+                        y = st["logits"]
+                        y = y[:len(rows)] if rows == list(range(len(rows))) else y[torch.tensor(rows, dtype=torch.int64, device=self.device)]
+                        logits = y.to(torch.float32, copy=True)
                 else:
                     hidden = self._run_decode_eager(rids)
             else:
                 hidden, _ = self._run_chunks(runs)
-            if rows:
+            if rows and logits is None:
                 idx = torch.tensor(rows, dtype=torch.int64, device=self.device)
                 logits = self.model.full_logits(hidden[idx].contiguous()).float()
             if self.cuda:
-                self._read_tokens(torch.zeros(1, dtype=torch.int32, device=self.device), 1)     # waits, and checks the status word
+                self._read_tokens(None, 0)           # waits, and checks the status word
         for key in end:
             rid = self._replays.pop(key, None)
             if rid is not None:

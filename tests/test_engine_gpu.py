@@ -97,3 +97,17 @@ def test_graph_and_eager_decode_agree_exactly():
 def test_smoke_entry():
     import __graft_entry__ as ge
     ge.smoke()
+
+
+def test_replayed_logits_are_the_steps_own():
+    _, g = _pair(False, 3)
+    eng = LLMEngine(g, num_pages=64, page_size=16, max_batch=4, prefill_chunk=128, max_model_len=128)
+    toks = {k: torch.randint(0, 1024, (20,), generator=torch.Generator().manual_seed(i)).tolist() for i, k in enumerate("abc")}
+    eng.replay([(k, toks[k][:17], [16]) for k in "abc"])
+    first = eng.replay([("a", toks["a"][17:18], [0]), ("b", toks["b"][17:18], [0]), ("c", toks["c"][17:18], [0])])
+    kept = first.clone()
+    hidden = next(iter(eng._graphs.values()))[1]["hidden"]
+    assert torch.equal(first, g.full_logits(hidden)[:3].float())
+    only = eng.replay([("a", toks["a"][18:19], []), ("b", toks["b"][18:19], [0]), ("c", toks["c"][18:19], [])])
+    assert torch.equal(only, g.full_logits(hidden)[1:2].float()) and torch.equal(first, kept)
+    assert eng.replay([("c", toks["c"][19:], [])], "abc") is None
