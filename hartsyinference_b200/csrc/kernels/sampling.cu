@@ -347,6 +347,11 @@ __device__ __forceinline__ unsigned long long ld_dsmem_u64(uint32_t addr) {
   asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned ld_dsmem_u32(uint32_t addr) {
+  unsigned v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint4 ld_dsmem_u32x4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
@@ -359,8 +364,10 @@ __device__ __forceinline__ uint4 ld_dsmem_u32x4(uint32_t addr) {
 struct RowHist {
   unsigned lo[kSampleBins], mid[kSampleBins], hi[kSampleBins];
 };
+constexpr int kRowRun = 32, kRowRuns = kSampleBins / kRowRun;      // bins whose sum a block gives its peers, and how many such runs
 struct RowShared {
   RowHist hist[2];                                    // levels alternate
+  unsigned long long runs[2][kRowRuns];               // sums of this block's runs of bins
   unsigned long long part[kSampleBins];               // the draw's masses per step and warp
   unsigned long long scan[kRowThreads / 32];
   unsigned long long front;                           // what lies in front of the chosen bin
@@ -410,7 +417,8 @@ __device__ __forceinline__ float row_select(RowShared& sh, int& level, const flo
 #pragma unroll 1
   for (int lv = 0; lv < 3; ++lv) {
     const int shift = lv == 0 ? 21 : lv == 1 ? 10 : 0, bits = lv == 2 ? 10 : 11, nb = 1 << bits;
-    RowHist& hist = sh.hist[level & 1];
+    const int parity = level & 1;
+    RowHist& hist = sh.hist[parity];
     ++level;
     for (int b = threadIdx.x; b < kSampleBins; b += kRowThreads) {
       hist.lo[b] = 0u;
@@ -433,32 +441,65 @@ __device__ __forceinline__ float row_select(RowShared& sh, int& level, const flo
         }
       }
     }
-    cluster_sync_all();
-    // every block adds up all blocks' bins; thread t takes four of them, the top ones first
-    const int b0 = kSampleBins - 4 - 4 * static_cast<int>(threadIdx.x);
-    unsigned long long c[4] = {0ull, 0ull, 0ull, 0ull};
+    __syncthreads();
+    // Sums of runs of bins first: the peers read 64 words of each block, and then the bins of the one run that the walk ends in. (All
+    // blocks' bins, 24 KB of each, took 12000 cycles a level and kept the blocks waiting for one another for as long.)
+    auto bin_of = [&](const RowHist& h, int at) {
+      unsigned long long m = h.lo[at];
+      if (!by_count) m += (static_cast<unsigned long long>(h.mid[at]) << 14) + (static_cast<unsigned long long>(h.hi[at]) << 28);
+      return m;
+    };
+    unsigned long long* const runs = sh.runs[parity];
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < kRowRuns; r += kRowThreads / 32) {
+      unsigned long long m = bin_of(hist, r * kRowRun + lane);
 #pragma unroll
-    for (int k = 0; k < kRowBlocks; ++k) {
-      const uint4 x = ld_dsmem_u32x4(dsmem_addr(hist.lo + b0, k));
-      uint4 y = make_uint4(0u, 0u, 0u, 0u), z = y;
-      if (!by_count) {
-        y = ld_dsmem_u32x4(dsmem_addr(hist.mid + b0, k));
-        z = ld_dsmem_u32x4(dsmem_addr(hist.hi + b0, k));
-      }
-      const unsigned xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w}, zs[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        c[j] += xs[j] + (static_cast<unsigned long long>(ys[j]) << 14) + (static_cast<unsigned long long>(zs[j]) << 28);
+      for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+      if (lane == 0) runs[r] = m;
     }
-    unsigned long long total;
-    unsigned long long front = before + row_scan(sh, c[0] + c[1] + c[2] + c[3], total);
+    cluster_sync_all();
+    // one warp walks, the top run first: a lane takes two runs, then one bin
+    if (threadIdx.x < 32) {
+      unsigned long long c[2] = {0ull, 0ull};
+      const int r0 = kRowRuns - 2 - 2 * lane;
 #pragma unroll
-    for (int j = 3; j >= 0; --j) {
-      const unsigned long long upto = front + c[j];
-      // one bin at most: what lies in front has not reached the target, with it it has
-      const bool hit = c[j] != 0ull && (by_count ? front < target && upto >= target : front <= target && upto > target);
-      if (hit) { sh.bin = b0 + j; sh.front = front; }
-      front = upto;
+      for (int k = 0; k < kRowBlocks; ++k) {
+        const uint4 x = ld_dsmem_u32x4(dsmem_addr(runs + r0, k));
+        c[0] += x.x | static_cast<unsigned long long>(x.y) << 32;
+        c[1] += x.z | static_cast<unsigned long long>(x.w) << 32;
+      }
+      auto in_front = [&](unsigned long long x) {            // sum over the lanes in front
+        unsigned long long incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        return incl - x;
+      };
+      // what lies in front has not reached the target, with this it has: of one run and one bin at most
+      auto ends = [&](unsigned long long front, unsigned long long x) {
+        return x != 0ull && (by_count ? front < target && front + x >= target : front <= target && front + x > target);
+      };
+      unsigned long long front = before + in_front(c[0] + c[1]);
+      int run = -1;
+      if (ends(front, c[1])) run = r0 + 1;
+      else if (ends(front + c[1], c[0])) { run = r0; front += c[1]; }
+      const unsigned who = __ballot_sync(0xffffffffu, run >= 0);
+      if (who) {
+        run = __shfl_sync(0xffffffffu, run, __ffs(who) - 1);
+        front = __shfl_sync(0xffffffffu, front, __ffs(who) - 1);
+        const int at = run * kRowRun + kRowRun - 1 - lane;
+        unsigned long long m = 0;
+#pragma unroll
+        for (int k = 0; k < kRowBlocks; ++k) {
+          m += ld_dsmem_u32(dsmem_addr(hist.lo + at, k));
+          if (!by_count) m += (static_cast<unsigned long long>(ld_dsmem_u32(dsmem_addr(hist.mid + at, k))) << 14) +
+                              (static_cast<unsigned long long>(ld_dsmem_u32(dsmem_addr(hist.hi + at, k))) << 28);
+        }
+        front += in_front(m);
+        if (ends(front, m)) { sh.bin = at; sh.front = front; }
+      }
     }
     __syncthreads();
     const int chosen = sh.bin;
@@ -474,8 +515,8 @@ __device__ __forceinline__ float row_select(RowShared& sh, int& level, const flo
 // The filter chain and the draw of sample_kernel with the row in registers: thread t of block b holds the values
 // (b * V + i) * 512 + t. Masses are 2^-40 fixed point throughout, so sums do not depend on their order.
 // Bound by the adds into the first histogram of a search, whose bins are few, and by the chain of exchanges, not by
-// memory. 64 rows of 128256: top-k 388 -> 95 us, top-p 432 -> 205, both 483 -> 257, neither 90 -> 42; one row with both
-// 469 -> 73 us.
+// memory. 64 rows of 128256 (a block per row / every block reading all bins of its peers / the run's bins only): top-p 393 / 205 /
+// 74 us, top-k and top-p 484 / 257 / 86, neither 66 / 42 / 32; one row with both 470 / 73 / 34 us.
 template <int V>
 __global__ void __launch_bounds__(kRowThreads, V <= 40 ? 2 : 1) sample_row_kernel(const SampleParams p) {
   extern __shared__ __align__(16) uint8_t row_smem[];
@@ -559,8 +600,9 @@ __global__ void __launch_bounds__(kRowThreads, V <= 40 ? 2 : 1) sample_row_kerne
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     unsigned long long m = v[i] >= tau ? static_cast<unsigned long long>(v[i] * kMassScale) : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    // 41 bits in two pieces whose sums over a warp fit 32: one instruction each
+    m = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(m) & 0xfffffu) +
+        (static_cast<unsigned long long>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(m >> 20))) << 20);
     if (lane == 0) part[i * (kRowThreads / 32) + wid] = m;
   }
   __syncthreads();
@@ -646,17 +688,20 @@ B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows,
   p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.min_p = min_p;
   p.seed = seed; p.counter = counter; p.out = out;
   const int each = (vocab + kRowBlocks * kRowThreads - 1) / (kRowBlocks * kRowThreads);      // values a thread holds
-  // A block of its own per row takes 24 us + a us per 350 logits with every filter, all rows of a wave at once. A cluster takes 58 to
-  // 105 us however short its rows are, and 37 of them (18 of the widest) fill the machine; from 16 to 40 values a thread a
-  // wave gets up to 1.4 times longer. Which filters a row asks for is known on the device only: with every one (us, block /
-  // cluster) 1 x 4096 34 / 54, 1 x 16384 69 / 54, 64 x 32000 121 / 208, 64 x 65536 252 / 214, 512 x 4096 136 / 1549,
-  // 128 x 100352 349 / 489, 128 x 202048 686 / 774, 148 x 128256 460 / 587; without filters 64 x 32000 32 / 18, 128 x 100352
-  // 74 / 73. The full chain, the longest a batch can take, decides.
-  const int sms = num_sms(), per_wave = (each <= 40 ? 2 * sms : sms) / kRowBlocks;
-  const double block_us = (24. + vocab / 350.) * ((rows + sms - 1) / sms);
-  const double cluster_us = rows <= 8 ? 58. : 2 * rows <= per_wave ? 75. :
-      105. * ((rows + per_wave - 1) / per_wave) * (each > 16 && each <= 40 ? 1. + (each - 16) / 64. : 1.);
-  if (rows < (1 << 27) && per_wave > 0 && cluster_us <= block_us) {
+  // A block of its own per row takes 28 us + a us per 290 logits with every filter, all rows of a wave at once, and 9 + one per 2100
+  // without. A cluster takes 24 to 44 us, twice that when they fill the machine, and from there 0.8 to 2.9 us a row by the
+  // values that a thread holds, and a third of that without filters. Which filters a row asks for is known on the device only:
+  // a cluster has to be a fifth faster in the full chain and no slower without one. With every filter (us, block / cluster)
+  // 1 x 4096 38 / 24, 1 x 128256 470 / 34, 16 x 2048 34 / 28, 37 x 4096 40 / 47, 48 x 16384 79 / 48, 96 x 16384 79 / 79, 64 x 128256
+  // 484 / 86, 128 x 151936 579 / 200, 512 x 16384 301 / 393; without 48 x 16384 15 / 15, 96 x 50257 30 / 28, 148 x 50257 30 / 42,
+  // 64 x 128256 66 / 32, 128 x 202048 110 / 134.
+  const int sms = num_sms(), waves = (rows + sms - 1) / sms;
+  const int width = each <= 8 ? 0 : each <= 16 ? 1 : each <= 32 ? 2 : each <= 40 ? 3 : 4;
+  constexpr double kRowUs[5] = {0.76, 0.93, 1.33, 1.6, 2.9}, kPlainUs[5] = {0.235, 0.285, 0.43, 0.6, 1.05};
+  const double block_us = (28. + vocab / 290.) * waves, block_plain = (9. + vocab / 2100.) * waves;
+  const double cluster_us = kRowUs[width] * (rows <= 8 ? 28. : rows <= 18 ? 36. : rows <= 49 ? 55. : rows + 6.);
+  const double cluster_plain = 3. + kPlainUs[width] * rows;
+  if (rows < (1 << 27) && sms >= kRowBlocks && cluster_us <= 0.8 * block_us && cluster_plain <= 1.05 * block_plain) {
     if (each <= 8) return launch_rows<8>(p, rows, stream);
     if (each <= 16) return launch_rows<16>(p, rows, stream);
     if (each <= 32) return launch_rows<32>(p, rows, stream);

@@ -59,7 +59,7 @@ def test_ties_and_infinities():
     assert set(_sample(x[:1].repeat(200, 1).contiguous(), 1.0, 1, 0.0, 0.0).tolist()) == {123, 39999}     # ties at the k-th value all stay
 
 
-@pytest.mark.parametrize("rows,vocab", [(300, 32000), (64, 8193), (9, 5000)])
+@pytest.mark.parametrize("rows,vocab", [(300, 32000), (300, 8193), (160, 5000)])
 def test_many_rows_as_few(rows, vocab):
     """Batches that a block per row is faster for, against the same rows a few at a time and the sampler's statement."""
     torch.manual_seed(rows)
@@ -85,3 +85,20 @@ def test_flat_rows_of_a_large_batch(t, k, p, mp):
     logits = (torch.randn(1000, 100000, device="cuda") * 0.1).to(torch.bfloat16)
     few = torch.cat([_sample(logits[i:i + 8], t, k, p, mp, seed=i) for i in range(0, 1000, 8)])
     assert torch.equal(_sample(logits, t, k, p, mp), few)
+
+
+# batches that go one block per row, and the same rows a few at a time, which go a cluster per row: the walk over runs of bins ends in
+# the first and the last run, in a bin that many values share, and nowhere
+@pytest.mark.parametrize("vocab", [2048, 4096, 16384])
+@pytest.mark.parametrize("t,k,p,mp", [(0.8, 50, 0.9, 0.05), (1.0, 1, 0.0, 0.0), (1.0, -1, 0.999999, 0.0), (0.7, 0, 1e-6, 0.0), (1.0, -1, 0.5, 1.0), (0.05, 0, 0.97, 0.0)])
+def test_blocks_and_clusters_draw_the_same(vocab, t, k, p, mp):
+    torch.manual_seed(vocab + 1)
+    x = torch.randn(160, vocab, device="cuda") * torch.linspace(0.01, 20, 160, device="cuda")[:, None]
+    x[3] = 1.5
+    x[4] = (torch.arange(vocab, device="cuda") % 7).float()
+    x[5, 1:] = float("-inf")
+    x[6] -= 50 * (torch.arange(vocab, device="cuda") % 2048 > 3)
+    k = vocab - 1 if k < 0 else k
+    many = _sample(x, t, k, p, mp)
+    few = torch.cat([_sample(x[i:i + 8], t, k, p, mp, seed=i) for i in range(0, 160, 8)])
+    assert torch.equal(many, few)
