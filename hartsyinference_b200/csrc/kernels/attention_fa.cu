@@ -32,7 +32,7 @@
 // One sample's V is read as it lies ([key][head dim], an MN-major operand) where it starts on a 16-byte boundary.
 // Otherwise, and in the segmented forms below, V is consumed transposed ([head dim][keys]) and padded; that transpose and
 // the int8 quantisation are small kernels of their own in front.
-#include "comm.cuh"
+#include "gemm_common.cuh"
 
 namespace b200 {
 
@@ -87,6 +87,12 @@ struct FaParams {
   long long out_col0;
   uint32_t* done_flags[8];   // rank s's "outputs have arrived" counter
   uint32_t* done_ctr;        // CTAs of this launch that have finished
+  // Quantised output: rows of out_q[0], from row q_split on rows of out_q[1], e4m3 with one UE8M0 scale per head (1x128) in the
+  // blocked layout; head h in columns q_col0 + h * 128
+  uint8_t* out_q[2];
+  uint8_t* out_sf[2];
+  long long q_ld[2];
+  int q_col0[2], q_kgroups[2], q_split;
 };
 
 // K and V^T tensor maps per source rank for the pull form (ring-style context parallelism without
@@ -108,7 +114,8 @@ __device__ __forceinline__ void fa_key_tile(const FaParams& p, int j, int& buf_t
 
 // kDirect: V is read as it lies ([key][dim], an MN-major operand) through tm_vt, nothing is transposed (a compile-time
 // matter: both forms in one kernel made the compiler spill inside the key loop, 15 % at 14040 keys).
-template <bool kI8, bool kDirect>
+// kQuant: the output leaves as e4m3 (one sample, no segments).
+template <bool kI8, bool kDirect, bool kQuant = false>
 __global__ void __launch_bounds__(kFaThreads, 1)
 attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
                const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_vt,
@@ -411,6 +418,32 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
       } else {
         tc_fence_after_sync();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+        if constexpr (kQuant) {
+          uint32_t y[4][16];
+          float amax = 0.f;
+#pragma unroll
+          for (int hc = 0; hc < 4; ++hc) {
+            uint32_t o[32];
+            tmem_ld_32x32(o_col + hc * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int u = 0; u < 16; ++u) y[hc][u] = pack_bf16x2(__uint_as_float(o[2 * u]) * inv, __uint_as_float(o[2 * u + 1]) * inv);
+            amax = words_max(y[hc], amax);
+          }
+          if (q_valid) {
+            const int part = q_idx >= p.q_split ? 1 : 0, r = q_idx - (part ? p.q_split : 0);
+            uint32_t eb;
+            const float scale = mx_scale_inv(amax, eb);
+            uint8_t* dst = p.out_q[part] + r * p.q_ld[part] + p.q_col0[part] + col0;
+#pragma unroll
+            for (int hc = 0; hc < 4; ++hc) {
+              uint32_t w[8];
+              fp8_words(y[hc], scale, w);
+              store_words8(dst + hc * 32, w);
+            }
+            store_sf(p.out_sf[part], r, (p.q_col0[part] + col0) >> 7, 128, p.q_kgroups[part], eb);
+          }
+        } else {
         // The Q tile is no longer read: 32 rows of 64 bytes per warp turn the rows that the lanes hold into
         // 64-byte runs of the output (16-byte pieces of 32 rows at a time leave half-written sectors). Pieces are
         // placed by (piece xor row / 2), which keeps the banks apart.
@@ -442,6 +475,7 @@ attn_fa_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_q,
             }
           }
           __syncwarp();
+        }
         }
       }
     }
@@ -942,6 +976,44 @@ B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out
   return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads), int8, stream, nullptr, direct);
 }
 
+// b200_attn_fa (bf16, V on a 16-byte boundary) for products that read e4m3: head h of query row r leaves as e4m3 with one 1x128 UE8M0 scale in
+// columns col0 + h * 128 of row r of q0, from row `split` on of row r - split of q1 (two streams that are projected apart);
+// scales in the blocked layout of kg words a row (4608 x 24 heads 352 + 17 us -> 358, 14040 x 40 3888 + 58 -> 3962). Values are rounded to bf16 first, so they are what a quantisation of
+// b200_attn_fa's output gives. -12: boundaries that it does not take.
+B200_API int b200_attn_fa_quant(const void* q, const void* k, const void* v, int sq, int sk, int heads, float scale, int split, void* q0, void* sf0,
+                                long long ld0, int col0, int kg0, void* q1, void* sf1, long long ld1, int col1, int kg1, void* status,
+                                cudaStream_t stream) {
+  if (sq <= 0 || sk <= 0) return 0;
+  const bool second = split < sq;
+  if (!fa_direct(v) || split < 0 || !q0 || !sf0 || (second && (!q1 || !sf1)) || ld0 % 32 != 0 || (second && ld1 % 32 != 0) || col0 % 128 != 0 || col1 % 128 != 0 ||
+      ((reinterpret_cast<uintptr_t>(q0) | (second ? reinterpret_cast<uintptr_t>(q1) : 0)) & 31))
+    return -12;
+  const long long ld = static_cast<long long>(heads) * kFaD;
+  FaParams p{};
+  p.sq = sq; p.sk = sk; p.heads = heads; p.batch = 1;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = static_cast<DeviceStatus*>(status);
+  p.n_tiles = fa_pad(sk, 128) / 128;
+  p.tiles_per_seg = p.n_tiles;
+  p.nseg = 1;
+  p.seg_len = sk;
+  p.seg_pad = p.n_tiles * 128;
+  p.out_q[0] = static_cast<uint8_t*>(q0);
+  p.out_q[1] = static_cast<uint8_t*>(q1);
+  p.out_sf[0] = static_cast<uint8_t*>(sf0);
+  p.out_sf[1] = static_cast<uint8_t*>(sf1);
+  p.q_ld[0] = ld0; p.q_ld[1] = ld1;
+  p.q_col0[0] = col0; p.q_col0[1] = col1;
+  p.q_kgroups[0] = kg0; p.q_kgroups[1] = kg1;
+  p.q_split = split;
+  CUtensorMap tq, tk, tv;
+  int rc = make_kmajor_map(&tq, q, 2, sq, ld, ld, 128);
+  if (rc == 0) rc = make_kmajor_map(&tk, k, 2, sk, ld, ld, 128);
+  if (rc == 0) rc = make_kmajor_map(&tv, v, 2, sk, ld, ld, 128);
+  if (rc) return rc;
+  return fa_launch(p, tq, tk, tv, dim3((sq + 2 * kFaTile - 1) / (2 * kFaTile), heads), 0, stream, nullptr, true);
+}
+
 static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid,
                      int int8, cudaStream_t stream, const FaPeerMaps* peers, bool direct) {
   static const FaPeerMaps no_peers{};
@@ -949,10 +1021,11 @@ static int fa_launch(const FaParams& p, const CUtensorMap& tq, const CUtensorMap
   const int qk_tile = int8 ? 128 * 128 : 128 * 128 * 2;
   const int stages = int8 ? 3 : 2;
   const int smem = 2 * qk_tile + stages * (qk_tile + 128 * 128 * 2) + static_cast<int>(sizeof(FaBarriers)) + 1024;
-  static PerDeviceOnce configured[4];
-  auto* kernel = int8 ? (direct ? attn_fa_kernel<true, true> : attn_fa_kernel<true, false>)
+  static PerDeviceOnce configured[5];
+  const bool quant = p.out_q[0] != nullptr;            // bf16 operands read in place only
+  auto* kernel = quant ? attn_fa_kernel<false, true, true> : int8 ? (direct ? attn_fa_kernel<true, true> : attn_fa_kernel<true, false>)
                       : (direct ? attn_fa_kernel<false, true> : attn_fa_kernel<false, false>);
-  if (configured[(int8 ? 2 : 0) + (direct ? 1 : 0)].first_time() &&
+  if (configured[quant ? 4 : (int8 ? 2 : 0) + (direct ? 1 : 0)].first_time() &&
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return -4;
   kernel<<<grid, kFaThreads, smem, stream>>>(p, tq, tk, tv, pm);

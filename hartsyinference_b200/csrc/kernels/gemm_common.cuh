@@ -161,6 +161,10 @@ struct GemmParams {
   uint8_t* glu_q;
   uint8_t* glu_sf;
   int glu_sf_rows;      // rows per block of the scale layout
+  // Quantised output (gemm_pair.cu): features from q_from on leave as e4m3 with 1x128 UE8M0 scales, in columns from q_col0 on of a
+  // matrix with rows q_ld bytes apart and q_kgroups scale words a row; the ones in front as bf16 to out
+  int q_from, q_col0, q_kgroups;
+  long long q_ld;
   int row_stores;       // large-token orientation: C (and bias, gate, residual) can be reached in 16-byte pieces
   int band;             // > 0, plain GEMM: tiles are walked in bands of this many A tiles (see decode_item)
 };
@@ -329,6 +333,25 @@ __device__ __forceinline__ void store_chunk_rows(const GemmParams& p, float (&v)
   __syncwarp();                                        // the strip is free for the next chunk
 }
 
+// 32 bytes a lane, one sector: what an epilogue of whole rows per lane writes without passing through shared memory, whose
+// 128 bytes a cycle the operands take (64 in by TMA, 64 out to the tensor core).
+__device__ __forceinline__ void store_words8(void* dst, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+__device__ __forceinline__ void load_words8(uint32_t* w, const void* src) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+               : "l"(src)
+               : "memory");
+}
+// Largest magnitude of 32 features, bf16 pairs
+__device__ __forceinline__ float words_max(const uint32_t (&y)[16], float mx) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(y[j] << 16)), fabsf(__uint_as_float(y[j] & 0xffff0000u))));
+  return mx;
+}
 // 32 features of act(gate) * up as bf16 pairs
 __device__ __forceinline__ void glu_words(const GemmParams& p, const uint32_t (&gate)[32], const uint32_t (&up)[32], uint32_t (&y)[16]) {
 #pragma unroll
@@ -403,6 +426,6 @@ int make_kmajor_map(CUtensorMap* out, const void* base, int elem_bytes, long lon
 int make_sf_map(CUtensorMap* out, const void* base, long long blocks);   // scale-factor blocks of 128 words; a box is one block
 // gemm_pair.cu: products on CTA pairs. p holds sizes, epilogue and scale factors; rows_a tokens, rows_b weight rows
 bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual);
-int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream);
+int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream, bool quant = false);
 
 }  // namespace b200

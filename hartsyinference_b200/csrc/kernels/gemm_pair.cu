@@ -85,19 +85,6 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// 32 bytes a lane, one sector: what an epilogue of whole rows per lane writes without passing through shared memory, whose
-// 128 bytes a cycle the operands take (64 in by TMA, 64 out to the tensor core).
-__device__ __forceinline__ void store_words8(void* dst, const uint32_t* w) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
-               "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
-}
-__device__ __forceinline__ void load_words8(uint32_t* w, const void* src) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-               : "l"(src)
-               : "memory");
-}
 // Epilogue of 32 columns from b0 on (all of them there) of one row: bias, activation, gate and residual, rounded to bf16 pairs.
 __device__ __forceinline__ void finish_row32(const GemmParams& p, const uint32_t (&r)[32], int row, int b0, uint32_t (&out)[16]) {
   uint32_t res[16];
@@ -161,7 +148,8 @@ struct alignas(16) PairBarriers {
 template <int kMode>
 constexpr int pair_stage_bytes() { return 2 * kStageBytesA + (kMode == 2 ? 2048 : 0); }
 
-template <int kMode, bool kGlu>
+// kQuant: see GemmParams::q_from. A warp's 128 columns are one group of a row's scales.
+template <int kMode, bool kGlu, bool kQuant = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb) {
@@ -370,9 +358,7 @@ gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, c
         if constexpr (kMx) {
           // the scale of a row's 128 features needs both halves, which sit in two warps: they exchange maxima behind a barrier of
           // their own, which a warp whose accumulator did not come still meets
-          float mx = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(y[j >> 4][j & 15] << 16)), fabsf(__uint_as_float(y[j >> 4][j & 15] & 0xffff0000u))));
+          float mx = words_max(y[1], words_max(y[0], 0.f));
           bars->amax[b][hsel * 128 + q * 32 + lane] = mx;
           asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
           mx = fmaxf(mx, bars->amax[b][(hsel ^ 1) * 128 + q * 32 + lane]);
@@ -391,6 +377,37 @@ gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, c
       } else if (ok) {
         tc_fence_after_sync();
         const int turn = holds_shared && b == 0 ? 3 : 0;
+        if constexpr (kQuant) {
+          const int group = tb * 256 + hsel * 128;
+          if (group >= p.q_from) {
+            uint32_t y[4][16];
+            float mx = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int c = hsel * 4 + ((u + turn) & 3);
+              uint32_t r[32];
+              tmem_ld_32x32(acc + c * 32, r);
+              tmem_ld_wait();
+              if (u == 0 && holds_shared) taken(true);
+              if (u == 3) taken(false);
+              if (group < p.rows_b) finish_row32(p, r, row, tb * 256 + c * 32, y[u]);
+              if (group < p.rows_b) mx = words_max(y[u], mx);
+            }
+            if (group < p.rows_b && row < p.rows_a) {
+              uint32_t eb;
+              const float inv = mx_scale_inv(mx, eb);
+              uint8_t* dst = p.glu_q + static_cast<long long>(row) * p.q_ld + p.q_col0 + (group - p.q_from);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                uint32_t w[8];
+                fp8_words(y[u], inv, w);
+                store_words8(dst + ((u + turn) & 3) * 32, w);
+              }
+              store_sf(p.glu_sf, row, (p.q_col0 + group - p.q_from) >> 7, 128, p.q_kgroups, eb);
+            }
+            continue;
+          }
+        }
 #pragma unroll 1
         for (int u = 0; u < 4; ++u) {
           const int c = hsel * 4 + ((u + turn) & 3), b0 = tb * 256 + c * 32;
@@ -429,12 +446,12 @@ gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, c
 }
 
 // ------------------------------------------------------------------------------------------ host side
-template <int kMode, bool kGlu>
+template <int kMode, bool kGlu, bool kQuant = false>
 static int launch_pair(const GemmParams& p, const CUtensorMap (&maps)[4], cudaStream_t stream) {
   const int smem = kPairStages * pair_stage_bytes<kMode>() + static_cast<int>(sizeof(PairBarriers)) + 1024;
   static PerDeviceOnce configured;
   if (configured.first_time()) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<kMode, kGlu>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<kMode, kGlu, kQuant>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return -static_cast<int>(e) - 200;
   }
   const int pairs = num_sms() / 2;
@@ -452,7 +469,7 @@ static int launch_pair(const GemmParams& p, const CUtensorMap (&maps)[4], cudaSt
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kMode, kGlu>, p, maps[0], maps[1], maps[2], maps[3]) != cudaSuccess) return -300;
+  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kMode, kGlu, kQuant>, p, maps[0], maps[1], maps[2], maps[3]) != cudaSuccess) return -300;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 300;
 }
@@ -478,7 +495,7 @@ bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long 
   return (3 * waves <= 5 * waves_one || k >= 3072) && (k >= 2048 || tiles > 36) && (tiles >= 32 || k <= 12288);
 }
 
-int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream) {
+int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream, bool quant) {
   const bool mx = dtype == 2, gated = p.glu_f > 0;
   const int esz = mx ? 1 : 2;
   p.num_tiles = (p.rows_a + 255) / 256 * (gated ? p.glu_f / 128 : (p.rows_b + 255) / 256);
@@ -489,8 +506,51 @@ int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long lo
   if (rc == 0 && mx) rc = make_sf_map(&maps[2], p.sf_a, (p.rows_a + 127ll) / 128 * p.sf_kgroups);
   if (rc == 0 && mx) rc = make_sf_map(&maps[3], p.sf_b, (p.rows_b + 127ll) / 128 * p.sf_kgroups);
   if (rc) return rc;
+  if (quant) return launch_pair<2, false, true>(p, maps, stream);
   if (mx) return gated ? launch_pair<2, true>(p, maps, stream) : launch_pair<2, false>(p, maps, stream);
   return gated ? launch_pair<0, true>(p, maps, stream) : launch_pair<0, false>(p, maps, stream);
 }
 
 }  // namespace b200
+
+using namespace b200;
+
+// Whether b200_gemm_quant takes m tokens by n features of depth k.
+B200_API int b200_gemm_quant_fits(int m, int n, int k) {
+  return m > 128 && n >= 128 && n % 128 == 0 && k >= 16 && k % 16 == 0 && pair_takes(m, n, k, 2, n, nullptr, nullptr) ? 1 : 0;
+}
+
+// act(x w^T + bias) of e4m3 operands with UE8M0 scales for a next product that reads e4m3: features from q_from on (a multiple of 128)
+// leave as e4m3 with 1x128 scales (rounded to bf16 first, as a quantisation of the stored product would find them) in columns from q_col0
+// on of out_q, rows q_ld bytes apart; scales in the blocked layout of q_kgroups words a row. The features in front leave as bf16 in
+// out [m][ldc]. What the quantisation kernel read and wrote stays away from memory: 4096 x 12288 of k 3072 with GELU 133 + 36 us -> 144,
+// 12288 features of 4608 x 21504 250 + 42 -> 259, 14040 x 13824 of k 5120 732 + 189 -> 827. act as in b200_gemm. -12: sizes or boundaries that it does not take.
+B200_API int b200_gemm_quant(const void* x, const void* w, void* out, void* out_q, void* out_sf, int m, int n, int k, long long ldx, long long ldw,
+                             long long ldc, const float* x_scale, const float* w_scale, const void* bias, int act, int q_from, long long q_ld,
+                             int q_col0, int q_kgroups, void* status, cudaStream_t stream) {
+  if (!b200_gemm_quant_fits(m, n, k) || q_from < 0 || q_from >= n || q_from % 128 != 0 || q_col0 < 0 || q_col0 % 128 != 0 || q_ld % 32 != 0 || !x_scale ||
+      !w_scale || !out_q || !out_sf || (q_from > 0 && (!out || ldc % 16 != 0)) || ldx % 16 != 0 || ldw % 16 != 0 || (act >> 8) % 8 != 0)
+    return -12;
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_q)) & 31) return -12;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(x_scale) |
+       reinterpret_cast<uintptr_t>(w_scale)) & 15)
+    return -12;
+  GemmParams p{};
+  p.k = k;
+  p.rows_a = m;
+  p.rows_b = n;
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.ldc = ldc;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.act = act & 255;
+  p.act_col = act >> 8;
+  p.status = static_cast<DeviceStatus*>(status);
+  p.glu_q = static_cast<uint8_t*>(out_q);
+  p.glu_sf = static_cast<uint8_t*>(out_sf);
+  p.q_from = q_from; p.q_ld = q_ld; p.q_col0 = q_col0; p.q_kgroups = q_kgroups;
+  p.row_stores = 1;
+  p.sf_a = reinterpret_cast<const uint32_t*>(x_scale);
+  p.sf_b = reinterpret_cast<const uint32_t*>(w_scale);
+  p.sf_kgroups = (k + 511) / 512;
+  return gemm_pair(p, x, w, ldx, ldw, 2, stream, true);
+}

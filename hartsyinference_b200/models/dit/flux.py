@@ -432,12 +432,16 @@ class FluxTransformer:
         # (ControlNet residual collection, the step cache) keeps the streams beyond the next block
         rp_fused = self._fused_rows(B * (S_i + S_t)) if (control is None and collect is None and step_cache is None) else None
 
+        # a projection that reads e4m3: the kernel in front can leave its output so
+        quant_ok = lambda w: B == 1 and self.tp == 1 and self.fp8 and x_i.is_cuda and isinstance(w, LinearWeight) and w.is_mx
+
         def stream_post(x, a, w: _StreamWeights, mod, S, slot):
             x = self._row_parallel(a, w.proj, x, mod[:, 2 * H:3 * H], S, rp_fused, slot)
             xn, _, xq = ops.norm(x, None, shift=mod[:, 3 * H:4 * H], scale=mod[:, 4 * H:5 * H], rows_per_batch=S,
                                  layernorm=True, emit_fp8=self.fp8 and w.mlp_in.is_fp8,
                                  emit_bf16=not (self.fp8 and w.mlp_in.is_fp8))
-            h = ops.linear(xq if xq is not None else xn, w.mlp_in, act="gelu_tanh")
+            h8 = ops.linear_quant(xq, w.mlp_in, act="gelu_tanh") if xq is not None and quant_ok(w.mlp_out) else None
+            h = h8[1] if h8 is not None else ops.linear(xq if xq is not None else xn, w.mlp_in, act="gelu_tanh")
             return self._row_parallel(h, w.mlp_out, x, mod[:, 5 * H:6 * H], S, rp_fused, slot + 1)
 
         whole = self.block_range == (0, cfg.num_double_blocks + cfg.num_single_blocks)
@@ -458,14 +462,18 @@ class FluxTransformer:
                 img_qkv, txt_qkv = stream_pre(x_i, wi, mod_i, S_i, cos_i, sin_i), stream_pre(x_t, wt, mod_t, S_t, cos_t, sin_t)
                 qkv = [torch.cat([torch.cat([a[i * S_t:(i + 1) * S_t], b[i * S_i:(i + 1) * S_i]], 0) for i in range(B)], 0)
                        for a, b in zip(txt_qkv, img_qkv)]
-            att = self._attend(*qkv, B)
-            if B == 1:
-                a_t, a_i = att[:S_t], att[S_t:]
+            if quant_ok(wi.proj) and quant_ok(wt.proj) and ops.attention_quant_fits(self.hl, self.hl, D, S):
+                a_t, a_i = (ops.empty_fp8_act(n, self.hl * D, self.device) for n in (S_t, S_i))
+                ops.attention_quant(*qkv, [(a_t, S_t, 0), (a_i, S_i, 0)])
+            elif B == 1:
+                att = self._attend(*qkv, B)
+                a_t, a_i = att[:S_t].contiguous(), att[S_t:].contiguous()
             else:
+                att = self._attend(*qkv, B)
                 a_t = torch.cat([att[i * S:i * S + S_t] for i in range(B)], 0)
                 a_i = torch.cat([att[i * S + S_t:(i + 1) * S] for i in range(B)], 0)
-            x_i = stream_post(x_i, a_i.contiguous(), wi, mod_i, S_i, 0)
-            x_t = stream_post(x_t, a_t.contiguous(), wt, mod_t, S_t, 2)
+            x_i = stream_post(x_i, a_i, wi, mod_i, S_i, 0)
+            x_t = stream_post(x_t, a_t, wt, mod_t, S_t, 2)
             if collect is not None:
                 collect[0].append(x_i)
             if control is not None and control[0]:
@@ -492,11 +500,18 @@ class FluxTransformer:
                                      emit_fp8=self.fp8 and w.qkv_mlp.is_fp8, emit_bf16=not (self.fp8 and w.qkv_mlp.is_fp8))
                 # [T, q | k | v | mlp]: the activation of the last part is the product's epilogue; once q, k and v are
                 # split off, the attention output takes the place of v, next to the part it is projected with
-                fused = ops.linear(xq if xq is not None else xn, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols)
+                split = ops.linear_quant(xq, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols, q_from=qkv_cols, lead=self.hl * D) \
+                    if xq is not None and quant_ok(w.out) and ops.attention_quant_fits(self.hl, self.hl, D, S) else None
+                fused = split[0] if split is not None else ops.linear(xq if xq is not None else xn, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols)
                 q, k, v = ops.dit_qkv(fused[:, :qkv_cols], self.hl, self.hl, D, q_norm_w=w.q_norm, k_norm_w=w.k_norm,
                                       cos=cj, sin=sj)
-                self._attend(q, k, v, B, out=fused[:, qkv_cols - self.hl * D:qkv_cols])
-                joint = self._row_parallel(fused[:, qkv_cols - self.hl * D:], w.out, joint, mod[:, 2 * H:3 * H], S, rp_fused, si & 1)
+                if split is not None:                # [T, attention | mlp] as e4m3, each part by the kernel that forms it
+                    a = split[1]
+                    ops.attention_quant(q, k, v, [(a, S, 0)])
+                else:
+                    self._attend(q, k, v, B, out=fused[:, qkv_cols - self.hl * D:qkv_cols])
+                    a = fused[:, qkv_cols - self.hl * D:]
+                joint = self._row_parallel(a, w.out, joint, mod[:, 2 * H:3 * H], S, rp_fused, si & 1)
                 if collect is not None or (control is not None and control[1]):
                     img_rows = slice(S_t, S) if B == 1 else None
                     if img_rows is None:

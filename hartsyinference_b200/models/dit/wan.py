@@ -180,6 +180,14 @@ class WanTransformer:
                 f.close()
         self._fused_exchange.clear()
 
+    def _attend_quant(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w) -> Optional[ops.Fp8Act]:
+        """Attention whose output ``w`` reads as e4m3, or None where it cannot leave so."""
+        if not (self.fp8 and q.is_cuda and isinstance(w, LinearWeight) and w.is_mx and ops.attention_quant_fits(q.shape[1], k.shape[1], q.shape[2], k.shape[0])):
+            return None
+        o = ops.empty_fp8_act(q.shape[0], q.shape[1] * q.shape[2], q.device)
+        ops.attention_quant(q, k, v, [(o, q.shape[0], 0)])
+        return o
+
     def _self_attention(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
         """q, k, v [S_local, heads, D] -> [S_local, heads * D]."""
         if self.sp == 1:
@@ -231,21 +239,26 @@ class WanTransformer:
             qkv = ops.linear(xq if xq is not None else xn, blk.qkv)                           # [S_l, 3H]
             q, k, v = ops.dit_qkv(qkv, heads, heads, D, q_norm_w=blk.norm_q, k_norm_w=blk.norm_k, cos=cos, sin=sin, eps=cfg.eps,
                                   row_norm=True)
-            att = self._self_attention(q, k, v)
+            att = self._attend_quant(q, k, v, blk.o) if self.sp == 1 else None
+            if att is None:
+                att = self._self_attention(q, k, v)
             x = ops.linear(att, blk.o, gate=m[0, 2 * H:3 * H].contiguous(), residual=x)
             # cross-attention to the text tokens (no gate, affine LayerNorm)
-            xn, _, _ = ops.norm(x, blk.norm3_w, bias=blk.norm3_b, layernorm=True, eps=cfg.eps)
-            cq, _, _ = ops.norm(ops.linear(xn, blk.cq), blk.cnorm_q, eps=cfg.eps)
+            xn, _, xq = ops.norm(x, blk.norm3_w, bias=blk.norm3_b, layernorm=True, eps=cfg.eps, emit_fp8=self.fp8 and blk.cq.is_fp8,
+                                 emit_bf16=not (self.fp8 and blk.cq.is_fp8))
+            cq, _, _ = ops.norm(ops.linear(xq if xq is not None else xn, blk.cq), blk.cnorm_q, eps=cfg.eps)
             ckv = ops.linear(context, blk.ckv)
             ck, _, _ = ops.norm(ckv[:, :H].contiguous(), blk.cnorm_k, eps=cfg.eps)
             L = context.shape[0]
-            co = ops.attention(cq.reshape(S_l, heads, D), ck.reshape(L, heads, D), ckv[:, H:].reshape(L, heads, D).contiguous())
-            x = ops.linear(co.reshape(S_l, H), blk.co, residual=x)
+            cross = cq.reshape(S_l, heads, D), ck.reshape(L, heads, D), ckv[:, H:].reshape(L, heads, D).contiguous()
+            co = self._attend_quant(*cross, blk.co)
+            x = ops.linear(co if co is not None else ops.attention(*cross).reshape(S_l, H), blk.co, residual=x)
             # feed-forward
             xn, _, xq = ops.norm(x, None, shift=m[:, 3 * H:4 * H], scale=m[:, 4 * H:5 * H], rows_per_batch=S_l,
                                  layernorm=True, eps=cfg.eps, emit_fp8=self.fp8 and blk.ffn_in.is_fp8,
                                  emit_bf16=not (self.fp8 and blk.ffn_in.is_fp8))
-            h = ops.linear(xq if xq is not None else xn, blk.ffn_in, act="gelu_tanh")
+            h8 = ops.linear_quant(xq, blk.ffn_in, act="gelu_tanh") if xq is not None and blk.ffn_out.is_mx else None
+            h = h8[1] if h8 is not None else ops.linear(xq if xq is not None else xn, blk.ffn_in, act="gelu_tanh")
             x = ops.linear(h, blk.ffn_out, gate=m[0, 5 * H:6 * H].contiguous(), residual=x)
         hm = (self.head_mod.float() + e.float()).to(dt).reshape(1, 2 * H).contiguous()         # shift, scale
         xn, _, _ = ops.norm(x, None, shift=hm[:, 0:H], scale=hm[:, H:2 * H], rows_per_batch=S_l, layernorm=True, eps=cfg.eps)

@@ -13,6 +13,8 @@ from .core import (  # noqa: F401
     LinearWeight,
     argmax,
     attention,
+    attention_quant,
+    attention_quant_fits,
     attn_decode,
     attn_paged_biased,
     attn_prefill_paged,
@@ -21,6 +23,7 @@ from .core import (  # noqa: F401
     colbatched_linear,
     dit_qkv,
     embedding,
+    empty_fp8_act,
     few_fits,
     fill_random_,
     fp8_mx,
@@ -38,6 +41,7 @@ from .core import (  # noqa: F401
     moe_dispatch,
     moe_route,
     linear,
+    linear_quant,
     mla_attn,
     mla_prep,
     cfg_renorm_euler_step,

@@ -227,6 +227,11 @@ def quant_fp8_act(x: torch.Tensor, tile_rows: int = 128, mx: Optional[bool] = No
     return Fp8Act(q, s)
 
 
+def empty_fp8_act(rows: int, k: int, device) -> Fp8Act:
+    """e4m3 activations with UE8M0 scales that kernels write in parts (``linear_quant``, ``attention_quant``)."""
+    return Fp8Act(torch.empty(rows, k, dtype=torch.uint8, device=device), None, _alloc_sf(rows, k, 128, device), 128)
+
+
 def quant_fp8_weight(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     """bf16 [N, K] -> (e4m3 bytes, scales [ceil(N/128), K/128]) with one scale per 128x128 block."""
     if not w.is_cuda or fp8_mx():
@@ -345,6 +350,28 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
                      ws.data_ptr(), ws.numel(), st.status.data_ptr(), N.stream())
     N.check(rc, "b200_gemm")
     return out
+
+
+def linear_quant(x, w, act: Optional[str] = None, act_from: int = 0, q_from: int = 0, lead: int = 0):
+    """``linear(x, w, act, act_from=act_from)`` of e4m3 operands in UE8M0 mode for a next product that reads e4m3: ``(y, q)`` with
+    the output features in front of ``q_from`` as bf16 y (None: there are none) and the others as :class:`Fp8Act` q, in its
+    columns from ``lead`` on (the ones in front are for another kernel to write). The same values as a quantisation of the
+    stored product. None, and nothing is done, where the product has no such form (few tokens, other operands)."""
+    if not (isinstance(x, Fp8Act) and isinstance(w, LinearWeight) and x.data.is_cuda and w.is_mx and x.sf is not None and x.tile_rows == 128):
+        return None
+    (m, k), n, xd = x.data.shape, w.weight.shape[0], x.data
+    if q_from % 128 or lead % 128 or w.weight.shape[1] != k or xd.stride(1) != 1 or w.weight.stride(1) != 1 or not N.lib().b200_gemm_quant_fits(m, n, k):
+        return None
+    y = torch.empty(m, q_from, dtype=torch.bfloat16, device=xd.device) if q_from else None
+    q = empty_fp8_act(m, lead + n - q_from, xd.device)
+    xs, ws = _scale_ptrs(x, w)
+    rc = N.lib().b200_gemm_quant(xd.data_ptr(), w.weight.data_ptr(), N.ptr(y), q.data.data_ptr(), q.sf.data_ptr(), m, n, k, xd.stride(0),
+                                 w.weight.stride(0), q_from, xs, ws, N.ptr(w.bias), act_code(act, act_from), q_from, q.data.stride(0), lead,
+                                 q.sf.shape[1], N.state(xd.device).status.data_ptr(), N.stream())
+    if rc == -12:                                    # boundaries that it does not take
+        return None
+    N.check(rc, "b200_gemm_quant")
+    return y, q
 
 
 def norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, *, bias: Optional[torch.Tensor] = None,
@@ -719,6 +746,32 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
                                    scale, softcap, N.stream())
     N.check(rc, "b200_attn_prefill")
     return dst
+
+
+def attention_quant_fits(hq: int, hkv: int, d: int, keys: int) -> bool:
+    """Whether dense attention of these sizes, in the modes that are set, can leave its output as e4m3 with UE8M0 scales."""
+    from .. import config
+    return (d == 128 and hq == hkv and keys >= 256 and fp8_mx() and _tc_attention() and bool(config.get("fa_attention"))
+            and not config.get("sage_attention"))
+
+
+def attention_quant(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, parts: list, scale: Optional[float] = None) -> None:
+    """``attention(q, k, v)`` (bidirectional, one sequence, ``attention_quant_fits``) with the output rows as e4m3 for products that read
+    it so. ``parts``: one or two (:class:`Fp8Act` from ``empty_fp8_act``, rows, first column): the first ``rows`` query rows go to
+    the columns of the first from that one on, the rest to the second. The same values as a quantisation of the stored output."""
+    tq, hq, d = q.shape
+    tk, hkv, _ = k.shape
+    if not (attention_quant_fits(hq, hkv, d, tk) and q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.is_contiguous()
+            and k.is_contiguous() and v.is_contiguous() and v.data_ptr() % 16 == 0 and sum(r for _, r, _ in parts) == tq
+            and all(a.sf is not None and a.tile_rows == 128 and a.data.shape[0] == r and c % 128 == 0 and c + hq * d <= a.data.shape[1] for a, r, c in parts)):
+        raise ValueError("attention_quant: sizes, types or layouts that it does not take")
+    args = []
+    for a, _, c in parts:
+        args += [a.data.data_ptr(), a.sf.data_ptr(), a.data.stride(0), c, a.sf.shape[1]]
+    args += [None, None, 0, 0, 0] * (2 - len(parts))
+    rc = N.lib().b200_attn_fa_quant(q.data_ptr(), k.data_ptr(), v.data_ptr(), tq, tk, hq, float(1.0 / math.sqrt(d) if scale is None else scale),
+                                    parts[0][1], *args, N.state(q.device).status.data_ptr(), N.stream())
+    N.check(rc, "b200_attn_fa_quant")
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) -> torch.Tensor:

@@ -125,3 +125,45 @@ def test_gated_tiles_fp8(m, f, k, act):
     assert ((got - ref).abs() <= ref.abs() * (2 ** -4 + 2 ** -7) + s * 2 ** -10 + 2 ** -9).all()
     mx = ref.abs().reshape(m, -1, 128).amax(-1)
     assert (q.scales_fp32().cpu() * 448 * (1 + 2 ** -6) + 2 ** -9 >= mx).all() and (q.scales_fp32().cpu() * 448 <= 2 * (1 + 2 ** -6) * mx + 2 ** -8).all()
+
+
+# products and attention that leave e4m3: the same bytes and scales as a quantisation of what they store otherwise
+@pytest.mark.parametrize("m,n,k,q_from,lead", [(256, 9472, 2048, 0, 0), (300, 12416, 3072, 0, 256), (2049, 2432, 4096, 0, 0), (1651, 4224, 2048, 1408, 384), (4100, 1280, 4096, 1152, 128)])
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+def test_quantised_product(m, n, k, q_from, lead, act):
+    if not ops.fp8_mx():
+        pytest.skip("block scales in fp32")
+    torch.manual_seed(m)
+    x = ops.quant_fp8_act(torch.randn(m, k, device="cuda").to(torch.bfloat16))
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16), torch.randn(n, device="cuda").to(torch.bfloat16), fp8=True)
+    y, q = ops.linear_quant(x, w, act=act, act_from=q_from if act else 0, q_from=q_from, lead=lead)
+    ref = ops.linear(x, w, act=act, act_from=q_from if act else 0)
+    assert (y is None) == (q_from == 0) and (y is None or torch.equal(y, ref[:, :q_from]))
+    want = ops.quant_fp8_act(ref[:, q_from:].contiguous())
+    assert torch.equal(q.data[:, lead:], want.data) and torch.equal(q.scales_fp32()[:, lead // 128:], want.scales_fp32())
+
+
+def test_small_products_are_not_quantised_in_place():
+    if not ops.fp8_mx():
+        pytest.skip("block scales in fp32")
+    w = ops.LinearWeight.from_dense(torch.randn(4096, 1024, device="cuda").to(torch.bfloat16), fp8=True)
+    x = torch.randn(1000, 1024, device="cuda").to(torch.bfloat16)
+    assert ops.linear_quant(ops.quant_fp8_act(x[:128]), w) is None and ops.linear_quant(x, w) is None
+    assert ops.linear_quant(ops.quant_fp8_act(x), w, q_from=64) is None
+
+
+@pytest.mark.parametrize("tq,tk,h,split,col", [(257, 256, 3, 257, 0), (600, 600, 2, 88, 128), (1000, 300, 1, 512, 0), (130, 777, 5, 130, 640)])
+def test_quantised_attention(tq, tk, h, split, col):
+    if not ops.attention_quant_fits(h, h, 128, tk):
+        pytest.skip("attention leaves bf16 in this mode")
+    torch.manual_seed(tq)
+    q = torch.randn(tq, h, 128, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn(tk, h, 128, device="cuda").to(torch.bfloat16) for _ in range(2))
+    sizes = [split, tq - split] if split < tq else [tq]
+    parts = [(ops.empty_fp8_act(r, h * 128 + col + 128 * i, "cuda"), r, col + 128 * i) for i, r in enumerate(sizes)]
+    ops.attention_quant(q, k, v, parts)
+    ref, at = ops.attention(q, k, v).reshape(tq, -1), 0
+    for a, r, c in parts:
+        want = ops.quant_fp8_act(ref[at:at + r].contiguous())
+        assert torch.equal(a.data[:, c:c + h * 128], want.data) and torch.equal(a.scales_fp32()[:, c // 128:c // 128 + h], want.scales_fp32())
+        at += r
