@@ -137,6 +137,10 @@ struct GemmParams {
   int num_tiles;
   int splits;
   int kblocks_per_split;
+  // > 0: even shares (small-token orientation, more tiles than CTAs): CTA c takes the c-th of share_ctas equal parts of all tiles'
+  // K groups in a row (share_groups a tile, share_kblocks k-blocks each). A share holds a tile at least, so a tile is cut by one
+  // boundary between shares at most; its two pieces meet in slot c = the CTA of the first one
+  int share_ctas, share_groups, share_kblocks;
   float* split_ws;          // [split tiles][splits][BN][128] fp32 partials
   uint32_t* split_counter;  // [split tiles], zero between launches
   long long ldc;            // leading dimension of C in elements

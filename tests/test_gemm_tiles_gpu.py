@@ -167,3 +167,24 @@ def test_quantised_attention(tq, tk, h, split, col):
         want = ops.quant_fp8_act(ref[at:at + r].contiguous())
         assert torch.equal(a.data[:, c:c + h * 128], want.data) and torch.equal(a.scales_fp32()[:, c // 128:c // 128 + h], want.scales_fp32())
         at += r
+
+
+# few tokens, more tiles than SMs: even shares of K groups, whose boundaries cut tiles into two pieces; rows of one group, ragged
+# groups, features that end inside a tile, every epilogue, and the same again from the counters that the first launch left
+@pytest.mark.parametrize("m,n,k", [(5, 19200, 640), (64, 28411, 1024), (17, 44416, 136), (128, 28672, 4096), (100, 24576, 1536), (33, 19100, 72), (1, 38528, 9216)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("act", [None, "silu", "gelu_tanh", "tanh"])
+def test_even_shares(m, n, k, fp8, act):
+    torch.manual_seed(m)
+    k = -(-k // 128) * 128 if fp8 else k
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    vec = lambda: torch.randn(n, device="cuda").to(torch.bfloat16) if act else None
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16), vec(), fp8=fp8)
+    gate = vec()
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16) if act else None
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    y = ops.linear(xq, w, act=act, act_from=8 if act == "tanh" else 0, gate=gate, residual=res)
+    ref = R.linear(xq.data if fp8 else x, w.weight, w.scale, xq.scales_fp32() if fp8 else None, w.bias, act, gate, res, torch.float32,
+                   act_from=8 if act == "tanh" else 0)
+    assert torch.allclose(y.float(), ref, rtol=2 ** -7, atol=2 ** -7), (y.float() - ref).abs().max()      # one rounding to bf16; fp32 sums
+    assert torch.equal(ops.linear(xq, w, act=act, act_from=8 if act == "tanh" else 0, gate=gate, residual=res), y)
