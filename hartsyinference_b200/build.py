@@ -47,7 +47,7 @@ NVCC_FLAGS = [
 # sources that make a smaller library for one kind of model; what a source uses of another one is in gemm_tcgen05.cu
 # (the launch switch, the number of processors, tensor maps) or used by it (gemv_bf16)
 KERNEL_GROUPS = {
-    "decoder": ("gemm_tcgen05", "gemm_pair", "gemv_bf16", "attention", "attention_pf", "delta", "delta_general", "fused_ops", "latent", "linear_f32", "mla", "moe", "residual_norm", "rotary", "sampling", "ssm"),
+    "decoder": ("gemm_tcgen05", "gemm_pair", "gemv_bf16", "attention", "attention_pf", "delta", "delta_general", "dense_layers", "fused_ops", "latent", "linear_f32", "mla", "moe", "residual_norm", "rotary", "sampling", "ssm"),
 }
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function", "-pthread"]
 

@@ -28,6 +28,7 @@ import torch
 from ... import config, ops
 from ...ops import LinearWeight
 from ...parallel.comm import Comm, SingleComm
+from ...utils import profiling
 from .config import RopeScaling, TransformerConfig, mixed_design
 from .rope import build_inv_freq
 
@@ -1043,23 +1044,42 @@ class DecoderModel:
             h = ex.reduce(res, self.final_norm if li == last else self.layers[li + 1].in_norm, cfg.rms_eps)
         return self.comm.all_gather(h.contiguous(), dim=0)
 
+    def _plain_stack(self, batch: ForwardBatch, x: torch.Tensor) -> bool:
+        """True when this pass runs all layers of a plain stack with bf16 weights on one device: norms, projections and a gated
+        feed-forward without extras of any kind."""
+        cfg = self.cfg
+        if (not x.is_cuda or self.tp > 1 or self.fp8 or cfg.residual_multiplier != 1.0 or cfg.mixed_layers or not (self.first_stage and self.last_stage)
+                or self.alibi_slopes is not None or self.inv_freq_local is not None or batch.slot_mapping is None or self.kv_cache is None
+                or not x.is_contiguous() or batch.positions.dtype != torch.int32 or batch.slot_mapping.dtype != torch.int64
+                or self.inv_freq.dtype != torch.float32 or self.kv_cache.dim() != 6 or not self.kv_cache.is_contiguous() or cfg.rotary_dim % 2):
+            return False
+        rows = (self.hq + 2 * self.hkv) * cfg.head_dim
+        return all(lw.ffn_module is None and lw.attn_module is None and lw.sinks is None and lw.q_norm is None and lw.k_norm is None
+                   and lw.post_attn_norm is None and lw.post_ffn_norm is None and isinstance(lw.in_norm, torch.Tensor) and isinstance(lw.post_norm, torch.Tensor)
+                   and all(isinstance(w, LinearWeight) and not w.is_fp8 for w in (lw.qkv, lw.o, lw.gate_up, lw.down))
+                   and lw.qkv.weight.shape[0] == rows and (lw.qkv.bias is None or lw.qkv.bias.dtype == torch.bfloat16) and lw.gate_up.bias is None
+                   for lw in self.layers)
+
     def _few_ok(self, batch: ForwardBatch, x: torch.Tensor) -> bool:
-        """True when this decode step is one token through a plain stack of bf16 layers, whose products take the norm in front of
+        """True when this decode step is one token through a plain stack, whose products take the norm in front of
         them along (five launches a layer instead of eight). One token: 24 layers of 896 features 630 -> 488 us, four of 4096
         features 375 both; two tokens 751 -> 750 and 408 -> 421, so they stay with the kernels apart."""
+        return (batch.is_decode and x.shape[0] == 1 and self._plain_stack(batch, x)
+                and all(ops.few_fits(x, lw.in_norm, lw.qkv) and ops.few_fits(x, lw.post_norm, lw.gate_up) for lw in self.layers))
+
+    def _prompt_layers(self, batch: ForwardBatch, x: torch.Tensor) -> Optional[torch.Tensor]:
+        """A batch of prompt tokens through a plain stack by ``ops.dense_prompt_layers``, or None: the same kernels as the loop of
+        ``forward_hidden`` launches, which stays where every op is to be timed on its own."""
         cfg = self.cfg
-        if (not batch.is_decode or not x.is_cuda or x.shape[0] != 1 or self.tp > 1 or self.fp8 or cfg.residual_multiplier != 1.0
-                or cfg.mixed_layers or not (self.first_stage and self.last_stage) or self.alibi_slopes is not None
-                or self.inv_freq_local is not None or batch.slot_mapping is None or self.kv_cache is None or not x.is_contiguous()):
-            return False
-        if (batch.positions.dtype != torch.int32 or batch.slot_mapping.dtype != torch.int64 or self.inv_freq.dtype != torch.float32
-                or self.kv_cache.dim() != 6 or not self.kv_cache.is_contiguous() or cfg.rotary_dim % 2):
-            return False
-        fits, rows = ops.few_fits, (self.hq + 2 * self.hkv) * cfg.head_dim
-        return all(lw.ffn_module is None and lw.attn_module is None and lw.sinks is None and lw.q_norm is None and lw.k_norm is None
-                   and lw.post_attn_norm is None and lw.post_ffn_norm is None and fits(x, lw.in_norm, lw.qkv) and fits(x, lw.post_norm, lw.gate_up)
-                   and lw.qkv.weight.shape[0] == rows and (lw.qkv.bias is None or lw.qkv.bias.dtype == torch.bfloat16) and lw.gate_up.bias is None
-                   and isinstance(lw.o, LinearWeight) and isinstance(lw.down, LinearWeight) for lw in self.layers)
+        if (batch.is_decode or batch.cu_q is None or profiling.active() or cfg.attn_softcap > 0 or cfg.sliding_window > 0 or cfg.activation not in ("silu", "gelu_tanh")
+                or not cfg.gated_ffn or not self._plain_stack(batch, x) or any(lw.o.bias is not None or lw.down.bias is not None for lw in self.layers)):
+            return None
+        layers = [(lw.in_norm, lw.qkv.weight, lw.qkv.bias, lw.o.weight, lw.post_norm, lw.gate_up.weight, lw.down.weight) for lw in self.layers]
+        return ops.dense_prompt_layers(x, layers, self.final_norm, self.kv_cache, batch.block_table, batch.kv_lens, batch.cu_q, batch.positions,
+                                       batch.slot_mapping, self.inv_freq, hq=self.hq, max_q_len=batch.max_q_len,
+                                       max_kv_len=batch.max_kv_len or batch.block_table.shape[1] * self.kv_cache.shape[4], rot=cfg.rotary_dim,
+                                       style=cfg.rope_style, theta=cfg.rope_theta, act=cfg.activation, eps=cfg.rms_eps, scale=self._attn_scale(),
+                                       weight_plus_one=cfg.norm_plus_one)
 
     def _forward_few(self, batch: ForwardBatch, x: torch.Tensor) -> torch.Tensor:
         """Layer loop of one decoded token (``_few_ok``): norm + qkv + rotation and cache write, attention, o + residual,
@@ -1110,6 +1130,10 @@ class DecoderModel:
 
         if hidden_in is None and self._few_ok(batch, x):
             return self._forward_few(batch, x)
+        if hidden_in is None:
+            out = self._prompt_layers(batch, x)
+            if out is not None:
+                return out
 
         # small batches: what goes straight into a norm is left as unsummed K ranges that the norm adds
         rows, on_device = x.shape[0], x.is_cuda

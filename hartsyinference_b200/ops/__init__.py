@@ -21,6 +21,7 @@ from .core import (  # noqa: F401
     causal_conv3d,
     cfg_euler_step,
     colbatched_linear,
+    dense_prompt_layers,
     dit_qkv,
     embedding,
     empty_fp8_act,

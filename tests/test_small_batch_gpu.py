@@ -149,3 +149,34 @@ def test_one_token_through_the_stack():
         # two layers of bf16 roundings that fall differently (one sum is no longer rounded ahead of the residual add)
         assert (y.float() - ref.float()).norm() <= 2e-2 * ref.float().norm()
         assert (cache.float() - model.kv_cache.float()).norm() <= 2e-3 * model.kv_cache.float().norm()
+
+
+# prompts through a plain stack: the same kernels whether the library or the loop of ops walks the layers, at the sizes where their choices
+# change (handful, ranges left unsummed, pair tiles, either attention kernel)
+@pytest.mark.parametrize("preset", ["qwen2.5-0.5b", "llama-3-8b"])
+@pytest.mark.parametrize("lens,held", [([1], 0), ([3], 5), ([17, 5, 7], 0), ([100, 28], 30), ([129], 0), ([700, 64, 260], 16)])
+def test_prompts_by_the_library_and_by_ops(preset, lens, held):
+    cfg = replace(C.PRESETS[preset], num_layers=2, vocab_size=512)
+    model = DecoderModel(cfg, "cuda")
+    model.random_init(seed=2)
+    per = [(n + held + 15) // 16 for n in lens]
+    model.alloc_kv(sum(per), 16)
+    model.kv_cache.normal_()
+    g = torch.Generator().manual_seed(3)
+    order, table, at = torch.randperm(sum(per), generator=g).to(torch.int32), torch.zeros(len(lens), max(per), dtype=torch.int32), 0
+    for i, c in enumerate(per):
+        table[i, :c] = order[at:at + c]
+        at += c
+    pos = torch.cat([torch.arange(held, held + n) for n in lens])
+    seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens))
+    slots = table[seq, pos // 16].long() * 16 + pos % 16
+    dev = lambda t, dt=torch.int32: torch.as_tensor(t).to(dt).cuda()
+    batch = ForwardBatch(tokens=dev(torch.randint(0, 512, (sum(lens),), generator=g)), positions=dev(pos), slot_mapping=dev(slots, torch.int64), block_table=dev(table),
+                         kv_lens=dev([n + held for n in lens]), is_decode=False, cu_q=dev(torch.tensor([0] + lens).cumsum(0)), max_q_len=max(lens),
+                         max_kv_len=max(lens) + held)
+    assert model._plain_stack(batch, torch.zeros(1, cfg.hidden_size, dtype=torch.bfloat16, device="cuda"))
+    before = model.kv_cache.clone()
+    y, cache = model.forward_hidden(batch), model.kv_cache.clone()
+    model.kv_cache.copy_(before)
+    model._prompt_layers = lambda *a: None
+    assert torch.equal(model.forward_hidden(batch), y) and torch.equal(model.kv_cache, cache)
