@@ -65,6 +65,36 @@ def test_decode_window_softcap():
     assert torch.allclose(out.float().cpu(), ref.float(), rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("b,hq,hkv,most", [(70, 64, 8, 1200), (16, 32, 32, 1100), (300, 16, 1, 4000), (150, 12, 4, 3000)])
+def test_decode_in_even_shares(b, hq, hkv, most, window):
+    """Lengths of nothing, one key, whole tiles and long runs; a tile of the sums per key head and block. Probabilities in bf16
+    (2^-9 each, of values up to about 2) and the bf16 result: 2e-2 as for the split form."""
+    from hartsyinference_b200.ops import _native as N
+    assert N.lib().b200_attn_decode_even_bytes(b, hq, hkv, 128, most) > 0
+    torch.manual_seed(b)
+    page, max_pages = 16, (most + 15) // 16
+    kc, vc = _pool(512, hkv, page, 128)
+    lens = torch.randint(1, most + 1, (b,), dtype=torch.int32)
+    lens[:8] = torch.tensor([0, 1, 63, 64, 65, 128, most, 0])
+    lens[-1] = 0
+    table = torch.randint(0, 512, (b, max_pages), dtype=torch.int32, device="cuda")
+    q = torch.randn(b, hq, 128, device="cuda").to(torch.bfloat16)
+    dev = lens.cuda()
+    out, o8 = ops.attn_decode(q, kc, vc, table, dev, window=window, max_kv_len=most, emit_fp8=True)
+    split = ops.attn_decode(q, kc, vc, table, dev, window=window, splits=2)
+    assert (out.float() - split.float()).abs().max() <= 2e-2
+    assert (out[dev == 0] == 0).all()
+    pick = [0, 1, 3, 4, 6, b // 2, b - 2, b - 1]
+    ref = ops.attn_decode(q[pick].cpu(), kc.cpu(), vc.cpu(), table[pick].cpu(), lens[pick].clamp(min=1), window=window).float()
+    ref[[0, 7]] = 0
+    assert torch.allclose(out[pick].float().cpu(), ref, rtol=2e-2, atol=2e-2)
+    deq = R.dequant_fp8_act(o8.data, o8.scales_fp32()).reshape(out.shape)
+    assert (deq - out.float()).norm() <= 5e-2 * out.float().norm()
+    again = ops.attn_decode(q, kc, vc, table, dev, window=window, max_kv_len=most)
+    assert torch.equal(again, out)
+
+
 @pytest.mark.parametrize("d,hq,hkv", [(128, 8, 2), (64, 14, 2)])
 def test_prefill_paged_chunked(d, hq, hkv):
     torch.manual_seed(2)
