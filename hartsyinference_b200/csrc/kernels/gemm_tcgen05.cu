@@ -24,9 +24,11 @@
 // Work items. Output tiles are dealt round-robin to the CTAs. When the tile count is not a
 // multiple of the grid, the tiles of the last, partial wave are split along K so that this wave
 // also covers every SM (a bandwidth-bound GEMM otherwise loses up to half its throughput to wave
-// quantisation); after full waves of 128 x 256 tiles only where rows are long. The CTAs of a split tile write fp32 partials to a scratch buffer and bump a
-// counter; whoever arrives last sums the partials in split order (deterministic) and runs the
-// epilogue. A GEMM with fewer tiles than SMs is split completely; its partials are summed by a
+// quantisation); after full waves of 128 x 256 tiles only where rows are long. The CTAs of a split tile
+// write fp32 partials to a scratch buffer and bump a counter; whoever arrives last sums the partials in
+// split order (deterministic) and runs the epilogue. With few tokens, full waves and a last wave that is
+// less than half full, every CTA takes an equal share of all tiles' K blocks instead (the rule stands by
+// the launch); a tile that two shares cut is finished by the CTA whose share starts it. A GEMM with fewer tiles than SMs is split completely; its partials are summed by a
 // second, machine-wide kernel (splitk_reduce_kernel) or, optionally, through the distributed
 // shared memory of a thread-block cluster (measured slower, off by default).
 //
@@ -1541,7 +1543,7 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
     a_ptr = x; lda = ldx; b_ptr = w; ldb = ldw;
     bn = fp8 && !i8 ? 128 : 256;
     // A 128 x 256 tile reads three quarters of the operand bytes per product of two 128 x 128 ones, which is
-    // what bounds one-byte operands (8192 x 57344 x 8192: 1.59 -> 2.32 PFLOP/s), but it fills the 512 columns of
+    // what bounds one-byte operands (8192 x 57344 x 8192: 1.59 -> 2.32 PFLOP/s; pair tiles 2.9, see pair_takes), but it fills the 512 columns of
     // TMEM with one accumulator and the scale factors; below one tile per SM the smaller ones balance
     // better (512 x 9216 x 3072: 30 us against 42 us with the larger tiles cut along K).
     if (mx && ar == nullptr && ag == nullptr &&
