@@ -31,6 +31,8 @@
 
 namespace b200 {
 
+int num_sms();      // of the current device, see gemm_tcgen05.cu
+
 constexpr int kTileTokens = 64;
 constexpr int kAttnThreads = 128;
 
@@ -975,11 +977,17 @@ B200_API long long b200_attn_decode_workspace_bytes(int seqs, int hq, int d, int
 
 static int g_decode_stages = 2;
 
-// Blocks of the decode kernel that the chip holds at once.
-static int decode_blocks() { return 148 * (g_decode_stages == 2 ? 3 : 2); }
+// Blocks of the decode kernel that the chip holds at once, with a ring of `stages` tiles.
+static int decode_blocks(int stages) { return num_sms() * (stages == 2 ? 3 : 2); }
+
+// Workspace of even shares on `slots` blocks: a row of sums per query head and piece, the first and last block of every key head
+static long long even_bytes(int slots, int seqs, int hq, int hkv, int d) {
+  const long long units = static_cast<long long>(seqs) * hkv;
+  return (slots + units) * (hq / hkv) * (d + 2) * 4 + units * 8;
+}
 
 // Number of KV splits for a decode batch, from a wave model fitted to B200 timings: the grid runs
-// in waves of (148 SMs x resident CTAs) and a CTA costs its tiles plus about four tiles' worth of
+// in waves of (SMs x resident CTAs) and a CTA costs its tiles plus about four tiles' worth of
 // prologue and merge, so the estimate is waves x (ceil(tiles / splits) + 4); ties go to fewer
 // splits (less partial traffic and a cheaper combine). Measured with the two-tile ring, 64-token
 // tiles, 2304-token contexts (CTAs before splitting: best splits, time): 16: 12, 13.5 us;
@@ -988,7 +996,7 @@ static int decode_blocks() { return 148 * (g_decode_stages == 2 ? 3 : 2); }
 B200_API int b200_attn_decode_pick_splits(int seqs, int hkv, int max_kv_len) {
   const int ctas = seqs * hkv > 0 ? seqs * hkv : 1;
   const int tiles = (max_kv_len + kTileTokens - 1) / kTileTokens;
-  const int slots = decode_blocks();
+  const int slots = decode_blocks(g_decode_stages);
   int best = 1;
   long long best_cost = -1;
   for (int sp = 1; sp <= 16 && sp <= tiles; ++sp) {
@@ -1017,23 +1025,27 @@ B200_API void b200_attn_set_decode_stages(int stages) { g_decode_stages = stages
 // Head size 64 keeps its splits: more than three of its blocks fit an SM, which this count of blocks does not know.
 B200_API long long b200_attn_decode_even_bytes(int seqs, int hq, int hkv, int d, int max_kv_len) {
   if (d != 128 || hkv <= 0 || hq % hkv != 0 || hq / hkv > 16) return 0;
-  const int slots = decode_blocks(), splits = b200_attn_decode_pick_splits(seqs, hkv, max_kv_len);
-  const long long units = static_cast<long long>(seqs) * hkv, rows = slots + units;
+  const int slots = decode_blocks(g_decode_stages), splits = b200_attn_decode_pick_splits(seqs, hkv, max_kv_len);
+  const long long units = static_cast<long long>(seqs) * hkv;
   const long long tiles = units * ((max_kv_len + kTileTokens - 1) / kTileTokens);
   if (splits == 1 || units * splits <= slots || tiles < 16ll * slots || tiles > 400ll * slots) return 0;
-  return rows * (hq / hkv) * (d + 2) * 4 + units * 8;
+  return even_bytes(slots, seqs, hq, hkv, d);
 }
 
+// workspace_bytes: of even shares, whose count of blocks follows the ring's depth at this call
 static int attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
                        const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
-                       int d, int page, int max_pages, int splits, bool even, void* workspace,
+                       int d, int page, int max_pages, int splits, bool even, void* workspace, long long workspace_bytes,
                        float scale, float softcap, int window, void* out_q, void* out_scale,
                        int sf_tile_rows, cudaStream_t stream) {
   if (seqs <= 0) return 0;
   if (out_q != nullptr && (d != 128 || (splits <= 1 && !even) || out_scale == nullptr)) return -6;   // combine kernel only
   if (d != 128 && (d != 64 || even)) return -2;
   if (hq % hkv != 0 || hq / hkv > 16) return -3;
+  const int stages = g_decode_stages == 2 ? 2 : 3;     // read once: grid, workspace and kernel go by the same depth
+  const int slots = decode_blocks(stages);
   if ((splits > 1 || even) && !workspace) return -5;
+  if (even && workspace_bytes < even_bytes(slots, seqs, hq, hkv, d)) return -5;
   AttnParams p{};
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k = static_cast<const __nv_bfloat16*>(k_cache);
@@ -1054,16 +1066,15 @@ static int attn_decode(const void* q, const void* k_cache, const void* v_cache, 
   p.sf_tile_rows = sf_tile_rows;
   dim3 grid(seqs, hkv, p.splits);
   if (p.splits > 1 || even) {
-    const long long rows = even ? (decode_blocks() + static_cast<long long>(seqs) * hkv) * (hq / hkv) : static_cast<long long>(seqs) * hq * p.splits;
+    const long long rows = even ? (slots + static_cast<long long>(seqs) * hkv) * (hq / hkv) : static_cast<long long>(seqs) * hq * p.splits;
     p.ws_o = static_cast<float*>(workspace);
     p.ws_ml = p.ws_o + rows * d;
     if (even) {
       p.ends = reinterpret_cast<int*>(p.ws_ml + rows * 2);
-      grid = dim3(decode_blocks());
+      grid = dim3(slots);
     }
   }
   // staging ring depth: 3 tiles (two CTAs per SM at d = 128) or 2 tiles (three CTAs per SM)
-  const int stages = g_decode_stages == 2 ? 2 : 3;
   const int smem = stages * 2 * kTileTokens * d * 2;
   static PerDeviceOnce attr_set[3][2];
   PerDeviceOnce& once = attr_set[even ? 2 : d == 128 ? 1 : 0][stages - 2];
@@ -1095,18 +1106,19 @@ B200_API int b200_attn_decode(const void* q, const void* k_cache, const void* v_
                               int d, int page, int max_pages, int splits, void* workspace,
                               float scale, float softcap, int window, void* out_q, void* out_scale,
                               int sf_tile_rows, cudaStream_t stream) {
-  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, splits, false, workspace, scale,
-                     softcap, window, out_q, out_scale, sf_tile_rows, stream);
+  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, splits, false, workspace, 0,
+                     scale, softcap, window, out_q, out_scale, sf_tile_rows, stream);
 }
 
-// The same in even shares of all tiles; workspace as b200_attn_decode_even_bytes says.
+// The same in even shares of all tiles; workspace as b200_attn_decode_even_bytes says. -5: it is smaller than the ring's depth at
+// this call asks for (b200_attn_set_decode_stages came in between).
 B200_API int b200_attn_decode_even(const void* q, const void* k_cache, const void* v_cache, void* out,
                                    const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
-                                   int d, int page, int max_pages, void* workspace,
+                                   int d, int page, int max_pages, void* workspace, long long workspace_bytes,
                                    float scale, float softcap, int window, void* out_q, void* out_scale,
                                    int sf_tile_rows, cudaStream_t stream) {
-  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, 1, true, workspace, scale,
-                     softcap, window, out_q, out_scale, sf_tile_rows, stream);
+  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, 1, true, workspace, workspace_bytes,
+                     scale, softcap, window, out_q, out_scale, sf_tile_rows, stream);
 }
 
 // Prefill / full attention. paged != 0: k, v are page pools read through block_table and kv_lens;

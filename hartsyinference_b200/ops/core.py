@@ -660,9 +660,10 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, b
         mk = max_kv_len if max_kv_len is not None else block_table.shape[1] * page
         even = L.b200_attn_decode_even_bytes(b, hq, hkv, d, min(mk, window + 63) if window > 0 else mk)
         splits = 1 if even else L.b200_attn_decode_pick_splits(b, hkv, mk)
-    ws = None
+    ws, ws_bytes = None, 0
     if even or splits > 1:
-        ws = N.state(q.device).scratch(even or L.b200_attn_decode_workspace_bytes(b, hq, d, splits)).data_ptr()
+        buf = N.state(q.device).scratch(even or L.b200_attn_decode_workspace_bytes(b, hq, d, splits))
+        ws, ws_bytes = buf.data_ptr(), buf.numel()
     fused_q = emit_fp8 and d == 128 and ws is not None
     out = torch.empty_like(q) if (emit_bf16 or not fused_q) else None
     oq = osc = None
@@ -672,8 +673,8 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, b
         osc = _alloc_sf(b, hq * d, 128, q.device) if mx else torch.empty(b, hq, dtype=torch.float32, device=q.device)
     at = (q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), N.ptr(out), block_table.data_ptr(), kv_lens.data_ptr(), b, hq, hkv, d,
           page, block_table.shape[1])
-    how = (ws, scale, softcap, window, N.ptr(oq), N.ptr(osc), 128 if (fused_q and mx) else 0, N.stream())
-    rc = L.b200_attn_decode_even(*at, *how) if even else L.b200_attn_decode(*at, splits, *how)
+    how = (scale, softcap, window, N.ptr(oq), N.ptr(osc), 128 if (fused_q and mx) else 0, N.stream())
+    rc = L.b200_attn_decode_even(*at, ws, ws_bytes, *how) if even else L.b200_attn_decode(*at, splits, ws, *how)
     N.check(rc, "b200_attn_decode", 2 if ws is not None else 1)
     if not emit_fp8:
         return out
