@@ -31,8 +31,6 @@
 
 namespace b200 {
 
-int num_sms();      // of the current device, see gemm_tcgen05.cu
-
 constexpr int kTileTokens = 64;
 constexpr int kAttnThreads = 128;
 
@@ -78,7 +76,6 @@ struct AttnParams {
   int head_gate;                // gate [tokens][gate_ld] holds one column per head
   long long out_ld;             // output row pitch (head h at h * dv)
   float cap_in, cap_out;        // softcap: cap_out * tanh(score / softcap), exp(2 score / softcap) = 2^(cap_in * q.k)
-  int* ends;                    // even shares: [seqs][hkv] first and last block of the key head's tiles; or null
 };
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kDistSmem = 4096;   // longest distance table that prefill blocks keep in shared memory
@@ -370,31 +367,26 @@ __device__ __forceinline__ float gate_of(const AttnParams& p, long long token, i
 // ------------------------------------------------------------------------------------------
 // decode
 // ------------------------------------------------------------------------------------------
-// The keys of one sequence that a decode step reads.
-struct DecodeSpan {
-  int kv_len, start_key, tile0, n_tiles;             // tiles [tile0, n_tiles)
-};
-__device__ __forceinline__ DecodeSpan decode_span(const AttnParams& p, int seq) {
-  DecodeSpan s;
-  s.kv_len = p.kv_lens[seq];
-  s.n_tiles = (s.kv_len + kTileTokens - 1) / kTileTokens;
-  s.start_key = p.window > 0 ? max(0, s.kv_len - p.window) : 0;
-  s.tile0 = s.start_key / kTileTokens;                          // tiles before the window are not read
-  return s;
-}
-
-// Tiles [tile_begin, tile_end) of one key head for the query heads on it: the result (one piece) or, with `partial`, the piece's
-// sums at rows first_row + r * row_step of the workspace for query head r of the group.
-template <int D, int kStages, bool kExt>
-__device__ __forceinline__ void decode_piece(const AttnParams& p, const DecodeSpan& span, int seq, int kvh, int kept, int tile_begin,
-                                             int tile_end, bool first_piece, bool partial, long long first_row, int row_step) {
+template <int D, int kStages, bool kExt = false>
+__global__ void __launch_bounds__(kAttnThreads)
+attn_decode_kernel(const AttnParams p) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int kTileBytes = kTileTokens * D * 2;
   extern __shared__ __align__(128) uint8_t smem[];
   const int stage_bytes = kExt && p.shared_kv ? kTileBytes : 2 * kTileBytes;
+  const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
   const int G = p.hq / p.hkv;
-  const int kv_len = span.kv_len, start_key = span.start_key, tile0 = span.tile0;
+  const int kv_len = p.kv_lens[seq];
+  const int n_tiles = (kv_len + kTileTokens - 1) / kTileTokens;
+  const int start_key = p.window > 0 ? max(0, kv_len - p.window) : 0;
+  const int tile0 = start_key / kTileTokens;                    // tiles before the window are not read
+  const int kept = kExt ? kept_tiles(p, tile0) : 0;             // except those of the kept first tokens
+  const int tiles_per_split = (n_tiles - tile0 + kept + p.splits - 1) / p.splits;
+  const int tile_begin = tile0 - kept + split * tiles_per_split;
+  const int tile_end = min(n_tiles, tile_begin + tiles_per_split);
   const int* table = p.block_table + static_cast<long long>(seq) * p.max_pages;
   const uint32_t smem_base = smem_u32(smem);
 
@@ -431,7 +423,7 @@ __device__ __forceinline__ void decode_piece(const AttnParams& p, const DecodeSp
       const int head = kvh * G + min(g + 8 * r, G - 1);
       if (p.slopes) row_slope[r] = p.slopes[head] * kLog2e;
       if (p.dist_bias) row_bias[r] = p.dist_bias + static_cast<long long>(head) * p.dist_len;
-      if (p.sinks && first_piece && warp == 0) {       // the sink enters the running sums once
+      if (p.sinks && split == 0 && warp == 0) {       // the sink enters the running sums once
         st.m[r] = p.sinks[head] * kLog2e;
         st.l[r] = 1.f;
       }
@@ -512,14 +504,14 @@ __device__ __forceinline__ void decode_piece(const AttnParams& p, const DecodeSp
       ll += sml[(w * 16 + r) * 2 + 1] * f;
     }
     const int head = kvh * G + r;
-    if (kExt && !partial) {
+    if (kExt && p.splits == 1) {
       if (c < p.dv)
         p.out[seq * p.out_ld + head * p.dv + c] = __float2bfloat16((ll > 0.f ? acc / ll : 0.f) * gate_of(p, seq, head, c));
-    } else if (!partial) {
+    } else if (p.splits == 1) {
       p.out[(static_cast<long long>(seq) * p.hq + head) * D + c] =
           __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
     } else {
-      const long long base = first_row + static_cast<long long>(r) * row_step;
+      const long long base = (static_cast<long long>(seq) * p.hq + head) * p.splits + split;
       p.ws_o[base * D + c] = acc;
       if (c == 0) {
         p.ws_ml[base * 2] = mm;
@@ -529,111 +521,21 @@ __device__ __forceinline__ void decode_piece(const AttnParams& p, const DecodeSp
   }
 }
 
-template <int D, int kStages, bool kExt = false>
-__global__ void __launch_bounds__(kAttnThreads)
-attn_decode_kernel(const AttnParams p) {
-  pdl_wait();
-  pdl_trigger();
-  const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
-  const DecodeSpan span = decode_span(p, seq);
-  const int kept = kExt ? kept_tiles(p, span.tile0) : 0;        // tiles of the kept first tokens, before the window
-  const int tiles_per_split = (span.n_tiles - span.tile0 + kept + p.splits - 1) / p.splits;
-  const int tile_begin = span.tile0 - kept + split * tiles_per_split;
-  const int tile_end = min(span.n_tiles, tile_begin + tiles_per_split);
-  const int G = p.hq / p.hkv;
-  decode_piece<D, kStages, kExt>(p, span, seq, kvh, kept, tile_begin, tile_end, split == 0, p.splits > 1,
-                                 (static_cast<long long>(seq) * p.hq + kvh * G) * p.splits + split, p.splits);
-}
-
-// Even shares: the tiles of all sequences and key heads, in this order, in equal runs over one wave of blocks, so that all blocks
-// are done at once whatever the lengths are. Bound by the cache's bytes and by the start of each piece (about four tiles' time):
-// 64 sequences of 2176 tokens on 8 key heads 138 -> 126 us, of 64 to 8192 on a logarithmic scale 161 -> 144. One ring of loads
-// that runs on from piece to piece cost more in every tile than it saved (134). A block's piece of key head u has the
-// workspace row (block + u), one more at each next piece; `ends` holds a key head's first and last block.
-template <int D, int kStages>
-__global__ void __launch_bounds__(kAttnThreads)
-attn_decode_even_kernel(const AttnParams p) {
-  pdl_wait();
-  pdl_trigger();
-  const int lane = threadIdx.x & 31, G = p.hq / p.hkv;
-  auto tiles_of = [&](int s) {
-    const DecodeSpan span = decode_span(p, s);
-    return max(0, span.n_tiles - span.tile0);
-  };
-  int sum = 0;
-  for (int s = lane; s < p.seqs; s += 32) sum += tiles_of(s);
-  sum = __reduce_add_sync(0xffffffffu, sum);
-  const long long all = static_cast<long long>(sum) * p.hkv;
-  const long long blocks = min(static_cast<long long>(gridDim.x), all);   // every one has a tile: a key head's pieces follow one another
-  if (blockIdx.x >= blocks) return;
-  long long at = all * blockIdx.x / blocks;
-  const long long end = all * (blockIdx.x + 1) / blocks;
-  // the sequence of the first tile: the tiles of one key head up to it are at most `upto`
-  const int upto = static_cast<int>(at / p.hkv);
-  int seq = 0, before = 0;
-  for (int s0 = 0; s0 < p.seqs; s0 += 32) {
-    const int t = s0 + lane < p.seqs ? tiles_of(s0 + lane) : 0;
-    int inc = t;
-#pragma unroll
-    for (int d = 1; d < 32; d *= 2) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += v;
-    }
-    const uint32_t past = __ballot_sync(0xffffffffu, upto < before + inc);
-    if (past != 0) {
-      const int l = __ffs(past) - 1;
-      seq = s0 + l;
-      before += __shfl_sync(0xffffffffu, inc - t, l);
-      break;
-    }
-    before += __shfl_sync(0xffffffffu, inc, 31);
-  }
-  const int in_seq = static_cast<int>(at - static_cast<long long>(before) * p.hkv);
-  DecodeSpan span = decode_span(p, seq);
-  int kvh = in_seq / (span.n_tiles - span.tile0), tile = span.tile0 + in_seq % (span.n_tiles - span.tile0);
-  for (;;) {
-    const int tile_end = static_cast<int>(min(static_cast<long long>(span.n_tiles), tile + (end - at)));
-    const int unit = seq * p.hkv + kvh;
-    if (threadIdx.x == 0) {
-      if (tile == span.tile0) p.ends[unit * 2] = blockIdx.x;
-      if (tile_end == span.n_tiles) p.ends[unit * 2 + 1] = blockIdx.x;
-    }
-    decode_piece<D, kStages, false>(p, span, seq, kvh, 0, tile, tile_end, false, true,
-                                    static_cast<long long>(blockIdx.x + unit) * G, 1);
-    at += tile_end - tile;
-    if (at >= end) return;
-    if (++kvh == p.hkv) {
-      kvh = 0;
-      do span = decode_span(p, ++seq); while (span.n_tiles <= span.tile0 && seq + 1 < p.seqs);
-    }
-    tile = span.tile0;
-    __syncthreads();                                 // the merge has read what the next loads overwrite
-  }
-}
-
 template <int D, bool kExt = false>
 __global__ void attn_combine_kernel(const AttnParams p) {
   pdl_wait();
   pdl_trigger();
   const int seq = blockIdx.x, head = blockIdx.y;
-  long long base = (static_cast<long long>(seq) * p.hq + head) * p.splits;
-  int n = p.splits, step = 1;
-  if (!kExt && p.ends) {
-    const int G = p.hq / p.hkv, unit = seq * p.hkv + head / G;
-    step = G;
-    n = p.kv_lens[seq] > 0 ? p.ends[unit * 2 + 1] - p.ends[unit * 2] + 1 : 0;   // a sequence without keys has no pieces
-    base = n > 0 ? static_cast<long long>(p.ends[unit * 2] + unit) * G + head % G : 0;
-  }
+  const long long base = (static_cast<long long>(seq) * p.hq + head) * p.splits;
   float mm = -INFINITY;
-  for (int s = 0; s < n; ++s) mm = fmaxf(mm, p.ws_ml[(base + s * step) * 2]);
+  for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, p.ws_ml[(base + s) * 2]);
   for (int c = threadIdx.x; c < D; c += blockDim.x) {
     float acc = 0.f, ll = 0.f;
-    for (int s = 0; s < n; ++s) {
-      const long long row = base + s * step;
-      const float ms = p.ws_ml[row * 2];
+    for (int s = 0; s < p.splits; ++s) {
+      const float ms = p.ws_ml[(base + s) * 2];
       const float f = ms == -INFINITY ? 0.f : exp2f(ms - mm);
-      acc += p.ws_o[row * D + c] * f;
-      ll += p.ws_ml[row * 2 + 1] * f;
+      acc += p.ws_o[(base + s) * D + c] * f;
+      ll += p.ws_ml[(base + s) * 2 + 1] * f;
     }
     if (kExt) {
       if (c < p.dv)
@@ -977,17 +879,8 @@ B200_API long long b200_attn_decode_workspace_bytes(int seqs, int hq, int d, int
 
 static int g_decode_stages = 2;
 
-// Blocks of the decode kernel that the chip holds at once, with a ring of `stages` tiles.
-static int decode_blocks(int stages) { return num_sms() * (stages == 2 ? 3 : 2); }
-
-// Workspace of even shares on `slots` blocks: a row of sums per query head and piece, the first and last block of every key head
-static long long even_bytes(int slots, int seqs, int hq, int hkv, int d) {
-  const long long units = static_cast<long long>(seqs) * hkv;
-  return (slots + units) * (hq / hkv) * (d + 2) * 4 + units * 8;
-}
-
 // Number of KV splits for a decode batch, from a wave model fitted to B200 timings: the grid runs
-// in waves of (SMs x resident CTAs) and a CTA costs its tiles plus about four tiles' worth of
+// in waves of (148 SMs x resident CTAs) and a CTA costs its tiles plus about four tiles' worth of
 // prologue and merge, so the estimate is waves x (ceil(tiles / splits) + 4); ties go to fewer
 // splits (less partial traffic and a cheaper combine). Measured with the two-tile ring, 64-token
 // tiles, 2304-token contexts (CTAs before splitting: best splits, time): 16: 12, 13.5 us;
@@ -996,7 +889,7 @@ static long long even_bytes(int slots, int seqs, int hq, int hkv, int d) {
 B200_API int b200_attn_decode_pick_splits(int seqs, int hkv, int max_kv_len) {
   const int ctas = seqs * hkv > 0 ? seqs * hkv : 1;
   const int tiles = (max_kv_len + kTileTokens - 1) / kTileTokens;
-  const int slots = decode_blocks(g_decode_stages);
+  const int slots = 148 * (g_decode_stages == 2 ? 3 : 2);
   int best = 1;
   long long best_cost = -1;
   for (int sp = 1; sp <= 16 && sp <= tiles; ++sp) {
@@ -1011,41 +904,16 @@ B200_API int b200_attn_decode_pick_splits(int seqs, int hkv, int max_kv_len) {
 // Depth of the decode kernel's K/V staging ring: 3 (two CTAs per SM at head dim 128) or 2 (three).
 B200_API void b200_attn_set_decode_stages(int stages) { g_decode_stages = stages == 2 ? 2 : 3; }
 
-
-// Workspace of a decode batch in even shares, 0 where b200_attn_decode stays the better one. Both measured for 1 to 512 sequences of up
-// to 300 to 32768 tokens on 1, 2, 8 and 32 key heads (times of even shares to the others'; all of one length, lengths down to the
-// half, lengths from 64 tokens on a logarithmic scale):
-//  - more than a wave of blocks in two splits or more: runs of 18 to 74 tiles 0.91 to 1.00, 0.89 to 0.97, 0.56 to 1.06; of 78 to 295 tiles
-//    0.97 to 0.99, 0.88 to 0.95, 0.7 to 0.98; batches far shorter than max_kv_len, where the splits are as many as for long ones, 0.55
-//    to 1.00 (1.08 at 300 tokens of 2304). Shorter runs pay for the start (6 tiles 1.02 to 1.25), runs of 440 and 590 tiles
-//    for the SMs' unequal speed, which many blocks even out (up to 1.05 and 1.08)
-//  - more than a wave without a split has no second kernel there: 74 tiles 1.10, 1.07, 1.24
-//  - up to a wave of blocks, one each, long runs gain as well (37 to 111 tiles 0.92 to 1.01, 0.78 to 1.00, 0.38 to 1.00), but a batch far shorter
-//    than max_kv_len, which a captured step does not know, loses (16 to 48 sequences of 300 tokens of 8192: 1.32 to 1.46).
-// Head size 64 keeps its splits: more than three of its blocks fit an SM, which this count of blocks does not know.
-B200_API long long b200_attn_decode_even_bytes(int seqs, int hq, int hkv, int d, int max_kv_len) {
-  if (d != 128 || hkv <= 0 || hq % hkv != 0 || hq / hkv > 16) return 0;
-  const int slots = decode_blocks(g_decode_stages), splits = b200_attn_decode_pick_splits(seqs, hkv, max_kv_len);
-  const long long units = static_cast<long long>(seqs) * hkv;
-  const long long tiles = units * ((max_kv_len + kTileTokens - 1) / kTileTokens);
-  if (splits == 1 || units * splits <= slots || tiles < 16ll * slots || tiles > 400ll * slots) return 0;
-  return even_bytes(slots, seqs, hq, hkv, d);
-}
-
-// workspace_bytes: of even shares, whose count of blocks follows the ring's depth at this call
-static int attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
-                       const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
-                       int d, int page, int max_pages, int splits, bool even, void* workspace, long long workspace_bytes,
-                       float scale, float softcap, int window, void* out_q, void* out_scale,
-                       int sf_tile_rows, cudaStream_t stream) {
+B200_API int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
+                              const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
+                              int d, int page, int max_pages, int splits, void* workspace,
+                              float scale, float softcap, int window, void* out_q, void* out_scale,
+                              int sf_tile_rows, cudaStream_t stream) {
   if (seqs <= 0) return 0;
-  if (out_q != nullptr && (d != 128 || (splits <= 1 && !even) || out_scale == nullptr)) return -6;   // combine kernel only
-  if (d != 128 && (d != 64 || even)) return -2;
+  if (out_q != nullptr && (d != 128 || splits <= 1 || out_scale == nullptr)) return -6;   // combine kernel only
+  if (d != 64 && d != 128) return -2;
   if (hq % hkv != 0 || hq / hkv > 16) return -3;
-  const int stages = g_decode_stages == 2 ? 2 : 3;     // read once: grid, workspace and kernel go by the same depth
-  const int slots = decode_blocks(stages);
-  if ((splits > 1 || even) && !workspace) return -5;
-  if (even && workspace_bytes < even_bytes(slots, seqs, hq, hkv, d)) return -5;
+  if (splits > 1 && !workspace) return -5;
   AttnParams p{};
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k = static_cast<const __nv_bfloat16*>(k_cache);
@@ -1064,34 +932,28 @@ static int attn_decode(const void* q, const void* k_cache, const void* v_cache, 
   p.out_q = static_cast<uint8_t*>(out_q);
   p.out_scale = out_scale;
   p.sf_tile_rows = sf_tile_rows;
-  dim3 grid(seqs, hkv, p.splits);
-  if (p.splits > 1 || even) {
-    const long long rows = even ? (slots + static_cast<long long>(seqs) * hkv) * (hq / hkv) : static_cast<long long>(seqs) * hq * p.splits;
+  if (p.splits > 1) {
     p.ws_o = static_cast<float*>(workspace);
-    p.ws_ml = p.ws_o + rows * d;
-    if (even) {
-      p.ends = reinterpret_cast<int*>(p.ws_ml + rows * 2);
-      grid = dim3(slots);
-    }
+    p.ws_ml = p.ws_o + static_cast<long long>(seqs) * hq * p.splits * d;
   }
+  dim3 grid(seqs, hkv, p.splits);
   // staging ring depth: 3 tiles (two CTAs per SM at d = 128) or 2 tiles (three CTAs per SM)
+  const int stages = g_decode_stages == 2 ? 2 : 3;
   const int smem = stages * 2 * kTileTokens * d * 2;
-  static PerDeviceOnce attr_set[3][2];
-  PerDeviceOnce& once = attr_set[even ? 2 : d == 128 ? 1 : 0][stages - 2];
+  static PerDeviceOnce attr_set[2][2];
+  PerDeviceOnce& once = attr_set[d == 128 ? 1 : 0][stages - 2];
   auto launch = [&](auto kernel) {
     if (once.first_time()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     launch_pdl(kernel, grid, dim3(kAttnThreads), smem, stream, p);
   };
-  if (even) {
-    if (stages == 2) launch(attn_decode_even_kernel<128, 2>); else launch(attn_decode_even_kernel<128, 3>);
-  } else if (d == 128) {
+  if (d == 128) {
     if (stages == 2) launch(attn_decode_kernel<128, 2>); else launch(attn_decode_kernel<128, 3>);
   } else {
     if (stages == 2) launch(attn_decode_kernel<64, 2>); else launch(attn_decode_kernel<64, 3>);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return -static_cast<int>(e) - 300;
-  if (p.splits > 1 || even) {
+  if (p.splits > 1) {
     dim3 cg(seqs, hq);
     if (d == 128) launch_pdl(attn_combine_kernel<128>, cg, dim3(128), 0, stream, p);
     else launch_pdl(attn_combine_kernel<64>, cg, dim3(64), 0, stream, p);
@@ -1099,26 +961,6 @@ static int attn_decode(const void* q, const void* k_cache, const void* v_cache, 
     if (e != cudaSuccess) return -static_cast<int>(e) - 400;
   }
   return 0;
-}
-
-B200_API int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
-                              const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
-                              int d, int page, int max_pages, int splits, void* workspace,
-                              float scale, float softcap, int window, void* out_q, void* out_scale,
-                              int sf_tile_rows, cudaStream_t stream) {
-  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, splits, false, workspace, 0,
-                     scale, softcap, window, out_q, out_scale, sf_tile_rows, stream);
-}
-
-// The same in even shares of all tiles; workspace as b200_attn_decode_even_bytes says. -5: it is smaller than the ring's depth at
-// this call asks for (b200_attn_set_decode_stages came in between).
-B200_API int b200_attn_decode_even(const void* q, const void* k_cache, const void* v_cache, void* out,
-                                   const int* block_table, const int* kv_lens, int seqs, int hq, int hkv,
-                                   int d, int page, int max_pages, void* workspace, long long workspace_bytes,
-                                   float scale, float softcap, int window, void* out_q, void* out_scale,
-                                   int sf_tile_rows, cudaStream_t stream) {
-  return attn_decode(q, k_cache, v_cache, out, block_table, kv_lens, seqs, hq, hkv, d, page, max_pages, 1, true, workspace, workspace_bytes,
-                     scale, softcap, window, out_q, out_scale, sf_tile_rows, stream);
 }
 
 // Prefill / full attention. paged != 0: k, v are page pools read through block_table and kv_lens;

@@ -113,8 +113,6 @@ _SIGNATURES = {
     "b200_dit_qkv_row": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, f32, vp]),
     "b200_fill_random": (i32, [vp, i64, u64, f32, i32, vp]),
     "b200_attn_decode": (i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, f32, f32, i32, vp, vp, i32, vp]),
-    "b200_attn_decode_even": (i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, i64, f32, f32, i32, vp, vp, i32, vp]),
-    "b200_attn_decode_even_bytes": (i64, [i32, i32, i32, i32, i32]),
     "b200_attn_decode_pick_splits": (i32, [i32, i32, i32]),
     "b200_attn_decode_workspace_bytes": (i64, [i32, i32, i32, i32]),
     "b200_attn_prefill": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32, vp]),

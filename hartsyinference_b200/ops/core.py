@@ -655,27 +655,24 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, b
         return (o, quant_fp8_act(o.reshape(b, hq * d))) if emit_fp8 else o
     assert block_table.dtype == torch.int32 and kv_lens.dtype == torch.int32
     L = N.lib()
-    even = 0                                             # workspace bytes of the form in even shares
     if splits is None:
         mk = max_kv_len if max_kv_len is not None else block_table.shape[1] * page
-        even = L.b200_attn_decode_even_bytes(b, hq, hkv, d, min(mk, window + 63) if window > 0 else mk)
-        splits = 1 if even else L.b200_attn_decode_pick_splits(b, hkv, mk)
-    ws, ws_bytes = None, 0
-    if even or splits > 1:
-        buf = N.state(q.device).scratch(even or L.b200_attn_decode_workspace_bytes(b, hq, d, splits))
-        ws, ws_bytes = buf.data_ptr(), buf.numel()
-    fused_q = emit_fp8 and d == 128 and ws is not None
+        splits = L.b200_attn_decode_pick_splits(b, hkv, mk)
+    ws = None
+    if splits > 1:
+        ws = N.state(q.device).scratch(L.b200_attn_decode_workspace_bytes(b, hq, d, splits)).data_ptr()
+    fused_q = emit_fp8 and d == 128 and splits > 1
     out = torch.empty_like(q) if (emit_bf16 or not fused_q) else None
     oq = osc = None
     mx = fp8_mx()
     if fused_q:
         oq = torch.empty(b, hq * d, dtype=torch.uint8, device=q.device)
         osc = _alloc_sf(b, hq * d, 128, q.device) if mx else torch.empty(b, hq, dtype=torch.float32, device=q.device)
-    at = (q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), N.ptr(out), block_table.data_ptr(), kv_lens.data_ptr(), b, hq, hkv, d,
-          page, block_table.shape[1])
-    how = (scale, softcap, window, N.ptr(oq), N.ptr(osc), 128 if (fused_q and mx) else 0, N.stream())
-    rc = L.b200_attn_decode_even(*at, ws, ws_bytes, *how) if even else L.b200_attn_decode(*at, splits, ws, *how)
-    N.check(rc, "b200_attn_decode", 2 if ws is not None else 1)
+    rc = L.b200_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), N.ptr(out),
+                            block_table.data_ptr(), kv_lens.data_ptr(), b, hq, hkv, d, page,
+                            block_table.shape[1], splits, ws, scale, softcap, window, N.ptr(oq), N.ptr(osc),
+                            128 if (fused_q and mx) else 0, N.stream())
+    N.check(rc, "b200_attn_decode", 2 if splits > 1 else 1)
     if not emit_fp8:
         return out
     if fused_q:

@@ -67,11 +67,9 @@ def test_decode_window_softcap():
 
 @pytest.mark.parametrize("window", [0, 100])
 @pytest.mark.parametrize("b,hq,hkv,most", [(70, 64, 8, 1200), (16, 32, 32, 1100), (300, 16, 1, 4000), (150, 12, 4, 3000)])
-def test_decode_in_even_shares(b, hq, hkv, most, window):
-    """Lengths of nothing, one key, whole tiles and long runs; a tile of the sums per key head and block. Probabilities in bf16
-    (2^-9 each, of values up to about 2) and the bf16 result: 2e-2 as for the split form."""
-    from hartsyinference_b200.ops import _native as N
-    assert N.lib().b200_attn_decode_even_bytes(b, hq, hkv, 128, most) > 0
+def test_decode_of_unequal_lengths(b, hq, hkv, most, window):
+    """Lengths of nothing, one key, whole tiles and long runs, in the splits that the library picks. Probabilities in bf16
+    (2^-9 each, of values up to about 2) and the bf16 result: 2e-2 as above."""
     torch.manual_seed(b)
     page, max_pages = 16, (most + 15) // 16
     kc, vc = _pool(512, hkv, page, 128)
@@ -93,6 +91,22 @@ def test_decode_in_even_shares(b, hq, hkv, most, window):
     assert (deq - out.float()).norm() <= 5e-2 * out.float().norm()
     again = ops.attn_decode(q, kc, vc, table, dev, window=window, max_kv_len=most)
     assert torch.equal(again, out)
+
+
+@pytest.mark.parametrize("b,hq,hkv,most", [(70, 64, 8, 1200), (64, 64, 8, 2304), (32, 32, 8, 8192)])
+def test_decode_of_a_sequence_whatever_its_neighbours_hold(b, hq, hkv, most):
+    """In a batch of one size, made for one longest length, a sequence's result has the same bits for all lengths of the others."""
+    torch.manual_seed(b + 1)
+    kc, vc = _pool(512, hkv, 16, 128)
+    table = torch.randint(0, 512, (b, (most + 15) // 16), dtype=torch.int32, device="cuda")
+    q = torch.randn(b, hq, 128, device="cuda").to(torch.bfloat16)
+    own = torch.randint(1, most + 1, (b // 2,), dtype=torch.int32, device="cuda")
+    outs = []
+    for others in (torch.ones_like(own), torch.randint(1, most + 1, own.shape, dtype=torch.int32, device="cuda"), torch.full_like(own, most)):
+        lens = torch.empty(b, dtype=torch.int32, device="cuda")
+        lens[0::2], lens[1::2] = own, others
+        outs.append(ops.attn_decode(q, kc, vc, table, lens, max_kv_len=most)[0::2])
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
 @pytest.mark.parametrize("d,hq,hkv", [(128, 8, 2), (64, 14, 2)])
