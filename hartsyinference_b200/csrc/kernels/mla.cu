@@ -28,8 +28,6 @@
 
 namespace b200 {
 
-int num_sms();      // of the current device, see gemm_tcgen05.cu
-
 constexpr int kLat = 512;            // latent width (also the value width)
 constexpr int kRopeDim = 64;
 constexpr int kRow = kLat + kRopeDim;        // 576
@@ -422,24 +420,12 @@ B200_API int b200_mla_prep(const void* kv, const void* kv_norm_w, const void* q,
 // Head groups of 16 that one CTA serves: two once a row has more than one group.
 static int mla_sets(int heads) { return heads > 16 ? 2 : 1; }
 
-// A block's shared memory fills a processor, so blocks run in waves of one per processor; a block takes its tiles and about half a tile more,
-// and ranges have to be combined. In tiles of 5 us (128 heads): 32 rows of 1024 keys 3 ranges 92.6 us, one 82.6; 16 of 4000 5 ranges
-// 187, 9 ranges 157; 128 of 1500 one 487, two 452; 8 of 2000 10 ranges 49.7, 4 ranges 45.6; 1 of 3000 24 ranges 18.2, 8 35.7.
+// Key ranges of a row: blocks for two on a processor, whatever max_kv_len is beyond that many tiles, since a captured step is made for
+// the longest length and its rows may be far shorter or unequal. A count that weighs waves of one block a processor against tiles
+// of max_kv_len gains up to a quarter where all rows have that length (128 heads, 32 rows of 1000 keys 92 -> 83 us) and loses
+// elsewhere (32 rows of 300 in a step made for 8192 39 -> 49 us, 48 rows of 300 for 32768 49 -> 90, 32 rows of 64 to 2304 on a
+// logarithmic scale 96 -> 151).
 B200_API int b200_mla_pick_splits(int rows, int heads, int max_kv_len) {
-  const int per_cta = 16 * mla_sets(heads);
-  const long long ctas = static_cast<long long>(rows) * ((heads + per_cta - 1) / per_cta);
-  const int tiles = (max_kv_len + kMlaTile - 1) / kMlaTile, sms = num_sms();
-  int best = 1;
-  double best_cost = 0.;
-  for (int s = 1; s <= 32 && (s == 1 || s <= tiles); ++s) {
-    const double cost = static_cast<double>((ctas * s + sms - 1) / sms) * ((tiles + s - 1) / s + 0.6) + (s > 1 ? 0.8 + 0.05 * s : 0.);
-    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
-  }
-  return best;
-}
-
-// For b200_latent_attn, whose shorter rows leave room for two blocks on a processor.
-B200_API int b200_latent_pick_splits(int rows, int heads, int max_kv_len) {
   const int per_cta = 16 * mla_sets(heads);
   const int ctas = rows * ((heads + per_cta - 1) / per_cta);
   const int tiles = (max_kv_len + kMlaTile - 1) / kMlaTile;

@@ -717,7 +717,7 @@ def latent_attn(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
     step = 32768                            # rows are the grid's second dimension
     for a in range(0, rows, step):
         b = min(a + step, rows)
-        splits = L.b200_latent_pick_splits(b - a, heads, longest)
+        splits = L.b200_mla_pick_splits(b - a, heads, longest)
         ws = None
         if splits > 1:
             ws = torch.empty(L.b200_mla_workspace_bytes(b - a, heads, splits), dtype=torch.uint8, device=q.device)
