@@ -1591,15 +1591,13 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
       first_split = tiles; s_eff = 1; p.kblocks_per_split = total_kblocks;
     }
   }
-  // More tiles than SMs and a last wave that is less than half full: equal shares of all tiles' K groups, so that every SM is done
-  // at once, instead of a last wave of tiles cut along K, whose ranges one CTA adds. Times of shares to those of cut tiles (row of
-  // 1024 / 4096 / 8192 values, 64 tokens): 165 tiles bf16 0.75 / 0.96 / 0.86, fp8 0.73 / 0.94 / 0.93, 222 tiles 0.94 / 0.81 / 0.92 and
-  // 0.62 / 0.71 / 0.83, 300 tiles 0.63 / 0.86 / 0.96 and 0.63 / 0.74 / 0.88; for 4 tokens 0.91 to 1.04. Fuller last waves were never
-  // cut: there a second and third epilogue a CTA cost more than the idle SMs (260 tiles 1.35 / 1.02 / 1.04 and 1.90 / 1.03 / 0.98), but
-  // up to 0.6 of a wave rows of 8 KB gain (224 tiles 1.34 / 0.93 / 0.91 and 1.30 / 0.96 / 0.89).
-  const int rest = tiles % sms;
-  if (swap && plain && splits == 0 && cs == nullptr && defer_ws == nullptr && tiles > sms && rest != 0 && workspace != nullptr &&
-      (2 * rest <= sms || (5 * rest <= 3 * sms && static_cast<long long>(k) * esz >= 8192)) &&
+  // More tiles than SMs and a last wave that the plan cuts along K (at most half full): equal shares of all tiles' K groups instead, so that
+  // every SM is done at once and no CTA adds all ranges of a tile. Times of shares to those of cut tiles (row of 1024 / 4096 / 8192
+  // values, 64 tokens): 165 tiles bf16 0.75 / 0.96 / 0.86, fp8 0.73 / 0.94 / 0.93, 222 tiles 0.94 / 0.81 / 0.92 and 0.62 / 0.71 / 0.83,
+  // 300 tiles 0.63 / 0.86 / 0.96 and 0.63 / 0.74 / 0.88; for 4 tokens 0.91 to 1.04. Products whose last wave is fuller stay whole: a second
+  // and third epilogue a CTA cost more than the idle SMs (260 tiles 1.35 / 1.02 / 1.04 and 1.90 / 1.03 / 0.98), and where rows of 8 KB would
+  // gain (224 tiles 0.93) they would need the scratch, which two streams of a device share; whole tiles run on both at once.
+  if (swap && plain && splits == 0 && cs == nullptr && defer_ws == nullptr && tiles > sms && first_split < tiles &&
       kSplitCounterBytes + sms * 2 * slot_bytes <= workspace_bytes) {
     p.share_ctas = sms;
     p.share_kblocks = mx ? 4 : 2;                      // ranges start on a scale-factor group, stages hold two K blocks

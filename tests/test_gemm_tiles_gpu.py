@@ -188,3 +188,26 @@ def test_even_shares(m, n, k, fp8, act):
                    act_from=8 if act == "tanh" else 0)
     assert torch.allclose(y.float(), ref, rtol=2 ** -7, atol=2 ** -7), (y.float() - ref).abs().max()      # one rounding to bf16; fp32 sums
     assert torch.equal(ops.linear(xq, w, act=act, act_from=8 if act == "tanh" else 0, gate=gate, residual=res), y)
+
+
+# Streams of one device share the scratch, so a product that does without it must leave it alone: few tokens and a last wave more than half
+# full (above all with long rows), rows of too few K blocks to cut, and many tokens on CTA pairs
+@pytest.mark.parametrize("m,n,k", [(6, 28672, 4096), (64, 28672, 4096), (128, 30720, 8192), (17, 29000, 4608), (33, 151936, 192), (5, 19200, 64), (300, 12288, 3072)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_whole_tiles_leave_the_scratch_alone(m, n, k, fp8):
+    if fp8 and k % 128:
+        pytest.skip("groups of 128")
+    from hartsyinference_b200.ops import _native as N
+    from hartsyinference_b200.ops import core
+    torch.manual_seed(n)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    w = ops.LinearWeight.from_dense((torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16), fp8=fp8)
+    xq = ops.quant_fp8_act(x) if fp8 else x
+    xs, ws = core._scale_ptrs(xq, w)
+    xd = xq.data if fp8 else xq
+    scratch = torch.zeros(64 << 20, dtype=torch.uint8, device="cuda")
+    scratch[16384:] = 0xA5                           # behind the counters, which are zero between launches
+    before, out = scratch.clone(), torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().b200_gemm(xd.data_ptr(), w.weight.data_ptr(), out.data_ptr(), m, n, k, k, k, n, core._gemm_dtype(w), xs, ws, None, None, None, 0, 0,
+                              scratch.data_ptr(), scratch.numel(), N.state(x.device).status.data_ptr(), N.stream()), "b200_gemm")
+    assert torch.equal(scratch, before) and torch.equal(out, ops.linear(xq, w))
