@@ -37,20 +37,33 @@ struct DenseSizes {
 
 static long long padded(long long bytes) { return (bytes + 255) / 256 * 256; }
 
-// Bytes of the K ranges that a product may leave unsummed
-static long long part_bytes(int tokens, int n, int k, long long ws_bytes) {
-  const int plan = tokens <= 128 ? b200_gemm_deferred_plan(tokens, n, k, 0, ws_bytes) : 0;
-  return static_cast<long long>((n + 127) / 128) * (plan & 0xffff) * (plan >> 16) * 128 * 4;
+// What the policy leaves unsummed of a layer's four products (see b200_gemm_deferred_plan), and the bytes of the ranges. The policy follows
+// switches that another thread can turn between the call that asks for the scratch's size and the launch, so a launch asks once, for all
+// layers, and compares with the size that it was given.
+struct DensePlan {
+  int qkv, o, gate_up, down;
+  long long part;
+};
+
+static DensePlan dense_plan(const DenseSizes& z, long long ws_bytes) {
+  DensePlan p{};
+  auto one = [&](int n, int k) {
+    const int plan = z.tokens <= 128 ? b200_gemm_deferred_plan(z.tokens, n, k, 0, ws_bytes) : 0;
+    const long long bytes = padded(static_cast<long long>((n + 127) / 128) * (plan & 0xffff) * (plan >> 16) * 128 * 4);
+    if (bytes > p.part) p.part = bytes;
+    return plan;
+  };
+  p.qkv = one(z.qkv(), z.hidden);
+  p.o = one(z.hidden, z.att());
+  p.gate_up = one(2 * z.ffn, z.hidden);
+  p.down = one(z.hidden, z.ffn);
+  return p;
 }
 
-static long long dense_part(const DenseSizes& z, long long ws_bytes) {
-  long long most = 0;
-  const int shapes[4][2] = {{z.qkv(), z.hidden}, {z.hidden, z.att()}, {2 * z.ffn, z.hidden}, {z.hidden, z.ffn}};
-  for (const auto& s : shapes) {
-    const long long b = part_bytes(z.tokens, s[0], s[1], ws_bytes);
-    if (b > most) most = b;
-  }
-  return padded(most);
+static long long dense_scratch(const DenseSizes& z, const DensePlan& plan) {
+  const long long t = z.tokens;
+  return 4 * padded(t * z.hidden * 2) + padded(t * z.qkv() * 2) + 2 * padded(t * z.att() * 2) + padded(t * 2 * z.ffn * 2) + padded(t * z.ffn * 2) +
+         plan.part;
 }
 
 // A product, or its unsummed ranges where the policy leaves them to the kernel behind it
@@ -66,22 +79,22 @@ using namespace b200;
 
 B200_API long long b200_dense_layers_scratch(int tokens, int hidden, int hq, int hkv, int d, int ffn, long long gemm_ws_bytes) {
   const DenseSizes z{tokens, hidden, hq, hkv, d, ffn};
-  const long long t = tokens;
-  return 4 * padded(t * hidden * 2) + padded(t * z.qkv() * 2) + 2 * padded(t * z.att() * 2) + padded(t * 2 * ffn * 2) + padded(t * ffn * 2) +
-         dense_part(z, gemm_ws_bytes);
+  return dense_scratch(z, dense_plan(z, gemm_ws_bytes));
 }
 
 // x [tokens][hidden] bf16 -> out = norm(stream) behind all layers. layer_ptrs: seven pointers a layer (in_norm, qkv, qkv bias or null, o,
 // post_norm, gate_up, down), rows of weights dense. kv: pools [layers][2][pages][hkv][page][d]. cu_q, kv_lens, block_table as in
 // b200_attn_prefill. scratch: b200_dense_layers_scratch bytes on a 256-byte boundary. Returns the number of ops launched, or the
-// negative code of the one that failed.
+// negative code of the one that failed; -14, and nothing is launched: the scratch is too small for the policy as it is now.
 B200_API int b200_dense_layers(const void* x, void* out, const void* const* layer_ptrs, const void* final_norm, void* kv, long long layer_stride,
                                long long v_offset, const int* block_table, const int* kv_lens, const int* cu_q, const int* positions,
                                const long long* slots, const float* inv_freq, int tokens, int seqs, int max_q_len, int max_kv_len, int layers,
                                int hidden, int hq, int hkv, int d, int ffn, int rot, int style, int page, int max_pages, long long pages, int act,
-                               int plus_one, float eps, float theta, float scale, void* gemm_ws, long long gemm_ws_bytes, void* scratch, void* status,
-                               cudaStream_t stream) {
+                               int plus_one, float eps, float theta, float scale, void* gemm_ws, long long gemm_ws_bytes, void* scratch,
+                               long long scratch_bytes, void* status, cudaStream_t stream) {
   const DenseSizes z{tokens, hidden, hq, hkv, d, ffn};
+  const DensePlan plans = dense_plan(z, gemm_ws_bytes);
+  if (dense_scratch(z, plans) > scratch_bytes) return -14;
   const long long t = tokens;
   uint8_t* at = static_cast<uint8_t*>(scratch);
   auto take = [&](long long bytes) {
@@ -98,10 +111,9 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
     ++launches;
     return code == 0;
   };
-  // dst [tokens][n] = in w^T (+ bias). defer: the kernel behind it adds K ranges (and the bias)
-  auto product = [&](const void* in, const void* w, const void* bias, __nv_bfloat16* dst, int n, int k, bool defer, Product& p) {
+  // dst [tokens][n] = in w^T (+ bias), or the K ranges of `plan`, which the kernel behind it adds (and the bias)
+  auto product = [&](const void* in, const void* w, const void* bias, __nv_bfloat16* dst, int n, int k, int plan, Product& p) {
     p = Product{};
-    const int plan = defer && tokens <= 128 ? b200_gemm_deferred_plan(tokens, n, k, 0, gemm_ws_bytes) : 0;
     if (plan) {
       p.part = part;
       p.splits = plan & 0xffff;
@@ -127,7 +139,7 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
     __nv_bfloat16* vc = kc + v_offset;
     if (!norm(cur, stream_in, stream_in ? res[0] : nullptr, w[0], h)) return rc;
     if (stream_in == nullptr) stream_in = x; else stream_in = res[0];
-    if (!product(h, w[1], w[2], qkv, z.qkv(), hidden, true, p)) return rc;
+    if (!product(h, w[1], w[2], qkv, z.qkv(), hidden, plans.qkv, p)) return rc;
     if (!ok(b200_rope_kv(p.y, q, kc, vc, nullptr, nullptr, positions, slots, nullptr, nullptr, inv_freq, tokens, hq, hkv, d, rot, style, page, theta, eps,
                          p.part, p.splits, p.bn, p.part ? w[2] : nullptr, stream)))
       return rc;
@@ -139,7 +151,7 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
       code = b200_attn_prefill(q, kc, vc, att, block_table, kv_lens, cu_q, nullptr, seqs, max_q_len, 0, 0, hq, hkv, d, page, max_pages, 1, 1, 0, scale, 0.f,
                                stream);
     if (!ok(code)) return rc;
-    if (!product(att, w[3], nullptr, y, hidden, z.att(), true, p)) return rc;
+    if (!product(att, w[3], nullptr, y, hidden, z.att(), plans.o, p)) return rc;
     if (!norm(p, stream_in, res[1], w[4], h)) return rc;
     // as ops.linear_glu: one kernel for a handful of tokens and for many, otherwise the product and the activation
     const int form = b200_glu_form(tokens, ffn, hidden, 0);
@@ -149,10 +161,10 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
     if (code != -12) {
       if (!ok(code)) return rc;
     } else {
-      if (!product(h, w[5], nullptr, gu, 2 * ffn, hidden, true, p)) return rc;
+      if (!product(h, w[5], nullptr, gu, 2 * ffn, hidden, plans.gate_up, p)) return rc;
       if (!ok(b200_glu(p.y, a, nullptr, nullptr, tokens, ffn, act, 0, p.part, p.splits, p.bn, stream))) return rc;
     }
-    if (!product(a, w[6], nullptr, y, hidden, ffn, true, cur)) return rc;
+    if (!product(a, w[6], nullptr, y, hidden, ffn, plans.down, cur)) return rc;
     stream_in = res[1];
   }
   if (!norm(cur, stream_in, res[0], final_norm, out)) return rc;

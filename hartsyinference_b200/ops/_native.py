@@ -99,7 +99,7 @@ _SIGNATURES = {
     "b200_gemm_deferred": (i32, [vp, vp, i32, i32, i32, i64, i64, i32, vp, vp, vp, i64, vp, vp, vp]),
     "b200_rope_kv": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, f32, vp, i32, i32, vp, vp]),
     "b200_dense_layers_scratch": (i64, [i32, i32, i32, i32, i32, i32, i64]),
-    "b200_dense_layers": (i32, [vp, vp, vp, vp, vp, i64, i64, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i64, i32, i32, f32, f32, f32, vp, i64, vp, vp, vp]),
+    "b200_dense_layers": (i32, [vp, vp, vp, vp, vp, i64, i64, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i64, i32, i32, f32, f32, f32, vp, i64, vp, i64, vp, vp]),
     "b200_embedding": (i32, [vp, vp, vp, i32, i32, i32, f32, vp]),
     "b200_argmax": (i32, [vp, vp, i32, i32, i64, i32, vp]),
     "b200_quant_int8_rows": (i32, [vp, vp, vp, vp, i64, i32, i64, i64, i32, vp]),

@@ -579,7 +579,9 @@ def dense_prompt_layers(x: torch.Tensor, layers: list, final_norm: torch.Tensor,
                              block_table.data_ptr(), kv_lens.data_ptr(), cu_q.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(),
                              inv_freq.data_ptr(), t, cu_q.numel() - 1, max_q_len, max_kv_len, len(layers), hidden, hq, hkv, d, ffn, rot, style, page,
                              block_table.shape[1], pages, 0 if act == "silu" else 1, int(weight_plus_one), eps, theta, scale, ws.data_ptr(), ws.numel(),
-                             scratch.data_ptr(), st.status.data_ptr(), N.stream())
+                             scratch.data_ptr(), scratch.numel(), st.status.data_ptr(), N.stream())
+    if rc == -14:                                        # the reduce form was switched since the size was asked for
+        return None
     N.check(min(rc, 0), "b200_dense_layers", rc)
     return out
 

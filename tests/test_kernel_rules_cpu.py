@@ -1,6 +1,7 @@
 """Sizes and choices that the kernels library settles on the host, before any launch: they need no device."""
 import pytest
 
+from hartsyinference_b200 import config
 from hartsyinference_b200.ops import _native as N
 
 pytestmark = pytest.mark.skipif(not N.available(), reason="kernels library not built")
@@ -16,3 +17,21 @@ def test_latent_attention_ranges_do_not_grow_with_the_longest_length(rows, heads
         s = N.lib().b200_mla_pick_splits(rows, heads, most)
         assert 1 <= s <= max(1, -(-2 * 148 // blocks))
         assert s * blocks >= min(2 * 148, 32 * blocks)
+
+
+def test_prompt_layers_refuse_scratch_of_another_reduce_form():
+    """The ranges that products leave unsummed need scratch only in one reduce form, which can be switched between the call that asks for
+    the size and the launch: the launch then returns an error before it touches anything."""
+    L, sizes, ws = N.lib(), (896, 14, 2, 64, 4864), 64 << 20
+    try:
+        L.b200_gemm_set_external_reduce(0)
+        small = L.b200_dense_layers_scratch(29, *sizes, ws)
+        L.b200_gemm_set_external_reduce(1)
+        need = L.b200_dense_layers_scratch(29, *sizes, ws)
+        assert small < need
+        hidden, hq, hkv, d, ffn = sizes
+        args = (None, None, None, None, None, 0, 0, None, None, None, None, None, None, 29, 1, 29, 29, 24, hidden, hq, hkv, d, ffn, d, 0, 16, 4, 64, 0, 0,
+                1e-6, 1e4, 0.125, None, ws, None)
+        assert L.b200_dense_layers(*args, small, None, None) == -14
+    finally:
+        L.b200_gemm_set_external_reduce(1 if config.get("splitk_second_kernel") else 0)
