@@ -42,6 +42,7 @@ static long long padded(long long bytes) { return (bytes + 255) / 256 * 256; }
 // layers, and compares with the size that it was given.
 struct DensePlan {
   int qkv, o, gate_up, down;
+  int form;                                            // of the gated product, see b200_glu_form
   long long part;
 };
 
@@ -57,13 +58,31 @@ static DensePlan dense_plan(const DenseSizes& z, long long ws_bytes) {
   p.o = one(z.hidden, z.att());
   p.gate_up = one(2 * z.ffn, z.hidden);
   p.down = one(z.hidden, z.ffn);
+  p.form = b200_glu_form(z.tokens, z.ffn, z.hidden, 0);
   return p;
 }
 
-static long long dense_scratch(const DenseSizes& z, const DensePlan& plan) {
-  const long long t = z.tokens;
-  return 4 * padded(t * z.hidden * 2) + padded(t * z.qkv() * 2) + 2 * padded(t * z.att() * 2) + padded(t * 2 * z.ffn * 2) + padded(t * z.ffn * 2) +
-         plan.part;
+// Where a layer's intermediates lie in the scratch, in bytes. The halves of a layer take turns in one region: q, k and v are dead when
+// attention has run, whose output takes the place of the packed projection and is dead when the product behind it has; the gate and up rows
+// exist only where the gated product does not form the activation itself. 8192 tokens of 4096 features with 32 + 16 heads of 128 and a
+// feed-forward of 14336: 1.2 GB with a place for each -> 0.5 GB.
+struct DenseLayout {
+  long long h, y, res[2], qkv, q, att, gu, a, part, total;
+};
+
+static DenseLayout dense_layout(const DenseSizes& z, const DensePlan& plan) {
+  const long long t = z.tokens, row = padded(t * z.hidden * 2), qkv = padded(t * z.qkv() * 2), att = padded(t * z.att() * 2), a = padded(t * z.ffn * 2);
+  const long long gu = plan.form == 0 ? padded(t * 2 * z.ffn * 2) : 0;
+  DenseLayout l{};
+  l.y = row;
+  l.res[0] = 2 * row;
+  l.res[1] = 3 * row;
+  l.qkv = l.att = l.a = 4 * row;
+  l.q = l.qkv + qkv;
+  l.gu = l.a + a;
+  l.part = 4 * row + (qkv + att > gu + a ? qkv + att : gu + a);
+  l.total = l.part + plan.part;
+  return l;
 }
 
 // A product, or its unsummed ranges where the policy leaves them to the kernel behind it
@@ -79,12 +98,12 @@ using namespace b200;
 
 B200_API long long b200_dense_layers_scratch(int tokens, int hidden, int hq, int hkv, int d, int ffn, long long gemm_ws_bytes) {
   const DenseSizes z{tokens, hidden, hq, hkv, d, ffn};
-  return dense_scratch(z, dense_plan(z, gemm_ws_bytes));
+  return dense_layout(z, dense_plan(z, gemm_ws_bytes)).total;
 }
 
 // x [tokens][hidden] bf16 -> out = norm(stream) behind all layers. layer_ptrs: seven pointers a layer (in_norm, qkv, qkv bias or null, o,
-// post_norm, gate_up, down), rows of weights dense. kv: pools [layers][2][pages][hkv][page][d]. cu_q, kv_lens, block_table as in
-// b200_attn_prefill. scratch: b200_dense_layers_scratch bytes on a 256-byte boundary. Returns the number of ops launched, or the
+// post_norm, gate_up, down), rows of weights dense, on 16-byte boundaries and multiples of 8 values long. kv: pools
+// [layers][2][pages][hkv][page][d]. cu_q, kv_lens, block_table as in b200_attn_prefill. scratch: b200_dense_layers_scratch bytes on a 256-byte boundary. Returns the number of ops launched, or the
 // negative code of the one that failed; -14, and nothing is launched: the scratch is too small for the policy as it is now.
 B200_API int b200_dense_layers(const void* x, void* out, const void* const* layer_ptrs, const void* final_norm, void* kv, long long layer_stride,
                                long long v_offset, const int* block_table, const int* kv_lens, const int* cu_q, const int* positions,
@@ -94,17 +113,12 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
                                long long scratch_bytes, void* status, cudaStream_t stream) {
   const DenseSizes z{tokens, hidden, hq, hkv, d, ffn};
   const DensePlan plans = dense_plan(z, gemm_ws_bytes);
-  if (dense_scratch(z, plans) > scratch_bytes) return -14;
-  const long long t = tokens;
-  uint8_t* at = static_cast<uint8_t*>(scratch);
-  auto take = [&](long long bytes) {
-    uint8_t* r = at;
-    at += padded(bytes);
-    return reinterpret_cast<__nv_bfloat16*>(r);
-  };
-  __nv_bfloat16 *h = take(t * hidden * 2), *y = take(t * hidden * 2), *res[2] = {take(t * hidden * 2), take(t * hidden * 2)};
-  __nv_bfloat16 *qkv = take(t * z.qkv() * 2), *q = take(t * z.att() * 2), *att = take(t * z.att() * 2), *gu = take(t * 2 * ffn * 2), *a = take(t * ffn * 2);
-  float* part = reinterpret_cast<float*>(at);
+  const DenseLayout at = dense_layout(z, plans);
+  if (at.total > scratch_bytes) return -14;
+  auto place = [&](long long offset) { return reinterpret_cast<__nv_bfloat16*>(static_cast<uint8_t*>(scratch) + offset); };
+  __nv_bfloat16 *const h = place(at.h), *const y = place(at.y), *const res[2] = {place(at.res[0]), place(at.res[1])};
+  __nv_bfloat16 *const qkv = place(at.qkv), *const q = place(at.q), *const att = place(at.att), *const gu = place(at.gu), *const a = place(at.a);
+  float* const part = reinterpret_cast<float*>(place(at.part));
   int launches = 0, rc = 0;
   auto ok = [&](int code) {
     rc = code;
@@ -154,11 +168,9 @@ B200_API int b200_dense_layers(const void* x, void* out, const void* const* laye
     if (!product(att, w[3], nullptr, y, hidden, z.att(), plans.o, p)) return rc;
     if (!norm(p, stream_in, res[1], w[4], h)) return rc;
     // as ops.linear_glu: one kernel for a handful of tokens and for many, otherwise the product and the activation
-    const int form = b200_glu_form(tokens, ffn, hidden, 0);
-    code = -12;
-    if (form == 1 && aligned(w[5])) code = b200_gemv_glu(h, w[5], a, tokens, ffn, hidden, hidden, hidden, ffn, act, stream);
-    else if (form == 2) code = b200_gemm_glu(h, w[5], a, nullptr, nullptr, tokens, ffn, hidden, hidden, hidden, ffn, 0, nullptr, nullptr, act, 128, status, stream);
-    if (code != -12) {
+    if (plans.form == 1) code = b200_gemv_glu(h, w[5], a, tokens, ffn, hidden, hidden, hidden, ffn, act, stream);
+    else if (plans.form == 2) code = b200_gemm_glu(h, w[5], a, nullptr, nullptr, tokens, ffn, hidden, hidden, hidden, ffn, 0, nullptr, nullptr, act, 128, status, stream);
+    if (plans.form != 0) {
       if (!ok(code)) return rc;
     } else {
       if (!product(h, w[5], nullptr, gu, 2 * ffn, hidden, plans.gate_up, p)) return rc;

@@ -35,3 +35,12 @@ def test_prompt_layers_refuse_scratch_of_another_reduce_form():
         assert L.b200_dense_layers(*args, small, None, None) == -14
     finally:
         L.b200_gemm_set_external_reduce(1 if config.get("splitk_second_kernel") else 0)
+
+
+@pytest.mark.parametrize("hidden,hq,hkv,d,ffn", [(4096, 32, 8, 128, 14336), (8192, 64, 8, 128, 28672), (896, 14, 2, 64, 4864)])
+@pytest.mark.parametrize("tokens", [2048, 8192])
+def test_prompt_layers_scratch_holds_what_lives_at_once(tokens, hidden, hq, hkv, d, ffn):
+    """Long prompts, whose gated product forms the activation itself: four rows of the stream's width, and the larger of what the two halves
+    of a layer hold (the packed projection and q, the activation); no gate and up rows."""
+    got = N.lib().b200_dense_layers_scratch(tokens, hidden, hq, hkv, d, ffn, 64 << 20)
+    assert got <= 2 * tokens * (4 * hidden + max((2 * hq + 2 * hkv) * d, ffn)) + 16 * 256
