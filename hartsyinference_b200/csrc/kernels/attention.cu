@@ -26,7 +26,7 @@
 // The score and PV products use warp-level mma.sync (m16n8k16, bf16): with one to sixteen query
 // rows per KV head the kernel is bound by KV bandwidth, not by tensor throughput, and a 128-row
 // tcgen05 tile would be mostly padding.
-#include "common.cuh"
+#include "layer_ops.cuh"
 #include "mma_sync.cuh"
 
 namespace b200 {

@@ -21,7 +21,7 @@
 //
 // Replaces the per-sequence prefill attention of the reference's scheduler (src/HartsyInference.LLM/Generation/
 // DynamicBatchScheduler.cs, AdmitAndPrefill:311-383).
-#include "common.cuh"
+#include "layer_ops.cuh"
 
 namespace b200 {
 

@@ -4,28 +4,7 @@
 // Why: a launch through the Python ops costs 15 us of host time (argument objects, output tensors, checks), so a short prompt
 // through 24 layers of a small model took 3.4 ms of which the device was busy for one; from here a launch costs 3 us. What
 // lies between the kernels is scratch that the caller allocates once for the whole stack.
-#include "common.cuh"
-
-extern "C" {
-int b200_norm(const void*, const void*, void*, const void*, const void*, const void*, const void*, void*, void*, float*, int, int, int, int,
-              float, int, int, int, const float*, int, int, cudaStream_t);
-int b200_gemm(const void*, const void*, void*, int, int, int, long long, long long, long long, int, const float*, const float*, const void*,
-              const void*, const void*, int, int, void*, long long, void*, cudaStream_t);
-int b200_gemm_deferred_plan(int, int, int, int, long long);
-int b200_gemm_deferred(const void*, const void*, int, int, int, long long, long long, int, const float*, const float*, void*, long long, float*,
-                       void*, cudaStream_t);
-int b200_rope_kv(const void*, void*, void*, void*, void*, void*, const int*, const long long*, const void*, const void*, const float*, int, int,
-                 int, int, int, int, int, float, float, const float*, int, int, const void*, cudaStream_t);
-int b200_attn_prefill_tc(const void*, const void*, const void*, void*, const int*, const int*, const int*, int, int, int, int, int, int, int,
-                         long long, int, float, void*, cudaStream_t);
-int b200_attn_prefill(const void*, const void*, const void*, void*, const int*, const int*, const int*, const int*, int, int, int, int, int, int,
-                      int, int, int, int, int, int, float, float, cudaStream_t);
-int b200_glu(const void*, void*, void*, float*, int, int, int, int, const float*, int, int, cudaStream_t);
-int b200_glu_form(int, int, int, int);
-int b200_gemm_glu(const void*, const void*, void*, void*, void*, int, int, int, long long, long long, long long, int, const float*, const float*,
-                  int, int, void*, cudaStream_t);
-int b200_gemv_glu(const void*, const void*, void*, int, int, int, long long, long long, long long, int, cudaStream_t);
-}
+#include "layer_ops.cuh"
 
 namespace b200 {
 

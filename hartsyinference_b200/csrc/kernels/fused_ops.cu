@@ -11,7 +11,7 @@
 // dit_fp8emit.cu) and its two-pass per-tensor fp8 quantiser (Kernels/dequant/fp8_quant.cu).
 // All rows are processed with 16-byte loads, one CTA per row (or several rows per CTA for short
 // rows), fp32 math, bf16 storage.
-#include "common.cuh"
+#include "layer_ops.cuh"
 
 namespace b200 {
 

@@ -50,6 +50,7 @@
 // small-token orientation the producer requests the first stages of WEIGHT tiles before
 // griddepcontrol.wait and the activation tiles after it; every other role waits first.
 #include "gemm_common.cuh"
+#include "layer_ops.cuh"
 
 namespace b200 {
 

@@ -13,7 +13,7 @@
 //
 // The norm in front (kNorm) and the rotation behind (kRope) can be taken along, and weights further on brought to L2 meanwhile: one
 // token through 24 layers of 896 features 630 us with eight launches a layer, 534 with five, 488 with the weights ahead.
-#include "common.cuh"
+#include "layer_ops.cuh"
 
 namespace b200 {
 
