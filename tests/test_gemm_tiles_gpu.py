@@ -190,6 +190,35 @@ def test_even_shares(m, n, k, fp8, act):
     assert torch.equal(ops.linear(xq, w, act=act, act_from=8 if act == "tanh" else 0, gate=gate, residual=res), y)
 
 
+# the two other operand types: s32 accumulators with row scales, and scales of 1x128 and 128x128 blocks, which a piece reads from the middle of
+# a row of them on
+@pytest.mark.parametrize("m,n,k", [(5, 19200, 640), (64, 28416, 1024), (17, 44416, 896), (100, 24576, 1536), (33, 19072, 512), (3, 38528, 4736)])
+@pytest.mark.parametrize("int8", [True, False])
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+def test_even_shares_other_types(m, n, k, int8, act):
+    torch.manual_seed(m)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    dense = (torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(n, device="cuda").to(torch.bfloat16) if act else None
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16) if act else None
+    if int8:
+        w = ops.Int8Weight.from_dense(dense, bias)
+        q, s = ops.quant_int8_act(x)
+        run = lambda: ops.linear(x, w, act=act, residual=res)
+        ref = (q.double() @ w.weight.double().T) * s.double()[:, None] * w.row_scale.double()[None]
+    else:
+        wq, wsc = R.quant_fp8_weight(dense)
+        xq, xsc = R.quant_fp8_act(x)
+        w = ops.LinearWeight(wq, wsc, bias)
+        run = lambda: ops.linear(ops.Fp8Act(xq, xsc), w, act=act, residual=res)
+        ref = R.linear(xq, wq, wsc, xsc, None, None, None, None, torch.float32).double()
+    ref = ref + bias.double() if act else ref
+    ref = torch.nn.functional.gelu(ref, approximate="tanh") + res.double() if act else ref
+    y = run()
+    assert torch.allclose(y.double(), ref, rtol=2 ** -7, atol=2 ** -7), (y.double() - ref).abs().max()      # one rounding to bf16; fp32 sums
+    assert torch.equal(run(), y)
+
+
 # Streams of one device share the scratch, so a product that does without it must leave it alone: few tokens and a last wave more than half
 # full (above all with long rows), rows of too few K blocks to cut, and many tokens on CTA pairs
 @pytest.mark.parametrize("m,n,k", [(6, 28672, 4096), (64, 28672, 4096), (128, 30720, 8192), (17, 29000, 4608), (33, 151936, 192), (5, 19200, 64), (300, 12288, 3072)])
