@@ -218,14 +218,15 @@ __device__ __forceinline__ void act_chunk(int act, float (&v)[32]) {
 // Stores 32 consecutive accumulator columns (B rows b0..b0+31) of A row `a_row` of a whole tile
 // to its destination: C, or (fused all-reduce) the staging buffer of the owning rank.
 // `b_end` is the end of the tile's B rows (a 16-row tile fills only half of a 32-column chunk; the
-// rest of the chunk is not this tile's data).
+// rest of the chunk is not this tile's data). kSwap: the small-token orientation (p.swap_out).
+template <bool kSwap>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, float (&v)[32], int a_row,
                                             int b0, int b_end, int split = 0) {
   if (a_row >= p.rows_a) return;
   if (p.ar.world > 0) {
     // fused all-reduce: raw bf16 partial of this K split into the rank's own [split][token][feature]
     // buffer (always the small-token orientation: a_row is the feature, the chunk walks tokens)
-    if (!p.swap_out) {
+    if constexpr (!kSwap) {
       // large-token orientation: a_row is the token, the chunk walks 32 features (whole chunks:
       // the feature count is a multiple of 128)
       if (b0 >= b_end) return;
@@ -243,7 +244,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, float (&v)[32],
       if (b0 + j < b_end) dst[static_cast<long long>(j) * p.rows_a] = __float2bfloat16(v[j]);
     return;
   }
-  if (!p.swap_out) {
+  if constexpr (!kSwap) {
     __nv_bfloat16* dst = p.out + static_cast<long long>(a_row) * p.ldc + b0;
     if (b0 + 32 <= b_end && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
       uint32_t w[16];

@@ -428,7 +428,7 @@ gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a, c
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_chunk(p, v, row, b0, p.rows_b);
+            store_chunk<false>(p, v, row, b0, p.rows_b);
           }
         }
       }

@@ -79,18 +79,22 @@ struct WorkItem {
   int bk;            // element offset of the group's columns in B (column-batched mode)
 };
 
+// kFew: the small-token orientation, the only one with even shares (a compile-time matter, as in emit_chunk: with their branch and the
+// small tokens' epilogue in their code the large-token kernels took 0.5 to 0.8 us more a launch, 512 x 4096 x 256 fp8 8.5 us against 7.9)
+template <bool kFew>
 __device__ __forceinline__ long long num_work_items(const GemmParams& p) {
   if (p.block_group != nullptr) return static_cast<long long>(*p.dyn_blocks) * (p.group_n / kTileA);
   // a share of s groups covers s / groups + 2 tiles at most, in part
-  if (p.share_ctas > 0) return p.share_ctas * ((static_cast<long long>(p.num_tiles) + p.share_ctas - 1) / p.share_ctas + 2);
+  if (kFew && p.share_ctas > 0) return p.share_ctas * ((static_cast<long long>(p.num_tiles) + p.share_ctas - 1) / p.share_ctas + 2);
   return p.first_split_tile + static_cast<long long>(p.num_tiles - p.first_split_tile) * p.splits;
 }
 
+template <bool kFew>
 __device__ __forceinline__ WorkItem decode_item(const GemmParams& p, long long w, int tiles_a,
                                                 int total_kblocks) {
   WorkItem it;
   long long tile;
-  if (p.share_ctas > 0) {
+  if (kFew && p.share_ctas > 0) {
     const long long all = static_cast<long long>(p.num_tiles) * p.share_groups;
     const int c = static_cast<int>(w % p.share_ctas), n = static_cast<int>(w / p.share_ctas);
     const int first = static_cast<int>(all * c / p.share_ctas), end = static_cast<int>(all * (c + 1) / p.share_ctas);
@@ -195,7 +199,7 @@ __device__ __forceinline__ void emit_chunk(const GemmParams& p, float (&v)[32], 
   if (it.slot >= 0 && p.ar.world == 0 && !(!kLarge && merge)) store_partial<BN>(p, v, row_local, chunk * 32, it);
   else if (kLarge && p.row_stores && it.tb * BN + chunk * 32 + 32 <= p.rows_b)
     store_chunk_rows(p, v, it.ta * kTileA + (row_local & ~31), it.tb * BN + chunk * 32, strip);
-  else store_chunk(p, v, it.ta * kTileA + row_local, it.tb * BN + chunk * 32, min(p.rows_b, (it.tb + 1) * BN),
+  else store_chunk<!kLarge>(p, v, it.ta * kTileA + row_local, it.tb * BN + chunk * 32, min(p.rows_b, (it.tb + 1) * BN),
                    it.split);
 }
 
@@ -659,7 +663,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, 
   pdl_trigger();
   const int e4 = blockIdx.x * blockDim.x + threadIdx.x;
   if (e4 >= bn * 32) return;
-  const WorkItem it = decode_item(p, p.first_split_tile + static_cast<long long>(blockIdx.y) * p.splits,
+  const WorkItem it = decode_item<false>(p, p.first_split_tile + static_cast<long long>(blockIdx.y) * p.splits,
                                   tiles_a, total_kblocks);
   if (it.skip) return;
   reduce_partials<8>(p, it, bn, e4);
@@ -714,7 +718,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
 
   const int tiles_a = (p.rows_a + kTileA - 1) / kTileA;
   const int total_kblocks = (p.k + kElemsPerAtom - 1) / kElemsPerAtom;
-  const long long work_items = num_work_items(p);
+  const long long work_items = num_work_items<kAtoms == 2>(p);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -809,7 +813,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       int pre = 0;                 // stage iterations of the first item already half-issued
       long long w_first = blockIdx.x;
       if (p.swap_out && p.group_n == 0 && w_first < work_items) {
-        const WorkItem it = decode_item(p, w_first, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kAtoms == 2>(p, w_first, tiles_a, total_kblocks);
         const int sfb = first_sfb(it);
         for (int kb = it.kb0; kb < it.kb1 && pre < stages; kb += kAtoms, ++pre) issue_stage(it, sfb, kb, pre, 1);
         pdl_wait();
@@ -823,7 +827,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       const uint32_t ag_call = p.ag.world > 0 ? *reinterpret_cast<volatile uint32_t*>(p.ag.ctr) + 1u : 0u;
       uint32_t ag_seen = 0;
       for (long long w = blockIdx.x; w < work_items && ok; w += gridDim.x) {
-        const WorkItem it = decode_item(p, w, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
         if (it.skip) continue;
         if (p.ag.world > 0 && !ag_wait_tile(p, it.ta, ag_call, ag_seen)) {
           report_status(p.status, kWaitTimeout, kKernelAllToAll, 12, blockIdx.x);
@@ -867,7 +871,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       bool ok = true;
       bool issued_any = false;
       for (long long w = blockIdx.x; w < work_items && ok; w += gridDim.x) {
-        const WorkItem it = decode_item(p, w, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
         if (it.skip) continue;
         if (!kFp8) {
           if (!mbar_wait(&bars->tmem_empty[abuf], aph ^ 1, abort_flag)) {
@@ -964,7 +968,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     bool ok = true;
     uint32_t glu_round = 0;
     for (long long w = blockIdx.x; w < work_items; w += gridDim.x) {
-      const WorkItem it = decode_item(p, w, tiles_a, total_kblocks);
+      const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
       if (it.skip) continue;
       if constexpr (kGlu) {
         if (ok && !__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[abuf], aph, abort_flag))) {
@@ -1180,7 +1184,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     // over all CTAs (fixed order: deterministic), applies the epilogue and stores C
     cluster_sync_all();
     if (warp >= 2) {
-      const WorkItem it = decode_item(p, blockIdx.x, tiles_a, total_kblocks);
+      const WorkItem it = decode_item<kAtoms == 2>(p, blockIdx.x, tiles_a, total_kblocks);
       const int et = threadIdx.x - 64;
       const uint32_t rank = cluster_ctarank();
       const int total4 = BN * 32;                                  // float4 groups of the tile
