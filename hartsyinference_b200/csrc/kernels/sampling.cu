@@ -14,7 +14,7 @@
 // A row of up to 262144 logits belongs to a cluster of eight blocks that keep it in registers: one read of
 // the row, histograms and prefix sums met through distributed shared memory. Longer rows go through one block that makes
 // eight passes over a row in L2, and so do short rows and many rows of moderate length, where the exchanges of a
-// cluster cost more than the passes (see b200_sample). Both forms sum masses in 2^-40, so a row's token is the
+// cluster cost more than the passes (see b200_sample_form). Both forms sum masses in 2^-40, so a row's token is the
 // same whatever batch it comes in (fp32 sums in the one block drew another token than the cluster in two or three of 1000 flat rows of 100000).
 //
 // The reference applies the same chain on the host, one request at a time, after copying the logits
@@ -677,6 +677,33 @@ static int launch_rows(const SampleParams& p, int rows, cudaStream_t stream) {
 
 using namespace b200;
 
+static int row_values(int vocab) { return (vocab + kRowBlocks * kRowThreads - 1) / (kRowBlocks * kRowThreads); }      // that a thread holds
+
+// Whether b200_sample gives a row to a cluster (1) or to one block (0). Which filters a row asks for is known on the device only. Every filter
+// asked for, a block takes 28 us + a us per 290 logits, all rows of a wave at once; a cluster 21 to 44 us, twice that when they fill the
+// machine, and from there 0.8 to 2.9 us a row by the values that a thread holds. Without filters a block takes 4 us + a us per 1950 to 2400
+// logits and 0.7 of that for each further wave; a cluster 7 to 18 us, a fifth more from 16 rows and nearly twice that from 37 on, where a
+// second wave starts, and 0.2 to 0.7 us a row beyond 49. A cluster has to be a fifth faster in the full chain and at most an eighth slower
+// without one (us, block / cluster: without filters, with all):
+//   1 x 2048      5.0 / 6.5, 30 / 21      8 x 8192      7.5 / 6.9, 47 / 22      37 x 8192     7.6 / 12.4, 47 / 45     48 x 16384    11.2 / 13.5, 69 / 47
+//   64 x 32000    22 / 16, 116 / 52       96 x 50257    26 / 27, 159 / 91       64 x 128256   64 / 37, 433 / 92      128 x 128256  65 / 71, 437 / 181
+//   148 x 128256  64 / 82, 435 / 214      200 x 202048  206 / 415, 1367 / 771   256 x 151936  152 / 235, 1033 / 480  512 x 100352  266 / 395, 1258 / 819
+// Rows of more than 163840 logits, one block of a cluster on a processor: there the full chain decides, with 105 us for 18 of them.
+B200_API int b200_sample_form(int rows, int vocab) {
+  const int each = row_values(vocab), sms = num_sms();
+  if (rows < 1 || rows >= (1 << 27) || sms < kRowBlocks || each > 64) return 0;
+  const int waves = (rows + sms - 1) / sms;
+  if (each > 40) return 105. * ((rows + 17) / 18) <= (24. + vocab / 350.) * waves ? 1 : 0;
+  const int width = each <= 8 ? 0 : each <= 16 ? 1 : each <= 32 ? 2 : 3;
+  constexpr double kRowUs[4] = {0.76, 0.93, 1.33, 1.6};                                        // with every filter
+  const double block_us = (28. + vocab / 290.) * waves, cluster_us = kRowUs[width] * (rows <= 8 ? 28. : rows <= 18 ? 36. : rows <= 49 ? 55. : rows + 6.);
+  constexpr double kFirst[4] = {6.9, 8., 15., 18.4}, kMore[4] = {0.205, 0.25, 0.52, 0.67}, kBase[4] = {1.5, 3., 4., 2.5};      // without
+  constexpr double kLogitsUs[4] = {2400., 2400., 2150., 1950.};
+  const double block_plain = 4.2 + vocab / kLogitsUs[width] * (1. + 0.72 * (waves - 1));
+  const double cluster_plain = rows <= 12 ? kFirst[width] : rows <= 36 ? 1.22 * kFirst[width] : rows <= 49 ? 1.9 * kFirst[width] : kBase[width] + kMore[width] * rows;
+  return cluster_us <= 0.8 * block_us && cluster_plain <= 1.12 * block_plain ? 1 : 0;
+}
+
 // logits [rows][ld] (fp32 when is_f32, else bf16); per-row device arrays as in SampleParams; out int32 [rows].
 B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows, int vocab, const float* temperature,
                          const int* top_k, const float* top_p, const float* min_p, const unsigned long long* seed,
@@ -687,21 +714,8 @@ B200_API int b200_sample(const void* logits, int is_f32, long long ld, int rows,
   p.logits = logits; p.is_f32 = is_f32; p.ld = ld; p.vocab = vocab;
   p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.min_p = min_p;
   p.seed = seed; p.counter = counter; p.out = out;
-  const int each = (vocab + kRowBlocks * kRowThreads - 1) / (kRowBlocks * kRowThreads);      // values a thread holds
-  // A block of its own per row takes 28 us + a us per 290 logits with every filter, all rows of a wave at once, and 9 + one per 2100
-  // without. A cluster takes 24 to 44 us, twice that when they fill the machine, and from there 0.8 to 2.9 us a row by the
-  // values that a thread holds, and a third of that without filters. Which filters a row asks for is known on the device only:
-  // a cluster has to be a fifth faster in the full chain and no slower without one. With every filter (us, block / cluster)
-  // 1 x 4096 38 / 24, 1 x 128256 470 / 34, 16 x 2048 34 / 28, 37 x 4096 40 / 47, 48 x 16384 79 / 48, 96 x 16384 79 / 79, 64 x 128256
-  // 484 / 86, 128 x 151936 579 / 200, 512 x 16384 301 / 393; without 48 x 16384 15 / 15, 96 x 50257 30 / 28, 148 x 50257 30 / 42,
-  // 64 x 128256 66 / 32, 128 x 202048 110 / 134.
-  const int sms = num_sms(), waves = (rows + sms - 1) / sms;
-  const int width = each <= 8 ? 0 : each <= 16 ? 1 : each <= 32 ? 2 : each <= 40 ? 3 : 4;
-  constexpr double kRowUs[5] = {0.76, 0.93, 1.33, 1.6, 2.9}, kPlainUs[5] = {0.235, 0.285, 0.43, 0.6, 1.05};
-  const double block_us = (28. + vocab / 290.) * waves, block_plain = (9. + vocab / 2100.) * waves;
-  const double cluster_us = kRowUs[width] * (rows <= 8 ? 28. : rows <= 18 ? 36. : rows <= 49 ? 55. : rows + 6.);
-  const double cluster_plain = 3. + kPlainUs[width] * rows;
-  if (rows < (1 << 27) && sms >= kRowBlocks && cluster_us <= 0.8 * block_us && cluster_plain <= 1.05 * block_plain) {
+  if (b200_sample_form(rows, vocab)) {
+    const int each = row_values(vocab);
     if (each <= 8) return launch_rows<8>(p, rows, stream);
     if (each <= 16) return launch_rows<16>(p, rows, stream);
     if (each <= 32) return launch_rows<32>(p, rows, stream);
