@@ -468,7 +468,7 @@ int make_kmajor_map(CUtensorMap* out, const void* base, int elem_bytes, long lon
 
 int make_sf_map(CUtensorMap* out, const void* base, long long blocks);   // scale-factor blocks of 128 words; a box is one block
 // gemm_pair.cu: products on CTA pairs. p holds sizes, epilogue and scale factors; rows_a tokens, rows_b weight rows
-bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual);
+bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual, bool fuses = false);
 int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream, bool quant = false);
 
 }  // namespace b200

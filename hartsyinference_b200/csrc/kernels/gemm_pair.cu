@@ -475,24 +475,34 @@ static int launch_pair(const GemmParams& p, const CUtensorMap (&maps)[4], cudaSt
 }
 
 // Whether a product of `tokens` rows by `rows_b` weight rows runs here and not on the tiles of one SM (gemm_tcgen05.cu). Both sides
-// measured over 24 shapes at depths 1024 to 12288 (bf16 256 x 9216 x 3072 47.4 -> 23.7 us, 2600 x 28672 x 4096 gated 535 -> 417,
+// measured over 1200 sizes of either type around the line (bf16 256 x 9216 x 3072 47.4 -> 23.7 us, 2600 x 28672 x 4096 gated 535 -> 417,
 // fp8 600 x 4096 x 3072 56.5 -> 17.0, 8192 x 8192 x 8192 480 -> 377, 4096 x 9216 x 3072 116 -> 92):
 //  - a wave of pair tiles takes 0.8 of the time of a wave of 128 x 256 tiles in bf16 and 0.6 to 0.7 in 8 bits, so tokens that leave
-//    the last 256 rows half empty stay there where that costs more waves (300 x 12288 x 4096, two waves against one: bf16
-//    47.1 us here and 38.7 there; fp8 16.3 and 15.0 at depth 1024, 25.4 and 26.7 at 3072)
-//  - few tiles of a long row are cut along K there (bf16 k 12288: 16 tiles 64.9 here and 45.4 there, 24 tiles 65.0 and 59.0, 32 tiles
-//    64.8 and 71.3; k 4096: 16 tiles 27.9 and 28.5), 8-bit ones of a short row are as fast (k 1024: 36 tiles 12.1 and 11.5, 40 tiles
-//    11.9 and 48.5, k 3072: 24 tiles 15.8 and 16.8).
+//    the last 256 rows half empty stay there where that costs more waves (bf16 five waves against four: 640 x 28672 x 1024 39.8 us there
+//    and 36.0 here, k 4096 118 both, k 8192 230 and 237, 2600 x 7168 x 14336 382 and 403; fp8 300 x 12288 x 1024 14.4 and 15.3)
+//  - few tiles of a long row are cut along K there: bf16 16 to 19 tiles k 3072 24.3 there and 21.8 here, k 4096 24.5 and 26.9, and where six
+//    ranges of a tile fit (300 x 2048) 21.1 and 21.7, 22.1 and 26.2; in three ranges (300 x 4096) k 6144 38.1 and 37.5, k 8192 44.1 and 46.8,
+//    k 14336 58 and 75; in two (512 x 4096) k 14336 76.6 and 75.7, k 18432 90.5 and 94.1. fp8 16 to 19 tiles k 8192 30.9 and 26.7,
+//    k 12288 34.3 and 37.2, in six ranges k 6144 22.1 and 22.2, k 8192 24.8 and 26.7; ones of a short row are as fast there
+//    (300 x 6144 x 1024 10.4 and 10.7, k 256 8.0 and 8.6)
+// fuses: the epilogue here does the work of a kernel that would follow a product there, and the line lies further out (gated 300 x 1024
+// of k 4096 24.7 there, 25.8 here; never slower over 264 sizes of either type otherwise).
 // Rows of the output (and residual) start on 32-byte boundaries: the epilogue's accesses.
-bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual) {
+bool pair_takes(long long tokens, long long rows_b, int k, int dtype, long long ldc, const void* out, const void* residual, bool fuses) {
   if (tokens <= 128 || (dtype != 0 && dtype != 2)) return false;
   if (ldc % 16 != 0 || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 31)) return false;
   const long long sms = num_sms(), cols = (rows_b + 255) / 256;
   const long long tiles = (tokens + 255) / 256 * cols, waves = (tiles + sms / 2 - 1) / (sms / 2);
-  const long long waves_one = ((tokens + 127) / 128 * cols + sms - 1) / sms;
+  const long long one = (tokens + 127) / 128 * cols, waves_one = (one + sms - 1) / sms;      // 128 x 256 tiles
   if (tiles < 16 || tiles >= 1ll << 30) return false;
-  if (dtype == 0) return 4 * waves <= 5 * waves_one && (tiles >= 32 || k <= 4096);
-  return (3 * waves <= 5 * waves_one || k >= 3072) && (k >= 2048 || tiles > 36) && (tiles >= 32 || k <= 12288);
+  if (dtype == 0) {
+    if (4 * waves > 5 * waves_one || (tiles < 32 && k > 4096)) return false;
+    if (fuses) return tiles >= 20 || k <= 3072 || 6 * one > sms;
+    return (4 * waves < 5 * waves_one || k <= 4096) && (tiles >= 20 || k <= (6 * one <= sms ? 2048 : 3072)) &&
+           (3 * one > sms || k <= 6144) && (2 * one > sms || k <= 14336);
+  }
+  if ((3 * waves > 5 * waves_one && k < 3072) || (k < 2048 && tiles <= 36) || (tiles < 32 && k > 12288)) return false;
+  return fuses || ((k >= 2048 || 2 * one > sms) && (tiles >= 20 || k <= (6 * one <= sms ? 6144 : 8192)));
 }
 
 int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long long ldw, int dtype, cudaStream_t stream, bool quant) {
@@ -515,9 +525,12 @@ int gemm_pair(GemmParams p, const void* x, const void* w, long long ldx, long lo
 
 using namespace b200;
 
+// Whether b200_gemm runs m tokens by n features of depth k on CTA pairs (operands and output dense).
+B200_API int b200_gemm_on_pairs(int m, int n, int k, int dtype) { return pair_takes(m, n, k, dtype, n, nullptr, nullptr) ? 1 : 0; }
+
 // Whether b200_gemm_quant takes m tokens by n features of depth k.
 B200_API int b200_gemm_quant_fits(int m, int n, int k) {
-  return m > 128 && n >= 128 && n % 128 == 0 && k >= 16 && k % 16 == 0 && pair_takes(m, n, k, 2, n, nullptr, nullptr) ? 1 : 0;
+  return m > 128 && n >= 128 && n % 128 == 0 && k >= 16 && k % 16 == 0 && pair_takes(m, n, k, 2, n, nullptr, nullptr, true) ? 1 : 0;
 }
 
 // act(x w^T + bias) of e4m3 operands with UE8M0 scales for a next product that reads e4m3: features from q_from on (a multiple of 128)

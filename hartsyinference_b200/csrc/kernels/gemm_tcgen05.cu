@@ -1770,7 +1770,7 @@ B200_API int b200_glu_form(int m, int f, int k, int dtype) {
   if (m < 1 || f < 1 || k < 1) return 0;
   if (f <= (1 << 30) && f % 8 == 0 && handful(m, 2 * f, k, dtype)) return 1;
   if (m <= 128 || f % 128 != 0 || (dtype != 0 && dtype != 2)) return 0;
-  if (pair_takes(m, 2ll * f, k, dtype, f, nullptr, nullptr)) return 2;
+  if (pair_takes(m, 2ll * f, k, dtype, f, nullptr, nullptr, true)) return 2;
   const long long tiles = (m + 127ll) / 128 * (f / 128), full = tiles / num_sms(), rest = tiles % num_sms();
   return full >= 3 || (full == 2 && (rest == 0 || 2 * rest > num_sms())) ? 2 : 0;
 }
@@ -1809,7 +1809,7 @@ B200_API int b200_gemm_glu(const void* x, const void* w, void* out, void* out_q,
   p.sf_b = reinterpret_cast<const uint32_t*>(w_scale);
   p.sf_kgroups = (k + 511) / 512;
   p.sf_tile_b = 128;
-  if (pair_takes(m, 2ll * f, k, dtype, mx ? f : ldc, mx ? out_q : out, nullptr)) return gemm_pair(p, x, w, ldx, ldw, dtype, stream);
+  if (pair_takes(m, 2ll * f, k, dtype, mx ? f : ldc, mx ? out_q : out, nullptr, true)) return gemm_pair(p, x, w, ldx, ldw, dtype, stream);
   if (tiles < num_sms()) return -12;
   p.num_tiles = p.first_split_tile = static_cast<int>(tiles);
   p.splits = 1;

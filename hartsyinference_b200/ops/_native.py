@@ -84,6 +84,7 @@ _SIGNATURES = {
     "b200_kv_store": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i32, vp]),
     "b200_glu_form": (i32, [i32, i32, i32, i32]),
     "b200_gemm_glu": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp, vp, i32, i32, vp, vp]),
+    "b200_gemm_on_pairs": (i32, [i32, i32, i32, i32]),
     "b200_gemm_quant_fits": (i32, [i32, i32, i32]),
     "b200_gemm_quant": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp, vp, i32, i32, i64, i32, i32, vp, vp]),
     "b200_attn_fa_quant": (i32, [vp, vp, vp, i32, i32, i32, f32, i32, vp, vp, i64, i32, i32, vp, vp, i64, i32, i32, vp, vp]),

@@ -52,3 +52,13 @@ def test_prompt_layers_scratch_holds_what_lives_at_once(tokens, hidden, hq, hkv,
     (1, 8192, 1), (8, 16384, 1), (64, 32000, 1), (96, 50257, 1), (64, 128256, 1), (128, 128256, 1), (128, 151936, 1), (1, 256000, 1), (1, 262145, 0), (1 << 28, 32000, 0)])
 def test_sampler_form(rows, vocab, cluster):
     assert N.lib().b200_sample_form(rows, vocab) == cluster
+
+
+# both kernels measured: CTA pairs where they are faster (dtype 0 bf16, 2 fp8)
+@pytest.mark.parametrize("m,n,k,dtype,pairs", [
+    (300, 4096, 14336, 0, 0), (300, 4096, 8192, 0, 0), (300, 2048, 4096, 0, 0), (129, 4096, 4096, 0, 0), (512, 4096, 18432, 0, 0), (2600, 7168, 14336, 0, 0),
+    (640, 28672, 8192, 0, 0), (300, 2048, 8192, 2, 0), (129, 4096, 12288, 2, 0), (300, 6144, 1024, 2, 0), (300, 6144, 256, 2, 0), (128, 28672, 4096, 0, 0),
+    (300, 4096, 6144, 0, 1), (300, 3072, 4096, 0, 1), (1024, 1024, 3072, 0, 1), (256, 9216, 3072, 0, 1), (640, 28672, 1024, 0, 1), (2600, 28672, 4096, 0, 1),
+    (1024, 1024, 8192, 2, 1), (300, 6144, 2048, 2, 1), (600, 4096, 3072, 2, 1), (4096, 9216, 3072, 2, 1)])
+def test_products_on_pairs(m, n, k, dtype, pairs):
+    assert N.lib().b200_gemm_on_pairs(m, n, k, dtype) == pairs
