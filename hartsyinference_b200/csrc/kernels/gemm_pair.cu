@@ -533,6 +533,12 @@ B200_API int b200_gemm_quant_fits(int m, int n, int k) {
   return m > 128 && n >= 128 && n % 128 == 0 && k >= 16 && k % 16 == 0 && pair_takes(m, n, k, 2, n, nullptr, nullptr, true) ? 1 : 0;
 }
 
+// Whether b200_gemm_quant is faster than b200_gemm and the quantisation of its output. The epilogue that quantises takes 3 to 6 us longer at
+// the end of the last wave, the other kernel 3 us and what it reads and writes: measured over 67 sizes (the two / this, us) 512 x 12288 of k 3072
+// 35.5 / 36.3, 256 x 13824 of k 5120 30 / 43, 1024 x 13824 69.6 / 72.0, 1024 x 12288 52.0 / 50.9, 1651 x 3072 of k 768 27.1 / 29.0, 1651 x 6144 of
+// k 1536 42.7 / 41.7, 2560 x 3072 30.5 / 29.5, 4608 x 12288 186 / 157, 14040 x 13824 917 / 781.
+B200_API int b200_gemm_quant_pays(int m, int n) { return m >= 1536 && static_cast<long long>(m) * n >= 7500000 ? 1 : 0; }
+
 // act(x w^T + bias) of e4m3 operands with UE8M0 scales for a next product that reads e4m3: features from q_from on (a multiple of 128)
 // leave as e4m3 with 1x128 scales (rounded to bf16 first, as a quantisation of the stored product would find them) in columns from q_col0
 // on of out_q, rows q_ld bytes apart; scales in the blocked layout of q_kgroups words a row. The features in front leave as bf16 in

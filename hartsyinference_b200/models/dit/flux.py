@@ -440,7 +440,7 @@ class FluxTransformer:
             xn, _, xq = ops.norm(x, None, shift=mod[:, 3 * H:4 * H], scale=mod[:, 4 * H:5 * H], rows_per_batch=S,
                                  layernorm=True, emit_fp8=self.fp8 and w.mlp_in.is_fp8,
                                  emit_bf16=not (self.fp8 and w.mlp_in.is_fp8))
-            h8 = ops.linear_quant(xq, w.mlp_in, act="gelu_tanh") if xq is not None and quant_ok(w.mlp_out) else None
+            h8 = ops.linear_quant(xq, w.mlp_in, act="gelu_tanh", if_faster=True) if xq is not None and quant_ok(w.mlp_out) else None
             h = h8[1] if h8 is not None else ops.linear(xq if xq is not None else xn, w.mlp_in, act="gelu_tanh")
             return self._row_parallel(h, w.mlp_out, x, mod[:, 5 * H:6 * H], S, rp_fused, slot + 1)
 
@@ -500,7 +500,7 @@ class FluxTransformer:
                                      emit_fp8=self.fp8 and w.qkv_mlp.is_fp8, emit_bf16=not (self.fp8 and w.qkv_mlp.is_fp8))
                 # [T, q | k | v | mlp]: the activation of the last part is the product's epilogue; once q, k and v are
                 # split off, the attention output takes the place of v, next to the part it is projected with
-                split = ops.linear_quant(xq, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols, q_from=qkv_cols, lead=self.hl * D) \
+                split = ops.linear_quant(xq, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols, q_from=qkv_cols, lead=self.hl * D, if_faster=True) \
                     if xq is not None and quant_ok(w.out) and ops.attention_quant_fits(self.hl, self.hl, D, S) else None
                 fused = split[0] if split is not None else ops.linear(xq if xq is not None else xn, w.qkv_mlp, act="gelu_tanh", act_from=qkv_cols)
                 q, k, v = ops.dit_qkv(fused[:, :qkv_cols], self.hl, self.hl, D, q_norm_w=w.q_norm, k_norm_w=w.k_norm,

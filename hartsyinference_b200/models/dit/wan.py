@@ -257,7 +257,7 @@ class WanTransformer:
             xn, _, xq = ops.norm(x, None, shift=m[:, 3 * H:4 * H], scale=m[:, 4 * H:5 * H], rows_per_batch=S_l,
                                  layernorm=True, eps=cfg.eps, emit_fp8=self.fp8 and blk.ffn_in.is_fp8,
                                  emit_bf16=not (self.fp8 and blk.ffn_in.is_fp8))
-            h8 = ops.linear_quant(xq, blk.ffn_in, act="gelu_tanh") if xq is not None and blk.ffn_out.is_mx else None
+            h8 = ops.linear_quant(xq, blk.ffn_in, act="gelu_tanh", if_faster=True) if xq is not None and isinstance(blk.ffn_out, LinearWeight) and blk.ffn_out.is_mx else None
             h = h8[1] if h8 is not None else ops.linear(xq if xq is not None else xn, blk.ffn_in, act="gelu_tanh")
             x = ops.linear(h, blk.ffn_out, gate=m[0, 5 * H:6 * H].contiguous(), residual=x)
         hm = (self.head_mod.float() + e.float()).to(dt).reshape(1, 2 * H).contiguous()         # shift, scale

@@ -86,6 +86,7 @@ _SIGNATURES = {
     "b200_gemm_glu": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp, vp, i32, i32, vp, vp]),
     "b200_gemm_on_pairs": (i32, [i32, i32, i32, i32]),
     "b200_gemm_quant_fits": (i32, [i32, i32, i32]),
+    "b200_gemm_quant_pays": (i32, [i32, i32]),
     "b200_gemm_quant": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp, vp, i32, i32, i64, i32, i32, vp, vp]),
     "b200_attn_fa_quant": (i32, [vp, vp, vp, i32, i32, i32, f32, i32, vp, vp, i64, i32, i32, vp, vp, i64, i32, i32, vp, vp]),
     "b200_gemv_glu": (i32, [vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp]),

@@ -352,15 +352,18 @@ def linear(x, w: LinearWeight, act: Optional[str] = None, gate: Optional[torch.T
     return out
 
 
-def linear_quant(x, w, act: Optional[str] = None, act_from: int = 0, q_from: int = 0, lead: int = 0):
+def linear_quant(x, w, act: Optional[str] = None, act_from: int = 0, q_from: int = 0, lead: int = 0, if_faster: bool = False):
     """``linear(x, w, act, act_from=act_from)`` of e4m3 operands in UE8M0 mode for a next product that reads e4m3: ``(y, q)`` with
     the output features in front of ``q_from`` as bf16 y (None: there are none) and the others as :class:`Fp8Act` q, in its
     columns from ``lead`` on (the ones in front are for another kernel to write). The same values as a quantisation of the
-    stored product. None, and nothing is done, where the product has no such form (few tokens, other operands)."""
+    stored product. None, and nothing is done, where the product has no such form (few tokens, other operands) and, with
+    ``if_faster``, where the product and a quantisation behind it take less time."""
     if not (isinstance(x, Fp8Act) and isinstance(w, LinearWeight) and x.data.is_cuda and w.is_mx and x.sf is not None and x.tile_rows == 128):
         return None
     (m, k), n, xd = x.data.shape, w.weight.shape[0], x.data
     if q_from % 128 or lead % 128 or w.weight.shape[1] != k or xd.stride(1) != 1 or w.weight.stride(1) != 1 or not N.lib().b200_gemm_quant_fits(m, n, k):
+        return None
+    if if_faster and not N.lib().b200_gemm_quant_pays(m, n):
         return None
     y = torch.empty(m, q_from, dtype=torch.bfloat16, device=xd.device) if q_from else None
     q = empty_fp8_act(m, lead + n - q_from, xd.device)

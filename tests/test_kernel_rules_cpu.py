@@ -62,3 +62,8 @@ def test_sampler_form(rows, vocab, cluster):
     (1024, 1024, 8192, 2, 1), (300, 6144, 2048, 2, 1), (600, 4096, 3072, 2, 1), (4096, 9216, 3072, 2, 1)])
 def test_products_on_pairs(m, n, k, dtype, pairs):
     assert N.lib().b200_gemm_on_pairs(m, n, k, dtype) == pairs
+
+
+@pytest.mark.parametrize("m,n,pays", [(200, 21504, 0), (512, 12288, 0), (1024, 13824, 0), (1651, 3072, 0), (1651, 6144, 1), (2560, 3072, 1), (4608, 12288, 1), (14040, 13824, 1)])
+def test_quantising_epilogue_pays(m, n, pays):
+    assert N.lib().b200_gemm_quant_pays(m, n) == pays
