@@ -39,6 +39,7 @@ struct GemvBf16Params {
   const long long* slots;         // < 0: k and v are not stored
   const float* inv_freq;          // [rot / 2]
   int hq, hkv, d, rot, style, page;
+  int early;                      // the kernel behind may be launched from the start on
   // kNorm: weights of products further on that are brought to L2 meanwhile
   const uint8_t* ahead[2];
   long long ahead_bytes[2];
@@ -121,8 +122,10 @@ __global__ void __launch_bounds__(256) gemv_bf16_kernel(const GemvBf16Params p) 
     pdl_wait();
     // With kRope attention follows, whose blocks share the keys: launched while the last blocks here still run they crowd the processors
     // that are free first, and the fullest one ends late (a layer of 4096 features and 9000 keys 117.4 us, without the trigger 110.1; of
-    // 1536 and 4000 53.2 and 48.7, and 40 44.8 and 43.5).
-    if (kForm != kRope) pdl_trigger();
+    // 1536 and 4000 53.2 and 48.7, and 40 44.8 and 43.5). Only few blocks of little work gain by being there early: heads of 64 values and
+    // at most 256 keys (896 features: 64 keys 20.5 us early, 20.9 late, 256 22.5 and 22.6, 512 23.6 and 23.5; heads of 128 42.4 and 42.6 for
+    // 128 keys, 43.3 and 42.6 for 256).
+    if (kForm != kRope || p.early) pdl_trigger();
     float ss[kTokens];
 #pragma unroll
     for (int t = 0; t < kTokens; ++t) {
@@ -351,11 +354,12 @@ B200_API int b200_gemv_norm_glu(const void* x, const void* norm_w, const void* w
 }
 
 // q | k | v = norm(x) w^T + bias of m decoded tokens with the rotary embedding (b200_rope_kv without head norms) in the epilogue: q to
-// q_out [m][hq][d], k and v into their pages. Three launches in one. d even, rot even and at most d, inv_freq [rot / 2].
+// q_out [m][hq][d], k and v into their pages. Three launches in one. early: the next kernel in the stream may be launched while this one runs. d even, rot even and at most d, inv_freq [rot / 2].
 B200_API int b200_gemv_norm_qkv(const void* x, const void* norm_w, const void* w, const void* bias, void* q_out, void* k_cache, void* v_cache,
                                 const int* positions, const long long* slots, const float* inv_freq, int m, int k, long long ldx, long long ldw,
                                 int hq, int hkv, int d, int rot, int style, int page, float eps, int plus_one,
-                                const void* ahead_a, long long ahead_a_bytes, const void* ahead_b, long long ahead_b_bytes, cudaStream_t stream) {
+                                const void* ahead_a, long long ahead_a_bytes, const void* ahead_b, long long ahead_b_bytes, int early,
+                                cudaStream_t stream) {
   const long long n = static_cast<long long>(hq + 2 * hkv) * d;
   if (hq < 1 || hkv < 1 || d < 2 || d % 2 != 0 || rot < 0 || rot % 2 != 0 || rot > d || page < 1 || n > (1 << 30) || (rot > 0 && inv_freq == nullptr) ||
       !b200_gemv_norm_fits(m, static_cast<int>(n), k) || ldx % 8 != 0 || ldw % 8 != 0 ||
@@ -374,6 +378,7 @@ B200_API int b200_gemv_norm_qkv(const void* x, const void* norm_w, const void* w
   p.slots = slots;
   p.inv_freq = inv_freq;
   p.hq = hq; p.hkv = hkv; p.d = d; p.rot = rot; p.style = style; p.page = page;
+  p.early = early;
   while (p.share < 8 && p.n * p.share < 2368 && k >= p.share * 32 * 8 * 2) p.share *= 2;      // half a round of loads each is enough: the chain counts
   const int per_block = 8 / p.share;
   const dim3 grid((p.n + per_block - 1) / per_block);

@@ -1088,11 +1088,13 @@ class DecoderModel:
         cfg, scale = self.cfg, self._attn_scale()
         kw = dict(eps=cfg.rms_eps, weight_plus_one=cfg.norm_plus_one)
         t = x.shape[0]
+        longest = batch.max_kv_len or batch.block_table.shape[1] * self.kv_cache.shape[4]
+        early = cfg.head_dim <= 64 and longest <= 256
         for li, lw in enumerate(self.layers):
             kc, vc = self.kv_cache[li, 0], self.kv_cache[li, 1]
             q = ops.norm_qkv_few(x, lw.in_norm, lw.qkv, batch.positions, self.hq, self.hkv, cfg.head_dim, k_cache=kc, v_cache=vc,
                                  slot_mapping=batch.slot_mapping, rot=cfg.rotary_dim, inv_freq=self.inv_freq, style=cfg.rope_style,
-                                 ahead=(lw.o, lw.gate_up), **kw)
+                                 ahead=(lw.o, lw.gate_up), early=early, **kw)
             att = ops.attn_decode(q, kc, vc, batch.block_table, batch.kv_lens, scale=scale, softcap=cfg.attn_softcap,
                                   window=cfg.layer_window(self.layer0 + li), max_kv_len=batch.max_kv_len or None)
             x = ops.linear(att.reshape(t, -1), lw.o, residual=x)

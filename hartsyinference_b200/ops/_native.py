@@ -92,7 +92,7 @@ _SIGNATURES = {
     "b200_gemv_glu": (i32, [vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, vp]),
     "b200_gemv_norm_fits": (i32, [i32, i32, i32]),
     "b200_gemv_norm_glu": (i32, [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, f32, i32, vp, i64, vp, i64, vp]),
-    "b200_gemv_norm_qkv": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i64, i64, i32, i32, i32, i32, i32, i32, f32, i32, vp, i64, vp, i64, vp]),
+    "b200_gemv_norm_qkv": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i64, i64, i32, i32, i32, i32, i32, i32, f32, i32, vp, i64, vp, i64, i32, vp]),
     "b200_norm": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32, i32, vp, i32, i32, vp]),
     "b200_quant_fp8": (i32, [vp, vp, vp, i32, i32, i64, i32, vp]),
     "b200_quant_fp8_weight": (i32, [vp, vp, vp, i32, i32, vp]),

@@ -519,9 +519,10 @@ def _ahead(weights) -> tuple:
 
 def norm_qkv_few(x: torch.Tensor, norm_w: torch.Tensor, w: LinearWeight, positions: torch.Tensor, hq: int, hkv: int, d: int, *,
                  k_cache: torch.Tensor, v_cache: torch.Tensor, slot_mapping: torch.Tensor, rot: int, inv_freq: torch.Tensor, style: int = 0,
-                 eps: float = 1e-6, weight_plus_one: bool = False, ahead: tuple = ()) -> Optional[torch.Tensor]:
+                 eps: float = 1e-6, weight_plus_one: bool = False, ahead: tuple = (), early: bool = False) -> Optional[torch.Tensor]:
     """``rope_kv(linear(norm(x), w))`` for a handful of decoded tokens with bf16 weights, in one launch: q [T, hq, d]. None (and
-    nothing is done) for operands that it does not take. ``ahead``: up to two weights of products further on, for L2."""
+    nothing is done) for operands that it does not take. ``ahead``: up to two weights of products further on, for L2. ``early``: the kernel
+    behind may be launched while this one runs (attention over few keys)."""
     if not (few_fits(x, norm_w, w) and w.weight.shape[0] == (hq + 2 * hkv) * d and k_cache.is_contiguous() and v_cache.is_contiguous()
             and positions.dtype == torch.int32 and slot_mapping.dtype == torch.int64 and inv_freq is not None and inv_freq.dtype == torch.float32
             and (w.bias is None or w.bias.dtype == torch.bfloat16)):
@@ -530,7 +531,7 @@ def norm_qkv_few(x: torch.Tensor, norm_w: torch.Tensor, w: LinearWeight, positio
     q = torch.empty(t, hq, d, dtype=torch.bfloat16, device=x.device)
     rc = N.lib().b200_gemv_norm_qkv(x.data_ptr(), norm_w.data_ptr(), w.weight.data_ptr(), N.ptr(w.bias), q.data_ptr(), k_cache.data_ptr(),
                                     v_cache.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(), inv_freq.data_ptr(), t, k, x.stride(0),
-                                    w.weight.stride(0), hq, hkv, d, rot, style, k_cache.shape[2], eps, int(weight_plus_one), *_ahead(ahead), N.stream())
+                                    w.weight.stride(0), hq, hkv, d, rot, style, k_cache.shape[2], eps, int(weight_plus_one), *_ahead(ahead), int(early), N.stream())
     N.check(rc, "b200_gemv_norm_qkv")
     return q
 
