@@ -978,7 +978,7 @@ B200_API int b200_attn_fa(const void* q, const void* k, const void* v, void* out
 
 // b200_attn_fa (bf16, V on a 16-byte boundary) for products that read e4m3: head h of query row r leaves as e4m3 with one 1x128 UE8M0 scale in
 // columns col0 + h * 128 of row r of q0, from row `split` on of row r - split of q1 (two streams that are projected apart);
-// scales in the blocked layout of kg words a row (4608 x 24 heads 352 + 17 us -> 358, 14040 x 40 3888 + 58 -> 3962). Values are rounded to bf16 first, so they are what a quantisation of
+// scales in the blocked layout of kg words a row (4608 x 24 heads 262 us the two -> 253, against 512 keys 56 -> 45, 14040 x 40 3946 -> 3962). Values are rounded to bf16 first, so they are what a quantisation of
 // b200_attn_fa's output gives. -12: boundaries that it does not take.
 B200_API int b200_attn_fa_quant(const void* q, const void* k, const void* v, int sq, int sk, int heads, float scale, int split, void* q0, void* sf0,
                                 long long ld0, int col0, int kg0, void* q1, void* sf1, long long ld1, int col1, int kg1, void* status,

@@ -6,7 +6,7 @@
 // Why pairs: a 128 x 256 tile of one SM takes 48 KB of operands from L2 for every 512 cycles of its tensor core
 // (96 bytes a cycle, more than an SM gets), so it ran at 0.6 of the core's rate in 8 and in 16 bits. Two SMs on one tile each
 // keep 128 rows of A and 128 rows of B, and the tensor cores read the other half of B from the neighbour's shared
-// memory: 32 KB for the same cycles, a third less, and a third less energy where the power limit holds the clock.
+// memory: 32 KB for the same cycles, a third less.
 //
 // Structure of one CTA (320 threads; persistent, pair i takes tiles i, i + pairs, ...):
 //   warp 0      one thread issues TMA loads of this CTA's 128 rows of either operand into its own shared memory; their
@@ -567,7 +567,6 @@ B200_API int b200_gemm_quant(const void* x, const void* w, void* out, void* out_
   p.glu_q = static_cast<uint8_t*>(out_q);
   p.glu_sf = static_cast<uint8_t*>(out_sf);
   p.q_from = q_from; p.q_ld = q_ld; p.q_col0 = q_col0; p.q_kgroups = q_kgroups;
-  p.row_stores = 1;
   p.sf_a = reinterpret_cast<const uint32_t*>(x_scale);
   p.sf_b = reinterpret_cast<const uint32_t*>(w_scale);
   p.sf_kgroups = (k + 511) / 512;

@@ -1763,7 +1763,8 @@ B200_API int b200_gemm(const void* x, const void* w, void* out, int m, int n, in
 // then b200_glu. dtype 0 (bf16) or 2 (UE8M0 fp8 with fp8 result). A handful of tokens: where the product itself leaves the
 // tensor core (1 x 9728 x 896 6.6 -> 5.1 us against the two kernels, 2 x 28672 x 4096 43.0 -> 41.0, 4 x 9728 x 896 10.5
 // both). Many: whole tiles only, from three full waves (bf16 512 x 28672 x 4096 170 -> 118 us, 8192 x 28672 x 4096 1609 ->
-// 1402, fp8 8192 x 57344 x 8192 3740 -> 3287), on CTA pairs always (the same tiles, see pair_takes), and from two where the plain product would not cut its last wave along K
+// 1402, fp8 8192 x 57344 x 8192 3740 -> 3287), on CTA pairs wherever
+// these take the product (the same tiles, see pair_takes), and from two where the plain product would not cut its last wave along K
 // (1187 x 9728 x 896 46 -> 40; swept from 376 to 690 tiles at depths 1024 to 8192, never slower). One wave and a half lost
 // (bf16 129 x 28672 x 4096 69.3 -> 71.4).
 B200_API int b200_glu_form(int m, int f, int k, int dtype) {
@@ -1780,7 +1781,9 @@ B200_API int b200_glu_form(int m, int f, int k, int dtype) {
 // e4m3 [m][f] (out_q) with 1x128 scales in the blocked layout of sf_rows rows per block (out_sf). A tile reads 128 gate
 // and 128 up rows, so neither product goes to memory: 8192 x 28672 of k 8192 writes 0.24 GB instead of 0.94, which the
 // activation kernel would read again (both 3740 us, this one 3287, fp8; bf16 8192 x 14336 of k 4096 1609 -> 1402). Bound
-// by the tensor core. Returns -12 for sizes that it does not take (f a multiple of 128, at least one tile per SM).
+// by the tensor core. CTA pairs take it where pair_takes says so and the rows of the output start on 32-byte boundaries (from 16 tiles of 256 x
+// 256 on), tiles of one SM where there is at least one for each and rows start on 16-byte boundaries. Returns -12 for other sizes and
+// boundaries, or where f is no multiple of 128.
 B200_API int b200_gemm_glu(const void* x, const void* w, void* out, void* out_q, void* out_sf, int m, int f, int k, long long ldx,
                            long long ldw, long long ldc, int dtype, const float* x_scale, const float* w_scale, int act, int sf_rows,
                            void* status, cudaStream_t stream) {
