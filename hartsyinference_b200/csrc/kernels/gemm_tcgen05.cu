@@ -79,22 +79,24 @@ struct WorkItem {
   int bk;            // element offset of the group's columns in B (column-batched mode)
 };
 
-// kFew: the small-token orientation, the only one with even shares (a compile-time matter, as in emit_chunk: with their branch and the
-// small tokens' epilogue in their code the large-token kernels took 0.5 to 0.8 us more a launch, 512 x 4096 x 256 fp8 8.5 us against 7.9)
-template <bool kFew>
+// kShare: even shares (small-token orientation). A kernel of its own, as the large-token orientation is in emit_chunk: with the branches of the
+// shares and of the other orientation's epilogue in their code the other kernels took longer, whatever they did with them (large-token tiles
+// 0.5 to 0.8 us a launch, 512 x 4096 x 256 fp8 8.5 us against 7.9; few tokens and tiles that are all cut 0.4 to 0.8 us, 6 x 1024 x 1024 bf16 6.95
+// against 6.1, 64 x 4096 x 1024 fp8 9.4 against 8.4).
+template <bool kShare>
 __device__ __forceinline__ long long num_work_items(const GemmParams& p) {
   if (p.block_group != nullptr) return static_cast<long long>(*p.dyn_blocks) * (p.group_n / kTileA);
   // a share of s groups covers s / groups + 2 tiles at most, in part
-  if (kFew && p.share_ctas > 0) return p.share_ctas * ((static_cast<long long>(p.num_tiles) + p.share_ctas - 1) / p.share_ctas + 2);
+  if (kShare) return p.share_ctas * ((static_cast<long long>(p.num_tiles) + p.share_ctas - 1) / p.share_ctas + 2);
   return p.first_split_tile + static_cast<long long>(p.num_tiles - p.first_split_tile) * p.splits;
 }
 
-template <bool kFew>
+template <bool kShare>
 __device__ __forceinline__ WorkItem decode_item(const GemmParams& p, long long w, int tiles_a,
                                                 int total_kblocks) {
   WorkItem it;
   long long tile;
-  if (kFew && p.share_ctas > 0) {
+  if (kShare) {
     const long long all = static_cast<long long>(p.num_tiles) * p.share_groups;
     const int c = static_cast<int>(w % p.share_ctas), n = static_cast<int>(w / p.share_ctas);
     const int first = static_cast<int>(all * c / p.share_ctas), end = static_cast<int>(all * (c + 1) / p.share_ctas);
@@ -186,17 +188,17 @@ __device__ __forceinline__ void store_partial(const GemmParams& p, const float (
 
 // Routes one 32-column chunk of accumulator values of work item `it`. kLarge: the large-token orientation (a
 // compile-time matter, because the code of its epilogue slowed the start of the short decode kernels by 2 us).
-template <int BN, bool kLarge>
+template <int BN, bool kLarge, bool kShare>
 __device__ __forceinline__ void emit_chunk(const GemmParams& p, float (&v)[32], const WorkItem& it,
                                            int row_local, int chunk, uint8_t* strip, bool merge) {
-  if (!kLarge && merge) {
+  if (kShare && merge) {
     // the other piece of the tile is there already: add it and finish the tile
     const float* ws = p.split_ws + (static_cast<long long>(it.slot) * p.splits + (it.split ^ 1)) * (BN * 128);
 #pragma unroll
     for (int j = 0; j < 32; ++j)
       if (chunk * 32 + j < BN) v[j] += __ldcg(ws + (chunk * 32 + j) * 128 + row_local);
   }
-  if (it.slot >= 0 && p.ar.world == 0 && !(!kLarge && merge)) store_partial<BN>(p, v, row_local, chunk * 32, it);
+  if (it.slot >= 0 && p.ar.world == 0 && !(kShare && merge)) store_partial<BN>(p, v, row_local, chunk * 32, it);
   else if (kLarge && p.row_stores && it.tb * BN + chunk * 32 + 32 <= p.rows_b)
     store_chunk_rows(p, v, it.ta * kTileA + (row_local & ~31), it.tb * BN + chunk * 32, strip);
   else store_chunk<!kLarge>(p, v, it.ta * kTileA + row_local, it.tb * BN + chunk * 32, min(p.rows_b, (it.tb + 1) * BN),
@@ -669,7 +671,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, 
   reduce_partials<8>(p, it, bn, e4);
 }
 
-template <int kMode, int BN, int kAtoms, bool kGlu = false>
+template <int kMode, int BN, int kAtoms, bool kGlu = false, bool kShare = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a,
                     const __grid_constant__ CUtensorMap tm_b) {
@@ -718,7 +720,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
 
   const int tiles_a = (p.rows_a + kTileA - 1) / kTileA;
   const int total_kblocks = (p.k + kElemsPerAtom - 1) / kElemsPerAtom;
-  const long long work_items = num_work_items<kAtoms == 2>(p);
+  const long long work_items = num_work_items<kShare>(p);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -813,7 +815,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       int pre = 0;                 // stage iterations of the first item already half-issued
       long long w_first = blockIdx.x;
       if (p.swap_out && p.group_n == 0 && w_first < work_items) {
-        const WorkItem it = decode_item<kAtoms == 2>(p, w_first, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kShare>(p, w_first, tiles_a, total_kblocks);
         const int sfb = first_sfb(it);
         for (int kb = it.kb0; kb < it.kb1 && pre < stages; kb += kAtoms, ++pre) issue_stage(it, sfb, kb, pre, 1);
         pdl_wait();
@@ -827,7 +829,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       const uint32_t ag_call = p.ag.world > 0 ? *reinterpret_cast<volatile uint32_t*>(p.ag.ctr) + 1u : 0u;
       uint32_t ag_seen = 0;
       for (long long w = blockIdx.x; w < work_items && ok; w += gridDim.x) {
-        const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kShare>(p, w, tiles_a, total_kblocks);
         if (it.skip) continue;
         if (p.ag.world > 0 && !ag_wait_tile(p, it.ta, ag_call, ag_seen)) {
           report_status(p.status, kWaitTimeout, kKernelAllToAll, 12, blockIdx.x);
@@ -871,7 +873,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       bool ok = true;
       bool issued_any = false;
       for (long long w = blockIdx.x; w < work_items && ok; w += gridDim.x) {
-        const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
+        const WorkItem it = decode_item<kShare>(p, w, tiles_a, total_kblocks);
         if (it.skip) continue;
         if (!kFp8) {
           if (!mbar_wait(&bars->tmem_empty[abuf], aph ^ 1, abort_flag)) {
@@ -968,7 +970,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     bool ok = true;
     uint32_t glu_round = 0;
     for (long long w = blockIdx.x; w < work_items; w += gridDim.x) {
-      const WorkItem it = decode_item<kAtoms == 2>(p, w, tiles_a, total_kblocks);
+      const WorkItem it = decode_item<kShare>(p, w, tiles_a, total_kblocks);
       if (it.skip) continue;
       if constexpr (kGlu) {
         if (ok && !__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[abuf], aph, abort_flag))) {
@@ -994,7 +996,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
       // Even shares: the piece that ends a tile was the first of the next CTA, so the one that starts it, the last of
       // this CTA, nearly always finds it done and finishes the tile from its own accumulator
       bool merge = false;
-      if (kAtoms == 2 && p.share_ctas > 0 && it.slot >= 0) {
+      if (kShare && it.slot >= 0) {
         if (threadIdx.x == 64) bars->flag = ld_acquire_gpu(p.split_counter + it.slot);
         epilogue_barrier();
         merge = bars->flag != 0;
@@ -1024,7 +1026,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[u][j]);
-                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, hsel + 2 * u, strip, merge);
+                emit_chunk<BN, kAtoms == 1, kShare>(p, v, it, row_local, hsel + 2 * u, strip, merge);
               }
               aph ^= 1;
             } else {
@@ -1054,7 +1056,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
                 for (int j = 0; j < 32; ++j)
                   if (c * 32 + j < BN) part[(c * 32 + j) * 128 + row_local] = v[j];
               } else {
-                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, c, strip, merge);
+                emit_chunk<BN, kAtoms == 1, kShare>(p, v, it, row_local, c, strip, merge);
               }
             }
             tc_fence_before_sync();
@@ -1162,13 +1164,13 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = acc[i * 32 + j];
-                emit_chunk<BN, kAtoms == 1>(p, v, it, row_local, c, strip, merge);
+                emit_chunk<BN, kAtoms == 1, kShare>(p, v, it, row_local, c, strip, merge);
               }
             }
           }
         }
       }
-      if (merge) {
+      if (kShare && merge) {
         if (threadIdx.x == 64) p.split_counter[it.slot] = 0;       // ready for the next launch
       } else {
         finish_item<BN>(p, it, ok, &bars->flag);
@@ -1184,7 +1186,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tm_a
     // over all CTAs (fixed order: deterministic), applies the epilogue and stores C
     cluster_sync_all();
     if (warp >= 2) {
-      const WorkItem it = decode_item<kAtoms == 2>(p, blockIdx.x, tiles_a, total_kblocks);
+      const WorkItem it = decode_item<kShare>(p, blockIdx.x, tiles_a, total_kblocks);
       const int et = threadIdx.x - 64;
       const uint32_t rank = cluster_ctarank();
       const int total4 = BN * 32;                                  // float4 groups of the tile
@@ -1314,14 +1316,14 @@ namespace b200 {
 static bool g_cluster_reduce = false;   // measured slower than the other two ways; opt-in
 static bool g_external_reduce = true;    // fully split GEMMs: second kernel (true) or last-arriving CTA (false)
 
-template <int kMode, int BN, int kAtoms, bool kGlu = false>
+template <int kMode, int BN, int kAtoms, bool kGlu = false, bool kShare = false>
 int launch_gemm(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& tb, int grid,
                 cudaStream_t stream) {
   const int stage_bytes = kAtoms * (kStageBytesA + BN * 128) + (kMode == 2 ? 2048 : 0);
   const int smem = p.stages * stage_bytes + static_cast<int>(sizeof(GemmBarriers)) + 1024 + (p.row_stores ? 8 * kStripBytes : 0);
   static PerDeviceOnce configured;
   if (configured.first_time()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu, kShare>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return -static_cast<int>(e) - 200;
   }
@@ -1342,9 +1344,14 @@ int launch_gemm(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& t
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
   }
-  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu>, p, ta, tb) != cudaSuccess) return -300;
+  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kMode, BN, kAtoms, kGlu, kShare>, p, ta, tb) != cudaSuccess) return -300;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 300;
+}
+
+template <int kMode, int BN>
+int launch_few(const GemmParams& p, const CUtensorMap& ta, const CUtensorMap& tb, int grid, cudaStream_t stream) {
+  return p.share_ctas > 0 ? launch_gemm<kMode, BN, 2, false, true>(p, ta, tb, grid, stream) : launch_gemm<kMode, BN, 2>(p, ta, tb, grid, stream);
 }
 
 static int g_num_sms[64] = {};
@@ -1668,10 +1675,10 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
     p.sa_ld = p.sb_ld = 1;
     if (swap) {
       switch (bn) {
-        case 16: rc = launch_gemm<3, 16, 2>(p, ta, tb, grid, stream); break;
-        case 32: rc = launch_gemm<3, 32, 2>(p, ta, tb, grid, stream); break;
-        case 64: rc = launch_gemm<3, 64, 2>(p, ta, tb, grid, stream); break;
-        default: rc = launch_gemm<3, 128, 2>(p, ta, tb, grid, stream); break;
+        case 16: rc = launch_few<3, 16>(p, ta, tb, grid, stream); break;
+        case 32: rc = launch_few<3, 32>(p, ta, tb, grid, stream); break;
+        case 64: rc = launch_few<3, 64>(p, ta, tb, grid, stream); break;
+        default: rc = launch_few<3, 128>(p, ta, tb, grid, stream); break;
       }
     } else if (bn == 128) {
       rc = launch_gemm<3, 128, 1>(p, ta, tb, grid, stream);
@@ -1681,10 +1688,10 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   } else if (mx) {
     if (swap) {
       switch (bn) {
-        case 16: rc = launch_gemm<2, 16, 2>(p, ta, tb, grid, stream); break;
-        case 32: rc = launch_gemm<2, 32, 2>(p, ta, tb, grid, stream); break;
-        case 64: rc = launch_gemm<2, 64, 2>(p, ta, tb, grid, stream); break;
-        default: rc = launch_gemm<2, 128, 2>(p, ta, tb, grid, stream); break;
+        case 16: rc = launch_few<2, 16>(p, ta, tb, grid, stream); break;
+        case 32: rc = launch_few<2, 32>(p, ta, tb, grid, stream); break;
+        case 64: rc = launch_few<2, 64>(p, ta, tb, grid, stream); break;
+        default: rc = launch_few<2, 128>(p, ta, tb, grid, stream); break;
       }
     } else if (bn == 128) {
       rc = launch_gemm<2, 128, 1>(p, ta, tb, grid, stream);
@@ -1694,10 +1701,10 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   } else if (fp8) {
     if (swap) {
       switch (bn) {
-        case 16: rc = launch_gemm<1, 16, 2>(p, ta, tb, grid, stream); break;
-        case 32: rc = launch_gemm<1, 32, 2>(p, ta, tb, grid, stream); break;
-        case 64: rc = launch_gemm<1, 64, 2>(p, ta, tb, grid, stream); break;
-        default: rc = launch_gemm<1, 128, 2>(p, ta, tb, grid, stream); break;
+        case 16: rc = launch_few<1, 16>(p, ta, tb, grid, stream); break;
+        case 32: rc = launch_few<1, 32>(p, ta, tb, grid, stream); break;
+        case 64: rc = launch_few<1, 64>(p, ta, tb, grid, stream); break;
+        default: rc = launch_few<1, 128>(p, ta, tb, grid, stream); break;
       }
     } else {
       rc = launch_gemm<1, 128, 1>(p, ta, tb, grid, stream);
@@ -1705,10 +1712,10 @@ int gemm_impl(const void* x, const void* w, void* out, int m, int n, int k, long
   } else {
     if (swap) {
       switch (bn) {
-        case 16: rc = launch_gemm<0, 16, 2>(p, ta, tb, grid, stream); break;
-        case 32: rc = launch_gemm<0, 32, 2>(p, ta, tb, grid, stream); break;
-        case 64: rc = launch_gemm<0, 64, 2>(p, ta, tb, grid, stream); break;
-        default: rc = launch_gemm<0, 128, 2>(p, ta, tb, grid, stream); break;
+        case 16: rc = launch_few<0, 16>(p, ta, tb, grid, stream); break;
+        case 32: rc = launch_few<0, 32>(p, ta, tb, grid, stream); break;
+        case 64: rc = launch_few<0, 64>(p, ta, tb, grid, stream); break;
+        default: rc = launch_few<0, 128>(p, ta, tb, grid, stream); break;
       }
     } else if (bn == 128) {
       rc = launch_gemm<0, 128, 1>(p, ta, tb, grid, stream);
